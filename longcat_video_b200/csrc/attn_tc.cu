@@ -17,16 +17,25 @@
 // and the two partial results are merged once at the end of the work item (as in split-KV decoding), so
 // the warpgroups never synchronise with each other inside the loop and one computes while the other waits.
 //
-//   warps 0-3, 4-7 : softmax warpgroups 0 and 1     warp 8  : TMA producer (Q tiles, K ring, V ring)
-//   warp 9         : S = Q K^T issuer               warp 10 : O += P V issuer      warp 11 : output TMA stores
+//   warps 0-3, 4-7 : softmax warpgroups 0 and 1     warp 8  : TMA producer of Q and K
+//   warp 9         : S = Q K^T issuer               warp 10 : O += P V issuer
+//   warp 11        : TMA producer of V, output TMA stores
 //
-// Per block i (warpgroup g = i & 1, its round r = i >> 1):  S = Q K^T  (M64 N64 K128, fp32 in TMEM, buffer
-// r & 1 of the warpgroup)  ->  the warpgroup reads S with tcgen05.ld, exp2 online softmax in registers, P in the
-// input dtype written over the first half of the same S buffer with tcgen05.st  ->  O_g += P V  (M64 N128
-// K64, A operand from TMEM).  The S of round r + 2 is issued into the buffer once that PV has finished, which
-// leaves a whole round of the warpgroup for it; a round costs the warpgroup one barrier wait and one arrival.
-// K and V have a ring of three slots each (a slot = the tiles of both query blocks), filled in the order in
-// which they are used: K0 K1 K2 K3 V0 K4 V1 ...
+// Once per item the softmax warpgroups move the Q rows from shared memory to TMEM, where they are the A operand of
+// every S of the item: with Q in shared memory an S reads as many bytes of Q as of K for every block.
+// Per block i (warpgroup g = i & 1):  S = Q K^T  (M64 N64 K128, A from TMEM, fp32 result in the warpgroup's S columns)
+// ->  the warpgroup reads S into registers with tcgen05.ld and releases the columns, so that the S of its next block is
+// computed under its arithmetic  ->  exp2 online softmax in registers, P in the input dtype into the warpgroup's P columns
+// with tcgen05.st, once its PV of the block before has finished  ->  O_g += P V  (M64 N128 K64, A operand from TMEM).
+// With P written over S, S of a block could not start before the PV of an earlier block was through.
+// K and V have a ring of three slots each (a slot = the tiles of both query blocks).  Each ring has a producer warp of
+// its own, and the copies are issued by one elected lane of the converged warp: one warp for both rings, issuing from a
+// divergent branch, needed about 950 cycles per ring slot and was what the rest waited for (V was requested 1700 cycles
+// after its P was ready).
+// What bounds it: M=64 MMAs, 16 x 32 + 8 x 64 = 1030 cycles of tensor pipe per block of a pair (an M=64 tile occupies the
+// pipe like an M=128 one); inside an item a block takes about 1040 cycles.  An item boundary costs some 10 000 more (the
+// softmax warps merge and store O before they take up the next item).  Attention launch, 480p grid, 32 heads, 39 of 624
+// blocks: 2.25 ms with one producer warp and P over S, 1.96 ms now.
 //
 // The MMAs are issued by whole converged warps with one elected lane (about 23 cycles per MMA for the
 // warp; a single lane inside a divergent branch needs 50 and more).
@@ -35,14 +44,13 @@
 // (the accumulated values stay finite and the result is unchanged after the final division), so O is
 // rarely rescaled in TMEM.
 //
-// TMEM columns, per warpgroup g at 256*g: S/P[buf] at 64*buf (the probabilities, two 16-bit values per
-// column, occupy the first 32 columns of the buffer), O at 128 (128 columns); the second tile of the
-// pair 16 lanes up in each.
+// TMEM columns: O of warpgroup g at 128 * g (128 columns), its S at 256 + 64 * g, its P at 384 + 32 * g (two 16-bit
+// values per column), Q at 448 (64 columns of 16-bit pairs); the second tile of the pair 16 lanes up in each.
 //
 // At the end of a work item both warpgroups exchange (maximum, row sum) through shared memory, each merges
 // and normalises one 64-column half of O and stages it in the V slot that the last PV has released; it
-// leaves by TMA store.  The Q tiles are released as soon as the last S of the item has been computed, so the
-// next item's Q, K and S are in flight while this one finishes.
+// leaves by TMA store.  The next item's Q goes to TMEM as soon as the last S of the item has been computed, so the
+// next item's K and S are in flight while this one finishes.
 //
 // Every wait on an mbarrier is bounded: when a wait runs out the CTA records where, raises an abort
 // flag that all roles poll, drains its outstanding bulk copies, frees its TMEM and returns.
@@ -62,22 +70,21 @@ constexpr int kHalfBytes = kTileBytes / 2;  // one 64-column half: 64 rows x 128
 constexpr int kTilesPerWork = 2;            // the two query blocks of a pair
 constexpr int kSlotBytes = kTilesPerWork * kTileBytes;  // a ring slot holds the K (or V) tiles of both query blocks
 constexpr int kKSlots = 3, kVSlots = 3;
-constexpr int kKLead = 4;                   // K blocks requested ahead of V: S runs two rounds of each warpgroup ahead
 constexpr int kThreads = 384;
 // setmaxnreg per warpgroup: (208 + 208 + 88) * 128 threads <= the 64 K registers of the SM
 constexpr int kRegsSoftmax = 208, kRegsOther = 88;
 
-// TMEM columns of warpgroup g: base 256 * g
-constexpr uint32_t kTmWg = 256, kTmS = 0, kTmO = 128;
+// TMEM columns: O accumulator of warpgroup g at 128 * g, its S at 256 + 64 * g, its P (16-bit pairs) at 384 + 32 * g; Q (16-bit pairs)
+constexpr uint32_t kTmO = 0, kTmS = 256, kTmP = 384, kTmQ = 448;
 
 // shared memory map (offsets from the 1024-byte aligned base of dynamic shared memory)
 constexpr int kOffQ = 0;
 constexpr int kOffK = kOffQ + kTilesPerWork * kTileBytes;
 constexpr int kOffV = kOffK + kKSlots * kSlotBytes;
 constexpr int kOffBar = kOffV + kVSlots * kSlotBytes;
-// barriers: k_full[3] k_empty[3] v_full[3] v_empty[3] q_full q_empty s_full[2][2] p_full[2][2] pv_done[2][2]
-//           ml_ready o_free o_staged
-constexpr int kNumBars = 2 * kKSlots + 2 * kVSlots + 2 + 12 + 3;
+// barriers: k_full[3] k_empty[3] v_full[3] v_empty[3] q_full q_empty s_full[2] s_free[2] p_full[2] pv_done[2]
+//           ml_ready o_free o_staged qt_full qt_free
+constexpr int kNumBars = 2 * kKSlots + 2 * kVSlots + 2 + 8 + 5;
 constexpr int kOffMisc = kOffBar + kNumBars * 8;      // abort flag, TMEM base
 constexpr int kOffMl = kOffMisc + 64;                 // [2 warpgroups][128 lanes] (maximum, row sum)
 constexpr int kSmemBytes = kOffMl + 2 * 128 * 8;
@@ -123,10 +130,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     auto bar_v_empty = [&](int s) { return bar0 + 8u * (2 * kKSlots + kVSlots + s); };
     constexpr int kB0 = 2 * kKSlots + 2 * kVSlots;
     const uint32_t bar_q_full = bar0 + 8u * kB0, bar_q_empty = bar0 + 8u * (kB0 + 1);
-    auto bar_s_full = [&](int wg, int buf) { return bar0 + 8u * (kB0 + 2 + 2 * wg + buf); };
-    auto bar_p_full = [&](int wg, int buf) { return bar0 + 8u * (kB0 + 6 + 2 * wg + buf); };
-    auto bar_pv_done = [&](int wg, int buf) { return bar0 + 8u * (kB0 + 10 + 2 * wg + buf); };
-    const uint32_t bar_ml_ready = bar0 + 8u * (kB0 + 14), bar_o_free = bar0 + 8u * (kB0 + 15), bar_o_staged = bar0 + 8u * (kB0 + 16);
+    auto bar_s_full = [&](int wg) { return bar0 + 8u * (kB0 + 2 + wg); };
+    auto bar_s_free = [&](int wg) { return bar0 + 8u * (kB0 + 4 + wg); };
+    auto bar_p_full = [&](int wg) { return bar0 + 8u * (kB0 + 6 + wg); };
+    auto bar_pv_done = [&](int wg) { return bar0 + 8u * (kB0 + 8 + wg); };
+    constexpr int kB1 = kB0 + 10;
+    const uint32_t bar_ml_ready = bar0 + 8u * kB1, bar_o_free = bar0 + 8u * (kB1 + 1), bar_o_staged = bar0 + 8u * (kB1 + 2);
+    const uint32_t bar_qt_full = bar0 + 8u * (kB1 + 3), bar_qt_free = bar0 + 8u * (kB1 + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kOffMisc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffMisc + 8);
     float2* ml = reinterpret_cast<float2*>(smem + kOffMl);  // [2][128]
@@ -146,13 +156,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             mbar_init(bar_v_empty(s), 1);
         }
         mbar_init(bar_q_full, 1);
-        mbar_init(bar_q_empty, 1);
-        for (int g = 0; g < 2; ++g)
-            for (int b = 0; b < 2; ++b) {
-                mbar_init(bar_s_full(g, b), 1);
-                mbar_init(bar_p_full(g, b), 4);  // one elected arrival per softmax warp
-                mbar_init(bar_pv_done(g, b), 1);
-            }
+        mbar_init(bar_q_empty, 8);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar_s_full(b), 1);
+            mbar_init(bar_s_free(b), 4);
+            mbar_init(bar_p_full(b), 4);  // one elected arrival per softmax warp
+            mbar_init(bar_pv_done(b), 1);
+        }
+        mbar_init(bar_qt_full, 8);
+        mbar_init(bar_qt_free, 1);
         mbar_init(bar_ml_ready, 8);
         mbar_init(bar_o_free, 8);
         mbar_init(bar_o_staged, 8);
@@ -180,42 +192,81 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
 
     const int groups = (P.nq + kTilesPerWork - 1) / kTilesPerWork;
     const long long total_work = start_ok ? (long long)P.bh_total * groups : 0;
+    // The CTA's items are blockIdx.x, blockIdx.x + gridDim.x, ...; every role steps through them as (head, group) pairs, since a
+    // 64-bit division per role and item costs more than a round.
+    const int first_bh = (int)(blockIdx.x / (unsigned)groups), first_g = (int)(blockIdx.x % (unsigned)groups);
+    const int step_bh = (int)(gridDim.x / (unsigned)groups), step_g = (int)(gridDim.x % (unsigned)groups);
+    auto next_item = [&](int& bh, int& g) {
+        bh += step_bh;
+        g += step_g;
+        if (g >= groups) {
+            g -= groups;
+            ++bh;
+        }
+    };
     constexpr bool bf16 = kBf16;
 
     // All roles walk the same list of work items and blocks.  Block number gb (counted over the whole kernel)
-    // uses K slot gb % 3 and V slot gb % 3; warpgroup g numbers its own rounds rr[g] over the whole kernel and
-    // round rr uses S/P buffer rr & 1.  Within an item block i belongs to warpgroup i & 1.
+    // uses K slot gb % 3 and V slot gb % 3.  Within an item block i belongs to warpgroup i & 1, which numbers its own rounds rr
+    // over the whole kernel.
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-      if (warp == 8) {
-        // ================================================================== TMA producer
+      if (warp == 8 || warp == 11) {
+        // ================================================================== TMA producers: warp 8 Q and K, warp 11 V and the output
+        // The output rows of an item are staged in the V slot its last PV released.  Warp 11 sends them off when it needs
+        // that slot again, at the latest before it requests the last V of the item behind it (the epilogue of that item
+        // completes the next phase of o_staged, so the wait is never a phase behind).
+        const bool is_k = warp == 8;
         unsigned gk = 0, gv = 0, wk = 0, nq_issued = 0;
+        int s_bh = first_bh, s_g = first_g;  // item whose output is stored next
+        unsigned ws_end = 0, ks = 0;        // blocks up to and including it, its number
         bool ok = true;
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), g = (int)(w % groups);
+        auto store_item = [&]() -> bool {
+            const int bh = s_bh, g = s_g;
+            const int b = bh / P.heads, h = bh % P.heads;
+            if (!mbar_wait_warp(bar_o_staged, ks & 1, ctl, 110, ks)) return false;
+            if (lane == 0) {
+                const unsigned last = ws_end - 1;
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int qq = g * kTilesPerWork + hf;
+                    if (qq >= P.nq) continue;
+                    Coord cc = block_coord(P.gq, qq, b, h, P.heads, P.merge_o, P.Tq);
+                    const CUtensorMap* tmo = &P.tm_o[0];
+                    if (P.o_frames > 0) {  // blocks never straddle ranks: o_frames is a multiple of the block's frames
+                        const int dst = cc.c3 / P.o_frames;
+                        cc.c3 -= dst * P.o_frames;
+                        tmo = &P.tm_o[dst];
+                    }
+                    const uint32_t src = sbase + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes;
+                    tma_store_5d(tmo, src, 0, cc.c1, cc.c2, cc.c3, cc.c4);
+                    tma_store_5d(tmo, src + kHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+                }
+                tma_store_commit();
+                tma_store_wait_read();
+                mbar_arrive(bar_v_empty(last % kVSlots));
+            }
+            __syncwarp();
+            next_item(s_bh, s_g);
+            ++ks;
+            return true;
+        };
+        int bh = first_bh, g = first_g, nx_bh = first_bh, nx_g = first_g;
+        int ca_n = 0, cb_n = 0;
+        auto peek = [&](bool there) {  // list lengths of item nx, read one item ahead
+            if (there) {
+                ca_n = clamp_cnt(P, nx_bh, nx_g * kTilesPerWork);
+                cb_n = clamp_cnt(P, nx_bh, nx_g * kTilesPerWork + 1);
+            }
+        };
+        peek(blockIdx.x < total_work);
+        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, g = nx_g) {
             const int b = bh / P.heads, h = bh % P.heads;
             const int qa = g * kTilesPerWork, qb = qa + 1;
-            const int ca = clamp_cnt(P, bh, qa), cb = clamp_cnt(P, bh, qb);
+            const int ca = ca_n, cb = cb_n;
             const int n_iter = max(1, max(ca, cb));
-            // Q tiles: the buffer is free once the last S of the previous item has been computed
-            ok = mbar_wait_warp(bar_q_empty, (wk & 1) ^ 1, ctl, 10, wk);
-            if (!ok) break;
-            ++nq_issued;
-            if (lane == 0) {
-                const int ntile = (qa < P.nq) + (qb < P.nq);
-                mbar_arrive_tx(bar_q_full, ntile * kTileBytes);
-                for (int hf = 0; hf < 2; ++hf) {
-                    const int qt = qa + hf;
-                    if (qt >= P.nq) continue;
-                    const Coord cc = block_coord(P.gq, qt, b, h, P.heads, P.merge_q, P.Tq);
-                    const uint32_t dst = sbase + kOffQ + hf * kTileBytes;
-                    tma_load_5d(dst, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                    tma_load_5d(dst + kHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
-                }
-            }
             // Block coordinates are fetched and decoded by the whole warp: lane L holds, for tile (L & 1) and
-            // block win + (L >> 1), the block's first token packed as t << 20 | h << 10 | w.  `prv` and `nxt`
-            // hold the windows of sixteen blocks before and after (V trails K by kKLead blocks).
+            // block win + (L >> 1), the block's first token packed as t << 20 | h << 10 | w.  `nxt` holds the window of
+            // sixteen blocks behind the current one.
             const int my_t = lane & 1, my_s = lane >> 1;
             const int my_c = my_t ? cb : ca;
             const int32_t* my_l = P.idx + ((long long)bh * P.nq + min(qa + my_t, P.nq - 1)) * P.cap;
@@ -236,65 +287,71 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                 block_coords(P.gk, blk, bt, bhh, bw);
                 return ((bt * P.gk.ct) << 20) | ((bhh * P.gk.ch) << 10) | (bw * P.gk.cw);
             };
-            int win = 0, prv = 0;
             int cur = fetch(my_s);
             int nxt = fetch(16 + my_s);
-            const int c3k = P.merge_k ? b * P.Tk : 0, c4k = P.merge_k ? h : b * P.heads + h;
-            const int c3v = P.merge_v ? b * P.Tk : 0, c4v = P.merge_v ? h : b * P.heads + h;
-            for (int j = 0; j < n_iter + kKLead && ok; ++j) {
-                if (j >= kKLead) {  // V(j - kKLead)
-                    const int jj = j - kKLead;
-                    const int src = jj >= win ? cur : prv;
-                    const int o = jj >= win ? jj - win : jj - (win - 16);
-                    const int pa = __shfl_sync(0xffffffffu, src, (o << 1) | 0);
-                    const int pb = __shfl_sync(0xffffffffu, src, (o << 1) | 1);
-                    const bool act_a = jj < ca, act_b = jj < cb;
-                    const int slot = gv % kVSlots;
-                    ok = mbar_wait_warp(bar_v_empty(slot), ((gv / kVSlots) & 1) ^ 1, ctl, 22, gv);
-                    if (!ok) break;
-                    ++gv;
-                    if (lane == 0) {
-                        mbar_arrive_tx(bar_v_full(slot), ((int)act_a + (int)act_b) * kTileBytes);
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf) {
-                            if (!(hf ? act_b : act_a)) continue;
-                            const int pk = hf ? pb : pa;
-                            const int cw = pk & 1023, chh = (pk >> 10) & 1023, ctt = (pk >> 20) + c3v;
-                            const uint32_t dst = sbase + kOffV + slot * kSlotBytes + hf * kTileBytes;
-                            tma_load_5d(dst, &P.tm_v, bar_v_full(slot), 0, cw, chh, ctt, c4v);
-                            tma_load_5d(dst + kHalfBytes, &P.tm_v, bar_v_full(slot), 64, cw, chh, ctt, c4v);
-                        }
+            next_item(nx_bh, nx_g);
+            peek(w + gridDim.x < total_work);
+            const bool mrg = is_k ? P.merge_k : P.merge_v;
+            const int c3 = mrg ? b * P.Tk : 0, c4 = mrg ? h : b * P.heads + h;
+            // the boxes of both query blocks' tiles of list position j into ring slot `dst`
+            auto request = [&](int j, const CUtensorMap* tm, uint32_t bar, uint32_t dst) {
+                const int pa = __shfl_sync(0xffffffffu, cur, (j & 15) << 1), pb = __shfl_sync(0xffffffffu, cur, ((j & 15) << 1) | 1);
+                mbar_arrive_tx_elect(bar, ((j < ca) + (j < cb)) * kTileBytes);
+                if (j < ca) {
+                    tma_load_5d_elect(dst, tm, bar, 0, pa & 1023, (pa >> 10) & 1023, (pa >> 20) + c3, c4);
+                    tma_load_5d_elect(dst + kHalfBytes, tm, bar, 64, pa & 1023, (pa >> 10) & 1023, (pa >> 20) + c3, c4);
+                }
+                if (j < cb) {
+                    tma_load_5d_elect(dst + kTileBytes, tm, bar, 0, pb & 1023, (pb >> 10) & 1023, (pb >> 20) + c3, c4);
+                    tma_load_5d_elect(dst + kTileBytes + kHalfBytes, tm, bar, 64, pb & 1023, (pb >> 10) & 1023, (pb >> 20) + c3, c4);
+                }
+                if ((j & 15) == 15) {
+                    cur = nxt;
+                    nxt = fetch(j + 17 + my_s);
+                }
+            };
+            if (is_k) {
+                // Q tiles: the buffer is free once the softmax warps have moved the previous item's Q to TMEM
+                ok = mbar_wait_warp(bar_q_empty, (wk & 1) ^ 1, ctl, 10, wk);
+                if (!ok) break;
+                ++nq_issued;
+                if (lane == 0) {
+                    const int ntile = (qa < P.nq) + (qb < P.nq);
+                    mbar_arrive_tx(bar_q_full, ntile * kTileBytes);
+                    for (int hf = 0; hf < 2; ++hf) {
+                        const int qt = qa + hf;
+                        if (qt >= P.nq) continue;
+                        const Coord cc = block_coord(P.gq, qt, b, h, P.heads, P.merge_q, P.Tq);
+                        const uint32_t dst = sbase + kOffQ + hf * kTileBytes;
+                        tma_load_5d(dst, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
+                        tma_load_5d(dst + kHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
                     }
                 }
-                if (j < n_iter) {  // K(j)
-                    while (j >= win + 16) {
-                        win += 16;
-                        prv = cur;
-                        cur = nxt;
-                        nxt = fetch(win + 16 + my_s);
-                    }
-                    const int pa = __shfl_sync(0xffffffffu, cur, ((j - win) << 1) | 0);
-                    const int pb = __shfl_sync(0xffffffffu, cur, ((j - win) << 1) | 1);
-                    const bool act_a = j < ca, act_b = j < cb;
+                __syncwarp();
+                for (int j = 0; j < n_iter; ++j) {
                     const int slot = gk % kKSlots;
                     ok = mbar_wait_warp(bar_k_empty(slot), ((gk / kKSlots) & 1) ^ 1, ctl, 20, gk);
                     if (!ok) break;
                     ++gk;
-                    if (lane == 0) {
-                        mbar_arrive_tx(bar_k_full(slot), ((int)act_a + (int)act_b) * kTileBytes);
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf) {
-                            if (!(hf ? act_b : act_a)) continue;
-                            const int pk = hf ? pb : pa;
-                            const int cw = pk & 1023, chh = (pk >> 10) & 1023, ctt = (pk >> 20) + c3k;
-                            const uint32_t dst = sbase + kOffK + slot * kSlotBytes + hf * kTileBytes;
-                            tma_load_5d(dst, &P.tm_k, bar_k_full(slot), 0, cw, chh, ctt, c4k);
-                            tma_load_5d(dst + kHalfBytes, &P.tm_k, bar_k_full(slot), 64, cw, chh, ctt, c4k);
-                        }
-                    }
+                    request(j, &P.tm_k, bar_k_full(slot), sbase + kOffK + slot * kSlotBytes);
                 }
+            } else {
+                for (int j = 0; j < n_iter; ++j) {
+                    if (ks < wk && (gv >= ws_end - 1 + kVSlots || j == n_iter - 1)) {
+                        ok = store_item();
+                        if (!ok) break;
+                    }
+                    const int slot = gv % kVSlots;
+                    ok = mbar_wait_warp(bar_v_empty(slot), ((gv / kVSlots) & 1) ^ 1, ctl, 22, gv);
+                    if (!ok) break;
+                    ++gv;
+                    request(j, &P.tm_v, bar_v_full(slot), sbase + kOffV + slot * kSlotBytes);
+                }
+                ws_end = gv;  // the item before has been stored
             }
         }
+        if (!is_k && ok && ks < wk) ok = store_item();
+        if (!is_k && lane == 0) tma_store_wait_all();
         if (!ok && lane == 0) {
             // drain: give the copies this warp issued a bounded time to land before the CTA exits
             const long long t0 = clock64();
@@ -313,47 +370,54 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
         const uint32_t idesc_s = instr_desc(bf16, 64, 64, 0);
         unsigned gb = 0, wk = 0, rr0 = 0, rr1 = 0;
         bool ok = true;
+        int bh = first_bh, g = first_g, ca_n = 0, cb_n = 0;
+        auto peek = [&](bool there) {  // list lengths of item (bh, g), which is then stepped: read one item ahead
+            if (!there) return;
+            ca_n = clamp_cnt(P, bh, g * kTilesPerWork);
+            cb_n = clamp_cnt(P, bh, g * kTilesPerWork + 1);
+            next_item(bh, g);
+        };
+        peek(blockIdx.x < total_work);
         for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), g = (int)(w % groups);
-            const int ca = clamp_cnt(P, bh, g * kTilesPerWork), cb = clamp_cnt(P, bh, g * kTilesPerWork + 1);
+            const int ca = ca_n, cb = cb_n;
+            peek(w + gridDim.x < total_work);
             const int n_iter = max(1, max(ca, cb));
-            ok = mbar_wait_warp(bar_q_full, wk & 1, ctl, 30, wk);
+            ok = mbar_wait_warp(bar_qt_full, wk & 1, ctl, 30, wk);  // Q of this item is in TMEM
             bool pre = false;
             for (int i = 0; i < n_iter && ok; ++i, ++gb) {
                 const int wg = i & 1;
                 const unsigned rr = wg ? rr1 : rr0;
-                const int slot = gb % kKSlots, buf = rr & 1;
+                const int slot = gb % kKSlots;
                 if (!pre) {  // not already seen ready by the look-ahead of the block before
                     ok = mbar_wait_warp(bar_k_full(slot), (gb / kKSlots) & 1, ctl, 40, gb);
-                    // the buffer held P of the warpgroup's round rr - 2: that PV has to be finished
-                    if (ok) ok = mbar_wait_warp(bar_pv_done(wg, buf), ((rr >> 1) & 1) ^ 1, ctl, 34 + wg, rr);
+                    // the warpgroup has the S of its round before in registers
+                    if (ok) ok = mbar_wait_warp(bar_s_free(wg), (rr & 1) ^ 1, ctl, 34 + wg, gb);
                     if (!ok) break;
                 }
                 // look ahead: probe the two barriers of the item's next block now, read the answer after the MMAs
                 bool nk = false, np = false;
                 if (i + 1 < n_iter) {
-                    const int wg2 = wg ^ 1;
-                    const unsigned rr2 = wg2 ? rr1 : rr0;  // that warpgroup's next round
                     nk = mbar_test(bar_k_full((gb + 1) % kKSlots), ((gb + 1) / kKSlots) & 1);
-                    np = mbar_test(bar_pv_done(wg2, rr2 & 1), ((rr2 >> 1) & 1) ^ 1);
+                    np = mbar_test(bar_s_free(wg ^ 1), ((wg ? rr0 : rr1) & 1) ^ 1);
                 }
                 tc_fence_after();
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
                     if (!(i < (hf ? cb : ca))) continue;  // warp-uniform
-                    const uint64_t qd = smem_desc(sbase + kOffQ + hf * kTileBytes, 16, 1024);
+                    const uint32_t qa = tmem + kTmQ + ((16u * hf) << 16);
                     const uint64_t kd = smem_desc(sbase + kOffK + slot * kSlotBytes + hf * kTileBytes, 16, 1024);
-                    const uint32_t d = tmem + kTmWg * wg + kTmS + 64u * buf + ((16u * hf) << 16);
+                    const uint32_t d = tmem + kTmS + 64u * wg + ((16u * hf) << 16);
 #pragma unroll
                     for (int j = 0; j < kD / 16; ++j) {
                         // 32 bytes per 16-column step inside a 64-column half, halves 8 KiB apart
                         const uint64_t off = (uint64_t)(((j >> 2) * kHalfBytes + (j & 3) * 32) >> 4);
-                        tc_mma(d, qd + off, kd + off, idesc_s, j > 0);
+                        tc_mma_ts(d, qa + 8u * j, kd + off, idesc_s, j > 0);
                     }
                 }
                 tc_commit(bar_k_empty(slot));  // K is free once these MMAs have read it
-                tc_commit(bar_s_full(wg, buf));
-                if (i == n_iter - 1) tc_commit(bar_q_empty);  // and so is Q after the last S of the item
+                tc_commit(bar_s_full(wg));
+                __syncwarp();
+                if (i == n_iter - 1) tc_commit(bar_qt_free);  // and so are Q's TMEM columns after the last S of the item
                 if (wg) ++rr1; else ++rr0;
                 pre = __all_sync(0xffffffffu, nk && np);
             }
@@ -363,9 +427,17 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
         const uint32_t idesc_pv = instr_desc(bf16, 64, 128, 1);
         unsigned gb = 0, wk = 0, rr0 = 0, rr1 = 0;
         bool ok = true;
+        int bh = first_bh, g = first_g, ca_n = 0, cb_n = 0;
+        auto peek = [&](bool there) {  // list lengths of item (bh, g), which is then stepped: read one item ahead
+            if (!there) return;
+            ca_n = clamp_cnt(P, bh, g * kTilesPerWork);
+            cb_n = clamp_cnt(P, bh, g * kTilesPerWork + 1);
+            next_item(bh, g);
+        };
+        peek(blockIdx.x < total_work);
         for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), g = (int)(w % groups);
-            const int ca = clamp_cnt(P, bh, g * kTilesPerWork), cb = clamp_cnt(P, bh, g * kTilesPerWork + 1);
+            const int ca = ca_n, cb = cb_n;
+            peek(w + gridDim.x < total_work);
             const int n_iter = max(1, max(ca, cb));
             // the epilogue of the previous item has read both O accumulators
             ok = mbar_wait_warp(bar_o_free, (wk & 1) ^ 1, ctl, 36, wk);
@@ -373,18 +445,16 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             for (int i = 0; i < n_iter && ok; ++i, ++gb) {
                 const int wg = i & 1;
                 const unsigned rr = wg ? rr1 : rr0;
-                const int slot = gb % kVSlots, buf = rr & 1;
+                const int slot = gb % kVSlots;
                 if (!pre) {
                     ok = mbar_wait_warp(bar_v_full(slot), (gb / kVSlots) & 1, ctl, 60, gb);
-                    if (ok) ok = mbar_wait_warp(bar_p_full(wg, buf), (rr >> 1) & 1, ctl, 50 + wg, rr);
+                    if (ok) ok = mbar_wait_warp(bar_p_full(wg), rr & 1, ctl, 50 + wg, gb);
                     if (!ok) break;
                 }
                 bool nv = false, np = false;  // look ahead to the item's next block
                 if (i + 1 < n_iter) {
-                    const int wg2 = wg ^ 1;
-                    const unsigned rr2 = wg2 ? rr1 : rr0;
                     nv = mbar_test(bar_v_full((gb + 1) % kVSlots), ((gb + 1) / kVSlots) & 1);
-                    np = mbar_test(bar_p_full(wg2, rr2 & 1), (rr2 >> 1) & 1);
+                    np = mbar_test(bar_p_full(wg ^ 1), (wg ? rr0 : rr1) & 1);
                 }
                 tc_fence_after();
                 // A: P in TMEM (first 32 columns of the S buffer), 8 columns per 16-key step; the second tile of
@@ -393,55 +463,21 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
                     if (!(i < (hf ? cb : ca))) continue;  // warp-uniform
-                    const uint32_t pa = tmem + kTmWg * wg + kTmS + 64u * buf + ((16u * hf) << 16);
+                    const uint32_t pa = tmem + kTmP + 32u * wg + ((16u * hf) << 16);
                     const uint64_t vd = smem_desc(sbase + kOffV + slot * kSlotBytes + hf * kTileBytes, kHalfBytes, 1024);
-                    const uint32_t d = tmem + kTmWg * wg + kTmO + ((16u * hf) << 16);
+                    const uint32_t d = tmem + kTmO + 128u * wg + ((16u * hf) << 16);
 #pragma unroll
                     for (int j = 0; j < kBlk / 16; ++j)
                         tc_mma_ts(d, pa + 8u * j, vd + (uint64_t)((j * 2048) >> 4), idesc_pv, (i > 1 || j > 0) ? 1u : 0u);
                 }
                 // the V slot of the item's last block goes to the epilogue, which stages O in it and frees it
                 if (i < n_iter - 1) tc_commit(bar_v_empty(slot));
-                tc_commit(bar_pv_done(wg, buf));
+                tc_commit(bar_pv_done(wg));
+                __syncwarp();
                 if (wg) ++rr1; else ++rr0;
                 pre = __all_sync(0xffffffffu, nv && np);
             }
         }
-      } else {
-        // ================================================================== output store warp
-        // Waits for the staged rows of a work item, sends them off by TMA and hands the V slot they were staged
-        // in back to the producer, so that the warpgroups do not wait for the store.
-        unsigned gb = 0, wk = 0;
-        bool ok = true;
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), g = (int)(w % groups);
-            const int b = bh / P.heads, h = bh % P.heads;
-            const int ca = clamp_cnt(P, bh, g * kTilesPerWork), cb = clamp_cnt(P, bh, g * kTilesPerWork + 1);
-            gb += max(1, max(ca, cb));
-            const unsigned last = gb - 1;
-            ok = mbar_wait_warp(bar_o_staged, wk & 1, ctl, 110, wk);
-            if (ok && lane == 0) {
-                for (int hf = 0; hf < 2; ++hf) {
-                    const int qq = g * kTilesPerWork + hf;
-                    if (qq >= P.nq) continue;
-                    Coord cc = block_coord(P.gq, qq, b, h, P.heads, P.merge_o, P.Tq);
-                    const CUtensorMap* tmo = &P.tm_o[0];
-                    if (P.o_frames > 0) {  // blocks never straddle ranks: o_frames is a multiple of the block's frames
-                        const int dst = cc.c3 / P.o_frames;
-                        cc.c3 -= dst * P.o_frames;
-                        tmo = &P.tm_o[dst];
-                    }
-                    const uint32_t src = sbase + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes;
-                    tma_store_5d(tmo, src, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                    tma_store_5d(tmo, src + kHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
-                }
-                tma_store_commit();
-                tma_store_wait_read();
-                mbar_arrive(bar_v_empty(last % kVSlots));
-            }
-            __syncwarp();
-        }
-        if (lane == 0) tma_store_wait_all();
       }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
@@ -451,18 +487,52 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
         const int hf = lane >> 4;         // tile of the pair this lane serves
         const int row = wq * 16 + (lane & 15);  // row of that tile
         const uint32_t t_lane = (uint32_t)(wq * 32) << 16;
-        const uint32_t tm_s = tmem + kTmWg * wg + kTmS + t_lane;
-        const uint32_t tm_o_mine = tmem + kTmWg * wg + kTmO + t_lane, tm_o_other = tmem + kTmWg * (wg ^ 1) + kTmO + t_lane;
+        const uint32_t tm_s = tmem + kTmS + 64u * wg + t_lane, tm_p = tmem + kTmP + 32u * wg + t_lane;
+        const uint32_t tm_o_mine = tmem + kTmO + 128u * wg + t_lane, tm_o_other = tmem + kTmO + 128u * (wg ^ 1) + t_lane;
         const int ml_idx = wq * 32 + lane;
-        unsigned rr = 0, wk = 0, gb = 0;
+        unsigned wk = 0, gb = 0, rr = 0;  // rr: rounds of this warpgroup over the whole kernel
         bool ok = true;
 
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), g = (int)(w % groups);
+        // Q of the CTA's work item number `item` from shared memory to TMEM: a thread moves its row, the warpgroup 64 of the 128 columns.
+        auto q_to_tmem = [&](unsigned item) -> bool {
+            // the last S of the item before has read the columns
+            if (item > 0 && !mbar_wait_warp(bar_qt_free, (item - 1) & 1, ctl, 106 + wg, item)) return false;
+            if (!mbar_wait_warp(bar_q_full, item & 1, ctl, 108 + wg, item)) return false;
+            tc_fence_after();
+            const unsigned char* src = smem + kOffQ + hf * kTileBytes + wg * kHalfBytes + row * 128;
+            uint32_t qr[32];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint4 v = *reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4));
+                qr[4 * c + 0] = v.x;
+                qr[4 * c + 1] = v.y;
+                qr[4 * c + 2] = v.z;
+                qr[4 * c + 3] = v.w;
+            }
+            tc_st32(tmem + kTmQ + 32u * wg + t_lane, qr);
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            mbar_arrive_elect(bar_q_empty);
+            mbar_arrive_elect(bar_qt_full);
+            return true;
+        };
+        if (blockIdx.x < total_work) ok = q_to_tmem(0);
+
+        int bh = first_bh, g = first_g, nx_bh = first_bh, nx_g = first_g, my_n = 0, other_n = 0;
+        auto peek = [&](bool there) {  // list lengths of item nx, read one item ahead
+            if (there) {
+                my_n = clamp_cnt(P, nx_bh, nx_g * kTilesPerWork + hf);
+                other_n = clamp_cnt(P, nx_bh, nx_g * kTilesPerWork + (hf ^ 1));
+            }
+        };
+        peek(blockIdx.x < total_work);
+        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, g = nx_g) {
             const int qt = g * kTilesPerWork + hf;
             const bool tile_valid = qt < P.nq;
-            const int my_cnt = clamp_cnt(P, bh, qt);
-            const int other_cnt = clamp_cnt(P, bh, g * kTilesPerWork + (hf ^ 1));
+            const int my_cnt = my_n, other_cnt = other_n;
+            next_item(nx_bh, nx_g);
+            peek(w + gridDim.x < total_work);
             const int n_iter = max(1, max(my_cnt, other_cnt));
             const int32_t* my_list = P.idx + ((long long)bh * P.nq + (tile_valid ? qt : 0)) * P.cap;
 
@@ -472,18 +542,21 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             // ragged grids: the block index of a round is fetched a round ahead, so that the global load never sits
             // between S and the softmax
             int blk_ahead = (kRagged && wg < my_cnt) ? my_list[wg] : 0;
+            // S of the warpgroup's round into registers; the buffer is then free for the S of its next round
+            uint32_t sr[64];
+            if (wg < n_iter) {
+                ok = mbar_wait_warp(bar_s_full(wg), rr & 1, ctl, 80 + wg, rr);
+                if (!ok) break;
+                tc_fence_after();
+                tc_ld64(tm_s, sr);
+                tc_wait_ld();
+                tc_fence_before();
+                mbar_arrive_elect(bar_s_free(wg));
+            }
             for (int i = wg; i < n_iter && ok; i += 2, ++rr) {
                 const bool active = i < my_cnt;
                 const int blk_now = blk_ahead;
                 if (kRagged && i + 2 < my_cnt) blk_ahead = my_list[i + 2];
-                const int buf = rr & 1;
-                const unsigned bph = (rr >> 1) & 1;
-                ok = mbar_wait_warp(bar_s_full(wg, buf), bph, ctl, 80 + wg, rr);
-                if (!ok) break;
-                tc_fence_after();
-                uint32_t sr[64];
-                tc_ld64(tm_s + 64u * buf, sr);
-                tc_wait_ld();
                 float alpha = 1.f;
                 bool need = false;
                 uint4 pk[8];  // this row of P in the input dtype, 8 keys per 16-byte chunk
@@ -503,9 +576,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                             }
                         }
                     }
-                    // One pass: the probabilities are computed against the current reference maximum while
-                    // the row maximum is tracked on the side; only if the maximum has moved by more than 2^8
-                    // (or this is the warpgroup's first block) is the pass repeated with the new reference.
+                    // One pass: the probabilities are computed against the current reference maximum while the row maximum is
+                    // tracked beside them (one basic block, so that the comparisons run under the exponentials); only if the
+                    // maximum has moved by more than 2^8 is the pass repeated with the new reference.  The warpgroup's first
+                    // block takes its own maximum as the reference.
                     auto probs = [&](float mref, float& rsum) {
                         // two keys per instruction where the machine has packed fp32 forms (fma, add); the four partial
                         // sums take the keys j = 0, 1, 2, 3 (mod 4) in ascending order
@@ -531,64 +605,38 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                         }
                         rsum = (r01.x + r01.y) + (r23.x + r23.y);
                     };
-                    // the reference maximum this row would have after this block (in units of log2)
-                    auto row_reference = [&]() {
+                    // the row maximum of this block, in units of log2
+                    auto row_max = [&]() {
                         float mx8[8];  // eight chains of eight values, three at a time
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
                             auto sv = [&](int i) { return __uint_as_float(sr[8 * i + k]); };
                             mx8[k] = fmaxf(max3(max3(max3(sv(0), sv(1), sv(2)), sv(3), sv(4)), sv(5), sv(6)), sv(7));
                         }
-                        const float mx = fmaxf(max3(max3(mx8[0], mx8[1], mx8[2]), mx8[3], mx8[4]), max3(mx8[5], mx8[6], mx8[7]));
-                        return fmaxf(m_ref, mx * P.scale2);
+                        return fmaxf(max3(max3(mx8[0], mx8[1], mx8[2]), mx8[3], mx8[4]), max3(mx8[5], mx8[6], mx8[7])) * P.scale2;
                     };
                     float rs = 0.f;
                     float m_new = m_ref;
-                    if (kRagged) {
-                        // the instantiation with the masking code: a single copy of the pass in the instruction stream.
-                        // The loop body runs once in the common case (pass, then the row maximum, which confirms the
-                        // reference) and twice when the reference moves; for the warpgroup's first block the first
-                        // pass is skipped.
-                        bool run_pass = !first, decided = false;
-#pragma unroll 1
-                        for (int turn = 0; turn < 2; ++turn) {
-                            if (run_pass) probs(m_ref, rs);
-                            if (decided) break;
-                            m_new = row_reference();
-                            run_pass = first || m_new - m_ref > 8.f;
-                            if (!run_pass) break;
-                            if (!first) {
-                                need = true;
-                                alpha = ex2(m_ref - m_new);
-                            }
-                            m_ref = (m_new == -INFINITY) ? 0.f : m_new;
-                            decided = true;
-                        }
-                    } else {
-                        // whole grids: straight-line code, the second copy of the pass off the common path
-                        if (!first) probs(m_ref, rs);
-                        m_new = row_reference();
-                        if (LCBSA_UNLIKELY(first || m_new - m_ref > 8.f)) {
-                            if (!first) {
-                                need = true;
-                                alpha = ex2(m_ref - m_new);
-                            }
-                            m_ref = (m_new == -INFINITY) ? 0.f : m_new;
-                            probs(m_ref, rs);
-                        }
+                    if (LCBSA_UNLIKELY(first)) {
+                        m_new = fmaxf(m_ref, row_max());
+                        m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+                    }
+                    probs(m_ref, rs);
+                    const float m_top = row_max();
+                    if (LCBSA_UNLIKELY(m_top - m_ref > 8.f)) {
+                        need = true;
+                        alpha = ex2(m_ref - m_top);
+                        m_ref = m_top;
+                        probs(m_ref, rs);
                     }
                     l_sum = l_sum * alpha + rs;  // alpha is 1 unless this row's reference maximum moved
                 }
                 first = false;
                 const bool any_need = __any_sync(0xffffffffu, need);
-                // O is rescaled only at rest: the warpgroup's PV of the round before has to be finished
-                // (need implies that this is not the warpgroup's first round of the item, so rr > 0)
-                if (LCBSA_UNLIKELY(any_need)) {
-                    ok = mbar_wait_warp(bar_pv_done(wg, buf ^ 1), ((rr - 1) >> 1) & 1, ctl, 92 + wg, rr);
-                    if (!ok) break;
-                }
-                {   // P overwrites the first half of the S buffer just read; all 32 lanes take part in the store
-                    // (a lane whose tile has run out of blocks writes don't-cares)
+                // P may be overwritten, and O rescaled, once the warpgroup's PV of the round before has finished
+                ok = mbar_wait_warp(bar_pv_done(wg), (rr & 1) ^ 1, ctl, 92 + wg, rr);
+                if (!ok) break;
+                {   // all 32 lanes take part in the store (a lane whose tile has run out of blocks writes don't-cares)
                     uint32_t pr[32];
 #pragma unroll
                     for (int cch = 0; cch < 8; ++cch) {
@@ -597,22 +645,38 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                         pr[4 * cch + 2] = pk[cch].z;
                         pr[4 * cch + 3] = pk[cch].w;
                     }
-                    tc_st32(tm_s + 64u * buf, pr);
+                    tc_st32(tm_p, pr);
                 }
                 if (LCBSA_UNLIKELY(any_need)) tc_scale_row128(tm_o_mine, alpha);  // rare: only when a row maximum jumps
-                tc_wait_st();
-                tc_fence_before();
-                mbar_arrive_elect(bar_p_full(wg, buf));
+                if (i + 2 < n_iter) {
+                    // The next round's S is on its way into the registers while P is being stored: it has usually been ready
+                    // for some hundred cycles, since it only waits for this round's S to be in registers.
+                    ok = mbar_wait_warp(bar_s_full(wg), (rr + 1) & 1, ctl, 80 + wg, rr);
+                    if (!ok) break;
+                    tc_fence_after();
+                    __syncwarp();
+                    tc_ld64(tm_s, sr);
+                    tc_wait_st();
+                    tc_fence_before();
+                    mbar_arrive_elect(bar_p_full(wg));
+                    tc_wait_ld();
+                    tc_fence_before();
+                    mbar_arrive_elect(bar_s_free(wg));
+                } else {
+                    tc_wait_st();
+                    tc_fence_before();
+                    mbar_arrive_elect(bar_p_full(wg));
+                }
             }
             if (!ok) break;
             gb += n_iter;
+            // Q of the next item, so that its S runs under this item's epilogue
+            if (w + gridDim.x < total_work && !q_to_tmem(wk + 1)) break;
 
             // ---- epilogue of this work item.  The warpgroup's PVs are finished once its last one is; it then
             // publishes (maximum, row sum) of its rows and waits for the other warpgroup to do the same.
-            const int my_rounds = (n_iter - wg + 1) >> 1;  // blocks wg, wg + 2, ... below n_iter
-            if (my_rounds > 0) {
-                const unsigned lr = rr - 1;
-                ok = mbar_wait_warp(bar_pv_done(wg, lr & 1), (lr >> 1) & 1, ctl, 100 + wg, lr);
+            if (n_iter > wg) {
+                ok = mbar_wait_warp(bar_pv_done(wg), (rr - 1) & 1, ctl, 100 + wg, rr);
                 if (!ok) break;
             }
             // the other warpgroup has read this warpgroup's entry of the previous item before it arrived on o_free
@@ -638,31 +702,37 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             // half-tile row per thread) in the V slot that the item's last PV has just released.
             const unsigned last = gb - 1;
             unsigned char* o_half = smem + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes + wg * kHalfBytes;
+            // a warpgroup that saw no block has weight 0; its accumulator holds garbage and is not used
+            const bool rd_mine = __any_sync(0xffffffffu, w_mine > 0.f), rd_oth = __any_sync(0xffffffffu, w_oth > 0.f);
+            const bool both = __all_sync(0xffffffffu, w_mine > 0.f && w_oth > 0.f);  // the usual case: no lane has to be masked
+            const float2 fm2 = make_float2(f_mine, f_mine), fo2 = make_float2(f_oth, f_oth);
 #pragma unroll
             for (int cch = 0; cch < 2; ++cch) {
                 uint32_t oa[32], ob[32];
-                // a warpgroup that saw no block has weight 0; its accumulator holds garbage and is not used
-                const bool rd_mine = __any_sync(0xffffffffu, w_mine > 0.f), rd_oth = __any_sync(0xffffffffu, w_oth > 0.f);
                 if (rd_mine) tc_ld32(tm_o_mine + 64 * wg + 32 * cch, oa);
                 if (rd_oth) tc_ld32(tm_o_other + 64 * wg + 32 * cch, ob);
                 tc_wait_ld();
+                if (LCBSA_UNLIKELY(!both)) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        if (!(w_mine > 0.f)) oa[j] = 0u;
+                        if (!(w_oth > 0.f)) ob[j] = 0u;
+                    }
+                }
                 if (tile_valid) {
 #pragma unroll
                     for (int q8 = 0; q8 < 4; ++q8) {
-                        float v[8];
+                        uint32_t pw[4];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float a = w_mine > 0.f ? __uint_as_float(oa[q8 * 8 + j]) * f_mine : 0.f;
-                            const float bb = w_oth > 0.f ? __uint_as_float(ob[q8 * 8 + j]) * f_oth : 0.f;
-                            v[j] = a + bb;
+                        for (int j = 0; j < 4; ++j) {
+                            const int e = q8 * 8 + 2 * j;
+                            const float2 a2 = __fmul2_rn(make_float2(__uint_as_float(oa[e]), __uint_as_float(oa[e + 1])), fm2);
+                            const float2 b2 = __fmul2_rn(make_float2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), fo2);
+                            const float2 v2 = __fadd2_rn(a2, b2);
+                            pw[j] = pack2(bf16, v2.x, v2.y);
                         }
-                        uint4 pk;
-                        pk.x = pack2(bf16, v[0], v[1]);
-                        pk.y = pack2(bf16, v[2], v[3]);
-                        pk.z = pack2(bf16, v[4], v[5]);
-                        pk.w = pack2(bf16, v[6], v[7]);
                         const int chunk = cch * 4 + q8;
-                        *reinterpret_cast<uint4*>(o_half + row * 128 + ((chunk ^ (row & 7)) << 4)) = pk;
+                        *reinterpret_cast<uint4*>(o_half + row * 128 + ((chunk ^ (row & 7)) << 4)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
                     }
                 }
             }

@@ -11,18 +11,25 @@
 // One persistent CTA per SM.  A work item is ONE query block of one head: a 128-row tile, i.e. M=128 tcgen05 MMAs
 // that run the tensor pipe at its full rate (the 64-row tiles of the other kernel occupy it like 128-row ones).  A
 // selected key block is processed as 2, 4 or 8 units of 64 keys (sub-boxes of the block, cut along its outermost even
-// axes), which keeps the S tile at 64 TMEM columns, so that every warpgroup has two S/P buffers beside its O
-// accumulator, exactly as in the 64-token kernel:
+// axes), which keeps the S tile at 64 TMEM columns, so that S, P and O of both warpgroups and Q fit, exactly as in the
+// 64-token kernel:
 //
 //   warps 0-3, 4-7 : softmax warpgroups 0 and 1 (units of even / odd number; thread = one query row)
-//   warp 8 : TMA producer (Q tile, K ring, V ring)   warp 9 : S = Q K^T issuer   warp 10 : O += P V issuer
-//   warp 11: output TMA stores
+//   warp 8 : TMA producer of Q and K   warp 9 : S = Q K^T issuer   warp 10 : O += P V issuer
+//   warp 11: TMA producer of V, output TMA stores
 //
-// Per unit i (warpgroup g = i & 1, its round r = i >> 1):  S = Q K^T (M128 N64 K128, buffer r & 1 of the warpgroup)
-// -> tcgen05.ld, exp2 online softmax in registers, P in the input dtype over the first half of the same buffer ->
+// Per unit i (warpgroup g = i & 1):  S = Q K^T (M128 N64 K128, A = Q from TMEM) -> tcgen05.ld, exp2 online softmax in registers, P in the input dtype into TMEM columns of its own ->
 // O_g += P V (M128 N128 K64, A from TMEM).  The two warpgroups keep separate maxima, row sums and accumulators and
 // are merged once per work item.  K and V rings: six slots of one 64-key tile (16 KiB) each.  The finished O
 // (128 rows x 256 B) is staged in the V slots of the item's last two units and leaves by TMA store.
+//
+// Q in TMEM: an S with both operands in shared memory reads 48 KB of them per unit, which takes longer than its MMAs
+// (M128 N64 K128: 256 cycles); with A from TMEM it reads 16 KB.
+// What bounds it: the softmax warps.  A unit's MMAs take 512 cycles, its exponentials 512 cycles of the transcendental
+// unit, and a warpgroup needs about 1900 cycles per round (two rounds per pair of units at the same time): the two
+// warpgroups run in step, so nobody uses the transcendental unit while both store P and fetch S.  720p grid, 90 of 720
+// blocks, 8 heads, attention launch: 5.08 ms with one producer warp, Q in shared memory and P over S; 4.0 ms now; with 32
+// heads (17 ms) the launch runs into the power cap of the GPU.
 //
 // Every wait on an mbarrier is bounded, as in attn_tc.cu.
 #include "tc_common.cuh"
@@ -44,22 +51,21 @@ constexpr int kHalfBytes = kTileBytes / 2;         // one 64-column half: 64 row
 constexpr int kSlotBytes = kTileBytes;             // a ring slot holds one unit's tile
 constexpr int kMaxUnits = 8;                       // units of 64 keys per key block: blocks of up to 512 tokens
 constexpr int kKSlots = 6, kVSlots = 6;            // even, like the number of units of an item: the last two units sit in a slot pair
-constexpr int kKLead = 4;                          // K units requested ahead of V: S runs two rounds of each warpgroup ahead
 constexpr int kThreads = 384;
 // setmaxnreg per warpgroup: (208 + 208 + 88) * 128 threads <= the 64 K registers of the SM
 constexpr int kRegsSoftmax = 208, kRegsOther = 88;
 
-// TMEM columns of warpgroup g: base 256 * g
-constexpr uint32_t kTmWg = 256, kTmS = 0, kTmO = 128;
+// TMEM columns: O accumulator of warpgroup g at 128 * g, its S at 256 + 64 * g, its P (16-bit pairs) at 384 + 32 * g; Q (16-bit pairs)
+constexpr uint32_t kTmO = 0, kTmS = 256, kTmP = 384, kTmQ = 448;
 
 // shared memory map (offsets from the 1024-byte aligned base of dynamic shared memory)
 constexpr int kOffQ = 0;
 constexpr int kOffK = kOffQ + kQTileBytes;
 constexpr int kOffV = kOffK + kKSlots * kSlotBytes;
 constexpr int kOffBar = kOffV + kVSlots * kSlotBytes;
-// barriers: k_full[6] k_empty[6] v_full[6] v_empty[6] q_full q_empty s_full[2][2] p_full[2][2] pv_done[2][2]
-//           ml_ready o_free o_staged
-constexpr int kNumBars = 2 * kKSlots + 2 * kVSlots + 2 + 12 + 3;
+// barriers: k_full[6] k_empty[6] v_full[6] v_empty[6] q_full q_empty s_full[2] s_free[2] p_full[2] pv_done[2]
+//           ml_ready o_free o_staged qt_full qt_free
+constexpr int kNumBars = 2 * kKSlots + 2 * kVSlots + 2 + 8 + 5;
 constexpr int kOffMisc = kOffBar + kNumBars * 8;      // abort flag, TMEM base
 constexpr int kOffMl = kOffMisc + 64;                 // [2 warpgroups][128 lanes] (maximum, row sum)
 constexpr int kSmemBytes = kOffMl + 2 * 128 * 8;
@@ -110,10 +116,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
     auto bar_v_empty = [&](int s) { return bar0 + 8u * (2 * kKSlots + kVSlots + s); };
     constexpr int kB0 = 2 * kKSlots + 2 * kVSlots;
     const uint32_t bar_q_full = bar0 + 8u * kB0, bar_q_empty = bar0 + 8u * (kB0 + 1);
-    auto bar_s_full = [&](int wg, int buf) { return bar0 + 8u * (kB0 + 2 + 2 * wg + buf); };
-    auto bar_p_full = [&](int wg, int buf) { return bar0 + 8u * (kB0 + 6 + 2 * wg + buf); };
-    auto bar_pv_done = [&](int wg, int buf) { return bar0 + 8u * (kB0 + 10 + 2 * wg + buf); };
-    const uint32_t bar_ml_ready = bar0 + 8u * (kB0 + 14), bar_o_free = bar0 + 8u * (kB0 + 15), bar_o_staged = bar0 + 8u * (kB0 + 16);
+    auto bar_s_full = [&](int wg) { return bar0 + 8u * (kB0 + 2 + wg); };
+    auto bar_s_free = [&](int wg) { return bar0 + 8u * (kB0 + 4 + wg); };
+    auto bar_p_full = [&](int wg) { return bar0 + 8u * (kB0 + 6 + wg); };
+    auto bar_pv_done = [&](int wg) { return bar0 + 8u * (kB0 + 8 + wg); };
+    constexpr int kB1 = kB0 + 10;
+    const uint32_t bar_ml_ready = bar0 + 8u * kB1, bar_o_free = bar0 + 8u * (kB1 + 1), bar_o_staged = bar0 + 8u * (kB1 + 2);
+    const uint32_t bar_qt_full = bar0 + 8u * (kB1 + 3), bar_qt_free = bar0 + 8u * (kB1 + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kOffMisc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffMisc + 8);
     float2* ml = reinterpret_cast<float2*>(smem + kOffMl);  // [2][128]
@@ -133,13 +142,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
             mbar_init(bar_v_empty(s), 1);
         }
         mbar_init(bar_q_full, 1);
-        mbar_init(bar_q_empty, 1);
-        for (int g = 0; g < 2; ++g)
-            for (int b = 0; b < 2; ++b) {
-                mbar_init(bar_s_full(g, b), 1);
-                mbar_init(bar_p_full(g, b), 4);  // one elected arrival per softmax warp
-                mbar_init(bar_pv_done(g, b), 1);
-            }
+        mbar_init(bar_q_empty, 8);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar_s_full(b), 1);
+            mbar_init(bar_s_free(b), 4);
+            mbar_init(bar_p_full(b), 4);  // one elected arrival per softmax warp
+            mbar_init(bar_pv_done(b), 1);
+        }
+        mbar_init(bar_qt_full, 8);
+        mbar_init(bar_qt_free, 1);
         mbar_init(bar_ml_ready, 8);
         mbar_init(bar_o_free, 8);
         mbar_init(bar_o_staged, 8);
@@ -167,36 +178,73 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
 
     const int groups = P.nq;  // one work item per query block
     const long long total_work = start_ok ? (long long)P.bh_total * groups : 0;
+    // The CTA's items are blockIdx.x, blockIdx.x + gridDim.x, ...; every role steps through them as (head, query block) pairs, since a
+    // 64-bit division per role and item costs more than a round.
+    const int first_bh = (int)(blockIdx.x / (unsigned)groups), first_g = (int)(blockIdx.x % (unsigned)groups);
+    const int step_bh = (int)(gridDim.x / (unsigned)groups), step_g = (int)(gridDim.x % (unsigned)groups);
+    auto next_item = [&](int& bh, int& g) {
+        bh += step_bh;
+        g += step_g;
+        if (g >= groups) {
+            g -= groups;
+            ++bh;
+        }
+    };
     constexpr bool bf16 = kBf16;
 
     // All roles walk the same list of work items and units.  Unit number gb (counted over the whole kernel)
-    // uses K slot gb % 6 and V slot gb % 6; warpgroup g numbers its own rounds rr[g] over the whole kernel and
-    // round rr uses S/P buffer rr & 1.  Within an item unit i belongs to warpgroup i & 1.
+    // uses K slot gb % 6 and V slot gb % 6.  Within an item unit i belongs to warpgroup i & 1.
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-      if (warp == 8) {
-        // ================================================================== TMA producer
+      if (warp == 8 || warp == 11) {
+        // ================================================================== TMA producers: warp 8 Q and K, warp 11 V and the output
+        // The output rows of an item are staged in the two V slots its last PVs released.  Warp 11 sends them off when it needs
+        // the first of them again, at the latest before it requests the last V of the item behind it (the epilogue of that item
+        // completes the next phase of o_staged, so the wait is never a phase behind).
+        const bool is_k = warp == 8;
         unsigned gk = 0, gv = 0, wk = 0, nq_issued = 0;
+        int s_bh = first_bh, s_g = first_g;  // item whose output is stored next
+        unsigned ws_end = 0, ks = 0;        // units up to and including it, its number
         bool ok = true;
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), qb = (int)(w % groups);
+        auto store_item = [&]() -> bool {
+            const int bh = s_bh, qb = s_g;
             const int b = bh / P.heads, h = bh % P.heads;
-            const int cnt = clamp_cnt(P, bh, qb);
+            const int s0 = (int)((ws_end - 2) % kVSlots);  // ws_end is even and so is the ring: slots s0 and s0 + 1
+            if (!mbar_wait_warp(bar_o_staged, ks & 1, ctl, 110, ks)) return false;
+            if (lane == 0) {
+                Coord cc = block_coord(P.gq, qb, b, h, P.heads, P.merge_o, P.Tq);
+                const CUtensorMap* tmo = &P.tm_o[0];
+                if (P.o_frames > 0) {  // blocks never straddle ranks: o_frames is a multiple of the block's frames
+                    const int dst = cc.c3 / P.o_frames;
+                    cc.c3 -= dst * P.o_frames;
+                    tmo = &P.tm_o[dst];
+                }
+                const uint32_t src = sbase + kOffV + s0 * kSlotBytes;
+                tma_store_5d(tmo, src, 0, cc.c1, cc.c2, cc.c3, cc.c4);
+                tma_store_5d(tmo, src + kQHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+                tma_store_commit();
+                tma_store_wait_read();
+                mbar_arrive(bar_v_empty(s0));
+                mbar_arrive(bar_v_empty(s0 + 1));
+            }
+            __syncwarp();
+            next_item(s_bh, s_g);
+            ++ks;
+            return true;
+        };
+        int bh = first_bh, qb = first_g, nx_bh = first_bh, nx_g = first_g;
+        int cnt_n = 0;
+        auto peek = [&](bool there) {  // list length of item nx, read one item ahead
+            if (there) cnt_n = clamp_cnt(P, nx_bh, nx_g);
+        };
+        peek(blockIdx.x < total_work);
+        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, qb = nx_g) {
+            const int b = bh / P.heads, h = bh % P.heads;
+            const int cnt = cnt_n;
             const int n_act = cnt << P.lg_units;  // units that exist: 2, 4 or 8 per listed key block
             const int n_iter = max(2, n_act);     // an empty list still goes through one (masked) pair of units
-            // Q tile: the buffer is free once the last S of the previous item has been computed
-            ok = mbar_wait_warp(bar_q_empty, (wk & 1) ^ 1, ctl, 10, wk);
-            if (!ok) break;
-            ++nq_issued;
-            if (lane == 0) {
-                mbar_arrive_tx(bar_q_full, kQTileBytes);
-                const Coord cc = block_coord(P.gq, qb, b, h, P.heads, P.merge_q, P.Tq);
-                tma_load_5d(sbase + kOffQ, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                tma_load_5d(sbase + kOffQ + kQHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
-            }
-            // Block coordinates are fetched and decoded by the whole warp: lane L holds list entry win + L as the
-            // block's first token packed t << 20 | h << 10 | w.  `prv` holds the window of thirty-two entries before
-            // (V trails K by kKLead units).
+            // Block coordinates are fetched and decoded by the whole warp: lane L holds list entry 32 n + L as the
+            // block's first token packed t << 20 | h << 10 | w.  `nxt` holds the thirty-two entries behind the current ones.
             const int32_t* my_l = P.idx + ((long long)bh * P.nq + qb) * P.cap;
             auto fetch = [&](int e) {
                 if (e >= cnt) return 0;
@@ -215,66 +263,63 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                 block_coords(P.gk, blk, bt, bhh, bw);
                 return ((bt * P.gk.ct) << 20) | ((bhh * P.gk.ch) << 10) | (bw * P.gk.cw);
             };
-            int win = 0, prv = 0;
             int cur = fetch(lane);
-            const int c3k = P.merge_k ? b * P.Tk : 0, c4k = P.merge_k ? h : b * P.heads + h;
-            const int c3v = P.merge_v ? b * P.Tk : 0, c4v = P.merge_v ? h : b * P.heads + h;
-            // coordinates of unit u: those of its block plus the offset of the unit inside the block
-            auto unit_coords = [&](int pk, int u, int& cw, int& chh, int& ctt) {
-                cw = pk & 1023;
-                chh = (pk >> 10) & 1023;
-                ctt = pk >> 20;
-                const int sub = u & ((1 << P.lg_units) - 1);
-                ctt += P.sub_t[sub];
-                chh += P.sub_h[sub];
-                cw += P.sub_w[sub];
-            };
-            for (int j = 0; j < n_iter + kKLead && ok; ++j) {
-                if (j >= kKLead) {  // V(j - kKLead)
-                    const int jj = j - kKLead, e = jj >> P.lg_units;
-                    const int pk = __shfl_sync(0xffffffffu, e >= win ? cur : prv, e >= win ? e - win : e - (win - 32));
-                    const bool act = jj < n_act;
-                    const int slot = gv % kVSlots;
-                    ok = mbar_wait_warp(bar_v_empty(slot), ((gv / kVSlots) & 1) ^ 1, ctl, 22, gv);
-                    if (!ok) break;
-                    ++gv;
-                    if (lane == 0) {
-                        mbar_arrive_tx(bar_v_full(slot), act ? kTileBytes : 0);
-                        if (act) {
-                            int cw, chh, ctt;
-                            unit_coords(pk, jj, cw, chh, ctt);
-                            const uint32_t dst = sbase + kOffV + slot * kSlotBytes;
-                            tma_load_5d(dst, &P.tm_v, bar_v_full(slot), 0, cw, chh, ctt + c3v, c4v);
-                            tma_load_5d(dst + kHalfBytes, &P.tm_v, bar_v_full(slot), 64, cw, chh, ctt + c3v, c4v);
-                        }
-                    }
+            int nxt = fetch(32 + lane);
+            next_item(nx_bh, nx_g);
+            peek(w + gridDim.x < total_work);
+            const bool mrg = is_k ? P.merge_k : P.merge_v;
+            const int c3 = mrg ? b * P.Tk : 0, c4 = mrg ? h : b * P.heads + h;
+            // the boxes of unit j: its block's first token plus the offset of the unit inside the block
+            auto request = [&](int j, const CUtensorMap* tm, uint32_t bar, uint32_t dst) {
+                const int e = j >> P.lg_units, u = j & ((1 << P.lg_units) - 1);
+                const int pk = __shfl_sync(0xffffffffu, cur, e & 31);
+                mbar_arrive_tx_elect(bar, j < n_act ? kTileBytes : 0);
+                if (j < n_act) {
+                    const int cw = (pk & 1023) + P.sub_w[u], chh = ((pk >> 10) & 1023) + P.sub_h[u], ctt = (pk >> 20) + P.sub_t[u] + c3;
+                    tma_load_5d_elect(dst, tm, bar, 0, cw, chh, ctt, c4);
+                    tma_load_5d_elect(dst + kHalfBytes, tm, bar, 64, cw, chh, ctt, c4);
                 }
-                if (j < n_iter) {  // K(j)
-                    const int e = j >> P.lg_units;
-                    while (e >= win + 32) {
-                        win += 32;
-                        prv = cur;
-                        cur = fetch(win + lane);
-                    }
-                    const int pk = __shfl_sync(0xffffffffu, cur, e - win);
-                    const bool act = j < n_act;
+                if ((e & 31) == 31 && u == (1 << P.lg_units) - 1) {
+                    cur = nxt;
+                    nxt = fetch(e + 33 + lane);
+                }
+            };
+            if (is_k) {
+                // Q tile: the buffer is free once the softmax warps have moved the previous item's Q to TMEM
+                ok = mbar_wait_warp(bar_q_empty, (wk & 1) ^ 1, ctl, 10, wk);
+                if (!ok) break;
+                ++nq_issued;
+                if (lane == 0) {
+                    mbar_arrive_tx(bar_q_full, kQTileBytes);
+                    const Coord cc = block_coord(P.gq, qb, b, h, P.heads, P.merge_q, P.Tq);
+                    tma_load_5d(sbase + kOffQ, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
+                    tma_load_5d(sbase + kOffQ + kQHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+                }
+                __syncwarp();
+                for (int j = 0; j < n_iter; ++j) {
                     const int slot = gk % kKSlots;
                     ok = mbar_wait_warp(bar_k_empty(slot), ((gk / kKSlots) & 1) ^ 1, ctl, 20, gk);
                     if (!ok) break;
                     ++gk;
-                    if (lane == 0) {
-                        mbar_arrive_tx(bar_k_full(slot), act ? kTileBytes : 0);
-                        if (act) {
-                            int cw, chh, ctt;
-                            unit_coords(pk, j, cw, chh, ctt);
-                            const uint32_t dst = sbase + kOffK + slot * kSlotBytes;
-                            tma_load_5d(dst, &P.tm_k, bar_k_full(slot), 0, cw, chh, ctt + c3k, c4k);
-                            tma_load_5d(dst + kHalfBytes, &P.tm_k, bar_k_full(slot), 64, cw, chh, ctt + c3k, c4k);
-                        }
-                    }
+                    request(j, &P.tm_k, bar_k_full(slot), sbase + kOffK + slot * kSlotBytes);
                 }
+            } else {
+                for (int j = 0; j < n_iter; ++j) {
+                    if (ks < wk && (gv >= ws_end - 2 + kVSlots || j == n_iter - 1)) {
+                        ok = store_item();
+                        if (!ok) break;
+                    }
+                    const int slot = gv % kVSlots;
+                    ok = mbar_wait_warp(bar_v_empty(slot), ((gv / kVSlots) & 1) ^ 1, ctl, 22, gv);
+                    if (!ok) break;
+                    ++gv;
+                    request(j, &P.tm_v, bar_v_full(slot), sbase + kOffV + slot * kSlotBytes);
+                }
+                ws_end = gv;  // the item before has been stored
             }
         }
+        if (!is_k && ok && ks < wk) ok = store_item();
+        if (!is_k && lane == 0) tma_store_wait_all();
         if (!ok && lane == 0) {
             // drain: give the copies this warp issued a bounded time to land before the CTA exits
             const long long t0 = clock64();
@@ -291,49 +336,52 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
       } else if (warp == 9) {
         // ================================================================== S = Q K^T issuer
         const uint32_t idesc_s = instr_desc(bf16, kQRows, kBlk, 0);
-        const uint64_t qd = smem_desc(sbase + kOffQ, 16, 1024);
         unsigned gb = 0, wk = 0, rr0 = 0, rr1 = 0;
         bool ok = true;
+        int bh = first_bh, g = first_g, cnt_n = 0;
+        auto peek = [&](bool there) {  // list length of item (bh, g), which is then stepped: read one item ahead
+            if (!there) return;
+            cnt_n = clamp_cnt(P, bh, g);
+            next_item(bh, g);
+        };
+        peek(blockIdx.x < total_work);
         for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), qb = (int)(w % groups);
-            const int n_act = clamp_cnt(P, bh, qb) << P.lg_units;
+            const int n_act = cnt_n << P.lg_units;
+            peek(w + gridDim.x < total_work);
             const int n_iter = max(2, n_act);
-            ok = mbar_wait_warp(bar_q_full, wk & 1, ctl, 30, wk);
+            ok = mbar_wait_warp(bar_qt_full, wk & 1, ctl, 30, wk);  // Q of this item is in TMEM
             bool pre = false;
             for (int i = 0; i < n_iter && ok; ++i, ++gb) {
                 const int wg = i & 1;
                 const unsigned rr = wg ? rr1 : rr0;
-                const int slot = gb % kKSlots, buf = rr & 1;
+                const int slot = gb % kKSlots;
                 if (!pre) {  // not already seen ready by the look-ahead of the unit before
                     ok = mbar_wait_warp(bar_k_full(slot), (gb / kKSlots) & 1, ctl, 40, gb);
-                    // the buffer held P of the warpgroup's round rr - 2: that PV has to be finished
-                    if (ok) ok = mbar_wait_warp(bar_pv_done(wg, buf), ((rr >> 1) & 1) ^ 1, ctl, 34 + wg, rr);
+                    // the warpgroup has the S of its round before in registers
+                    if (ok) ok = mbar_wait_warp(bar_s_free(wg), (rr & 1) ^ 1, ctl, 34 + wg, gb);
                     if (!ok) break;
                 }
                 // look ahead: probe the two barriers of the item's next unit now, read the answer after the MMAs
                 bool nk = false, np = false;
                 if (i + 1 < n_iter) {
-                    const int wg2 = wg ^ 1;
-                    const unsigned rr2 = wg2 ? rr1 : rr0;  // that warpgroup's next round
                     nk = mbar_test(bar_k_full((gb + 1) % kKSlots), ((gb + 1) / kKSlots) & 1);
-                    np = mbar_test(bar_pv_done(wg2, rr2 & 1), ((rr2 >> 1) & 1) ^ 1);
+                    np = mbar_test(bar_s_free(wg ^ 1), ((wg ? rr0 : rr1) & 1) ^ 1);
                 }
                 tc_fence_after();
                 if (i < n_act) {
                     const uint64_t kd = smem_desc(sbase + kOffK + slot * kSlotBytes, 16, 1024);
-                    const uint32_t d = tmem + kTmWg * wg + kTmS + 64u * buf;
+                    const uint32_t d = tmem + kTmS + 64u * wg;
 #pragma unroll
                     for (int j = 0; j < kD / 16; ++j) {
-                        // 32 bytes per 16-column step inside a 64-column half; the halves are 16 KiB (Q) and
-                        // 8 KiB (K) apart
-                        const uint64_t qoff = (uint64_t)(((j >> 2) * kQHalfBytes + (j & 3) * 32) >> 4);
+                        // 32 bytes per 16-column step inside a 64-column half, halves 8 KiB apart
                         const uint64_t koff = (uint64_t)(((j >> 2) * kHalfBytes + (j & 3) * 32) >> 4);
-                        tc_mma(d, qd + qoff, kd + koff, idesc_s, j > 0);
+                        tc_mma_ts(d, tmem + kTmQ + 8u * j, kd + koff, idesc_s, j > 0);
                     }
                 }
                 tc_commit(bar_k_empty(slot));  // K is free once these MMAs have read it
-                tc_commit(bar_s_full(wg, buf));
-                if (i == n_iter - 1) tc_commit(bar_q_empty);  // and so is Q after the last S of the item
+                tc_commit(bar_s_full(wg));
+                __syncwarp();
+                if (i == n_iter - 1) tc_commit(bar_qt_free);  // and so are Q's TMEM columns after the last S of the item
                 if (wg) ++rr1; else ++rr0;
                 pre = __all_sync(0xffffffffu, nk && np);
             }
@@ -343,9 +391,16 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
         const uint32_t idesc_pv = instr_desc(bf16, kQRows, kD, 1);
         unsigned gb = 0, wk = 0, rr0 = 0, rr1 = 0;
         bool ok = true;
+        int bh = first_bh, g = first_g, cnt_n = 0;
+        auto peek = [&](bool there) {  // list length of item (bh, g), which is then stepped: read one item ahead
+            if (!there) return;
+            cnt_n = clamp_cnt(P, bh, g);
+            next_item(bh, g);
+        };
+        peek(blockIdx.x < total_work);
         for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), qb = (int)(w % groups);
-            const int n_act = clamp_cnt(P, bh, qb) << P.lg_units;
+            const int n_act = cnt_n << P.lg_units;
+            peek(w + gridDim.x < total_work);
             const int n_iter = max(2, n_act);
             // the epilogue of the previous item has read both O accumulators
             ok = mbar_wait_warp(bar_o_free, (wk & 1) ^ 1, ctl, 36, wk);
@@ -353,68 +408,36 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
             for (int i = 0; i < n_iter && ok; ++i, ++gb) {
                 const int wg = i & 1;
                 const unsigned rr = wg ? rr1 : rr0;
-                const int slot = gb % kVSlots, buf = rr & 1;
+                const int slot = gb % kVSlots;
                 if (!pre) {
                     ok = mbar_wait_warp(bar_v_full(slot), (gb / kVSlots) & 1, ctl, 60, gb);
-                    if (ok) ok = mbar_wait_warp(bar_p_full(wg, buf), (rr >> 1) & 1, ctl, 50 + wg, rr);
+                    if (ok) ok = mbar_wait_warp(bar_p_full(wg), rr & 1, ctl, 50 + wg, gb);
                     if (!ok) break;
                 }
                 bool nv = false, np = false;  // look ahead to the item's next unit
                 if (i + 1 < n_iter) {
-                    const int wg2 = wg ^ 1;
-                    const unsigned rr2 = wg2 ? rr1 : rr0;
                     nv = mbar_test(bar_v_full((gb + 1) % kVSlots), ((gb + 1) / kVSlots) & 1);
-                    np = mbar_test(bar_p_full(wg2, rr2 & 1), (rr2 >> 1) & 1);
+                    np = mbar_test(bar_p_full(wg ^ 1), (wg ? rr0 : rr1) & 1);
                 }
                 tc_fence_after();
                 // A: P in TMEM (first 32 columns of the S buffer), 8 columns per 16-key step.
                 // B: V tile, MN-major: 64-column halves 8 KiB apart (LBO), 8-key groups 1 KiB apart (SBO).
                 if (i < n_act) {
-                    const uint32_t pa = tmem + kTmWg * wg + kTmS + 64u * buf;
+                    const uint32_t pa = tmem + kTmP + 32u * wg;
                     const uint64_t vd = smem_desc(sbase + kOffV + slot * kSlotBytes, kHalfBytes, 1024);
-                    const uint32_t d = tmem + kTmWg * wg + kTmO;
+                    const uint32_t d = tmem + kTmO + 128u * wg;
 #pragma unroll
                     for (int j = 0; j < kBlk / 16; ++j)
                         tc_mma_ts(d, pa + 8u * j, vd + (uint64_t)((j * 2048) >> 4), idesc_pv, (i > 1 || j > 0) ? 1u : 0u);
                 }
                 // the V slots of the item's last two units go to the epilogue, which stages O in them and frees them
                 if (i < n_iter - 2) tc_commit(bar_v_empty(slot));
-                tc_commit(bar_pv_done(wg, buf));
+                tc_commit(bar_pv_done(wg));
+                __syncwarp();
                 if (wg) ++rr1; else ++rr0;
                 pre = __all_sync(0xffffffffu, nv && np);
             }
         }
-      } else {
-        // ================================================================== output store warp
-        // Waits for the staged rows of a work item, sends them off by TMA and hands the two V slots they were staged
-        // in back to the producer, so that the warpgroups do not wait for the store.
-        unsigned gb = 0, wk = 0;
-        bool ok = true;
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), qb = (int)(w % groups);
-            const int b = bh / P.heads, h = bh % P.heads;
-            gb += max(2, clamp_cnt(P, bh, qb) << P.lg_units);
-            const int s0 = (int)((gb - 2) % kVSlots);  // gb is even and so is the ring: slots s0 and s0 + 1
-            ok = mbar_wait_warp(bar_o_staged, wk & 1, ctl, 110, wk);
-            if (ok && lane == 0) {
-                Coord cc = block_coord(P.gq, qb, b, h, P.heads, P.merge_o, P.Tq);
-                const CUtensorMap* tmo = &P.tm_o[0];
-                if (P.o_frames > 0) {  // blocks never straddle ranks: o_frames is a multiple of the block's frames
-                    const int dst = cc.c3 / P.o_frames;
-                    cc.c3 -= dst * P.o_frames;
-                    tmo = &P.tm_o[dst];
-                }
-                const uint32_t src = sbase + kOffV + s0 * kSlotBytes;
-                tma_store_5d(tmo, src, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                tma_store_5d(tmo, src + kQHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
-                tma_store_commit();
-                tma_store_wait_read();
-                mbar_arrive(bar_v_empty(s0));
-                mbar_arrive(bar_v_empty(s0 + 1));
-            }
-            __syncwarp();
-        }
-        if (lane == 0) tma_store_wait_all();
       }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
@@ -423,15 +446,44 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
         const int wq = warp & 3;          // TMEM quadrant of this warp
         const int row = wq * 32 + lane;   // row of the query block = TMEM lane
         const uint32_t t_lane = (uint32_t)(wq * 32) << 16;
-        const uint32_t tm_s = tmem + kTmWg * wg + kTmS + t_lane;
-        const uint32_t tm_o_mine = tmem + kTmWg * wg + kTmO + t_lane, tm_o_other = tmem + kTmWg * (wg ^ 1) + kTmO + t_lane;
+        const uint32_t tm_s = tmem + kTmS + 64u * wg + t_lane, tm_p = tmem + kTmP + 32u * wg + t_lane;
+        const uint32_t tm_o_mine = tmem + kTmO + 128u * wg + t_lane, tm_o_other = tmem + kTmO + 128u * (wg ^ 1) + t_lane;
         const int ml_idx = row;
-        unsigned rr = 0, wk = 0, gb = 0;
+        unsigned wk = 0, gb = 0, rr = 0;  // rr: rounds of this warpgroup over the whole kernel
         bool ok = true;
 
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
-            const int bh = (int)(w / groups), qt = (int)(w % groups);
-            const int n_act = clamp_cnt(P, bh, qt) << P.lg_units;
+        // Q of the CTA's work item number `item` from shared memory to TMEM: a thread moves its row, the warpgroup 64 of the 128 columns.
+        auto q_to_tmem = [&](unsigned item) -> bool {
+            // the last S of the item before has read the columns
+            if (item > 0 && !mbar_wait_warp(bar_qt_free, (item - 1) & 1, ctl, 106 + wg, item)) return false;
+            if (!mbar_wait_warp(bar_q_full, item & 1, ctl, 108 + wg, item)) return false;
+            tc_fence_after();
+            const unsigned char* src = smem + kOffQ + wg * kQHalfBytes + row * 128;
+            uint32_t qr[32];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                const uint4 v = *reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4));
+                qr[4 * c + 0] = v.x;
+                qr[4 * c + 1] = v.y;
+                qr[4 * c + 2] = v.z;
+                qr[4 * c + 3] = v.w;
+            }
+            tc_st32(tmem + kTmQ + 32u * wg + t_lane, qr);
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            mbar_arrive_elect(bar_q_empty);
+            mbar_arrive_elect(bar_qt_full);
+            return true;
+        };
+        if (blockIdx.x < total_work) ok = q_to_tmem(0);
+
+        int bh = first_bh, qt = first_g, nx_bh = first_bh, nx_g = first_g, cnt_n = 0;
+        if (blockIdx.x < total_work) cnt_n = clamp_cnt(P, bh, qt);
+        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, qt = nx_g) {
+            const int n_act = cnt_n << P.lg_units;
+            next_item(nx_bh, nx_g);
+            if (w + gridDim.x < total_work) cnt_n = clamp_cnt(P, nx_bh, nx_g);  // read one item ahead
             const int n_iter = max(2, n_act);
             const int32_t* my_list = P.idx + ((long long)bh * P.nq + qt) * P.cap;
 
@@ -441,18 +493,21 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
             // ragged grids: the block index of a round is fetched a round ahead, so that the global load never sits
             // between S and the softmax (unit i belongs to list entry i >> lg_units)
             int blk_ahead = (kRagged && wg < n_act) ? my_list[0] : 0;
+            // S of the warpgroup's round into registers; the buffer is then free for the S of its next round
+            uint32_t sr[64];
+            if (wg < n_iter) {
+                ok = mbar_wait_warp(bar_s_full(wg), rr & 1, ctl, 80 + wg, rr);
+                if (!ok) break;
+                tc_fence_after();
+                tc_ld64(tm_s, sr);
+                tc_wait_ld();
+                tc_fence_before();
+                mbar_arrive_elect(bar_s_free(wg));
+            }
             for (int i = wg; i < n_iter && ok; i += 2, ++rr) {
                 const bool active = i < n_act;
                 const int blk_now = blk_ahead;
                 if (kRagged && i + 2 < n_act) blk_ahead = my_list[(i + 2) >> P.lg_units];
-                const int buf = rr & 1;
-                const unsigned bph = (rr >> 1) & 1;
-                ok = mbar_wait_warp(bar_s_full(wg, buf), bph, ctl, 80 + wg, rr);
-                if (!ok) break;
-                tc_fence_after();
-                uint32_t sr[64];
-                tc_ld64(tm_s + 64u * buf, sr);
-                tc_wait_ld();
                 float alpha = 1.f;
                 bool need = false;
                 uint4 pk[8];  // this row of P in the input dtype, 8 keys per 16-byte chunk
@@ -477,9 +532,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                             }
                         }
                     }
-                    // One pass: the probabilities are computed against the current reference maximum while
-                    // the row maximum is tracked on the side; only if the maximum has moved by more than 2^8
-                    // (or this is the warpgroup's first block) is the pass repeated with the new reference.
+                    // One pass: the probabilities are computed against the current reference maximum while the row maximum is
+                    // tracked beside them (one basic block, so that the comparisons run under the exponentials); only if the
+                    // maximum has moved by more than 2^8 is the pass repeated with the new reference.  The warpgroup's first
+                    // unit takes its own maximum as the reference.
                     auto probs = [&](float mref, float& rsum) {
                         // two keys per instruction where the machine has packed fp32 forms (fma, add); the four partial
                         // sums take the keys j = 0, 1, 2, 3 (mod 4) in ascending order
@@ -505,89 +561,90 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                         }
                         rsum = (r01.x + r01.y) + (r23.x + r23.y);
                     };
-                    // the reference maximum this row would have after this block (in units of log2)
-                    auto row_reference = [&]() {
+                    // the row maximum of this unit, in units of log2
+                    auto row_max = [&]() {
                         float mx8[8];  // eight chains of eight values, three at a time
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
                             auto sv = [&](int i) { return __uint_as_float(sr[8 * i + k]); };
                             mx8[k] = fmaxf(max3(max3(max3(sv(0), sv(1), sv(2)), sv(3), sv(4)), sv(5), sv(6)), sv(7));
                         }
-                        const float mx = fmaxf(max3(max3(mx8[0], mx8[1], mx8[2]), mx8[3], mx8[4]), max3(mx8[5], mx8[6], mx8[7]));
-                        return first ? mx * P.scale2 : fmaxf(m_ref, mx * P.scale2);  // no reference yet: m_ref is a placeholder
+                        return fmaxf(max3(max3(mx8[0], mx8[1], mx8[2]), mx8[3], mx8[4]), max3(mx8[5], mx8[6], mx8[7])) * P.scale2;
                     };
                     float rs = 0.f;
                     float m_new = m_ref;
-                    if (kRagged) {
-                        // the instantiation with the masking code: a single copy of the pass in the instruction stream.
-                        // The loop body runs once in the common case (pass, then the row maximum, which confirms the
-                        // reference) and twice when the reference moves; for the warpgroup's first block the first
-                        // pass is skipped.
-                        bool run_pass = !first, decided = false;
-#pragma unroll 1
-                        for (int turn = 0; turn < 2; ++turn) {
-                            if (run_pass) probs(m_ref, rs);
-                            if (decided) break;
-                            m_new = row_reference();
-                            run_pass = first || m_new - m_ref > 8.f;
-                            if (!run_pass) break;
-                            if (!first) {
-                                need = true;
-                                alpha = ex2(m_ref - m_new);
-                            }
-                            m_ref = (m_new == -INFINITY) ? 0.f : m_new;
-                            decided = true;
-                        }
-                    } else {
-                        // whole grids: straight-line code, the second copy of the pass off the common path
-                        if (!first) probs(m_ref, rs);
-                        m_new = row_reference();
-                        if (LCBSA_UNLIKELY(first || m_new - m_ref > 8.f)) {
-                            if (!first) {
-                                need = true;
-                                alpha = ex2(m_ref - m_new);
-                            }
-                            m_ref = (m_new == -INFINITY) ? 0.f : m_new;
-                            probs(m_ref, rs);
-                        }
+                    if (LCBSA_UNLIKELY(first)) {
+                        m_new = row_max();
+                        m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+                    }
+                    first = first && m_new == -INFINITY;  // a unit wholly outside a ragged grid leaves no reference behind
+                    probs(m_ref, rs);
+                    const float m_top = row_max();
+                    if (LCBSA_UNLIKELY(m_top - m_ref > 8.f)) {
+                        need = true;
+                        alpha = ex2(m_ref - m_top);
+                        m_ref = m_top;
+                        probs(m_ref, rs);
                     }
                     l_sum = l_sum * alpha + rs;  // alpha is 1 unless this row's reference maximum moved
-                    // a unit that lies wholly outside a ragged grid leaves no reference behind: the next one is the first
-                    first = first && m_new == -INFINITY;
                 } else {
                     first = false;
                 }
                 const bool any_need = __any_sync(0xffffffffu, need);
-                // O is rescaled only at rest: the warpgroup's PV of the round before has to be finished
-                // (need implies that this is not the warpgroup's first round of the item, so rr > 0)
-                if (LCBSA_UNLIKELY(any_need)) {
-                    ok = mbar_wait_warp(bar_pv_done(wg, buf ^ 1), ((rr - 1) >> 1) & 1, ctl, 92 + wg, rr);
+                // P may be overwritten, and O rescaled, once the warpgroup's PV of the round before has finished.  The next S
+                // only waits for this one to be in registers, so it is usually there too: both barriers are probed at once
+                // (a wait costs its warp 200 cycles even on a completed phase) and the next S is fetched under the store of P.
+                const bool more = i + 2 < n_iter;
+                const bool pv_ok = mbar_test(bar_pv_done(wg), (rr & 1) ^ 1), s_ok = !more || mbar_test(bar_s_full(wg), (rr + 1) & 1);
+                const bool ready = __all_sync(0xffffffffu, pv_ok && s_ok);
+                if (!ready) {
+                    ok = mbar_wait_warp(bar_pv_done(wg), (rr & 1) ^ 1, ctl, 92 + wg, rr);
                     if (!ok) break;
                 }
-                {   // P overwrites the first half of the S buffer just read (don't-cares for a unit that does not exist)
-                    uint32_t pr[32];
+                uint32_t pr[32];  // all 32 lanes take part in the store (don't-cares for a unit that does not exist)
 #pragma unroll
-                    for (int cch = 0; cch < 8; ++cch) {
-                        pr[4 * cch + 0] = pk[cch].x;
-                        pr[4 * cch + 1] = pk[cch].y;
-                        pr[4 * cch + 2] = pk[cch].z;
-                        pr[4 * cch + 3] = pk[cch].w;
-                    }
-                    tc_st32(tm_s + 64u * buf, pr);
+                for (int cch = 0; cch < 8; ++cch) {
+                    pr[4 * cch + 0] = pk[cch].x;
+                    pr[4 * cch + 1] = pk[cch].y;
+                    pr[4 * cch + 2] = pk[cch].z;
+                    pr[4 * cch + 3] = pk[cch].w;
                 }
                 if (LCBSA_UNLIKELY(any_need)) tc_scale_row128(tm_o_mine, alpha);  // rare: only when a row maximum jumps
-                tc_wait_st();
-                tc_fence_before();
-                mbar_arrive_elect(bar_p_full(wg, buf));
+                if (ready && more) {
+                    tc_fence_after();
+                    tc_st32(tm_p, pr);
+                    tc_ld64(tm_s, sr);
+                    tc_wait_st();
+                    tc_fence_before();
+                    mbar_arrive_elect(bar_p_full(wg));
+                    tc_wait_ld();
+                    tc_fence_before();
+                    mbar_arrive_elect(bar_s_free(wg));
+                } else {
+                    tc_st32(tm_p, pr);
+                    tc_wait_st();
+                    tc_fence_before();
+                    mbar_arrive_elect(bar_p_full(wg));
+                    if (more) {
+                        ok = mbar_wait_warp(bar_s_full(wg), (rr + 1) & 1, ctl, 80 + wg, rr);
+                        if (!ok) break;
+                        tc_fence_after();
+                        tc_ld64(tm_s, sr);
+                        tc_wait_ld();
+                        tc_fence_before();
+                        mbar_arrive_elect(bar_s_free(wg));
+                    }
+                }
             }
             if (!ok) break;
             gb += n_iter;
+            // Q of the next item, so that its S runs under this item's epilogue
+            if (w + gridDim.x < total_work && !q_to_tmem(wk + 1)) break;
 
             // ---- epilogue of this work item.  The warpgroup's PVs are finished once its last one is; it then
             // publishes (maximum, row sum) of its rows and waits for the other warpgroup to do the same.
             {   // n_iter is even and at least 2: every warpgroup has had a round
-                const unsigned lr = rr - 1;
-                ok = mbar_wait_warp(bar_pv_done(wg, lr & 1), (lr >> 1) & 1, ctl, 100 + wg, lr);
+                ok = mbar_wait_warp(bar_pv_done(wg), (rr - 1) & 1, ctl, 100 + wg, rr);
                 if (!ok) break;
             }
             // the other warpgroup has read this warpgroup's entry of the previous item before it arrived on o_free
@@ -613,31 +670,37 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
             // half-tile row per thread) in the V slot that its own last PV has just released: the last two units of
             // the item sit in slots s0 (warpgroup 0) and s0 + 1 (warpgroup 1), s0 even.
             unsigned char* o_half = smem + kOffV + ((gb - 2) % kVSlots + wg) * kSlotBytes;
+            // a warpgroup that saw no block has weight 0; its accumulator holds garbage and is not used
+            const bool rd_mine = __any_sync(0xffffffffu, w_mine > 0.f), rd_oth = __any_sync(0xffffffffu, w_oth > 0.f);
+            const bool both = __all_sync(0xffffffffu, w_mine > 0.f && w_oth > 0.f);  // the usual case: no lane has to be masked
+            const float2 fm2 = make_float2(f_mine, f_mine), fo2 = make_float2(f_oth, f_oth);
 #pragma unroll
             for (int cch = 0; cch < 2; ++cch) {
                 uint32_t oa[32], ob[32];
-                // a warpgroup that saw no block has weight 0; its accumulator holds garbage and is not used
-                const bool rd_mine = __any_sync(0xffffffffu, w_mine > 0.f), rd_oth = __any_sync(0xffffffffu, w_oth > 0.f);
                 if (rd_mine) tc_ld32(tm_o_mine + 64 * wg + 32 * cch, oa);
                 if (rd_oth) tc_ld32(tm_o_other + 64 * wg + 32 * cch, ob);
                 tc_wait_ld();
+                if (LCBSA_UNLIKELY(!both)) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        if (!(w_mine > 0.f)) oa[j] = 0u;
+                        if (!(w_oth > 0.f)) ob[j] = 0u;
+                    }
+                }
                 {
 #pragma unroll
                     for (int q8 = 0; q8 < 4; ++q8) {
-                        float v[8];
+                        uint32_t pw[4];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const float a = w_mine > 0.f ? __uint_as_float(oa[q8 * 8 + j]) * f_mine : 0.f;
-                            const float bb = w_oth > 0.f ? __uint_as_float(ob[q8 * 8 + j]) * f_oth : 0.f;
-                            v[j] = a + bb;
+                        for (int j = 0; j < 4; ++j) {
+                            const int e = q8 * 8 + 2 * j;
+                            const float2 a2 = __fmul2_rn(make_float2(__uint_as_float(oa[e]), __uint_as_float(oa[e + 1])), fm2);
+                            const float2 b2 = __fmul2_rn(make_float2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), fo2);
+                            const float2 v2 = __fadd2_rn(a2, b2);
+                            pw[j] = pack2(bf16, v2.x, v2.y);
                         }
-                        uint4 pk;
-                        pk.x = pack2(bf16, v[0], v[1]);
-                        pk.y = pack2(bf16, v[2], v[3]);
-                        pk.z = pack2(bf16, v[4], v[5]);
-                        pk.w = pack2(bf16, v[6], v[7]);
                         const int chunk = cch * 4 + q8;
-                        *reinterpret_cast<uint4*>(o_half + row * 128 + ((chunk ^ (row & 7)) << 4)) = pk;
+                        *reinterpret_cast<uint4*>(o_half + row * 128 + ((chunk ^ (row & 7)) << 4)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
                     }
                 }
             }
