@@ -126,8 +126,16 @@ __global__ void __launch_bounds__(kThreads) score_topk_kernel(const T* __restric
     for (int i = 0; i < QPW; ++i) {
         const int qrow = q0 + warp * QPW + i;
         if (qrow >= Nq) break;
-        select_row<Key>(keys + (long long)(warp * QPW + i) * nk_pad, Nk, nk_pad, nsel, cap, idx + ((long long)bh * Nq + qrow) * cap,
-                        cnt + (long long)bh * Nq + qrow, lane);
+        const Key* row = keys + (long long)(warp * QPW + i) * nk_pad;
+        int32_t* out = idx + ((long long)bh * Nq + qrow) * cap;
+        int32_t* n_out = cnt + (long long)bh * Nq + qrow;
+        if constexpr (sizeof(Key) == 2) {
+            if (nk_pad <= 64 * kRegWords) {
+                select_row_regs<kRegWords>(row, nk_pad, nsel, cap, out, n_out, lane);
+                continue;
+            }
+        }
+        select_row<Key>(row, Nk, nk_pad, nsel, cap, out, n_out, lane);
     }
 }
 

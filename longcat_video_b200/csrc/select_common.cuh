@@ -6,7 +6,7 @@
 namespace lcbsa {
 namespace sel {
 
-constexpr int kRegWords = 24;  // 32-bit words of a 16-bit key row that a lane may keep in registers (rows up to 1536 keys)
+constexpr int kRegWords = 24;  // 32-bit words of a 16-bit key row that a lane may keep in registers (select_row_regs: rows up to 1536 keys)
 
 template <typename T> struct KeyOf { using type = uint16_t; };
 template <> struct KeyOf<float> { using type = uint32_t; };
@@ -31,11 +31,7 @@ __device__ __forceinline__ uint32_t make_key(float v) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-__device__ __forceinline__ int warp_sum(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
+__device__ __forceinline__ int warp_sum(int v) { return __reduce_add_sync(0xffffffffu, v); }
 
 // Number of keys of a row that are >= cand (gt == false) or > cand (gt == true).
 __device__ __forceinline__ int count_row(const uint16_t* row, int nk_pad, uint32_t cand, bool gt, int lane) {
@@ -66,63 +62,100 @@ struct KeyMask {
     __device__ __forceinline__ bool operator()(int j) const { return period == 0 || ((j / hw) % period) < split; }
 };
 
-// The nsel largest keys of one row (ties at the threshold broken towards the lower block index), emitted as
-// ascending block indices by one warp; the cap - nsel trailing entries are set to -1.  `row` may be shared or
-// global memory; nk_pad (a multiple of 64) entries are readable and those past Nk hold key 0.
+// The nsel largest keys of one row of 16-bit keys (ties at the threshold broken towards the lower block index), emitted as
+// ascending block indices by one warp; the cap - nsel trailing entries are set to -1.  nk_pad (a multiple of 64, at most
+// 64 * NW) entries are readable and those past Nk hold key 0, which no block that may be selected has.
+//
+// Issue bound: the row is read once (2 bytes per key) and then counted up to 16 times.  Every lane keeps its share of the
+// row in registers (word i: keys 2 (lane + 32 i) and the one behind it), the low key of a word shifted up in a register of
+// its own, so that a count is a compare and an add per key; NW follows the row (a fixed 24 words spent 60 % of the work of a 624-key row on padding); the
+// bisection ends as soon as a candidate is reached by exactly nsel keys; and the indices are emitted from the registers.
+// Before, with 24 words for every row, five shuffles per count, all 17 counts and a second read of the row: 19 968 rows of
+// 624 keys 76 us, now 33 us; 46 080 rows of 1440 keys 199 us, now 185 us (there 23 of the 24 words were needed all along).
+template <int NW>
+__device__ __forceinline__ void select_row_regs(const uint16_t* row, int nk_pad, int nsel, int cap, int32_t* out, int32_t* cnt_out, int lane,
+                                                const KeyMask mask = KeyMask{1, 0, 0}) {
+    if (lane == 0) *cnt_out = nsel;
+    if (nsel > 0) {
+        const uint32_t* r32 = reinterpret_cast<const uint32_t*>(row);
+        const int nwords = nk_pad / 2;
+        uint32_t hi[NW], lo[NW];  // hi: the word itself (its upper key decides a comparison with c << 16), lo: the lower key << 16
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            uint32_t w = (lane + 32 * i < nwords) ? r32[lane + 32 * i] : 0u;  // key 0 is never counted
+            if (mask.period != 0) {  // keys of blocks this row may not select become key 0
+                const int j = 2 * (lane + 32 * i);
+                if (!mask(j)) w &= 0xffff0000u;
+                if (!mask(j + 1)) w &= 0x0000ffffu;
+            }
+            hi[i] = w;
+            lo[i] = w << 16;
+        }
+        auto count = [&](uint32_t c) {  // keys >= c, 1 <= c <= 0xffff
+            int n = 0;
+            const uint32_t cc = c << 16;
+#pragma unroll
+            for (int i = 0; i < NW; ++i) n += (int)(hi[i] >= cc) + (int)(lo[i] >= cc);
+            return warp_sum(n);
+        };
+        uint32_t thr = 0;
+        bool exact = false;  // exactly nsel keys reach the threshold
+#pragma unroll 1
+        for (int bit = 15; bit >= 0; --bit) {
+            const uint32_t cand = thr | (1u << bit);
+            const int n = count(cand);
+            if (n >= nsel) thr = cand;
+            if (n == nsel) {
+                exact = true;
+                break;
+            }
+        }
+        // otherwise thr is the nsel-th largest key and more than nsel keys reach it
+        const int take_eq = exact ? 0 : nsel - (thr < 0xffffu ? count(thr + 1u) : 0);  // ties to keep, lowest block index first
+        const uint32_t tt = thr << 16;
+        const unsigned lt_mask = (1u << lane) - 1u;
+        int n_out = 0, n_eq = 0;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) {
+            if (64 * i >= nk_pad) break;
+            bool t0 = lo[i] >= tt, t1 = hi[i] >= tt;
+            if (!exact) {
+                const bool e0 = lo[i] == tt, e1 = (hi[i] & 0xffff0000u) == tt;
+                const unsigned m0 = __ballot_sync(0xffffffffu, e0), m1 = __ballot_sync(0xffffffffu, e1);
+                const int before = n_eq + __popc(m0 & lt_mask) + __popc(m1 & lt_mask);
+                if (e0) t0 = before < take_eq;
+                if (e1) t1 = before + (int)e0 < take_eq;
+                n_eq += __popc(m0) + __popc(m1);
+            }
+            const unsigned s0 = __ballot_sync(0xffffffffu, t0), s1 = __ballot_sync(0xffffffffu, t1);
+            const int at = n_out + __popc(s0 & lt_mask) + __popc(s1 & lt_mask);
+            if (t0) out[at] = 2 * (lane + 32 * i);
+            if (t1) out[at + (int)t0] = 2 * (lane + 32 * i) + 1;
+            n_out += __popc(s0) + __popc(s1);
+        }
+    }
+    for (int j = nsel + lane; j < cap; j += 32) out[j] = -1;
+}
+
+// The same for a row of any length and either key type, counted where it lies: `row` may be shared or global memory.
 template <typename Key>
 __device__ __forceinline__ void select_row(const Key* row, int Nk, int nk_pad, int nsel, int cap, int32_t* out, int32_t* cnt_out,
-                                           int lane, const KeyMask mask = KeyMask{1, 0, 0}) {
+                                           int lane) {
     constexpr int kKeyBits = sizeof(Key) * 8;
     if (lane == 0) *cnt_out = nsel;
     if (nsel > 0) {
         uint32_t thr = 0;
-        int above;
-        if (sizeof(Key) == 2 && nk_pad <= 2 * 32 * kRegWords) {
-            // 16-bit keys of a row that fits: every lane keeps its share of the row (two keys per word) in registers,
-            // so the 17 counting passes of the bisection read the row once
-            const uint32_t* r32 = reinterpret_cast<const uint32_t*>(row);
-            const int nwords = nk_pad / 2;
-            uint32_t w[kRegWords];
-#pragma unroll
-            for (int i = 0; i < kRegWords; ++i) w[i] = (lane + 32 * i < nwords) ? r32[lane + 32 * i] : 0u;  // key 0 is never counted
-            if (mask.period != 0) {  // keys of blocks this row may not select become key 0
-#pragma unroll
-                for (int i = 0; i < kRegWords; ++i) {
-                    const int j = 2 * (lane + 32 * i);
-                    if (!mask(j)) w[i] &= 0xffff0000u;
-                    if (!mask(j + 1)) w[i] &= 0x0000ffffu;
-                }
-            }
-            auto count = [&](uint32_t c) {  // keys >= c, c >= 1
-                int n = 0;
-#pragma unroll
-                for (int i = 0; i < kRegWords; ++i) n += ((w[i] & 0xffffu) >= c) + ((w[i] >> 16) >= c);
-                return warp_sum(n);
-            };
-            for (int bit = kKeyBits - 1; bit >= 0; --bit) {
-                const uint32_t cand = thr | (1u << bit);
-                if (count(cand) >= nsel) thr = cand;
-            }
-            above = count(thr + 1u);
-        } else if (mask.period != 0) {
-            // a masked row is only handled where it fits in registers (the host checks this before the launch):
-            // select nothing rather than something wrong
-            if (lane == 0) *cnt_out = 0;
-            for (int j = lane; j < cap; j += 32) out[j] = -1;
-            return;
-        } else {
-            for (int bit = kKeyBits - 1; bit >= 0; --bit) {
-                const uint32_t cand = thr | (1u << bit);
-                if (count_row(row, nk_pad, cand, false, lane) >= nsel) thr = cand;
-            }
-            above = count_row(row, nk_pad, thr, true, lane);
+        for (int bit = kKeyBits - 1; bit >= 0; --bit) {
+            const uint32_t cand = thr | (1u << bit);
+            if (count_row(row, nk_pad, cand, false, lane) >= nsel) thr = cand;
         }
+        const int above = count_row(row, nk_pad, thr, true, lane);
         const int take_eq = nsel - above;  // ties at the threshold to keep, lowest block index first
         int n_out = 0, n_eq = 0;
         const unsigned lt_mask = (1u << lane) - 1u;
         for (int j0 = 0; j0 < Nk; j0 += 32) {
             const int j = j0 + lane;
-            const bool ok = (j < Nk) && mask(j);
+            const bool ok = j < Nk;
             const uint32_t key = ok ? (uint32_t)row[j] : 0u;
             const bool gt = key > thr;
             const bool eq = (key == thr) && ok;
