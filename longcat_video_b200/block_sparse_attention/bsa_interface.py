@@ -32,16 +32,12 @@ def _prod(x: Sequence[int]) -> int:
 
 
 def num_blocks(latent_shape: Sequence[int], chunk: Sequence[int]) -> int:
-    g = L.grid_desc(latent_shape, chunk)
-    n = L.lib().lcbsa_num_blocks(ctypes.byref(g))
-    if n < 0:
-        L.check(n)
-    return n
+    return L.grid_plan(latent_shape, chunk)[1]
 
 
 def num_selected(sparsity: float, n_k_blocks: int) -> int:
     """``int((1 - sparsity) * Nk)`` -- bsa_interface.py:214, evaluated in double precision."""
-    return int(L.lib().lcbsa_num_selected(float(sparsity), int(n_k_blocks)))
+    return int((1.0 - float(sparsity)) * int(n_k_blocks))
 
 
 def _as_abi(t: torch.Tensor) -> torch.Tensor:
@@ -55,7 +51,7 @@ def mean_pooling_compression_3d(x: torch.Tensor, latent_shape, chunk_3d_shape) -
     nb = num_blocks(latent_shape, chunk_3d_shape)
     out = torch.empty(B, H, nb, D, dtype=x.dtype, device=x.device)
     xd, g = L.tensor_desc(x), L.grid_desc(latent_shape, chunk_3d_shape)
-    with torch.cuda.device(x.device):
+    with L.on_device(x.device):
         L.check(L.lib().lcbsa_pool(ctypes.byref(xd), ctypes.byref(g), ctypes.c_void_p(out.data_ptr()),
                                    L.current_stream(x.device)))
     return out
@@ -80,7 +76,7 @@ def get_select_indices_from_pooled(q_cmp: torch.Tensor, k_cmp: torch.Tensor, spa
     dt = L.dtype_code(q_cmp.dtype)
     keys_bytes = L.lib().lcbsa_score_keys_bytes(dt, B * H, Nq, Nk, D)  # 0: only the fused kernel applies
     ws = torch.empty(max(keys_bytes, 16), dtype=torch.uint8, device=q_cmp.device)
-    with torch.cuda.device(q_cmp.device):
+    with L.on_device(q_cmp.device):
         L.check(L.lib().lcbsa_score_topk_ws(q_cmp.data_ptr(), k_cmp.data_ptr(), dt, B * H, Nq, Nk, D, nsel, cap,
                                             idx.data_ptr(), cnt.data_ptr(), ws.data_ptr(), keys_bytes,
                                             L.current_stream(q_cmp.device)))
@@ -104,7 +100,7 @@ def get_select_indices_from_pooled_split(q_cmp: torch.Tensor, k_cmp: torch.Tenso
     keys_bytes = L.lib().lcbsa_score_keys_bytes(dt, B * H, Nq, Nk, D)
     ws = torch.empty(max(keys_bytes, 16), dtype=torch.uint8, device=q_cmp.device)
     sp = L.LcbsaSplit(hw_q, period_q, split_q, hw_k, period_k, split_k, nsel_first)
-    with torch.cuda.device(q_cmp.device):
+    with L.on_device(q_cmp.device):
         L.check(L.lib().lcbsa_score_topk_split(q_cmp.data_ptr(), k_cmp.data_ptr(), dt, B * H, Nq, Nk, D, ctypes.byref(sp), nsel, cap,
                                                idx.data_ptr(), cnt.data_ptr(), ws.data_ptr(), keys_bytes, L.current_stream(q_cmp.device)))
     return idx, cnt
@@ -116,8 +112,7 @@ def get_select_indices_split(q, k, latent_shape_q, latent_shape_k, sparsity, chu
     splits in frame blocks."""
     q, k = _as_abi(q), _as_abi(k)
     B, H, _, D = q.shape
-    gq, gk = L.grid_desc(latent_shape_q, chunk_3d_shape_q), L.grid_desc(latent_shape_k, chunk_3d_shape_k)
-    nq, nk = num_blocks(latent_shape_q, chunk_3d_shape_q), num_blocks(latent_shape_k, chunk_3d_shape_k)
+    (gq, nq), (gk, nk) = L.grid_plan(latent_shape_q, chunk_3d_shape_q), L.grid_plan(latent_shape_k, chunk_3d_shape_k)
     hw_k = nk // (-(-int(latent_shape_k[0]) // int(chunk_3d_shape_k[0])))
     nk_first = nk // hw_k // period_tk * split_tk * hw_k
     nsel, nsel_first = num_selected(sparsity, nk), num_selected(sparsity, nk_first)
@@ -127,7 +122,7 @@ def get_select_indices_split(q, k, latent_shape_q, latent_shape_k, sparsity, chu
     ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=q.device)
     idx = torch.empty(B, H, nq, cap, dtype=torch.int32, device=q.device)
     cnt = torch.empty(B, H, nq, dtype=torch.int32, device=q.device)
-    with torch.cuda.device(q.device):
+    with L.on_device(q.device):
         L.check(L.lib().lcbsa_block_select_split(ctypes.byref(qd), ctypes.byref(kd), ctypes.byref(gq), ctypes.byref(gk), int(period_tq),
                                                  int(split_tq), int(period_tk), int(split_tk), nsel_first, nsel, cap, idx.data_ptr(),
                                                  cnt.data_ptr(), ws.data_ptr(), ws_bytes, L.current_stream(q.device)))
@@ -144,7 +139,7 @@ def _select_cdf(q_cmp: torch.Tensor, k_cmp: torch.Tensor, cdf_threshold: float, 
     cnt = torch.empty(B, H, Nq, dtype=torch.int32, device=q_cmp.device)
     keys_bytes = L.lib().lcbsa_score_keys_bytes(dt, B * H, Nq, Nk, D)
     ws = torch.empty(max(keys_bytes, 16), dtype=torch.uint8, device=q_cmp.device)
-    with torch.cuda.device(q_cmp.device):
+    with L.on_device(q_cmp.device):
         L.check(L.lib().lcbsa_score_cdf(q_cmp.data_ptr(), k_cmp.data_ptr(), dt, B * H, Nq, Nk, D, ctypes.c_float(1 / D ** 0.5),
                                         ctypes.c_float(cdf_threshold), int(nsel_min), idx.data_ptr(), cnt.data_ptr(),
                                         ws.data_ptr(), keys_bytes, L.current_stream(q_cmp.device)))
@@ -162,8 +157,7 @@ def get_select_indices(q: torch.Tensor, k: torch.Tensor, latent_shape_q, latent_
                                               mean_pooling_compression_3d(k, latent_shape_k, chunk_3d_shape_k), sparsity, cdf_threshold)
     q, k = _as_abi(q), _as_abi(k)
     B, H, _, D = q.shape
-    gq, gk = L.grid_desc(latent_shape_q, chunk_3d_shape_q), L.grid_desc(latent_shape_k, chunk_3d_shape_k)
-    nq, nk = num_blocks(latent_shape_q, chunk_3d_shape_q), num_blocks(latent_shape_k, chunk_3d_shape_k)
+    (gq, nq), (gk, nk) = L.grid_plan(latent_shape_q, chunk_3d_shape_q), L.grid_plan(latent_shape_k, chunk_3d_shape_k)
     nsel = num_selected(sparsity, nk)
     cap = max(nsel, 1)
     qd, kd = L.tensor_desc(q), L.tensor_desc(k)
@@ -171,7 +165,7 @@ def get_select_indices(q: torch.Tensor, k: torch.Tensor, latent_shape_q, latent_
     ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=q.device)
     idx = torch.empty(B, H, nq, cap, dtype=torch.int32, device=q.device)
     cnt = torch.empty(B, H, nq, dtype=torch.int32, device=q.device)
-    with torch.cuda.device(q.device):
+    with L.on_device(q.device):
         L.check(L.lib().lcbsa_block_select(ctypes.byref(qd), ctypes.byref(kd), ctypes.byref(gq), ctypes.byref(gk), nsel, cap,
                                            idx.data_ptr(), cnt.data_ptr(), ws.data_ptr(), ws_bytes,
                                            L.current_stream(q.device)))
@@ -191,9 +185,9 @@ def attn_fwd_bsa_varlen(q, k, v, sm_scale, block_indices, block_indices_lens, la
     lse = torch.empty(B, H, Sq, dtype=torch.float32, device=q.device) if return_lse else None
     idx = block_indices.to(torch.int32).contiguous()
     cnt = block_indices_lens.to(torch.int32).contiguous()
-    gq, gk = L.grid_desc(latent_shape_q, chunk_3d_shape_q), L.grid_desc(latent_shape_k, chunk_3d_shape_k)
+    gq, gk = L.grid_plan(latent_shape_q, chunk_3d_shape_q)[0], L.grid_plan(latent_shape_k, chunk_3d_shape_k)[0]
     qd, kd, vd, od = L.tensor_desc(q), L.tensor_desc(k), L.tensor_desc(v), L.tensor_desc(out)
-    with torch.cuda.device(q.device):
+    with L.on_device(q.device):
         L.check(L.lib().lcbsa_attn_fwd(ctypes.byref(qd), ctypes.byref(kd), ctypes.byref(vd), ctypes.byref(gq), ctypes.byref(gk),
                                        idx.data_ptr(), cnt.data_ptr(), idx.shape[-1], float(sm_scale), ctypes.byref(od),
                                        lse.data_ptr() if lse is not None else None, int(impl),
@@ -211,9 +205,9 @@ def attn_bwd_bsa_varlen(do, q, k, v, o, lse, sm_scale, block_indices, block_indi
     idx = block_indices.to(torch.int32).contiguous()
     cnt = block_indices_lens.to(torch.int32).contiguous()
     lse = lse.to(torch.float32).contiguous()
-    gq, gk = L.grid_desc(latent_shape_q, chunk_3d_shape_q), L.grid_desc(latent_shape_k, chunk_3d_shape_k)
+    gq, gk = L.grid_plan(latent_shape_q, chunk_3d_shape_q)[0], L.grid_plan(latent_shape_k, chunk_3d_shape_k)[0]
     d = {n: L.tensor_desc(t) for n, t in dict(q=q, k=k, v=v, o=o, do=do, dq=dq, dk=dk, dv=dv).items()}
-    with torch.cuda.device(q.device):
+    with L.on_device(q.device):
         need = L.lib().lcbsa_attn_bwd_workspace_bytes(ctypes.byref(d["q"]), ctypes.byref(gq), ctypes.byref(gk), idx.shape[-1])
         ws = torch.empty(max(need, 256), dtype=torch.uint8, device=q.device)
         L.check(L.lib().lcbsa_attn_bwd(ctypes.byref(d["q"]), ctypes.byref(d["k"]), ctypes.byref(d["v"]), ctypes.byref(d["o"]),
