@@ -75,19 +75,22 @@ __device__ __forceinline__ void count_row_cdf(const uint32_t* row, int Nk, float
     if (lane == 0) *cnt = max(min(n, Nk), nsel_min);
 }
 
-// Rows of up to 2048 entries: thread t keeps entries 8 t .. 8 t + 7 in registers from the load to the sorted row.
-// Of the 66 compare-exchange stages of the 2048-wide bitonic network, the 30 with a distance below 8 stay inside a
-// thread, the 30 with a distance of 8 .. 128 entries go through warp shuffles, and only the 6 with a distance of
-// 256 .. 1024 entries cross warps through shared memory.
+// Rows of up to 8 kT = 512, 1024 or 2048 entries: thread t of kT keeps entries 8 t .. 8 t + 7 in registers from the load to
+// the sorted row.  Of the 66 compare-exchange stages of the 2048-wide bitonic network, the 30 with a distance below 8 stay
+// inside a thread, the 30 with a distance of 8 .. 128 entries go through warp shuffles, and only the 6 with a distance of
+// 256 .. 1024 entries cross warps through shared memory.  The kernel is bound by the issue of those stages, so a row takes
+// the narrowest network that holds it: 1024 entries are 55 stages on half the threads (4992 rows of 624 entries: 43 us,
+// 100 us on the 2048-wide network).  The denominator is the same at every width: the warps that are missing would add zeros.
 constexpr int kFastE = 8;
 constexpr int kFastP = kFastE * kCdfThreads;
 
-template <typename T>
-__global__ void __launch_bounds__(kCdfThreads) cdf_rows_fast_kernel(const uint16_t* __restrict__ keys, int Nk, int nk_pad, float sm_scale,
+template <typename T, int kT>
+__global__ void __launch_bounds__(kT) cdf_rows_fast_kernel(const uint16_t* __restrict__ keys, int Nk, int nk_pad, float sm_scale,
                                                                    float threshold, int nsel_min, int32_t* __restrict__ idx,
                                                                    int32_t* __restrict__ cnt) {
-    __shared__ __align__(16) uint32_t row[kFastP];
-    __shared__ float red[kCdfThreads / 32];
+    constexpr int kP = kFastE * kT;
+    __shared__ __align__(16) uint32_t row[kP];
+    __shared__ float red[kT / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long r = blockIdx.x;
     const int base = tid * kFastE;
@@ -112,7 +115,7 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_rows_fast_kernel(const uint16
     __syncthreads();
     m = red[0];
 #pragma unroll
-    for (int w = 1; w < kCdfThreads / 32; ++w) m = fmaxf(m, red[w]);
+    for (int w = 1; w < kT / 32; ++w) m = fmaxf(m, red[w]);
     __syncthreads();
 
     // e = exp(x - m) and the denominator
@@ -128,16 +131,16 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_rows_fast_kernel(const uint16
     for (int o = 16; o > 0; o >>= 1) part = __fadd_rn(part, __shfl_xor_sync(0xffffffffu, part, o));
     if (lane == 0) red[warp] = part;
     __syncthreads();
-    float grp[kCdfThreads / 32];
+    float grp[kT / 32];
 #pragma unroll
-    for (int w = 0; w < kCdfThreads / 32; ++w) grp[w] = red[w];
+    for (int w = 0; w < kT / 32; ++w) grp[w] = red[w];
 #pragma unroll
-    for (int o = kCdfThreads / 64; o > 0; o >>= 1) {
-        float nxt[kCdfThreads / 32];
+    for (int o = kT / 64; o > 0; o >>= 1) {
+        float nxt[kT / 32];
 #pragma unroll
-        for (int w = 0; w < kCdfThreads / 32; ++w) nxt[w] = __fadd_rn(grp[w], grp[w ^ o]);
+        for (int w = 0; w < kT / 32; ++w) nxt[w] = __fadd_rn(grp[w], grp[w ^ o]);
 #pragma unroll
-        for (int w = 0; w < kCdfThreads / 32; ++w) grp[w] = nxt[w];
+        for (int w = 0; w < kT / 32; ++w) grp[w] = nxt[w];
     }
     const float sum = grp[0];
 
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_rows_fast_kernel(const uint16
 
     // bitonic network, descending: entry i and entry i ^ j; the lower index keeps the larger key where (i & k) == 0
 #pragma unroll
-    for (int k = 2; k <= kFastP; k <<= 1) {
+    for (int k = 2; k <= kP; k <<= 1) {
 #pragma unroll
         for (int j = k >> 1; j > 0; j >>= 1) {
             if (j < kFastE) {
@@ -196,7 +199,7 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_rows_fast_kernel(const uint16
     }
     __syncthreads();
     int32_t* out = idx + r * Nk;
-    for (int j = tid; j < Nk; j += kCdfThreads) out[j] = (int32_t)(0xffffu - (row[j] & 0xffffu));
+    for (int j = tid; j < Nk; j += kT) out[j] = (int32_t)(0xffffu - (row[j] & 0xffffu));
     if (warp == 0) count_row_cdf<T>(row, Nk, threshold, nsel_min, cnt + r, lane);
 }
 
@@ -289,6 +292,18 @@ __global__ void __launch_bounds__(kCdfThreads) cdf_rows_kernel(const uint16_t* _
     if (warp == 0) count_row_cdf<T>(row, Nk, threshold, nsel_min, cnt + r, lane);
 }
 
+template <typename T>
+cudaError_t launch_fast(const uint16_t* keys, long long rows, int Nk, int nk_pad, float sm_scale, float threshold, int nsel_min, int32_t* idx,
+                        int32_t* cnt, cudaStream_t st) {
+    if (Nk <= kFastP / 4)
+        cdf_rows_fast_kernel<T, kCdfThreads / 4><<<(unsigned)rows, kCdfThreads / 4, 0, st>>>(keys, Nk, nk_pad, sm_scale, threshold, nsel_min, idx, cnt);
+    else if (Nk <= kFastP / 2)
+        cdf_rows_fast_kernel<T, kCdfThreads / 2><<<(unsigned)rows, kCdfThreads / 2, 0, st>>>(keys, Nk, nk_pad, sm_scale, threshold, nsel_min, idx, cnt);
+    else
+        cdf_rows_fast_kernel<T, kCdfThreads><<<(unsigned)rows, kCdfThreads, 0, st>>>(keys, Nk, nk_pad, sm_scale, threshold, nsel_min, idx, cnt);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_cdf_rows(int dtype, const void* keys, long long rows, int Nk, float sm_scale, float threshold, int nsel_min,
@@ -305,11 +320,8 @@ cudaError_t launch_cdf_rows(int dtype, const void* keys, long long rows, int Nk,
     const int nk_pad = (Nk + 63) / 64 * 64;
     const uint16_t* kp0 = static_cast<const uint16_t*>(keys);
     if (Nk <= kFastP) {
-        if (dtype == LCBSA_BF16)
-            cdf_rows_fast_kernel<__nv_bfloat16><<<(unsigned)rows, kCdfThreads, 0, st>>>(kp0, Nk, nk_pad, sm_scale, threshold, nsel_min, idx, cnt);
-        else
-            cdf_rows_fast_kernel<__half><<<(unsigned)rows, kCdfThreads, 0, st>>>(kp0, Nk, nk_pad, sm_scale, threshold, nsel_min, idx, cnt);
-        return cudaGetLastError();
+        if (dtype == LCBSA_BF16) return launch_fast<__nv_bfloat16>(kp0, rows, Nk, nk_pad, sm_scale, threshold, nsel_min, idx, cnt, st);
+        return launch_fast<__half>(kp0, rows, Nk, nk_pad, sm_scale, threshold, nsel_min, idx, cnt, st);
     }
     int P = 2;
     while (P < Nk) P <<= 1;
