@@ -38,7 +38,7 @@ enum { LCBSA_BF16 = 0, LCBSA_FP16 = 1, LCBSA_FP32 = 2 };
 /* Which attention kernel lcbsa_attn_fwd runs. */
 enum {
     LCBSA_ATTN_AUTO = 0, /* tcgen05 kernel when the shape allows it, otherwise the generic one */
-    LCBSA_ATTN_TC = 1,   /* TMA + tcgen05 + TMEM kernel (head_dim 128, 64-token blocks, bf16/fp16) */
+    LCBSA_ATTN_TC = 1,   /* TMA + tcgen05 + TMEM kernels at head_dim 128 (AUTO also takes the one for 64-token blocks at 64) */
     LCBSA_ATTN_MMA = 2   /* generic warp-level MMA kernel (other block sizes / head dims) */
 };
 

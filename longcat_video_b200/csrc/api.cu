@@ -328,6 +328,8 @@ int lcbsa_attn_fwd(const LcbsaTensor* q, const LcbsaTensor* k, const LcbsaTensor
     // two tcgen05 kernels: one for 64-token blocks, one for 128-token blocks (the reference's default [4, 4, 8])
     const char* why128 = "";
     const bool tc64 = lcbsa::attn_tc_supported(a, &why), tc128 = !tc64 && lcbsa::attn_tc128_supported(a, &why128);
+    // LCBSA_ATTN_TC names the kernels' head_dim 128 forms; the head_dim 64 form of the first is reached by LCBSA_ATTN_AUTO
+    if (impl == LCBSA_ATTN_TC && a.D != 128) return fail(LCBSA_EUNSUPPORTED, "attn_fwd (tcgen05): needs head_dim 128");
     if (impl == LCBSA_ATTN_AUTO) impl = (tc64 || tc128) ? LCBSA_ATTN_TC : LCBSA_ATTN_MMA;
     if (impl == LCBSA_ATTN_TC) {
         if (!tc64 && !tc128) return fail(LCBSA_EUNSUPPORTED, "attn_fwd (tcgen05): %s", a.gq.bs == 128 ? why128 : why);
@@ -374,6 +376,7 @@ int lcbsa_attn_fwd_scatter(const LcbsaTensor* q, const LcbsaTensor* k, const Lcb
     if (!a.status) return fail(LCBSA_ECUDA, "attn_fwd_scatter: cannot resolve the device status words");
     const char* why = "";
     const char* why128 = "";
+    if (a.D != 128) return fail(LCBSA_EUNSUPPORTED, "attn_fwd_scatter (tcgen05): needs head_dim 128");
     const bool tc64 = lcbsa::attn_tc_supported(a, &why), tc128 = !tc64 && lcbsa::attn_tc128_supported(a, &why128);
     if (!tc64 && !tc128) return fail(LCBSA_EUNSUPPORTED, "attn_fwd_scatter (tcgen05): %s", a.gq.bs == 128 ? why128 : why);
     cudaError_t e = tc64 ? lcbsa::launch_attn_tc(a, static_cast<cudaStream_t>(stream), &why)

@@ -5,7 +5,9 @@
 // three rearrange copies before it and the one after it (bsa_interface.py:650-659): the 3-D token
 // blocks are fetched and the output is written by 5-D TMA boxes straight from/to T,H,W order.
 //
-// Shape handled: head_dim 128, query and key blocks of 64 tokens, bf16 or fp16.
+// Shape handled: head_dim 128 or 64, query and key blocks of 64 tokens, bf16 or fp16.  The figures below are those of
+// head_dim 128; at 64 a tile is one 64-column half, the rings have six slots, an S is half as many MMAs and a P V half as wide
+// (2 x 16 heads of a 12x16x24 grid in fp16, 18 of 72 blocks: 114 us, 248 us on the warp-level kernel that served it before).
 //
 // One persistent CTA per SM.  A work item is a pair of consecutive query blocks of one head.  Each
 // query block is a 64-row tile, i.e. an M=64 tcgen05 MMA whose accumulator occupies 16 lanes of every
@@ -63,13 +65,9 @@ namespace {
 
 using namespace tc;
 
-constexpr int kD = 128;
 constexpr int kBlk = 64;                    // tokens per query / key block
-constexpr int kTileBytes = kBlk * kD * 2;   // 16 KiB: one Q, K, V or O tile
-constexpr int kHalfBytes = kTileBytes / 2;  // one 64-column half: 64 rows x 128 B, 128B-swizzled
+constexpr int kHalfBytes = kBlk * 128;      // one 64-column half of a tile: 64 rows x 128 B, 128B-swizzled
 constexpr int kTilesPerWork = 2;            // the two query blocks of a pair
-constexpr int kSlotBytes = kTilesPerWork * kTileBytes;  // a ring slot holds the K (or V) tiles of both query blocks
-constexpr int kKSlots = 3, kVSlots = 3;
 constexpr int kThreads = 384;
 // setmaxnreg per warpgroup: (208 + 208 + 88) * 128 threads <= the 64 K registers of the SM
 constexpr int kRegsSoftmax = 208, kRegsOther = 88;
@@ -78,16 +76,22 @@ constexpr int kRegsSoftmax = 208, kRegsOther = 88;
 constexpr uint32_t kTmO = 0, kTmS = 256, kTmP = 384, kTmQ = 448;
 
 // shared memory map (offsets from the 1024-byte aligned base of dynamic shared memory)
-constexpr int kOffQ = 0;
-constexpr int kOffK = kOffQ + kTilesPerWork * kTileBytes;
-constexpr int kOffV = kOffK + kKSlots * kSlotBytes;
-constexpr int kOffBar = kOffV + kVSlots * kSlotBytes;
-// barriers: k_full[3] k_empty[3] v_full[3] v_empty[3] q_full q_empty s_full[2] s_free[2] p_full[2] pv_done[2]
-//           ml_ready o_free o_staged qt_full qt_free
-constexpr int kNumBars = 2 * kKSlots + 2 * kVSlots + 2 + 8 + 5;
-constexpr int kOffMisc = kOffBar + kNumBars * 8;      // abort flag, TMEM base
-constexpr int kOffMl = kOffMisc + 64;                 // [2 warpgroups][128 lanes] (maximum, row sum)
-constexpr int kSmemBytes = kOffMl + 2 * 128 * 8;
+template <int kD> struct Lay {
+    static constexpr int halves = kD / 64;
+    static constexpr int tile = halves * kHalfBytes;     // one Q, K, V or O tile: 16 KiB at head_dim 128
+    static constexpr int slot = kTilesPerWork * tile;    // a ring slot holds the K (or V) tiles of both query blocks
+    static constexpr int slots = kD == 128 ? 3 : 6;      // of the K ring and of the V ring: 96 KiB each
+    static constexpr int offQ = 0;
+    static constexpr int offK = offQ + kTilesPerWork * tile;
+    static constexpr int offV = offK + slots * slot;
+    static constexpr int offBar = offV + slots * slot;
+    // barriers: k_full[slots] k_empty[slots] v_full[slots] v_empty[slots] q_full q_empty s_full[2] s_free[2] p_full[2] pv_done[2]
+    //           ml_ready o_free o_staged qt_full qt_free
+    static constexpr int numBars = 4 * slots + 2 + 8 + 5;
+    static constexpr int offMisc = offBar + numBars * 8;  // abort flag, TMEM base
+    static constexpr int offMl = offMisc + 64;            // [2 warpgroups][128 lanes] (maximum, row sum)
+    static constexpr int smem = offMl + 2 * 128 * 8;
+};
 
 struct TcParams {
     CUtensorMap tm_q, tm_k, tm_v;
@@ -119,8 +123,11 @@ __device__ __forceinline__ int clamp_cnt(const TcParams& P, int bh, int qt) {
 
 // kRagged: the key grid has partial blocks.  The masking code exists only in that instantiation, which keeps the
 // instruction stream of the softmax loop of whole grids short (the loop is sensitive to instruction fetch).
-template <bool kBf16, bool kRagged>
+template <bool kBf16, bool kRagged, int kD>
 __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_constant__ TcParams P) {
+    using Ly = Lay<kD>;
+    constexpr int kHalves = Ly::halves, kTileBytes = Ly::tile, kSlotBytes = Ly::slot, kKSlots = Ly::slots, kVSlots = Ly::slots;
+    constexpr int kOffQ = Ly::offQ, kOffK = Ly::offK, kOffV = Ly::offV, kOffBar = Ly::offBar, kOffMisc = Ly::offMisc, kOffMl = Ly::offMl;
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t sbase = smem_u32(smem);
     const uint32_t bar0 = sbase + kOffBar;
@@ -207,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     constexpr bool bf16 = kBf16;
 
     // All roles walk the same list of work items and blocks.  Block number gb (counted over the whole kernel)
-    // uses K slot gb % 3 and V slot gb % 3.  Within an item block i belongs to warpgroup i & 1, which numbers its own rounds rr
+    // uses slot gb % slots of the K ring and of the V ring.  Within an item block i belongs to warpgroup i & 1, which numbers its own rounds rr
     // over the whole kernel.
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
@@ -239,7 +246,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                     }
                     const uint32_t src = sbase + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes;
                     tma_store_5d(tmo, src, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                    tma_store_5d(tmo, src + kHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+                    if (kHalves == 2) tma_store_5d(tmo, src + kHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
                 }
                 tma_store_commit();
                 tma_store_wait_read();
@@ -299,11 +306,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                 mbar_arrive_tx_elect(bar, ((j < ca) + (j < cb)) * kTileBytes);
                 if (j < ca) {
                     tma_load_5d_elect(dst, tm, bar, 0, pa & 1023, (pa >> 10) & 1023, (pa >> 20) + c3, c4);
-                    tma_load_5d_elect(dst + kHalfBytes, tm, bar, 64, pa & 1023, (pa >> 10) & 1023, (pa >> 20) + c3, c4);
+                    if (kHalves == 2) tma_load_5d_elect(dst + kHalfBytes, tm, bar, 64, pa & 1023, (pa >> 10) & 1023, (pa >> 20) + c3, c4);
                 }
                 if (j < cb) {
                     tma_load_5d_elect(dst + kTileBytes, tm, bar, 0, pb & 1023, (pb >> 10) & 1023, (pb >> 20) + c3, c4);
-                    tma_load_5d_elect(dst + kTileBytes + kHalfBytes, tm, bar, 64, pb & 1023, (pb >> 10) & 1023, (pb >> 20) + c3, c4);
+                    if (kHalves == 2) tma_load_5d_elect(dst + kTileBytes + kHalfBytes, tm, bar, 64, pb & 1023, (pb >> 10) & 1023, (pb >> 20) + c3, c4);
                 }
                 if ((j & 15) == 15) {
                     cur = nxt;
@@ -324,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                         const Coord cc = block_coord(P.gq, qt, b, h, P.heads, P.merge_q, P.Tq);
                         const uint32_t dst = sbase + kOffQ + hf * kTileBytes;
                         tma_load_5d(dst, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                        tma_load_5d(dst + kHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+                        if (kHalves == 2) tma_load_5d(dst + kHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
                     }
                 }
                 __syncwarp();
@@ -424,7 +431,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
         }
       } else if (warp == 10) {
         // ================================================================== O += P V issuer
-        const uint32_t idesc_pv = instr_desc(bf16, 64, 128, 1);
+        const uint32_t idesc_pv = instr_desc(bf16, 64, kD, 1);
         unsigned gb = 0, wk = 0, rr0 = 0, rr1 = 0;
         bool ok = true;
         int bh = first_bh, g = first_g, ca_n = 0, cb_n = 0;
@@ -493,23 +500,27 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
         unsigned wk = 0, gb = 0, rr = 0;  // rr: rounds of this warpgroup over the whole kernel
         bool ok = true;
 
-        // Q of the CTA's work item number `item` from shared memory to TMEM: a thread moves its row, the warpgroup 64 of the 128 columns.
+        // Q of the CTA's work item number `item` from shared memory to TMEM: a thread moves its row, the warpgroup half of the columns.
         auto q_to_tmem = [&](unsigned item) -> bool {
             // the last S of the item before has read the columns
             if (item > 0 && !mbar_wait_warp(bar_qt_free, (item - 1) & 1, ctl, 106 + wg, item)) return false;
             if (!mbar_wait_warp(bar_q_full, item & 1, ctl, 108 + wg, item)) return false;
             tc_fence_after();
-            const unsigned char* src = smem + kOffQ + hf * kTileBytes + wg * kHalfBytes + row * 128;
-            uint32_t qr[32];
+            // head_dim 128: the warpgroup's 64-column half, eight chunks of 16 bytes; 64: its four chunks of the only half
+            constexpr int kChunks = kD / 16;
+            const unsigned char* src = smem + kOffQ + hf * kTileBytes + (kD == 128 ? wg * kHalfBytes : 0) + row * 128;
+            const int c0 = kD == 128 ? 0 : 4 * wg;
+            uint32_t qr[4 * kChunks];
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint4 v = *reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4));
+            for (int c = 0; c < kChunks; ++c) {
+                const uint4 v = *reinterpret_cast<const uint4*>(src + (((c0 + c) ^ (row & 7)) << 4));
                 qr[4 * c + 0] = v.x;
                 qr[4 * c + 1] = v.y;
                 qr[4 * c + 2] = v.z;
                 qr[4 * c + 3] = v.w;
             }
-            tc_st32(tmem + kTmQ + 32u * wg + t_lane, qr);
+            if constexpr (kD == 128) tc_st32(tmem + kTmQ + 32u * wg + t_lane, qr);
+            else tc_st16(tmem + kTmQ + 16u * wg + t_lane, qr);
             tc_wait_st();
             tc_fence_before();
             __syncwarp();
@@ -647,7 +658,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                     }
                     tc_st32(tm_p, pr);
                 }
-                if (LCBSA_UNLIKELY(any_need)) tc_scale_row128(tm_o_mine, alpha);  // rare: only when a row maximum jumps
+                if (LCBSA_UNLIKELY(any_need)) tc_scale_row<kD>(tm_o_mine, alpha);  // rare: only when a row maximum jumps
                 if (i + 2 < n_iter) {
                     // The next round's S is on its way into the registers while P is being stored: it has usually been ready
                     // for some hundred cycles, since it only waits for this round's S to be in registers.
@@ -698,19 +709,19 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             const float l_all = l_sum * w_mine + oth.y * w_oth;
             const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
             const float f_mine = w_mine * inv, f_oth = w_oth * inv;
-            // This warpgroup merges and stages columns 64*wg .. 64*wg+63 of O (input dtype, one 128B-swizzled
-            // half-tile row per thread) in the V slot that the item's last PV has just released.
+            // This warpgroup merges and stages half of the columns of O (input dtype, 128B-swizzled rows of 64 columns) in the V slot that the item's last PV has just released.
             const unsigned last = gb - 1;
-            unsigned char* o_half = smem + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes + wg * kHalfBytes;
+            unsigned char* o_half = smem + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes + (kD == 128 ? wg * kHalfBytes : 0);
+            constexpr int kMine = kD / 2;  // columns kMine * wg ..
             // a warpgroup that saw no block has weight 0; its accumulator holds garbage and is not used
             const bool rd_mine = __any_sync(0xffffffffu, w_mine > 0.f), rd_oth = __any_sync(0xffffffffu, w_oth > 0.f);
             const bool both = __all_sync(0xffffffffu, w_mine > 0.f && w_oth > 0.f);  // the usual case: no lane has to be masked
             const float2 fm2 = make_float2(f_mine, f_mine), fo2 = make_float2(f_oth, f_oth);
 #pragma unroll
-            for (int cch = 0; cch < 2; ++cch) {
+            for (int cch = 0; cch < kMine / 32; ++cch) {
                 uint32_t oa[32], ob[32];
-                if (rd_mine) tc_ld32(tm_o_mine + 64 * wg + 32 * cch, oa);
-                if (rd_oth) tc_ld32(tm_o_other + 64 * wg + 32 * cch, ob);
+                if (rd_mine) tc_ld32(tm_o_mine + kMine * wg + 32 * cch, oa);
+                if (rd_oth) tc_ld32(tm_o_other + kMine * wg + 32 * cch, ob);
                 tc_wait_ld();
                 if (LCBSA_UNLIKELY(!both)) {
 #pragma unroll
@@ -731,7 +742,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                             const float2 v2 = __fadd2_rn(a2, b2);
                             pw[j] = pack2(bf16, v2.x, v2.y);
                         }
-                        const int chunk = cch * 4 + q8;
+                        const int chunk = (kD == 128 ? 0 : 4 * wg) + cch * 4 + q8;
                         *reinterpret_cast<uint4*>(o_half + row * 128 + ((chunk ^ (row & 7)) << 4)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
                     }
                 }
@@ -782,7 +793,7 @@ int attn_sm_reserve() { return g_sm_reserve.load(); }
 
 bool attn_tc_supported(const AttnArgs& a, const char** why) {
     if (a.dtype != LCBSA_BF16 && a.dtype != LCBSA_FP16) { *why = "needs bf16 or fp16"; return false; }
-    if (a.D != kD) { *why = "needs head_dim 128"; return false; }
+    if (a.D != 128 && a.D != 64) { *why = "needs head_dim 64 or 128"; return false; }
     if (a.gq.bs != kBlk || a.gk.bs != kBlk) { *why = "needs 64-token query and key blocks"; return false; }
     if (a.gq.ct > 256 || a.gq.ch > 256 || a.gq.cw > 256 || a.gk.ct > 256 || a.gk.ch > 256 || a.gk.cw > 256) {
         *why = "block axis above the TMA box limit";
@@ -814,8 +825,8 @@ cudaError_t launch_attn_tc(const AttnArgs& a, cudaStream_t st, const char** why)
     TcParams P;
     const int mq = merge_mode(a.q, a.B, a.H, a.gq), mk = merge_mode(a.k, a.B, a.H, a.gk);
     const int mv = merge_mode(a.v, a.B, a.H, a.gk), mo = merge_mode(a.o, a.B, a.H, a.gq);
-    if (!make_map(&P.tm_q, a.dtype, a.q, a.B, a.H, a.gq, mq) || !make_map(&P.tm_k, a.dtype, a.k, a.B, a.H, a.gk, mk) ||
-        !make_map(&P.tm_v, a.dtype, a.v, a.B, a.H, a.gk, mv)) {
+    if (!make_map(&P.tm_q, a.dtype, a.q, a.B, a.H, a.gq, mq, a.D) || !make_map(&P.tm_k, a.dtype, a.k, a.B, a.H, a.gk, mk, a.D) ||
+        !make_map(&P.tm_v, a.dtype, a.v, a.B, a.H, a.gk, mv, a.D)) {
         *why = "cuTensorMapEncodeTiled rejected a tensor";
         return cudaErrorInvalidValue;
     }
@@ -828,12 +839,12 @@ cudaError_t launch_attn_tc(const AttnArgs& a, cudaStream_t st, const char** why)
         for (int r = 0; r < a.n_out_dst; ++r) {
             View vo = a.o;
             vo.data = a.out_dst[r];
-            if (!make_map(&P.tm_o[r], a.dtype, vo, 1, a.H, gl, 0)) {
+            if (!make_map(&P.tm_o[r], a.dtype, vo, 1, a.H, gl, 0, a.D)) {
                 *why = "cuTensorMapEncodeTiled rejected a destination of the scattered output";
                 return cudaErrorInvalidValue;
             }
         }
-    } else if (!make_map(&P.tm_o[0], a.dtype, a.o, a.B, a.H, a.gq, mo)) {
+    } else if (!make_map(&P.tm_o[0], a.dtype, a.o, a.B, a.H, a.gq, mo, a.D)) {
         *why = "cuTensorMapEncodeTiled rejected a tensor";
         return cudaErrorInvalidValue;
     }
@@ -856,11 +867,18 @@ cudaError_t launch_attn_tc(const AttnArgs& a, cudaStream_t st, const char** why)
         ds.sm_count.store(sm_count, std::memory_order_relaxed);
     }
     const bool ragged = a.gk.ragged;
-    auto kern = P.is_bf16 ? (ragged ? attn_tc_kernel<true, true> : attn_tc_kernel<true, false>)
-                          : (ragged ? attn_tc_kernel<false, true> : attn_tc_kernel<false, false>);
-    const int bit = 1 << ((P.is_bf16 ? 0 : 1) + (ragged ? 2 : 0));  // bits 0-3 of attr_set
+    using Kern = void (*)(const TcParams);
+    Kern kern;
+    if (a.D == 128)
+        kern = P.is_bf16 ? (ragged ? attn_tc_kernel<true, true, 128> : attn_tc_kernel<true, false, 128>)
+                         : (ragged ? attn_tc_kernel<false, true, 128> : attn_tc_kernel<false, false, 128>);
+    else
+        kern = P.is_bf16 ? (ragged ? attn_tc_kernel<true, true, 64> : attn_tc_kernel<true, false, 64>)
+                         : (ragged ? attn_tc_kernel<false, true, 64> : attn_tc_kernel<false, false, 64>);
+    const int smem_bytes = a.D == 128 ? Lay<128>::smem : Lay<64>::smem;
+    const int bit = (a.D == 128 ? 1 : 256) << ((P.is_bf16 ? 0 : 1) + (ragged ? 2 : 0));  // bits 0-3 and 8-11 of attr_set
     if (!(ds.attr_set.load(std::memory_order_relaxed) & bit)) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
         if (e != cudaSuccess) return e;
         ds.attr_set.fetch_or(bit, std::memory_order_relaxed);
     }
@@ -868,7 +886,7 @@ cudaError_t launch_attn_tc(const AttnArgs& a, cudaStream_t st, const char** why)
     const long long work = groups * a.B * a.H;
     const int usable = sm_count - g_sm_reserve.load() > 0 ? sm_count - g_sm_reserve.load() : 1;
     const int grid = (int)(work < usable ? work : usable);
-    kern<<<grid, kThreads, kSmemBytes, st>>>(P);
+    kern<<<grid, kThreads, smem_bytes, st>>>(P);
     return cudaGetLastError();
 }
 

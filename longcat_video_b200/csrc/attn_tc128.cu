@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                     pr[4 * cch + 2] = pk[cch].z;
                     pr[4 * cch + 3] = pk[cch].w;
                 }
-                if (LCBSA_UNLIKELY(any_need)) tc_scale_row128(tm_o_mine, alpha);  // rare: only when a row maximum jumps
+                if (LCBSA_UNLIKELY(any_need)) tc_scale_row<kD>(tm_o_mine, alpha);  // rare: only when a row maximum jumps
                 if (ready && more) {
                     tc_fence_after();
                     tc_st32(tm_p, pr);

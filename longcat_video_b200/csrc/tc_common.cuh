@@ -245,11 +245,12 @@ __device__ __forceinline__ uint32_t pack2(bool bf16, float lo, float hi) {
 }
 
 // Rare path of the online softmax, as a rolled loop so that it takes little room in the instruction stream of the loop:
-// multiply this thread's row of a 128-column fp32 accumulator in TMEM by alpha.  Warp-collective.
-__device__ __forceinline__ void tc_scale_row128(uint32_t taddr, float alpha) {
+// multiply this thread's row of a kCols-column fp32 accumulator in TMEM by alpha.  Warp-collective.
+template <int kCols>
+__device__ __forceinline__ void tc_scale_row(uint32_t taddr, float alpha) {
     tc_fence_after();
 #pragma unroll 1
-    for (int cch = 0; cch < 4; ++cch) {
+    for (int cch = 0; cch < kCols / 32; ++cch) {
         uint32_t orr[32];
         tc_ld32(taddr + 32 * cch, orr);
         tc_wait_ld();
@@ -341,11 +342,11 @@ inline int merge_mode(const View& v, int B, int H, const Geom& g) {
     return -1;
 }
 
-inline bool encode_map(CUtensorMap* tm, int dtype, const View& v, int B, int H, const Geom& g, int merge) {
+inline bool encode_map(CUtensorMap* tm, int dtype, const View& v, int B, int H, const Geom& g, int merge, int D) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     const cuuint64_t es = 2;
-    cuuint64_t dims[5] = {(cuuint64_t)128, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)(merge ? (long long)g.T * B : g.T),
+    cuuint64_t dims[5] = {(cuuint64_t)D, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)(merge ? (long long)g.T * B : g.T),
                           (cuuint64_t)(merge ? H : (long long)B * H)};
     cuuint64_t strides[4] = {(cuuint64_t)v.ss * es, (cuuint64_t)v.ss * g.W * es, (cuuint64_t)v.ss * g.W * g.H * es,
                              (cuuint64_t)v.sh * es};
@@ -357,15 +358,15 @@ inline bool encode_map(CUtensorMap* tm, int dtype, const View& v, int B, int H, 
     return r == CUDA_SUCCESS;
 }
 
-// Tensor maps are a pure function of (pointer, dtype, strides, batch, heads, grid, block, fold mode); a DiT calls the
+// Tensor maps are a pure function of (pointer, dtype, strides, batch, heads, grid, block, fold mode, head_dim); a DiT calls the
 // op with the same few buffers layer after layer, so the last encodings are kept per host thread and reused.
 struct MapKey {
     const void* data;
     long long sb, sh, ss;
-    int dtype, B, H, T, Hh, W, ct, ch, cw, merge;
+    int dtype, B, H, T, Hh, W, ct, ch, cw, merge, D;
     bool operator==(const MapKey& o) const {
         return data == o.data && sb == o.sb && sh == o.sh && ss == o.ss && dtype == o.dtype && B == o.B && H == o.H && T == o.T &&
-               Hh == o.Hh && W == o.W && ct == o.ct && ch == o.ch && cw == o.cw && merge == o.merge;
+               Hh == o.Hh && W == o.W && ct == o.ct && ch == o.ch && cw == o.cw && merge == o.merge && D == o.D;
     }
 };
 constexpr int kMapCache = 32;
@@ -375,15 +376,15 @@ struct MapCache {
     int used = 0, next = 0;
 };
 
-inline bool make_map(CUtensorMap* tm, int dtype, const View& v, int B, int H, const Geom& g, int merge) {
+inline bool make_map(CUtensorMap* tm, int dtype, const View& v, int B, int H, const Geom& g, int merge, int D = 128) {
     static thread_local MapCache cache;
-    const MapKey k{v.data, v.sb, v.sh, v.ss, dtype, B, H, g.T, g.H, g.W, g.ct, g.ch, g.cw, merge};
+    const MapKey k{v.data, v.sb, v.sh, v.ss, dtype, B, H, g.T, g.H, g.W, g.ct, g.ch, g.cw, merge, D};
     for (int i = 0; i < cache.used; ++i)
         if (cache.key[i] == k) {
             *tm = cache.map[i];
             return true;
         }
-    if (!encode_map(tm, dtype, v, B, H, g, merge)) return false;
+    if (!encode_map(tm, dtype, v, B, H, g, merge, D)) return false;
     const int slot = cache.next;
     cache.key[slot] = k;
     cache.map[slot] = *tm;
@@ -396,7 +397,7 @@ inline bool make_map(CUtensorMap* tm, int dtype, const View& v, int B, int H, co
 constexpr int kMaxDevices = 64;
 struct DeviceState {
     std::atomic<int> sm_count{0};
-    std::atomic<int> attr_set{0};  // one bit per kernel instantiation: bits 0-3 64-token blocks (dtype, ragged), bits 4-7 128-token blocks
+    std::atomic<int> attr_set{0};  // one bit per kernel instantiation: bits 0-3 64-token blocks (dtype, ragged), bits 4-7 128-token blocks, bits 8-11 64-token blocks of head_dim 64
 };
 DeviceState* device_states();  // defined once, in attn_tc.cu
 int attn_sm_reserve();           // SMs the persistent attention kernels leave idle (lcbsa_set_attn_sm_reserve)
