@@ -1,6 +1,6 @@
 // Generic block-sparse flash-attention forward on warp-level MMA (mma.sync m16n8k16).
 //
-// Covers the shapes the tcgen05 kernel does not: head_dim 64, 128-token blocks, and serves as the
+// Covers the shapes the tcgen05 kernels do not: head_dim 64 outside 64-token blocks, other block sizes, and serves as the
 // on-device comparator for it.  Same contract as the Triton kernels it stands in for
 // (longcat_video/block_sparse_attention/flash_attn_bsa_varlen_mask.py:172-285 and :35-153):
 // one CTA keeps a query block resident and walks that block's list of selected K/V blocks with an

@@ -738,8 +738,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                         for (int j = 0; j < 4; ++j) {
                             const int e = q8 * 8 + 2 * j;
                             const float2 a2 = __fmul2_rn(make_float2(__uint_as_float(oa[e]), __uint_as_float(oa[e + 1])), fm2);
-                            const float2 b2 = __fmul2_rn(make_float2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), fo2);
-                            const float2 v2 = __fadd2_rn(a2, b2);
+                            const float2 v2 = __ffma2_rn(make_float2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), fo2, a2);
                             pw[j] = pack2(bf16, v2.x, v2.y);
                         }
                         const int chunk = (kD == 128 ? 0 : 4 * wg) + cch * 4 + q8;
