@@ -76,6 +76,10 @@ constexpr int kRegsSoftmax = 208, kRegsOther = 88;
 constexpr uint32_t kTmO = 0, kTmS = 256, kTmP = 384, kTmQ = 448;
 
 // shared memory map (offsets from the 1024-byte aligned base of dynamic shared memory)
+// Ring of the key masks of ragged grids, indexed by block number.  The K producer writes the masks of a block before it
+// requests its tiles, at most six (the K ring) ahead of an S that waited for a softmax warpgroup to have read the masks of
+// a block at most three further back: sixteen entries are never overwritten unread.
+constexpr int kMaskRing = 16;
 template <int kD> struct Lay {
     static constexpr int halves = kD / 64;
     static constexpr int tile = halves * kHalfBytes;     // one Q, K, V or O tile: 16 KiB at head_dim 128
@@ -90,7 +94,8 @@ template <int kD> struct Lay {
     static constexpr int numBars = 4 * slots + 2 + 8 + 5;
     static constexpr int offMisc = offBar + numBars * 8;  // abort flag, TMEM base
     static constexpr int offMl = offMisc + 64;            // [2 warpgroups][128 lanes] (maximum, row sum)
-    static constexpr int smem = offMl + 2 * 128 * 8;
+    static constexpr int offMask = offMl + 2 * 128 * 8;   // ragged grids: [kMaskRing][2 tiles] which keys of a block are present
+    static constexpr int smem = offMask + kMaskRing * 16;
 };
 
 struct TcParams {
@@ -128,6 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     using Ly = Lay<kD>;
     constexpr int kHalves = Ly::halves, kTileBytes = Ly::tile, kSlotBytes = Ly::slot, kKSlots = Ly::slots, kVSlots = Ly::slots;
     constexpr int kOffQ = Ly::offQ, kOffK = Ly::offK, kOffV = Ly::offV, kOffBar = Ly::offBar, kOffMisc = Ly::offMisc, kOffMl = Ly::offMl;
+    constexpr int kOffMask = Ly::offMask;
     extern __shared__ __align__(1024) unsigned char smem[];
     const uint32_t sbase = smem_u32(smem);
     const uint32_t bar0 = sbase + kOffBar;
@@ -147,6 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kOffMisc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffMisc + 8);
     float2* ml = reinterpret_cast<float2*>(smem + kOffMl);  // [2][128]
+    unsigned long long* masks = reinterpret_cast<unsigned long long*>(smem + kOffMask);  // [kMaskRing][2]
     const Ctl ctl{abort_flag, P.status};
 
     const int tid = threadIdx.x, lane = tid & 31;
@@ -335,12 +342,24 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                     }
                 }
                 __syncwarp();
+                // ragged grids: which keys of this lane's list entry lie inside the grid (decoded here once per entry; the softmax
+                // warps spent two divisions per round and thread on it: 720p with 45 rows, 8 heads, 2.73 ms, 2.61 ms with masks
+                // from here and the single copy of the pass below)
+                auto entry_mask = [&]() {
+                    return slot_mask64(P.gk.ct, P.gk.ch, P.gk.cw, P.gk.T - (cur >> 20), P.gk.H - ((cur >> 10) & 1023), P.gk.W - (cur & 1023));
+                };
+                unsigned long long my_mask = kRagged ? entry_mask() : 0ull;
                 for (int j = 0; j < n_iter; ++j) {
                     const int slot = gk % kKSlots;
                     ok = mbar_wait_warp(bar_k_empty(slot), ((gk / kKSlots) & 1) ^ 1, ctl, 20, gk);
                     if (!ok) break;
+                    if (kRagged) {
+                        if (my_s == (j & 15)) masks[(gk % kMaskRing) * 2 + my_t] = my_mask;
+                        __syncwarp();
+                    }
                     ++gk;
                     request(j, &P.tm_k, bar_k_full(slot), sbase + kOffK + slot * kSlotBytes);
+                    if (kRagged && (j & 15) == 15) my_mask = entry_mask();
                 }
             } else {
                 for (int j = 0; j < n_iter; ++j) {
@@ -545,14 +564,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             next_item(nx_bh, nx_g);
             peek(w + gridDim.x < total_work);
             const int n_iter = max(1, max(my_cnt, other_cnt));
-            const int32_t* my_list = P.idx + ((long long)bh * P.nq + (tile_valid ? qt : 0)) * P.cap;
 
             float m_ref = -INFINITY, l_sum = 0.f;
             bool first = true;  // no block of this item seen yet by this warpgroup
 
-            // ragged grids: the block index of a round is fetched a round ahead, so that the global load never sits
-            // between S and the softmax
-            int blk_ahead = (kRagged && wg < my_cnt) ? my_list[wg] : 0;
+            unsigned long long present = ~0ull;  // ragged grids: which keys of the round's block lie inside the grid
             // S of the warpgroup's round into registers; the buffer is then free for the S of its next round
             uint32_t sr[64];
             if (wg < n_iter) {
@@ -560,25 +576,19 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                 if (!ok) break;
                 tc_fence_after();
                 tc_ld64(tm_s, sr);
+                if (kRagged) present = masks[((gb + wg) % kMaskRing) * 2 + hf];
                 tc_wait_ld();
                 tc_fence_before();
                 mbar_arrive_elect(bar_s_free(wg));
             }
             for (int i = wg; i < n_iter && ok; i += 2, ++rr) {
                 const bool active = i < my_cnt;
-                const int blk_now = blk_ahead;
-                if (kRagged && i + 2 < my_cnt) blk_ahead = my_list[i + 2];
                 float alpha = 1.f;
                 bool need = false;
                 uint4 pk[8];  // this row of P in the input dtype, 8 keys per 16-byte chunk
                 if (active) {
                     if (kRagged) {  // keys of a partial block that lie outside the grid
-                        const int blk = blk_now;
-                        int bt, bhh, bw;
-                        block_coords(P.gk, blk, bt, bhh, bw);
-                        const int vt = P.gk.T - bt * P.gk.ct, vh = P.gk.H - bhh * P.gk.ch, vw = P.gk.W - bw * P.gk.cw;
-                        if (vt < P.gk.ct || vh < P.gk.ch || vw < P.gk.cw) {
-                            const uint64_t present = slot_mask64(P.gk.ct, P.gk.ch, P.gk.cw, vt, vh, vw);
+                        if (present != ~0ull) {
                             const uint32_t p_lo = (uint32_t)present, p_hi = (uint32_t)(present >> 32);
 #pragma unroll
                             for (int j = 0; j < 32; ++j) {
@@ -627,18 +637,39 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                         return fmaxf(max3(max3(mx8[0], mx8[1], mx8[2]), mx8[3], mx8[4]), max3(mx8[5], mx8[6], mx8[7])) * P.scale2;
                     };
                     float rs = 0.f;
-                    float m_new = m_ref;
-                    if (LCBSA_UNLIKELY(first)) {
-                        m_new = fmaxf(m_ref, row_max());
-                        m_ref = (m_new == -INFINITY) ? 0.f : m_new;
-                    }
-                    probs(m_ref, rs);
-                    const float m_top = row_max();
-                    if (LCBSA_UNLIKELY(m_top - m_ref > 8.f)) {
-                        need = true;
-                        alpha = ex2(m_ref - m_top);
-                        m_ref = m_top;
+                    if (kRagged) {
+                        // the instantiation with the masking code: a single copy of the pass in the instruction stream.  The loop
+                        // body runs once in the common case (pass, then the row maximum, which confirms the reference) and twice
+                        // when the reference moves; for the warpgroup's first block the first pass is skipped.
+                        bool run_pass = !first, decided = false;
+#pragma unroll 1
+                        for (int turn = 0; turn < 2; ++turn) {
+                            if (run_pass) probs(m_ref, rs);
+                            if (decided) break;
+                            const float m_new = fmaxf(m_ref, row_max());
+                            run_pass = first || m_new - m_ref > 8.f;
+                            if (!run_pass) break;
+                            if (!first) {
+                                need = true;
+                                alpha = ex2(m_ref - m_new);
+                            }
+                            m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+                            decided = true;
+                        }
+                    } else {
+                        float m_new = m_ref;
+                        if (LCBSA_UNLIKELY(first)) {
+                            m_new = fmaxf(m_ref, row_max());
+                            m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+                        }
                         probs(m_ref, rs);
+                        const float m_top = row_max();
+                        if (LCBSA_UNLIKELY(m_top - m_ref > 8.f)) {
+                            need = true;
+                            alpha = ex2(m_ref - m_top);
+                            m_ref = m_top;
+                            probs(m_ref, rs);
+                        }
                     }
                     l_sum = l_sum * alpha + rs;  // alpha is 1 unless this row's reference maximum moved
                 }
@@ -667,6 +698,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                     tc_fence_after();
                     __syncwarp();
                     tc_ld64(tm_s, sr);
+                    if (kRagged) present = masks[((gb + i + 2) % kMaskRing) * 2 + hf];
                     tc_wait_st();
                     tc_fence_before();
                     mbar_arrive_elect(bar_p_full(wg));
