@@ -678,6 +678,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                 // P may be overwritten, and O rescaled, once the warpgroup's PV of the round before has finished
                 ok = mbar_wait_warp(bar_pv_done(wg), (rr & 1) ^ 1, ctl, 92 + wg, rr);
                 if (!ok) break;
+                tc_fence_after();  // orders the store of P behind the MMAs that read the columns (no other barrier does)
                 {   // all 32 lanes take part in the store (a lane whose tile has run out of blocks writes don't-cares)
                     uint32_t pr[32];
 #pragma unroll

@@ -601,6 +601,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                     ok = mbar_wait_warp(bar_pv_done(wg), (rr & 1) ^ 1, ctl, 92 + wg, rr);
                     if (!ok) break;
                 }
+                tc_fence_after();  // orders the store of P behind the MMAs that read the columns (no other barrier does)
                 uint32_t pr[32];  // all 32 lanes take part in the store (don't-cares for a unit that does not exist)
 #pragma unroll
                 for (int cch = 0; cch < 8; ++cch) {
@@ -611,7 +612,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                 }
                 if (LCBSA_UNLIKELY(any_need)) tc_scale_row<kD>(tm_o_mine, alpha);  // rare: only when a row maximum jumps
                 if (ready && more) {
-                    tc_fence_after();
                     tc_st32(tm_p, pr);
                     tc_ld64(tm_s, sr);
                     tc_wait_st();

@@ -1,0 +1,61 @@
+"""Ordering rules of the tcgen05 kernels that no run can be relied on to violate, checked on the source text.
+
+A tcgen05 access (ld, st, mma) that follows a wait on an mbarrier is only ordered behind the tcgen05 work which that
+barrier reports if a ``tcgen05.fence::after_thread_sync`` stands between the two.  The scan below walks a kernel source in
+textual order: a wait or a probe of a barrier clears "fenced", a fence sets it, and an access needs it.  A fence inside a
+block of braces counts for that block alone; an unfenced wait inside a block counts behind it too.  The branches of an
+if / else start from the same state.
+"""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "longcat_video_b200", "csrc")
+TOKEN = re.compile(r"[{}]|\b(?:mbar_wait_warp|mbar_wait_thread|mbar_test|mbar_try|tc_fence_after|tc_ld32|tc_ld64|tc_st16|tc_st32|tc_mma|tc_mma_ts)(?=\()")
+
+
+def _unfenced(text):
+    """Line numbers of tcgen05 accesses without a fence behind the last wait."""
+    text = re.sub(r"//[^\n]*", "", text)
+    found, stack, fenced = [], [], True
+    branch = True  # state at the end of the branches before this one, while an else is open
+    for m in TOKEN.finditer(text):
+        tok = m.group()
+        if tok == "{":
+            stack.append((fenced, branch))
+            branch = True
+        elif tok == "}":
+            before, others = stack.pop()
+            end = fenced and others
+            if re.match(r"\s*else\b", text[m.end():]):
+                fenced, branch = before, end
+            else:
+                fenced, branch = before and end, True
+        elif tok.startswith("mbar"):
+            fenced = False
+        elif tok == "tc_fence_after":
+            fenced = True
+        elif not fenced:
+            found.append(text.count("\n", 0, m.start()) + 1)
+    assert not stack
+    return found
+
+
+def _source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return f.read()
+
+
+@pytest.mark.parametrize("name", ["attn_tc.cu", "attn_tc128.cu", "attn_bwd_tc.cu"])
+def test_every_tcgen05_access_behind_a_wait_is_fenced(name):
+    assert _unfenced(_source(name)) == []
+
+
+def test_the_scan_sees_a_missing_fence():
+    ok = "{ mbar_wait_warp(b); tc_fence_after(); { tc_st32(x); } }"
+    assert _unfenced(ok) == []
+    assert _unfenced(ok.replace("tc_fence_after();", "")) == [1]
+    assert _unfenced("{ mbar_test(b); if (r) { tc_fence_after(); tc_st32(x); } else {\n tc_st32(x); } }") == [2]
+    assert _unfenced("{ tc_fence_after(); if (!pre) { mbar_wait_warp(b); }\n tc_mma(x); }") == [2]
+    assert _unfenced("{ if (k) { mbar_wait_warp(b); } else { mbar_wait_warp(c); tc_fence_after(); tc_ld32(x); }\n tc_ld32(x); }") == [2]
