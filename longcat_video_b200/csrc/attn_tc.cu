@@ -79,6 +79,7 @@ constexpr uint32_t kTmO = 0, kTmS = 256, kTmP = 384, kTmQ = 448;
 // Ring of the key masks of ragged grids, indexed by block number.  The K producer writes the masks of a block before it
 // requests its tiles, at most six (the K ring) ahead of an S that waited for a softmax warpgroup to have read the masks of
 // a block at most three further back: sixteen entries are never overwritten unread.
+// They become visible through threads' arrivals alone: the producer's on k_full, then the S issuer's on s_full.
 constexpr int kMaskRing = 16;
 template <int kD> struct Lay {
     static constexpr int halves = kD / 64;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
         mbar_init(bar_q_full, 1);
         mbar_init(bar_q_empty, 8);
         for (int b = 0; b < 2; ++b) {
-            mbar_init(bar_s_full(b), 1);
+            mbar_init(bar_s_full(b), kRagged ? 2 : 1);  // the MMAs; ragged grids: and the issuer, for the masks
             mbar_init(bar_s_free(b), 4);
             mbar_init(bar_p_full(b), 4);  // one elected arrival per softmax warp
             mbar_init(bar_pv_done(b), 1);
@@ -441,6 +442,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                     }
                 }
                 tc_commit(bar_k_empty(slot));  // K is free once these MMAs have read it
+                // The softmax warps read the block's key masks once s_full completes.  The masks are generic stores of the K
+                // producer, which its arrival on k_full released to this warp; the commit only reports MMAs, so an arrival
+                // of this warp passes them on.
+                if (kRagged) mbar_arrive_elect(bar_s_full(wg));
                 tc_commit(bar_s_full(wg));
                 __syncwarp();
                 if (i == n_iter - 1) tc_commit(bar_qt_free);  // and so are Q's TMEM columns after the last S of the item

@@ -59,3 +59,14 @@ def test_the_scan_sees_a_missing_fence():
     assert _unfenced("{ mbar_test(b); if (r) { tc_fence_after(); tc_st32(x); } else {\n tc_st32(x); } }") == [2]
     assert _unfenced("{ tc_fence_after(); if (!pre) { mbar_wait_warp(b); }\n tc_mma(x); }") == [2]
     assert _unfenced("{ if (k) { mbar_wait_warp(b); } else { mbar_wait_warp(c); tc_fence_after(); tc_ld32(x); }\n tc_ld32(x); }") == [2]
+
+
+def test_key_masks_are_handed_on_by_arrivals_of_threads():
+    """Ragged grids: the key masks are plain stores of the K producer.  Its arrival on k_full releases them to the issuer of
+    S; the arrival of a tcgen05.commit reports MMAs and nothing else, so the issuer has to arrive on s_full itself."""
+    src = re.sub(r"//[^\n]*", "", _source("attn_tc.cu"))
+    store, full = src.index("masks[(gk %"), src.index("request(j, &P.tm_k")
+    assert store < full and "__syncwarp()" in src[store:full]
+    issue = src[src.index("mbar_wait_warp(bar_k_full(slot)"):src.index("tc_commit(bar_s_full(wg))")]
+    assert "if (kRagged) mbar_arrive_elect(bar_s_full(wg));" in issue
+    assert "mbar_init(bar_s_full(b), kRagged ? 2 : 1);" in src
