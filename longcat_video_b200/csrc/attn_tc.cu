@@ -740,20 +740,22 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             if (!ok) break;
             tc_fence_after();
             const float2 oth = ml[(wg ^ 1) * 128 + ml_idx];
-            // merged scale of both partial sums: everything relative to the larger reference maximum
-            const float m_all = fmaxf(m_ref, oth.x);
-            const float w_mine = l_sum > 0.f ? ex2(m_ref - m_all) : 0.f;
-            const float w_oth = oth.y > 0.f ? ex2(oth.x - m_all) : 0.f;
+            // merged scale of both partial sums: everything relative to the larger reference maximum.  A row with a NaN or an
+            // infinite score has a NaN sum and comes out as NaN, like on the warp-level kernel; a warpgroup that saw no block has
+            // the maximum -inf, hence the weight 0.
+            const float m_all = fmaxf(m_ref, oth.x), m_base = m_all == -INFINITY ? 0.f : m_all;
+            const float w_mine = ex2(m_ref - m_base), w_oth = ex2(oth.x - m_base);
             const float l_all = l_sum * w_mine + oth.y * w_oth;
-            const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
+            const float inv = l_all == 0.f ? 0.f : 1.f / l_all;
             const float f_mine = w_mine * inv, f_oth = w_oth * inv;
             // This warpgroup merges and stages half of the columns of O (input dtype, 128B-swizzled rows of 64 columns) in the V slot that the item's last PV has just released.
             const unsigned last = gb - 1;
             unsigned char* o_half = smem + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes + (kD == 128 ? wg * kHalfBytes : 0);
             constexpr int kMine = kD / 2;  // columns kMine * wg ..
-            // a warpgroup that saw no block has weight 0; its accumulator holds garbage and is not used
-            const bool rd_mine = __any_sync(0xffffffffu, w_mine > 0.f), rd_oth = __any_sync(0xffffffffu, w_oth > 0.f);
-            const bool both = __all_sync(0xffffffffu, w_mine > 0.f && w_oth > 0.f);  // the usual case: no lane has to be masked
+            // the accumulator of a warpgroup that saw no block holds garbage and is not used
+            const bool saw_mine = my_cnt > wg, saw_oth = my_cnt > (wg ^ 1);
+            const bool rd_mine = __any_sync(0xffffffffu, saw_mine), rd_oth = __any_sync(0xffffffffu, saw_oth);
+            const bool both = __all_sync(0xffffffffu, saw_mine && saw_oth);  // the usual case: no lane has to be masked
             const float2 fm2 = make_float2(f_mine, f_mine), fo2 = make_float2(f_oth, f_oth);
 #pragma unroll
             for (int cch = 0; cch < kMine / 32; ++cch) {
@@ -764,8 +766,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                 if (LCBSA_UNLIKELY(!both)) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
-                        if (!(w_mine > 0.f)) oa[j] = 0u;
-                        if (!(w_oth > 0.f)) ob[j] = 0u;
+                        if (!saw_mine) oa[j] = 0u;
+                        if (!saw_oth) ob[j] = 0u;
                     }
                 }
                 if (tile_valid) {

@@ -652,40 +652,39 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                 ok = mbar_wait_warp(bar_o_free, (wk - 1) & 1, ctl, 102 + wg, wk);
                 if (!ok) break;
             }
-            ml[wg * 128 + ml_idx] = make_float2(m_ref, l_sum);
+            const float m_pub = first ? -INFINITY : m_ref;  // no key seen: m_ref is a placeholder
+            ml[wg * 128 + ml_idx] = make_float2(m_pub, l_sum);
             __syncwarp();
             mbar_arrive_elect(bar_ml_ready);
             ok = mbar_wait_warp(bar_ml_ready, wk & 1, ctl, 104 + wg, wk);
             if (!ok) break;
             tc_fence_after();
             const float2 oth = ml[(wg ^ 1) * 128 + ml_idx];
-            // merged scale of both partial sums: everything relative to the larger reference maximum
-            const float m_all = fmaxf(l_sum > 0.f ? m_ref : -INFINITY, oth.y > 0.f ? oth.x : -INFINITY);  // a side that saw no key has no maximum
-            const float w_mine = l_sum > 0.f ? ex2(m_ref - m_all) : 0.f;
-            const float w_oth = oth.y > 0.f ? ex2(oth.x - m_all) : 0.f;
+            // merged scale of both partial sums: everything relative to the larger reference maximum.  A row with a NaN or an
+            // infinite score has a NaN sum and comes out as NaN, like on the warp-level kernel; a side that saw no key has the
+            // maximum -inf, hence the weight 0.
+            const float m_all = fmaxf(m_pub, oth.x), m_base = m_all == -INFINITY ? 0.f : m_all;
+            const float w_mine = ex2(m_pub - m_base), w_oth = ex2(oth.x - m_base);
             const float l_all = l_sum * w_mine + oth.y * w_oth;
-            const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
+            const float inv = l_all == 0.f ? 0.f : 1.f / l_all;
             const float f_mine = w_mine * inv, f_oth = w_oth * inv;
             // This warpgroup merges and stages columns 64*wg .. 64*wg+63 of O (input dtype, one 128B-swizzled
             // half-tile row per thread) in the V slot that its own last PV has just released: the last two units of
             // the item sit in slots s0 (warpgroup 0) and s0 + 1 (warpgroup 1), s0 even.
             unsigned char* o_half = smem + kOffV + ((gb - 2) % kVSlots + wg) * kSlotBytes;
-            // a warpgroup that saw no block has weight 0; its accumulator holds garbage and is not used
-            const bool rd_mine = __any_sync(0xffffffffu, w_mine > 0.f), rd_oth = __any_sync(0xffffffffu, w_oth > 0.f);
-            const bool both = __all_sync(0xffffffffu, w_mine > 0.f && w_oth > 0.f);  // the usual case: no lane has to be masked
+            const bool saw = n_act > 0;  // an empty list: the accumulators hold garbage and are not used
             const float2 fm2 = make_float2(f_mine, f_mine), fo2 = make_float2(f_oth, f_oth);
 #pragma unroll
             for (int cch = 0; cch < 2; ++cch) {
                 uint32_t oa[32], ob[32];
-                if (rd_mine) tc_ld32(tm_o_mine + 64 * wg + 32 * cch, oa);
-                if (rd_oth) tc_ld32(tm_o_other + 64 * wg + 32 * cch, ob);
+                if (saw) {
+                    tc_ld32(tm_o_mine + 64 * wg + 32 * cch, oa);
+                    tc_ld32(tm_o_other + 64 * wg + 32 * cch, ob);
+                }
                 tc_wait_ld();
-                if (LCBSA_UNLIKELY(!both)) {
+                if (LCBSA_UNLIKELY(!saw)) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        if (!(w_mine > 0.f)) oa[j] = 0u;
-                        if (!(w_oth > 0.f)) ob[j] = 0u;
-                    }
+                    for (int j = 0; j < 32; ++j) oa[j] = ob[j] = 0u;
                 }
                 {
 #pragma unroll
