@@ -42,9 +42,9 @@
 // The MMAs are issued by whole converged warps with one elected lane (about 23 cycles per MMA for the
 // warp; a single lane inside a divergent branch needs 50 and more).
 //
-// The running maximum baked into O is only refreshed when the row maximum grows by more than 2^8
+// head_dim 128: the running maximum baked into O is only refreshed when the row maximum grows by more than 2^8
 // (the accumulated values stay finite and the result is unchanged after the final division), so O is
-// rarely rescaled in TMEM.
+// rarely rescaled in TMEM.  head_dim 64 takes every new maximum, for its precision (see the softmax loop).
 //
 // TMEM columns: O of warpgroup g at 128 * g (128 columns), its S at 256 + 64 * g, its P at 384 + 32 * g (two 16-bit
 // values per column), Q at 448 (64 columns of 16-bit pairs); the second tile of the pair 16 lanes up in each.
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                             }
                         }
                     }
-                    // One pass: the probabilities are computed against the current reference maximum while the row maximum is
+                    // head_dim 128, one pass: the probabilities are computed against the current reference maximum while the row maximum is
                     // tracked beside them (one basic block, so that the comparisons run under the exponentials); only if the
                     // maximum has moved by more than 2^8 is the pass repeated with the new reference.  The warpgroup's first
                     // block takes its own maximum as the reference.
@@ -642,7 +642,18 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                         return fmaxf(max3(max3(mx8[0], mx8[1], mx8[2]), mx8[3], mx8[4]), max3(mx8[5], mx8[6], mx8[7])) * P.scale2;
                     };
                     float rs = 0.f;
-                    if (kRagged) {
+                    if constexpr (kD == 64) {
+                        // The reference is the running maximum itself, as in the warp-level kernel that served head_dim 64 before:
+                        // the largest probability of a row, which carries most of its weight, is then exactly 1 and not rounded
+                        // to the input type.  With a reference that lags the error against float64 was 5 to 12 % larger.
+                        const float m_new = fmaxf(m_ref, row_max());
+                        if (!first && m_new > m_ref) {
+                            need = true;
+                            alpha = ex2(m_ref - m_new);
+                        }
+                        m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+                        probs(m_ref, rs);
+                    } else if (kRagged) {
                         // the instantiation with the masking code: a single copy of the pass in the instruction stream.  The loop
                         // body runs once in the common case (pass, then the row maximum, which confirms the reference) and twice
                         // when the reference moves; for the warpgroup's first block the first pass is skipped.
@@ -695,7 +706,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                     }
                     tc_st32(tm_p, pr);
                 }
-                if (LCBSA_UNLIKELY(any_need)) tc_scale_row<kD>(tm_o_mine, alpha);  // rare: only when a row maximum jumps
+                // head_dim 128: rare, only when a row maximum jumps
+                if (kD == 64 ? any_need : LCBSA_UNLIKELY(any_need)) tc_scale_row<kD>(tm_o_mine, alpha);
                 if (i + 2 < n_iter) {
                     // The next round's S is on its way into the registers while P is being stored: it has usually been ready
                     // for some hundred cycles, since it only waits for this round's S to be in registers.

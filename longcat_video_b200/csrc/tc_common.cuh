@@ -244,8 +244,9 @@ __device__ __forceinline__ uint32_t pack2(bool bf16, float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Rare path of the online softmax, as a rolled loop so that it takes little room in the instruction stream of the loop:
-// multiply this thread's row of a kCols-column fp32 accumulator in TMEM by alpha.  Warp-collective.
+// Multiply this thread's row of a kCols-column fp32 accumulator in TMEM by alpha.  Warp-collective.  A rolled loop: at head_dim
+// 128 it is the rare path of the online softmax and should take little room in the instruction stream of the loop; at
+// head_dim 64, where most rounds come here, an unrolled one costs 11 spilled registers.
 template <int kCols>
 __device__ __forceinline__ void tc_scale_row(uint32_t taddr, float alpha) {
     tc_fence_after();

@@ -1,0 +1,50 @@
+"""head_dim 64: precision against float64, which kernel a call takes, and the calls that stay on the warp-level kernel."""
+import pytest
+import torch
+
+from longcat_video_b200 import _lib as L
+from longcat_video_b200.block_sparse_attention import bsa_interface as B
+from longcat_video_b200.synthetic import Workload, make_qkv
+from oracle import bsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense(q, k, v, gq, gk, chunk, idx, cnt):
+    """float64 softmax over the keys of every list, on the device."""
+    tq, tk = O.token_map(gq, chunk).cuda(), O.token_map(gk, chunk).cuda()
+    out = torch.zeros(q.shape, dtype=torch.float64, device="cuda")
+    for b in range(q.shape[0]):
+        for h in range(q.shape[1]):
+            for n in range(tq.shape[0]):
+                rows = tq[n][tq[n] >= 0]
+                keys = tk[idx[b, h, n, : int(cnt[b, h, n])].long()].flatten()
+                keys = keys[keys >= 0]
+                s = (q[b, h, rows].double() @ k[b, h, keys].double().T) * q.shape[-1] ** -0.5
+                out[b, h, rows] = torch.softmax(s, -1) @ v[b, h, keys].double()
+    return out
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", ["normal", "scaled_lowrank"])
+@pytest.mark.parametrize("gq,gk,chunk,sparsity", [
+    ((12, 16, 24), (12, 16, 24), (4, 4, 4), 0.75),
+    ((4, 16, 16), (8, 16, 16), (4, 4, 4), 0.5),
+    ((8, 15, 22), (8, 15, 22), (2, 4, 8), 0.875),
+    ((8, 16, 24), (8, 16, 24), (4, 4, 4), 0.96875),
+])
+def test_no_further_from_float64_than_the_warp_level_kernel(gq, gk, chunk, sparsity, kind, dtype):
+    """Both round P to the input type; where a row's largest probability is exactly 1 its rounding does not count, so the
+    reference has to be the running maximum.  The errors are norms over 130 000 elements and more, whose spread is
+    1 / sqrt(2 n) < 0.2 %: 1 % is allowed for it."""
+    wl = Workload("d64", 9400, 1, 2, 64, gq, gk, chunk, sparsity, dtype, kind)
+    q, k, v = (t.cuda() for t in make_qkv(wl))
+    idx, cnt = B.get_select_indices(q, k, gq, gk, sparsity, None, chunk, chunk)
+    want = _dense(q, k, v, gq, gk, chunk, idx, cnt)
+    err = {}
+    for impl in (L.ATTN_AUTO, L.ATTN_MMA):
+        got = B.attn_fwd_bsa_varlen(q, k, v, 64 ** -0.5, idx, cnt, gq, gk, chunk, chunk, impl=impl).double()
+        err[impl] = float((got - want).norm() / want.norm())
+    L.check(L.lib().lcbsa_check_device_status())
+    print(f"D64 {gq} {sparsity} {kind} {dtype}: AUTO {err[L.ATTN_AUTO]:.4e} warp-level {err[L.ATTN_MMA]:.4e}")
+    assert err[L.ATTN_AUTO] <= 1.01 * err[L.ATTN_MMA]
