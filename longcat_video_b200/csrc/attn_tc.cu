@@ -69,6 +69,9 @@ constexpr int kBlk = 64;                    // tokens per query / key block
 constexpr int kHalfBytes = kBlk * 128;      // one 64-column half of a tile: 64 rows x 128 B, 128B-swizzled
 constexpr int kTilesPerWork = 2;            // the two query blocks of a pair
 constexpr int kThreads = 384;
+// Reference of a row whose blocks so far scored -inf throughout: finite, so that their probabilities are 0 and not NaN, and far
+// enough below every score that the first one above -inf replaces it.
+constexpr float kNoScore = -1e30f;
 // setmaxnreg per warpgroup: (208 + 208 + 88) * 128 threads <= the 64 K registers of the SM
 constexpr int kRegsSoftmax = 208, kRegsOther = 88;
 
@@ -651,7 +654,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                             need = true;
                             alpha = ex2(m_ref - m_new);
                         }
-                        m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+                        m_ref = fmaxf(m_new, kNoScore);
                         probs(m_ref, rs);
                     } else if (kRagged) {
                         // the instantiation with the masking code: a single copy of the pass in the instruction stream.  The loop
@@ -669,14 +672,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                                 need = true;
                                 alpha = ex2(m_ref - m_new);
                             }
-                            m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+                            m_ref = fmaxf(m_new, kNoScore);
                             decided = true;
                         }
                     } else {
                         float m_new = m_ref;
                         if (LCBSA_UNLIKELY(first)) {
                             m_new = fmaxf(m_ref, row_max());
-                            m_ref = (m_new == -INFINITY) ? 0.f : m_new;
+                            m_ref = fmaxf(m_new, kNoScore);
                         }
                         probs(m_ref, rs);
                         const float m_top = row_max();

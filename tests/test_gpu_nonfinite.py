@@ -51,7 +51,9 @@ def _dense(q, k, v, gq, gk, chunk, idx, cnt):
                 continue
             keys = torch.cat([_tokens(gk, chunk, int(j)) for j in idx[0, h, b, :n]])
             s = (q[0, h, rows].double() @ k[0, h, keys].double().T) * q.shape[-1] ** -0.5
-            out[0, h, rows] = torch.softmax(s, -1) @ v[0, h, keys].double()
+            p = torch.softmax(s, -1)
+            p[s.amax(-1) == float("-inf")] = 0.0  # no key at all: a row of zeros
+            out[0, h, rows] = p @ v[0, h, keys].double()
     return out
 
 
@@ -85,3 +87,16 @@ def test_nan_and_inf_reach_the_rows_they_belong_to(name, where):
         v[0, 0, 5, 3] = v[0, 1, -1, 4] = val
     want = _compare(q, k, v, gq, gk, chunk, idx, cnt, dt)
     assert not torch.isfinite(want).all() and torch.isfinite(want).any()
+
+
+@pytest.mark.parametrize("name", sorted(SHAPES))
+def test_blocks_of_minus_inf_scores_leave_no_reference(name):
+    """The first two blocks of every list score -inf throughout, the others far below zero: whatever stands in for the
+    missing maximum of the first two must not be taken for a score (the rest would underflow against it)."""
+    d, chunk, gq, gk, dt, q, k, v, idx, cnt = _case(name)
+    q[..., 0] = 1.0
+    k[..., 0] = -3000.0
+    for block in (0, 1):
+        k[:, :, _tokens(gk, chunk, block), 0] = float("-inf")
+    want = _compare(q, k, v, gq, gk, chunk, idx, cnt, dt)
+    assert torch.isfinite(want).all() and (want[0, 0] != 0).all()
