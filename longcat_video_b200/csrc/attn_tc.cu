@@ -848,6 +848,13 @@ int attn_sm_reserve() { return g_sm_reserve.load(); }
 bool attn_tc_supported(const AttnArgs& a, const char** why) {
     if (a.dtype != LCBSA_BF16 && a.dtype != LCBSA_FP16) { *why = "needs bf16 or fp16"; return false; }
     if (a.D != 128 && a.D != 64) { *why = "needs head_dim 64 or 128"; return false; }
+    if (a.D == 64 && a.sm_scale < 0.f) {
+        // The reference is the maximum of the raw scores times the scale, here the smallest scaled score of a block, and P grows
+        // with the range of the scores.  Two partial results with references of their own let an fp16 P overflow where the one
+        // of the warp-level kernel, which has always served head_dim 64 with such a scale, does not.
+        *why = "head_dim 64 needs a scale that is not negative";
+        return false;
+    }
     if (a.gq.bs != kBlk || a.gk.bs != kBlk) { *why = "needs 64-token query and key blocks"; return false; }
     if (a.gq.ct > 256 || a.gq.ch > 256 || a.gq.cw > 256 || a.gk.ct > 256 || a.gk.ch > 256 || a.gk.cw > 256) {
         *why = "block axis above the TMA box limit";

@@ -25,3 +25,19 @@ def rel_l2(a, b):
 
 def max_abs(a, b):
     return float((a.double() - b.double()).abs().max())
+
+
+def kernels_of_capture(fn):
+    """Mangled names of the kernels that ``fn`` launches, from the nodes of a graph captured around a second call."""
+    import re
+    import tempfile
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    with tempfile.TemporaryDirectory() as d:
+        path = os.path.join(d, "graph.dot")
+        graph.debug_dump(path)
+        with open(path) as f:
+            return re.findall(r"_Z\w+", f.read())

@@ -1,4 +1,8 @@
-"""head_dim 64: precision against float64, which kernel a call takes, and the calls that stay on the warp-level kernel."""
+"""head_dim 64: precision against float64, which kernel a call takes, and the calls that stay on the warp-level kernel.
+
+The kernel is read off the nodes of a captured graph: a forced ``ATTN_TC`` refuses head_dim 64, so the tcgen05 form is only
+reached by ``ATTN_AUTO``, and a comparison with ``ATTN_MMA`` alone would also pass if that chose the warp-level kernel.
+"""
 import pytest
 import torch
 
@@ -6,6 +10,7 @@ from longcat_video_b200 import _lib as L
 from longcat_video_b200.block_sparse_attention import bsa_interface as B
 from longcat_video_b200.synthetic import Workload, make_qkv
 from oracle import bsa_oracle as O
+from tests.helpers import kernels_of_capture
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +53,22 @@ def test_no_further_from_float64_than_the_warp_level_kernel(gq, gk, chunk, spars
     L.check(L.lib().lcbsa_check_device_status())
     print(f"D64 {gq} {sparsity} {kind} {dtype}: AUTO {err[L.ATTN_AUTO]:.4e} warp-level {err[L.ATTN_MMA]:.4e}")
     assert err[L.ATTN_AUTO] <= 1.01 * err[L.ATTN_MMA]
+
+
+def _call(gq, gk, chunk, dtype, d=64):
+    g = torch.Generator().manual_seed(0)
+    q, k, v = (torch.randn(1, 2, s[0] * s[1] * s[2], d, generator=g).to(dtype).cuda() for s in (gq, gk, gk))
+    nq, nk = O.num_blocks(gq, chunk), O.num_blocks(gk, chunk)
+    idx = torch.arange(nk, dtype=torch.int32).expand(1, 2, nq, nk).contiguous().cuda()
+    cnt = torch.full((1, 2, nq), nk, dtype=torch.int32).cuda()
+    return lambda impl, scale=d ** -0.5: B.attn_fwd_bsa_varlen(q, k, v, scale, idx, cnt, gq, gk, chunk, chunk, impl=impl)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_a_negative_scale_stays_on_the_warp_level_kernel(dtype):
+    """Bit for bit what the warp-level kernel gives, at scales where an fp16 P comes near its largest value."""
+    call = _call((4, 8, 8), (4, 8, 16), (4, 4, 4), dtype)
+    for scale in (-0.125, -0.25):
+        assert torch.equal(call(L.ATTN_AUTO, scale).view(torch.int16), call(L.ATTN_MMA, scale).view(torch.int16))
+    L.check(L.lib().lcbsa_check_device_status())
+    assert any("attn_mma_kernel" in k for k in kernels_of_capture(lambda: call(L.ATTN_AUTO, -0.125)))
