@@ -157,6 +157,20 @@ cudaError_t launch_topk(const uint16_t* keys, long long rows, int Nq, int Nk, in
     return cudaGetLastError();
 }
 
+// The narrowest register row that holds nk_pad keys, in steps of 128 keys: the work of a count is proportional to the words a
+// lane keeps, and with two words a step no row counts more than one word of padding.  Rows above 64 * kRegWords keys are
+// counted where they lie.
+template <int NW>
+cudaError_t launch_topk_for(const uint16_t* keys, long long rows, int Nq, int Nk, int nk_pad, const SelectSplit* split, int nsel, int cap, int32_t* idx,
+                            int32_t* cnt, cudaStream_t st) {
+    if constexpr (NW <= kRegWords) {
+        if (nk_pad <= 64 * NW) return launch_topk<NW>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
+        return launch_topk_for<NW + 2>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
+    } else {
+        return launch_topk<0>(keys, rows, Nq, Nk, nk_pad, nullptr, nsel, cap, idx, cnt, st);
+    }
+}
+
 template <typename T, int D>
 cudaError_t launch_gemm(const void* qc, const void* kc, int BH, int Nq, int Nk, int nk_pad, uint16_t* keys, cudaStream_t st) {
     dim3 grid((nk_pad + kTile - 1) / kTile, (Nq + kTile - 1) / kTile, BH);
@@ -205,17 +219,11 @@ cudaError_t launch_score_gemm_topk(int dtype, const void* qc, const void* kc, in
         e = D == 128 ? launch_gemm<__half, 128>(qc, kc, BH, Nq, Nk, nk_pad, keys, st) : launch_gemm<__half, 64>(qc, kc, BH, Nq, Nk, nk_pad, keys, st);
     if (e != cudaSuccess) return e;
     const long long rows = (long long)BH * Nq;
-    // the smallest register row that holds nk_pad keys: the work of a count is proportional to it
-    const int words = nk_pad / 64;
-    if (words <= 4) return launch_topk<4>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
-    if (words <= 10) return launch_topk<10>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
-    if (words <= 16) return launch_topk<16>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
-    if (words <= kRegWords) return launch_topk<kRegWords>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
-    if (split != nullptr) {
+    if (split != nullptr && nk_pad > 64 * kRegWords) {
         *why = "the split selection handles up to 1536 key blocks";
         return cudaErrorInvalidValue;
     }
-    return launch_topk<0>(keys, rows, Nq, Nk, nk_pad, nullptr, nsel, cap, idx, cnt, st);
+    return launch_topk_for<2>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
 }
 
 }  // namespace lcbsa

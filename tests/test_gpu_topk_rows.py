@@ -8,7 +8,7 @@ from oracle import bsa_oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nk", [1, 63, 64, 65, 255, 256, 257, 640, 641, 1024, 1025, 1536, 1537])
+@pytest.mark.parametrize("nk", [1, 63, 64, 65, 255] + [n + i for n in range(128, 1537, 128) for i in (0, 1)])
 @pytest.mark.parametrize("distinct", [3, 4000])
 def test_topk_row_lengths(nk, distinct):
     """Both sides of every row length at which the top-k kernel changes, with rows full of ties and rows with few."""
