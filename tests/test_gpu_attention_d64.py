@@ -10,7 +10,9 @@ from longcat_video_b200 import _lib as L
 from longcat_video_b200.block_sparse_attention import bsa_interface as B
 from longcat_video_b200.synthetic import Workload, make_qkv
 from oracle import bsa_oracle as O
-from tests.helpers import kernels_of_capture
+from tests.golden.cases import CASES
+from tests.helpers import kernels_of_capture, load_golden, rel_l2
+from tests.test_gpu_attention_items import LONG, SHAPES
 
 pytestmark = pytest.mark.gpu
 
@@ -72,3 +74,41 @@ def test_a_negative_scale_stays_on_the_warp_level_kernel(dtype):
         assert torch.equal(call(L.ATTN_AUTO, scale).view(torch.int16), call(L.ATTN_MMA, scale).view(torch.int16))
     L.check(L.lib().lcbsa_check_device_status())
     assert any("attn_mma_kernel" in k for k in kernels_of_capture(lambda: call(L.ATTN_AUTO, -0.125)))
+
+
+FORMS = {n: c for n, c in {**SHAPES, **LONG}.items() if c[2] == 64}
+
+
+@pytest.mark.parametrize("name", sorted(FORMS))
+def test_64_token_blocks_take_the_tcgen05_kernel(name):
+    """The shapes that the head_dim 64 tests of this kernel use reach it: dtype, ragged form and head_dim of the instantiation."""
+    b, h, d, gq, gk, chunk, dt = FORMS[name]
+    ragged = any(n % c for n, c in zip(gk, chunk))
+    names = kernels_of_capture(lambda c=_call(gq, gk, chunk, dt, d): c(L.ATTN_AUTO))
+    want = f"attn_tc_kernelILb{int(dt == torch.bfloat16)}ELb{int(ragged)}ELi64E"
+    assert any(want in k for k in names) and not any("attn_mma_kernel" in k for k in names), names
+
+
+def test_128_token_blocks_stay_on_the_warp_level_kernel():
+    names = kernels_of_capture(lambda c=_call((4, 8, 16), (4, 8, 16), (4, 4, 8), torch.bfloat16): c(L.ATTN_AUTO))
+    assert any("attn_mma_kernel" in k for k in names) and not any("attn_tc" in k for k in names), names
+
+
+def test_golden_case_on_the_kernel_that_serves_it():
+    """Lists and result of the reference's own functions at head_dim 64 (fixture fp16_d64), through the dispatch of a user's call."""
+    wl, _ = CASES["fp16_d64"]
+    gold = load_golden("fp16_d64")
+    q, k, v = make_qkv(wl)
+    idx = torch.sort(torch.from_numpy(gold["idx"].astype("int32")), dim=-1).values.contiguous().cuda()
+    cnt = torch.from_numpy(gold["lens"].astype("int32")).cuda()
+    ref = torch.from_numpy(gold["attn"])
+    q, k, v = q.cuda(), k.cuda(), v.cuda()
+
+    def call():
+        return B.attn_fwd_bsa_varlen(q, k, v, wl.head_dim ** -0.5, idx, cnt, wl.grid_q, wl.grid_k, wl.chunk, wl.chunk)
+
+    names = kernels_of_capture(call)
+    assert any("attn_tc_kernel" in n for n in names), names
+    out = call().float().cpu()
+    L.check(L.lib().lcbsa_check_device_status())
+    assert rel_l2(out, ref) <= 1.3e-3  # fp16: P is rounded to 2^-12 relative

@@ -1,8 +1,10 @@
 """The tcgen05 forward kernels where their work items are at their smallest and most uneven, and at head_dim 64.
 
 A CTA walks over many items, prefetches the next one and stores an item's output behind its back, so the lists here mix
-lengths from zero to the whole grid and there are several items per CTA.  Tolerance against the fp32 oracle: rel-L2 <=
-1e-2 in bf16 and 1.3e-3 in fp16 (P is rounded to the input type, 2^-9 and 2^-12 relative, before the second contraction).
+lengths from zero to the whole grid; the calls on fewer SMs give every CTA four of them.  Tolerance against the fp32
+oracle: rel-L2 <= 1e-2 in bf16 and 1.3e-3 in fp16 (P is rounded to the input type, 2^-9 and 2^-12 relative, before the
+second contraction).  Log-sum-exp of two kernels: 1e-3 absolute; a score is an fp32 sum of up to 128 products of unit
+variance, at most 128 * 2^-24 * 128 * 0.09 = 1e-4 off whatever the order, and the sums of the probabilities add less.
 """
 import pytest
 import torch
@@ -24,7 +26,7 @@ SHAPES = {
     "d64_fp16_batch2": (2, 2, 64, (8, 8, 8), (8, 8, 8), (4, 4, 4), torch.float16),
     "d64_fp16_ragged": (1, 2, 64, (5, 7, 9), (6, 7, 10), (4, 4, 4), torch.float16),
     "d64_block248": (1, 2, 64, (4, 8, 16), (4, 8, 16), (2, 4, 8), torch.bfloat16),
-    "d64_items": (1, 12, 64, (8, 16, 24), (4, 8, 8), (4, 4, 4), torch.bfloat16),        # 288 items: two or more per CTA
+    "d64_items": (1, 12, 64, (8, 16, 24), (4, 8, 8), (4, 4, 4), torch.bfloat16),        # 288 items: two for most CTAs
     "d128_items": (1, 12, 128, (8, 16, 24), (4, 8, 8), (4, 4, 4), torch.bfloat16),
     "d128_items_ragged": (1, 10, 128, (8, 15, 23), (4, 7, 9), (4, 4, 4), torch.bfloat16),
     "blocks128_items": (1, 14, 128, (8, 16, 24), (4, 8, 16), (4, 4, 8), torch.bfloat16),  # 336 items of one block
@@ -32,11 +34,43 @@ SHAPES = {
 }
 
 
+# 336 items (84 CTAs below), key grids of 56 and more blocks (128-token blocks: 36): lists that span several windows of sixteen (128-token blocks: thirty-two) entries, and
+# rings of K, V and, on ragged grids, key masks that turn over several times within an item.
+LONG = {
+    "long_d64_bf16": (1, 14, 64, (8, 16, 24), (8, 16, 28), (4, 4, 4), torch.bfloat16),
+    "long_d64_fp16": (2, 7, 64, (8, 16, 24), (8, 16, 32), (4, 4, 4), torch.float16),
+    "long_d64_ragged_bf16": (1, 14, 64, (8, 15, 23), (8, 15, 27), (4, 4, 4), torch.bfloat16),
+    "long_d64_ragged_fp16": (1, 14, 64, (7, 11, 30), (7, 15, 27), (2, 4, 8), torch.float16),
+    "long_d128": (1, 14, 128, (8, 16, 24), (8, 16, 28), (4, 4, 4), torch.bfloat16),
+    "long_d128_ragged": (1, 14, 128, (8, 15, 23), (8, 15, 27), (4, 4, 4), torch.float16),
+    "long_blocks128": (1, 14, 128, (8, 16, 24), (8, 24, 24), (4, 4, 8), torch.bfloat16),
+    "long_blocks128_ragged": (1, 14, 128, (8, 16, 23), (8, 23, 23), (4, 4, 8), torch.float16),
+}
+
+
+@pytest.fixture
+def fewer_sms():
+    """The persistent kernels leave as many SMs idle as the library allows: 84 CTAs on a B200."""
+    old = L.lib().lcbsa_set_attn_sm_reserve(64)
+    assert old >= 0
+    yield
+    assert L.lib().lcbsa_set_attn_sm_reserve(old) == 64
+
+
+@pytest.mark.parametrize("name", sorted(LONG))
+def test_many_items_per_cta_and_long_lists(name, fewer_sms):
+    _check_uneven(name, 9300 + sorted(LONG).index(name), LONG[name], "mixed")
+
+
 @pytest.mark.parametrize("lists", ["short", "mixed"])
 @pytest.mark.parametrize("name", sorted(SHAPES))
 def test_uneven_lists(name, lists):
-    b, h, d, gq, gk, chunk, dt = SHAPES[name]
-    wl = Workload(name, 9100 + sorted(SHAPES).index(name), b, h, d, gq, gk, chunk, 0.5, dt, "normal")
+    _check_uneven(name, 9100 + sorted(SHAPES).index(name), SHAPES[name], lists)
+
+
+def _check_uneven(name, seed, shape, lists):
+    b, h, d, gq, gk, chunk, dt = shape
+    wl = Workload(name, seed, b, h, d, gq, gk, chunk, 0.5, dt, "normal")
     q, k, v = make_qkv(wl)
     nq, nk = O.num_blocks(gq, chunk), O.num_blocks(gk, chunk)
     gen = torch.Generator().manual_seed(wl.seed)
@@ -61,19 +95,34 @@ def test_uneven_lists(name, lists):
     assert rel_l2(out.float(), other.float()) <= TOL[dt]
 
 
-@pytest.mark.parametrize("d", [64, 128])
-def test_growing_maximum_rescales(d):
-    """Key blocks whose scores grow by far more than 2^8 from one to the next: every round moves the reference maximum."""
-    gq, gk, chunk = (4, 8, 8), (4, 16, 16), (4, 4, 4)
+# growth of the scores from one block to the next, as a multiple of what moves the reference between two rounds of a warpgroup
+@pytest.mark.parametrize("steep", [1, 4])
+@pytest.mark.parametrize("gk", [(4, 16, 16), (4, 15, 15)], ids=["whole", "ragged"])
+@pytest.mark.parametrize("d,chunk", [(64, (4, 4, 4)), (128, (4, 4, 4)), (128, (4, 4, 8))], ids=["d64", "d128", "blocks128"])
+def test_growing_maximum_rescales(d, chunk, gk, steep):
+    """Key blocks whose scores grow by more than 2^8 from one round of a warpgroup to its next: every round moves the reference
+    maximum and rescales what has been accumulated.  One coordinate carries the growth (a step per block that bf16 holds
+    exactly), the others carry scores of a quarter of the usual spread."""
+    gq = (4, 8, 8)
     wl = Workload("grow", 9200 + d, 1, 2, d, gq, gk, chunk, 0.0, torch.bfloat16, "normal")
     q, k, v = make_qkv(wl)
     nq, nk = O.num_blocks(gq, chunk), O.num_blocks(gk, chunk)
-    q = q.abs()
+    bs = chunk[0] * chunk[1] * chunk[2]
+    # a warpgroup takes every second block of 64 tokens, and one of the two halves of every block of 128
+    per_round = 2 if bs == 64 else 1
+    step = {64: 28.0, 128: 36.0}[d] * (2 // per_round) * steep  # 5.0 and 4.6 (2^...) per block of 64 tokens
+    tm = O.token_map(gk, chunk).long()
     order = torch.empty(gk[0] * gk[1] * gk[2])
-    order[O.token_map(gk, chunk).long().flatten()] = torch.arange(nk).repeat_interleave(64).float()
-    k = (k.abs() * 0.2 * (1.0 + order)[None, None, :, None]).to(k.dtype)
+    order[tm[tm >= 0]] = torch.arange(nk).repeat_interleave(bs)[tm.flatten() >= 0].float()
+    q, k = (0.25 * q).to(q.dtype), k.clone()
+    q[..., 0] = 1.0
+    k[..., 0] = (step * order).to(k.dtype)
+    log2_scores = torch.einsum("bhqd,bhkd->bhqk", q.float(), k.float()) * d ** -0.5 * 1.4427
+    top = torch.stack([log2_scores[..., order == n].amax(-1) for n in range(nk)], -1)
+    assert float((top[..., per_round:] - top[..., :-per_round]).min()) > 8.0
     idx = torch.arange(nk, dtype=torch.int32).expand(1, 2, nq, nk).contiguous()
     cnt = torch.full((1, 2, nq), nk, dtype=torch.int32)
     ref, _ = O.attention(q, k, v, gq, gk, chunk, chunk, idx, cnt)
     out = B.attn_fwd_bsa_varlen(q.cuda(), k.cuda(), v.cuda(), 1 / d ** 0.5, idx.cuda(), cnt.cuda(), gq, gk, chunk, chunk, impl=TC[d])
+    L.check(L.lib().lcbsa_check_device_status())
     assert rel_l2(out.float().cpu(), ref) <= TOL[torch.bfloat16]
