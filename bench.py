@@ -46,15 +46,14 @@ from longcat_video_b200.synthetic import WORKLOADS, make_qkv  # noqa: E402
 METRIC = "bsa_fwd_effective_tflops"
 UNIT = "TFLOP/s"
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
-# dram__bytes_read.sum + dram__bytes_write.sum of one attn_tc_kernel launch over the bytes of q, k, v and out, from
-# the ncu capture summarised in profiles/attn_tc_kernel_480p_16heads.md (454.0 MB read + 150.7 MB written against
-# 654.3 MB).  K and V of a head are re-read from L2, so the traffic of a launch grows with the tensors, not with the
-# selected blocks.
-NCU_ATTN_DRAM_PER_IO_BYTE = (454.0 + 150.7) / 654.3
-# the same for the block-select stage at 720p / 32 heads (profiles/select_kernels_720p_32heads.md): the pool launch
-# reads q and k once (1524 MB read, 65 MB written against 1415.6 MB of q and k), the score launch adds 23.6 + 76 MB
-# and the top-k launch 135.7 + 8.6 MB (its 16-bit keys no longer fit in L2 at this size).
-NCU_SELECT_DRAM_PER_IO_BYTE = (1524.0 + 65.0 + 23.6 + 76.0 + 135.7 + 8.6) / 1415.6
+# dram__bytes_read.sum + dram__bytes_write.sum of one attention launch over the bytes of q, k, v and out, by tokens per
+# block, from the ncu capture summarised in profiles/forward_kernels_counters.md (16 heads; MB read + MB written).  K and V
+# of a head are re-read from L2, so the traffic of a launch grows with the tensors, not with the selected blocks.
+NCU_ATTN_DRAM_PER_IO_BYTE = {64: (493.2 + 148.1) / 654.3, 128: (530.0 + 162.3) / 704.6}
+# the same for the block-select stage at 720p / 32 heads (same capture): the pool launch reads q and k once (1524 MB read,
+# 65.5 MB written against 1415.6 MB of q and k), the score launch adds 23.6 + 76.5 MB and the top-k launch 135.7 + 8.7 MB
+# (its 16-bit keys no longer fit in L2 at this size).
+NCU_SELECT_DRAM_PER_IO_BYTE = (1524.1 + 65.5 + 23.6 + 76.5 + 135.7 + 8.7) / 1415.6
 
 def load_peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
@@ -336,8 +335,8 @@ def main():
                 "frac_of_sustained_peak": attn_tf / peaks["bf16_tflops_sustained"],
                 "peak_source": f"{peak_src} (burst cuBLAS bf16); sustained {peaks['bf16_tflops_sustained']}",
                 "ms_per_launch": ms_attn,
-                "traffic": NCU_ATTN_DRAM_PER_IO_BYTE * attn_io_bytes,
-                "traffic_source": "ncu capture of 480p_legal/16 heads scaled by the bytes of q,k,v,out"}
+                "traffic": NCU_ATTN_DRAM_PER_IO_BYTE[128 if block_tokens == 128 else 64] * attn_io_bytes,
+                "traffic_source": "ncu capture of the kernel at a 480p grid/16 heads scaled by the bytes of q,k,v,out"}
     sel_gbs = select_bytes / ms_select / 1e6
     roofline_select = {"bound": "hbm", "kernel": "pool_kernel + score_gemm_kernel + topk_rows_kernel", "achieved": sel_gbs, "peak": peaks["hbm_gbs"],
                        "unit": "GB/s", "frac": sel_gbs / peaks["hbm_gbs"], "peak_source": peak_src, "ms_per_stage": ms_select,

@@ -38,7 +38,7 @@ enum { LCBSA_BF16 = 0, LCBSA_FP16 = 1, LCBSA_FP32 = 2 };
 /* Which attention kernel lcbsa_attn_fwd runs. */
 enum {
     LCBSA_ATTN_AUTO = 0, /* tcgen05 kernel when the shape allows it, otherwise the generic one */
-    LCBSA_ATTN_TC = 1,   /* TMA + tcgen05 + TMEM kernels at head_dim 128 (AUTO also takes the one for 64-token blocks at 64) */
+    LCBSA_ATTN_TC = 1,   /* TMA + tcgen05 + TMEM kernels at head_dim 128 (AUTO also takes the one for 64-token blocks at 64, sm_scale >= 0) */
     LCBSA_ATTN_MMA = 2   /* generic warp-level MMA kernel (other block sizes / head dims) */
 };
 
@@ -176,6 +176,7 @@ int lcbsa_block_select(const LcbsaTensor* q, const LcbsaTensor* k, const LcbsaGr
  *      kernel reads zeros for it; either way the device status is flagged (lcbsa_check_device_status returns
  *      LCBSA_EDEVICE naming the entry) and the rows of that query block are finite but unspecified.
  * out: [B, H, Sq, D], dtype of q.   lse: nullable, fp32 dense [B*H, Sq], natural log.
+ *      A row with an empty list is 0, its lse -inf.  A row with a NaN or +inf score is NaN, its lse -inf too.
  * impl: LCBSA_ATTN_*.
  */
 int lcbsa_attn_fwd(const LcbsaTensor* q, const LcbsaTensor* k, const LcbsaTensor* v, const LcbsaGrid* gq,

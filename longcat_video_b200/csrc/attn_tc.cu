@@ -7,7 +7,7 @@
 //
 // Shape handled: head_dim 128 or 64, query and key blocks of 64 tokens, bf16 or fp16.  The figures below are those of
 // head_dim 128; at 64 a tile is one 64-column half, the rings have six slots, an S is half as many MMAs and a P V half as wide
-// (2 x 16 heads of a 12x16x24 grid in fp16, 18 of 72 blocks: 114 us, 248 us on the warp-level kernel that served it before).
+// (2 x 16 heads of a 12x16x24 grid in fp16, 18 of 72 blocks: 120 us, 255 us on the warp-level kernel that served it before).
 //
 // One persistent CTA per SM.  A work item is a pair of consecutive query blocks of one head.  Each
 // query block is a 64-row tile, i.e. an M=64 tcgen05 MMA whose accumulator occupies 16 lanes of every
@@ -34,10 +34,10 @@
 // its own, and the copies are issued by one elected lane of the converged warp: one warp for both rings, issuing from a
 // divergent branch, needed about 950 cycles per ring slot and was what the rest waited for (V was requested 1700 cycles
 // after its P was ready).
-// What bounds it: M=64 MMAs, 16 x 32 + 8 x 64 = 1030 cycles of tensor pipe per block of a pair (an M=64 tile occupies the
-// pipe like an M=128 one); inside an item a block takes about 1040 cycles.  An item boundary costs some 10 000 more (the
-// softmax warps merge and store O before they take up the next item).  Attention launch, 480p grid, 32 heads, 39 of 624
-// blocks: 2.25 ms with one producer warp and P over S, 1.96 ms now.
+// What bounds it: M=64 MMAs, 16 x 32 + 8 x 64 = 1024 cycles of tensor pipe per block of a pair (an M=64 tile occupies the
+// pipe like an M=128 one); inside an item a block takes 1025 to 1040 cycles.  An item boundary costs some 8000 more, last PV
+// to first PV (the softmax warps merge and store O before they take up the next item).  Attention launch, 480p grid, 32
+// heads, 39 of 624 blocks: 2.25 ms with one producer warp and P over S, 1.91 ms now.
 //
 // The MMAs are issued by whole converged warps with one elected lane (about 23 cycles per MMA for the
 // warp; a single lane inside a divergent branch needs 50 and more).
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                     np = mbar_test(bar_p_full(wg ^ 1), (wg ? rr0 : rr1) & 1);
                 }
                 tc_fence_after();
-                // A: P in TMEM (first 32 columns of the S buffer), 8 columns per 16-key step; the second tile of
+                // A: P in the warpgroup's 32 P columns, 8 columns per 16-key step; the second tile of
                 // the pair sits 16 lanes up, like its accumulators.
                 // B: V tile, MN-major: 64-column halves 8 KiB apart (LBO), 8-key groups 1 KiB apart (SBO).
 #pragma unroll

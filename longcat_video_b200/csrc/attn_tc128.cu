@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                     np = mbar_test(bar_p_full(wg ^ 1), (wg ? rr0 : rr1) & 1);
                 }
                 tc_fence_after();
-                // A: P in TMEM (first 32 columns of the S buffer), 8 columns per 16-key step.
+                // A: P in the warpgroup's 32 P columns, 8 columns per 16-key step.
                 // B: V tile, MN-major: 64-column halves 8 KiB apart (LBO), 8-key groups 1 KiB apart (SBO).
                 if (i < n_act) {
                     const uint32_t pa = tmem + kTmP + 32u * wg;

@@ -63,7 +63,6 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 
 // Branches that are rarely taken and whose code should not sit in the instruction stream of a hot loop.
 #define LCBSA_UNLIKELY(x) __builtin_expect(!!(x), 0)
-#define LCBSA_LIKELY(x) __builtin_expect(!!(x), 1)
 
 struct Ctl {
     volatile int* abort;    // shared flag
