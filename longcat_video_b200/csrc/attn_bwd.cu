@@ -774,7 +774,8 @@ BwdLayout bwd_layout(long long BH, const Geom& gq, const Geom& gk, int cap) {
     l.toff = off;   off += up((size_t)BH * (Nk + 1) * sizeof(int32_t));
     l.tidx = off;   off += up((size_t)BH * Nq * capu * sizeof(int32_t));
     l.bitmap = off; off += up((size_t)BH * Nk * ((Nq + 31) / 32) * sizeof(uint32_t));
-    l.stats = off;  off += up((size_t)BH * Sq * 2 * sizeof(float));
+    // one pair per slot of every block: on a ragged grid more slots than tokens
+    l.stats = off;  off += up((size_t)BH * gq.nblk * gq.bs * 2 * sizeof(float));
     const size_t rewritten = Uq * Uk > 1 ? 1 : 0;  // 64-token blocks on both sides: the lists are used as they are
     l.idx_u = off;  off += up(rewritten * BH * Nq * capu * sizeof(int32_t));
     l.cnt_u = off;  off += up(rewritten * BH * Nq * sizeof(int32_t));

@@ -532,7 +532,7 @@ bool attn_bwd_tc_supported(const BwdArgs& a, const BwdTcPlan& p) {
 }
 
 // a.delta, the lists of the plan and (for the dK/dV pass) their transposition are ready on the stream; a.stats is scratch
-// of B*H*Sq*2 floats
+// of two floats per slot of every query block (B*H*Sq*2 floats on whole grids, more on ragged ones)
 cudaError_t launch_attn_bwd_tc(const BwdArgs& a, const BwdTcPlan& p, cudaStream_t st, const char** why) {
     const long long Sq = (long long)a.gq.T * a.gq.H * a.gq.W;
     const long long BH = (long long)a.B * a.H;
