@@ -27,19 +27,25 @@
 //
 //   warps 0-7 : arithmetic.  A thread serves one TMEM lane = one row of the kM x 64 tile (an M=128 accumulator has row r in
 //               lane r, an M=64 one occupies lanes 0-15 of every 32-lane quadrant)
-//   warp 8    : TMA producer: the CTA's own tiles once, then a ring of five (four for kM = 128) (B1, B2) slots; in the
-//               dK/dV pass also the query block's 64 (lse * log2 e) and 64 delta values per slot, by a bulk copy onto the
-//               same barrier (bwd_stats_kernel lays them out per block)
-//   warp 9    : issues every MMA, one elected lane
+//   warps 8, 11 : TMA producers of B1 and of B2 into a ring of five (four for kM = 128) slots; warp 8 also brings the CTA's
+//               own tiles once, and in the dK/dV pass the query block's 64 (lse * log2 e) and 64 delta values per slot, by a
+//               bulk copy onto the same barrier (bwd_stats_kernel lays them out, negated, per block)
+//   warp 9    : issues S and dP (SS)    warp 10 : issues the gradient MMAs (TS); one elected lane each
 //
 // TMEM and the order of the MMAs.  P and dS (16-bit pairs) have columns of their own, twice, in both passes: the values
-// of entry s + 2 go where those of entry s were and are written after s_full(s + 2), a commit the issuer makes behind
-// TS(s), so no buffer is rewritten while an MMA may still read it.
+// of entry s + 2 go where those of entry s were, once TS(s) has read them (ts_done).
 //   dQ pass (448 columns): S and dP have two buffers; warps 0-3 take the even entries, warps 4-7 the odd ones.
-//       SS(0) SS(1) | TS(0) SS(2) | TS(1) SS(3) | ...        TS(s) after x_full(s), which also frees S/dP of entry s
 //   dK/dV pass (512 columns, two accumulators): S^T and dP^T have ONE buffer; all eight warps work on every entry (warps
-//       0-3 columns 0-31, warps 4-7 columns 32-63) and release the buffer as soon as they hold it in registers (s_free).
-//       SS(0) | SS(1) TS(0) | SS(2) TS(1) | ...               SS(s+1) after s_free(s),  TS(s) after x_full(s)
+//       0-3 columns 0-31, warps 4-7 columns 32-63).
+//   In both, SS of the entry that takes the buffer next waits until the arithmetic warps hold S and dP in registers
+//   (s_free), and TS(s) for x_full(s), the P and dS of entry s.
+// The own tiles are moved to TMEM once, where they are the A operands of every S and dP (kM = 128, dK/dV pass: only K, TMEM is
+// full): an M=64 S with both operands in shared memory reads 128 bytes a cycle of it, all that it gives, beside the incoming
+// tiles.  At kM = 64 the second of two things sits in the lanes 16-31 that an M=64 tile leaves free (see Cols).
+// What bounds it: the tensor pipe, 512 + 256 cycles per entry in the dQ pass and 512 + 512 in the dK/dV pass whether M is 64 or
+// 128.  Measured per entry (in-kernel time stamps; 64-token blocks of the 480p grid, 128-token blocks of 24x32x56), before with
+// one issuer and one producer and both operands in shared memory, and now: dQ 1071 -> 948 and 1200 -> 958 cycles, dK/dV
+// 1336 -> 1165.  A CTA adds some 10000 cycles of its own before its first and behind its last entry.
 // Every mbarrier wait is bounded; when one runs out the CTA flags the status word, drains its copies, frees TMEM, returns.
 #include <cstdlib>
 #include <cstring>
@@ -69,30 +75,51 @@ template <int kM> struct Lay {
     static constexpr int slots = kM == 64 ? 5 : 4;   // ring of (B1, B2) tile pairs
     static constexpr int offA = 0;
     static constexpr int offB = offA + 2 * aTile;
-    static constexpr int offStats = offB + slots * kSlotBytes;  // per slot: lse2[64], delta[64] of the streamed query block
+    static constexpr int offStats = offB + slots * kSlotBytes;  // per slot: -lse2[64], -delta[64] of the streamed query block
     static constexpr int offBar = offStats + slots * kStatsBytes;
-    // barriers: a_full, full[slots], empty[slots], s_full[2], s_free, x_full[2], acc_done
-    static constexpr int numBars = 1 + 2 * slots + 2 + 1 + 2 + 1;
+    // barriers: a_full, full[slots], empty[slots], s_full[2], s_free[2], x_full[2], ts_done[2], acc_done, at_full
+    static constexpr int numBars = 1 + 2 * slots + 8 + 2;
     static constexpr int offMisc = offBar + numBars * 8;  // abort flag, TMEM base
     static constexpr int smem = offMisc + 64;
 };
 
-// TMEM columns.  dQ pass: dQ 0..127, S[buf] 128 + 128 buf, dP[buf] 192 + 128 buf, dS[buf] 384 + 32 buf.
-// dK/dV pass: dK 0..127, dV 128..255, S^T 256..319, dP^T 320..383, P^T[buf] 384 + 64 buf, dS^T[buf] 416 + 64 buf.
-template <int kMode> struct Cols;
-template <> struct Cols<0> {
-    static constexpr uint32_t acc1 = 0, acc2 = 0;
-    __device__ static __forceinline__ uint32_t s(int buf) { return 128u + 128u * buf; }
-    __device__ static __forceinline__ uint32_t dp(int buf) { return 192u + 128u * buf; }
-    __device__ static __forceinline__ uint32_t xp(int buf) { return 384u + 32u * buf; }  // unused in this pass
-    __device__ static __forceinline__ uint32_t xd(int buf) { return 384u + 32u * buf; }
+// Where things are in TMEM: column plus (lane offset << 16).  own1, own2: the CTA's own tiles as 16-bit pairs (64 columns);
+// s, dp: fp32, 64 columns; xp, xd: P and dS as 16-bit pairs, 32 columns; acc1, acc2: fp32, 128 columns.  sbufs: buffers of S, xbufs: of P
+// and dS; split: both warpgroups work on every entry (half the columns each) instead of on every other one.
+//
+// An M=64 tile takes lanes 0-15 of every 32-lane quadrant, so at kM = 64 two things share their columns: S and dP, P and dS, dV and
+// dK, A1 and A2, the second of each 16 lanes up (the A operand and the result of an MMA are always in the same lanes).
+constexpr uint32_t kUp = 16u << 16;
+template <int kMode, int kM> struct Cols;
+template <int kMode> struct Cols<kMode, 64> {
+    static constexpr uint32_t acc2 = 0, acc1 = kMode == 0 ? 0 : kUp;
+    static constexpr uint32_t own1 = 320, own2 = 320 + kUp;
+    static constexpr int sbufs = 2, xbufs = 2;
+    static constexpr bool split = false;
+    __device__ static __forceinline__ uint32_t s(int buf) { return 128u + 64u * buf; }
+    __device__ static __forceinline__ uint32_t dp(int buf) { return 128u + 64u * buf + kUp; }
+    __device__ static __forceinline__ uint32_t xp(int buf) { return 256u + 32u * buf; }
+    __device__ static __forceinline__ uint32_t xd(int buf) { return 256u + 32u * buf + (kMode == 0 ? 0u : kUp); }
 };
-template <> struct Cols<1> {
-    static constexpr uint32_t acc1 = 0, acc2 = 128;
+// kM = 128, dQ pass: dQ 0, S 128 and 192, dP 256 (one buffer), dS 320 and 352, Q 384, dO 448
+template <> struct Cols<0, 128> {
+    static constexpr uint32_t acc1 = 0, acc2 = 0, own1 = 384, own2 = 448;
+    static constexpr int sbufs = 2, xbufs = 2;
+    static constexpr bool split = false;
+    __device__ static __forceinline__ uint32_t s(int buf) { return 128u + 64u * buf; }
+    __device__ static __forceinline__ uint32_t dp(int) { return 256u; }
+    __device__ static __forceinline__ uint32_t xp(int) { return 0u; }  // unused in this pass
+    __device__ static __forceinline__ uint32_t xd(int buf) { return 320u + 32u * buf; }
+};
+// kM = 128, dK/dV pass: dK 0, dV 128, S^T 256, dP^T 320, P^T 384, dS^T 416 (one buffer each), K 448; V stays in shared memory
+template <> struct Cols<1, 128> {
+    static constexpr uint32_t acc1 = 0, acc2 = 128, own1 = 448, own2 = 0;
+    static constexpr int sbufs = 1, xbufs = 1;
+    static constexpr bool split = true;
     __device__ static __forceinline__ uint32_t s(int) { return 256u; }
     __device__ static __forceinline__ uint32_t dp(int) { return 320u; }
-    __device__ static __forceinline__ uint32_t xp(int buf) { return 384u + 64u * buf; }
-    __device__ static __forceinline__ uint32_t xd(int buf) { return 416u + 64u * buf; }
+    __device__ static __forceinline__ uint32_t xp(int) { return 384u; }
+    __device__ static __forceinline__ uint32_t xd(int) { return 416u; }
 };
 
 struct BwdTcParams {
@@ -101,7 +128,7 @@ struct BwdTcParams {
     const int32_t* cnt;    // dQ pass: [BH][n_own]
     const int32_t* toff;   // dK/dV pass: [BH][n_own + 1]
     long long list_stride;
-    const float* stats;    // dK/dV pass: [BH][n_stream][2][64] of the streamed 64-token query blocks
+    const float* stats;    // dK/dV pass: [BH][n_stream][2][64] of the streamed 64-token query blocks: -lse * log2(e), -delta
     const float* lse;      // dQ pass: [BH][Sq] natural log, of the own rows
     const float* delta;    // dQ pass: [BH][Sq]
     long long Sq;
@@ -115,19 +142,17 @@ struct BwdTcParams {
     float scale, scale2;   // sm_scale, sm_scale * log2(e)
 };
 
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
-                 "r"(bytes), "r"(bar)
-                 : "memory");
+// called by a whole converged warp with warp-uniform operands, like the _elect copies of tc_common.cuh
+__device__ __forceinline__ void bulk_load_elect(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}"
+        ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+        : "memory");
 }
 
-// the two 64-column boxes of one [64 tokens x 128] tile
-__device__ __forceinline__ void load_tile_pair(uint32_t dst, const CUtensorMap* tm, uint32_t bar, const Coord& c) {
-    tma_load_5d(dst, tm, bar, 0, c.c1, c.c2, c.c3, c.c4);
-    tma_load_5d(dst + kHalfBytes, tm, bar, 64, c.c1, c.c2, c.c3, c.c4);
-}
-
-// lse * log2(e) and delta of every query row, laid out per 64-token block in slot order, so that a block's 128 values are
+// -lse * log2(e) and -delta of every query row, laid out per 64-token block in slot order, so that a block's 128 values are
 // one contiguous 512-byte piece.  Slots of a partial block that lie outside the grid get zeros (their q and dO rows are
 // zero-filled by TMA, so every term they enter is a finite number times zero).
 __global__ void __launch_bounds__(256) bwd_stats_kernel(const float* lse, const float* delta, Geom g, long long Sq, long long total,
@@ -145,8 +170,8 @@ __global__ void __launch_bounds__(256) bwd_stats_kernel(const float* lse, const 
     const bool inside = tt < g.T && hh < g.H && ww < g.W;
     const long long tok = ((long long)tt * g.H + hh) * g.W + ww;
     float* dst = stats + (bh * g.nblk + blk) * kStatsFloats;
-    dst[r] = inside ? lse[bh * Sq + tok] * 1.4426950408889634f : 0.f;
-    dst[kBlk + r] = inside ? delta[bh * Sq + tok] : 0.f;
+    dst[r] = inside ? -(lse[bh * Sq + tok] * 1.4426950408889634f) : 0.f;
+    dst[kBlk + r] = inside ? -delta[bh * Sq + tok] : 0.f;
 }
 
 // 32 columns of this thread's accumulator row -> 64 bytes of the row in global memory (input dtype)
@@ -166,7 +191,7 @@ __device__ __forceinline__ void store_row32(unsigned char* row_ptr, int col0, co
 // kMode 0: dQ pass, 1: dK/dV pass.  Grid: (blocks of the CTA's own grid, batch * heads).
 template <bool kBf16, int kMode, int kM>
 __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_constant__ BwdTcParams P) {
-    using C = Cols<kMode>;
+    using C = Cols<kMode, kM>;
     using Ly = Lay<kM>;
     constexpr int kSlots = Ly::slots, kOffA = Ly::offA, kOffB = Ly::offB, kOffStats = Ly::offStats, kOffBar = Ly::offBar, kOffMisc = Ly::offMisc;
     constexpr int kATile = Ly::aTile, kAHalf = Ly::aHalf;
@@ -176,10 +201,16 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
     const uint32_t bar_a_full = bar0;
     auto bar_full = [&](int s) { return bar0 + 8u * (1 + s); };
     auto bar_empty = [&](int s) { return bar0 + 8u * (1 + kSlots + s); };
-    auto bar_s_full = [&](int buf) { return bar0 + 8u * (1 + 2 * kSlots + (kMode == 0 ? buf : 0)); };
-    const uint32_t bar_s_free = bar0 + 8u * (3 + 2 * kSlots);
-    auto bar_x_full = [&](int buf) { return bar0 + 8u * (4 + 2 * kSlots + buf); };
-    const uint32_t bar_acc_done = bar0 + 8u * (6 + 2 * kSlots);
+    // entry s: S and dP in buffer s % kSBufs, P and dS in buffer s % kXBufs
+    constexpr int kB = 1 + 2 * kSlots, kSBufs = C::sbufs, kXBufs = C::xbufs;
+    constexpr bool kSplit = C::split;
+    constexpr bool kOneDp = kM == 128 && kMode == 0;  // two buffers of S, one of dP
+    constexpr bool kOwn2Smem = kM == 128 && kMode == 1;  // A2 is read from shared memory
+    auto bar_s_full = [&](int sbuf) { return bar0 + 8u * (kB + sbuf); };
+    auto bar_s_free = [&](int sbuf) { return bar0 + 8u * (kB + 2 + sbuf); };
+    auto bar_x_full = [&](int buf) { return bar0 + 8u * (kB + 4 + buf); };
+    auto bar_ts_done = [&](int buf) { return bar0 + 8u * (kB + 6 + buf); };
+    const uint32_t bar_acc_done = bar0 + 8u * (kB + 8), bar_at_full = bar0 + 8u * (kB + 9);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kOffMisc);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffMisc + 8);
     const Ctl ctl{abort_flag, P.status};
@@ -205,15 +236,17 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
         *abort_flag = 0;
         mbar_init(bar_a_full, 1);
         for (int s = 0; s < kSlots; ++s) {
-            mbar_init(bar_full(s), 1);
+            mbar_init(bar_full(s), 2);  // one arrival per producer
             mbar_init(bar_empty(s), 1);
         }
-        mbar_init(bar0 + 8u * (1 + 2 * kSlots), 1);  // s_full[0], s_full[1]
-        mbar_init(bar0 + 8u * (2 + 2 * kSlots), 1);
-        mbar_init(bar_s_free, 8);  // one elected arrival per arithmetic warp
-        mbar_init(bar_x_full(0), kMode == 0 ? 4 : 8);  // the warps that work on an entry
-        mbar_init(bar_x_full(1), kMode == 0 ? 4 : 8);
+        for (int buf = 0; buf < 2; ++buf) {
+            mbar_init(bar_s_full(buf), 1);
+            mbar_init(bar_s_free(buf), kSplit ? 8 : 4);  // one elected arrival per warp that works on an entry
+            mbar_init(bar_x_full(buf), kSplit ? 8 : 4);
+            mbar_init(bar_ts_done(buf), 1);
+        }
         mbar_init(bar_acc_done, 1);
+        mbar_init(bar_at_full, 8);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // the tiles are 128B-swizzled, which ties their layout to address bits 7-9: refuse to run on an unaligned base
         if (sbase & 1023u) {
@@ -237,93 +270,128 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
 
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-        if (warp == 8 && n > 0) {
-            // ================================================================== TMA producer
-            if (lane == 0) {
+        if ((warp == 8 || warp == 11) && n > 0) {
+            // ================================================================== TMA producers: warp 8 B1, the own tiles and the stats, warp 11 B2
+            const bool is_b1 = warp == 8;
+            const CUtensorMap* tm = is_b1 ? &P.tm_b1 : &P.tm_b2;
+            const int mrg = is_b1 ? P.merge_b1 : P.merge_b2;
+            const int c3 = mrg ? b * P.gb.T : 0, c4 = mrg ? h : b * P.heads + h;
+            // The list is fetched and decoded by the whole warp, 32 entries at a time and one window ahead: lane L holds entry
+            // 32 w + L as the block's first token packed t << 20 | h << 10 | w.
+            auto fetch = [&](int e) { return e < n ? list[e] : 0; };
+            auto decode = [&](int blk) {
+                // an entry outside the grid never becomes an address: the box is placed at w = W, wholly outside the map, and
+                // TMA fills the tiles with zeros (the list transposition has flagged the call)
+                if ((unsigned)blk >= (unsigned)P.gb.nblk) return P.gb.W;
+                int bt, bhh, bw;
+                block_coords(P.gb, blk, bt, bhh, bw);
+                return ((bt * P.gb.ct) << 20) | ((bhh * P.gb.ch) << 10) | (bw * P.gb.cw);
+            };
+            int blk = fetch(lane), blk_n = fetch(32 + lane);
+            if (is_b1) {
                 // one box of kM rows per 64-column half (the own grid's block is the box)
-                mbar_arrive_tx(bar_a_full, 2 * kATile);
-                const Coord c1 = block_coord(P.ga, own, b, h, P.heads, P.merge_a1, P.ga.T), c2 = block_coord(P.ga, own, b, h, P.heads, P.merge_a2, P.ga.T);
-                tma_load_5d(sbase + kOffA, &P.tm_a1, bar_a_full, 0, c1.c1, c1.c2, c1.c3, c1.c4);
-                tma_load_5d(sbase + kOffA + kAHalf, &P.tm_a1, bar_a_full, 64, c1.c1, c1.c2, c1.c3, c1.c4);
-                tma_load_5d(sbase + kOffA + kATile, &P.tm_a2, bar_a_full, 0, c2.c1, c2.c2, c2.c3, c2.c4);
-                tma_load_5d(sbase + kOffA + kATile + kAHalf, &P.tm_a2, bar_a_full, 64, c2.c1, c2.c2, c2.c3, c2.c4);
+                mbar_arrive_tx_elect(bar_a_full, 2 * kATile);
+                const Coord a1 = block_coord(P.ga, own, b, h, P.heads, P.merge_a1, P.ga.T), a2 = block_coord(P.ga, own, b, h, P.heads, P.merge_a2, P.ga.T);
+                tma_load_5d_elect(sbase + kOffA, &P.tm_a1, bar_a_full, 0, a1.c1, a1.c2, a1.c3, a1.c4);
+                tma_load_5d_elect(sbase + kOffA + kAHalf, &P.tm_a1, bar_a_full, 64, a1.c1, a1.c2, a1.c3, a1.c4);
+                tma_load_5d_elect(sbase + kOffA + kATile, &P.tm_a2, bar_a_full, 0, a2.c1, a2.c2, a2.c3, a2.c4);
+                tma_load_5d_elect(sbase + kOffA + kATile + kAHalf, &P.tm_a2, bar_a_full, 64, a2.c1, a2.c2, a2.c3, a2.c4);
             }
+            int pos = decode(blk);
             bool ok = true;
-            int win = 0, issued = 0;
+            int issued = 0;
             for (int s = 0; s < n; ++s) {
-                if ((s & 31) == 0) win = (s + lane < n) ? list[s + lane] : 0;
-                const int blk = __shfl_sync(0xffffffffu, win, s & 31);
                 const int slot = s % kSlots;
                 ok = mbar_wait_warp(bar_empty(slot), ((s / kSlots) & 1) ^ 1, ctl, 210 + kMode, s);
                 if (!ok) break;
                 ++issued;
-                if (lane == 0) {
-                    mbar_arrive_tx(bar_full(slot), 2 * kTileBytes + (kMode == 1 ? kStatsBytes : 0));
-                    Coord c1, c2;
-                    if ((unsigned)blk < (unsigned)P.gb.nblk) {
-                        c1 = block_coord(P.gb, blk, b, h, P.heads, P.merge_b1, P.gb.T);
-                        c2 = block_coord(P.gb, blk, b, h, P.heads, P.merge_b2, P.gb.T);
-                    } else {
-                        // an entry outside the grid never becomes an address: the box is placed at w = W, wholly outside
-                        // the map, and TMA fills the tiles with zeros (the list transposition has flagged the call)
-                        c1 = Coord{P.gb.W, 0, 0, 0};
-                        c2 = c1;
-                    }
-                    const uint32_t dst = sbase + kOffB + slot * kSlotBytes;
-                    load_tile_pair(dst, &P.tm_b1, bar_full(slot), c1);
-                    load_tile_pair(dst + kTileBytes, &P.tm_b2, bar_full(slot), c2);
-                    if (kMode == 1)  // transposed lists only hold blocks of the grid
-                        bulk_load(sbase + kOffStats + slot * kStatsBytes, P.stats + ((long long)bh * P.n_stream + blk) * kStatsFloats, kStatsBytes,
-                                  bar_full(slot));
+                const int pk = __shfl_sync(0xffffffffu, pos, s & 31);
+                const bool stats = kMode == 1 && is_b1;
+                mbar_arrive_tx_elect(bar_full(slot), kTileBytes + (stats ? kStatsBytes : 0));
+                const uint32_t dst = sbase + kOffB + slot * kSlotBytes + (is_b1 ? 0 : kTileBytes);
+                tma_load_5d_elect(dst, tm, bar_full(slot), 0, pk & 1023, (pk >> 10) & 1023, (pk >> 20) + c3, c4);
+                tma_load_5d_elect(dst + kHalfBytes, tm, bar_full(slot), 64, pk & 1023, (pk >> 10) & 1023, (pk >> 20) + c3, c4);
+                if (stats) {  // transposed lists only hold blocks of the grid
+                    const int bk = __shfl_sync(0xffffffffu, blk, s & 31);
+                    bulk_load_elect(sbase + kOffStats + slot * kStatsBytes, P.stats + ((long long)bh * P.n_stream + bk) * kStatsFloats, kStatsBytes,
+                                    bar_full(slot));
                 }
-                __syncwarp();
+                if ((s & 31) == 31) {
+                    blk = blk_n;
+                    pos = decode(blk);
+                    blk_n = fetch(s + 33 + lane);
+                }
             }
             if (!ok && lane == 0) {
                 // drain: give the copies this warp issued a bounded time to land before the CTA exits
                 const long long t0 = clock64();
-                while (!mbar_try(bar_a_full, 0) && clock64() - t0 < 40000000ll) {
+                while (is_b1 && !mbar_try(bar_a_full, 0) && clock64() - t0 < 40000000ll) {
                 }
                 for (int r = issued > kSlots ? issued - kSlots : 0; r < issued; ++r)
                     while (!mbar_try(bar_full(r % kSlots), (r / kSlots) & 1) && clock64() - t0 < 40000000ll) {
                     }
             }
         } else if (warp == 9 && n > 0) {
-            // ================================================================== MMA issuer
-            const uint32_t idesc_ss = instr_desc(kBf16, kM, 64, 0), idesc_ts = instr_desc(kBf16, kM, 128, 1);
-            const uint64_t a1d = smem_desc(sbase + kOffA, 16, 1024), a2d = smem_desc(sbase + kOffA + kATile, 16, 1024);
-            bool ok = mbar_wait_warp(bar_a_full, 0, ctl, 220 + kMode, 0);
-            // S (or S^T) and dP (or dP^T) of entry s
-            auto issue_ss = [&](int s) -> bool {
-                const int slot = s % kSlots, buf = s & 1;
-                if (!mbar_wait_warp(bar_full(slot), (s / kSlots) & 1, ctl, 222 + kMode, s)) return false;
-                // dK/dV pass: the arithmetic warps hold S^T and dP^T of entry s - 1 in registers.  (dQ pass: the buffer
-                // was entry s - 2's, whose x_full the issuer has seen before TS(s - 2).)
-                if (kMode == 1 && s > 0 && !mbar_wait_warp(bar_s_free, (s - 1) & 1, ctl, 226, s)) return false;
+            // ================================================================== issuer of S and dP (S^T and dP^T)
+            const uint32_t idesc_ss = instr_desc(kBf16, kM, 64, 0);
+            const uint64_t a2d = smem_desc(sbase + kOffA + kATile, 16, 1024);  // kOwn2Smem
+            bool ok = mbar_wait_warp(bar_at_full, 0, ctl, 220 + kMode, 0), pre = false;  // the own tiles are in TMEM
+            for (int s = 0; s < n && ok; ++s) {
+                const int slot = s % kSlots, sbuf = s % kSBufs;
+                if (!pre) {  // not already seen ready by the look-ahead of the entry before
+                    ok = mbar_wait_warp(bar_full(slot), (s / kSlots) & 1, ctl, 222 + kMode, s);
+                    // the arithmetic warps hold the buffer's last S and dP in registers (kOneDp: seen before the dP of entry s - 1)
+                    if (ok && !kOneDp) ok = mbar_wait_warp(bar_s_free(sbuf), ((s / kSBufs) & 1) ^ 1, ctl, 226, s);
+                    if (!ok) break;
+                }
+                bool nf = false, ns = kOneDp;  // look ahead: probe the next entry's barriers now, read the answer after the MMAs
+                if (s + 1 < n) {
+                    nf = mbar_test(bar_full((s + 1) % kSlots), ((s + 1) / kSlots) & 1);
+                    if (!kOneDp) ns = mbar_test(bar_s_free((s + 1) % kSBufs), (((s + 1) / kSBufs) & 1) ^ 1);
+                }
                 tc_fence_after();
                 const uint32_t tile = sbase + kOffB + slot * kSlotBytes;
                 const uint64_t b1d = smem_desc(tile, 16, 1024), b2d = smem_desc(tile + kTileBytes, 16, 1024);
 #pragma unroll
                 for (int j = 0; j < kD / 16; ++j) {
-                    // 32 bytes per 16-column step inside a 64-column half; the halves are kM x 128 B (own tile) and 8 KiB
-                    // (streamed tile) apart
-                    const uint64_t aoff = (uint64_t)(((j >> 2) * kAHalf + (j & 3) * 32) >> 4);
+                    // 32 bytes per 16-column step inside a 64-column half, the halves 8 KiB apart; 8 TMEM columns per step
                     const uint64_t off = (uint64_t)(((j >> 2) * kHalfBytes + (j & 3) * 32) >> 4);
-                    tc_mma(tmem + C::s(buf), a1d + aoff, b1d + off, idesc_ss, j > 0);
+                    tc_mma_ts(tmem + C::s(sbuf), tmem + C::own1 + 8u * j, b1d + off, idesc_ss, j > 0);
+                }
+                if (kOneDp && s > 0) {  // dP of the entry before is in registers
+                    ok = mbar_wait_warp(bar_s_free((s - 1) & 1), ((s - 1) >> 1) & 1, ctl, 227, s);
+                    if (!ok) break;
+                    tc_fence_after();
                 }
 #pragma unroll
                 for (int j = 0; j < kD / 16; ++j) {
-                    const uint64_t aoff = (uint64_t)(((j >> 2) * kAHalf + (j & 3) * 32) >> 4);
                     const uint64_t off = (uint64_t)(((j >> 2) * kHalfBytes + (j & 3) * 32) >> 4);
-                    tc_mma(tmem + C::dp(buf), a2d + aoff, b2d + off, idesc_ss, j > 0);
+                    const uint64_t aoff = (uint64_t)(((j >> 2) * kAHalf + (j & 3) * 32) >> 4);  // the halves of an own tile are kM x 128 B apart
+                    if (kOwn2Smem) tc_mma(tmem + C::dp(sbuf), a2d + aoff, b2d + off, idesc_ss, j > 0);
+                    else tc_mma_ts(tmem + C::dp(sbuf), tmem + C::own2 + 8u * j, b2d + off, idesc_ss, j > 0);
                 }
-                tc_commit(bar_s_full(buf));
-                return true;
-            };
-            // the gradient MMAs of entry e: A from TMEM (8 columns per 16-row step), B the streamed tile, MN-major
-            // (64-column halves 8 KiB apart = LBO, 8-row groups 1 KiB apart = SBO, 16 rows = 2 KiB per step)
-            auto issue_ts = [&](int e) -> bool {
-                const int slot = e % kSlots, buf = e & 1;
-                if (!mbar_wait_warp(bar_x_full(buf), (e >> 1) & 1, ctl, 224 + kMode, e)) return false;
+                tc_commit(bar_s_full(sbuf));
+                __syncwarp();
+                pre = __all_sync(0xffffffffu, nf && ns);
+            }
+        } else if (warp == 10 && n > 0) {
+            // ================================================================== issuer of the gradient MMAs: A from TMEM (8 columns
+            // per 16-row step), B the streamed tile, MN-major (64-column halves 8 KiB apart = LBO, 8-row groups 1 KiB apart =
+            // SBO, 16 rows = 2 KiB per step)
+            const uint32_t idesc_ts = instr_desc(kBf16, kM, 128, 1);
+            bool ok = true, pre = false;
+            for (int e = 0; e < n && ok; ++e) {
+                const int slot = e % kSlots, buf = e % kXBufs;
+                if (!pre) {
+                    ok = mbar_wait_warp(bar_full(slot), (e / kSlots) & 1, ctl, 228 + kMode, e);
+                    if (ok) ok = mbar_wait_warp(bar_x_full(buf), (e / kXBufs) & 1, ctl, 224 + kMode, e);
+                    if (!ok) break;
+                }
+                bool nf = false, nx = false;
+                if (e + 1 < n) {
+                    nf = mbar_test(bar_full((e + 1) % kSlots), ((e + 1) / kSlots) & 1);
+                    nx = mbar_test(bar_x_full((e + 1) % kXBufs), ((e + 1) / kXBufs) & 1);
+                }
                 tc_fence_after();
                 const uint32_t tile = sbase + kOffB + slot * kSlotBytes;
                 const uint64_t b1m = smem_desc(tile, kHalfBytes, 1024), b2m = smem_desc(tile + kTileBytes, kHalfBytes, 1024);
@@ -336,21 +404,10 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
                 for (int j = 0; j < kBlk / 16; ++j)  // dQ += dS K, or dK += dS^T Q
                     tc_mma_ts(tmem + C::acc1, tmem + C::xd(buf) + 8u * j, b1m + (uint64_t)((j * 2048) >> 4), idesc_ts, (e > 0 || j > 0) ? 1u : 0u);
                 tc_commit(bar_empty(slot));  // the streamed tiles are free once these MMAs have read them
+                tc_commit(bar_ts_done(buf)); // and so are P and dS
                 if (e == n - 1) tc_commit(bar_acc_done);
-                return true;
-            };
-            if (ok) ok = issue_ss(0);
-            if (kMode == 0) {
-                if (ok && n > 1) ok = issue_ss(1);
-                for (int i = 0; i < n && ok; ++i) {
-                    ok = issue_ts(i);
-                    if (ok && i + 2 < n) ok = issue_ss(i + 2);
-                }
-            } else {
-                for (int i = 0; i < n && ok; ++i) {
-                    if (i + 1 < n) ok = issue_ss(i + 1);
-                    if (ok) ok = issue_ts(i);
-                }
+                __syncwarp();
+                pre = __all_sync(0xffffffffu, nf && nx);
             }
         }
     } else {
@@ -374,65 +431,131 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
             row_inside = tt < P.ga.T && hh < P.ga.H && ww < P.ga.W;
             tok = ((long long)tt * P.ga.H + hh) * P.ga.W + ww;
         }
-        // dQ pass: this thread's query row has one lse and one delta for the whole list
-        float my_l2 = 0.f, my_dl = 0.f;
-        if (kMode == 0 && n > 0 && row_inside) {
-            my_l2 = P.lse[(long long)bh * P.Sq + tok] * 1.4426950408889634f;
-            my_dl = P.delta[(long long)bh * P.Sq + tok];
-        }
-        // 32 columns of S and dP -> 16 columns of P and of dS in the input dtype.  st4: the slot's lse and delta values
-        // of those 32 columns (dK/dV pass, where columns are query rows)
-        auto columns32 = [&](const uint32_t (&sr)[32], const uint32_t (&dr)[32], const float4* l4, const float4* d4, uint32_t* xp, uint32_t* xd) {
-#pragma unroll
-            for (int c4 = 0; c4 < 8; ++c4) {
-                float4 l2 = make_float4(my_l2, my_l2, my_l2, my_l2), dl = make_float4(my_dl, my_dl, my_dl, my_dl);
-                if (kMode == 1) {
-                    l2 = l4[c4];
-                    dl = d4[c4];
-                }
-                const float p0 = ex2(fmaf(__uint_as_float(sr[4 * c4 + 0]), P.scale2, -l2.x));
-                const float p1 = ex2(fmaf(__uint_as_float(sr[4 * c4 + 1]), P.scale2, -l2.y));
-                const float p2 = ex2(fmaf(__uint_as_float(sr[4 * c4 + 2]), P.scale2, -l2.z));
-                const float p3 = ex2(fmaf(__uint_as_float(sr[4 * c4 + 3]), P.scale2, -l2.w));
-                const float g0 = p0 * (__uint_as_float(dr[4 * c4 + 0]) - dl.x) * P.scale;
-                const float g1 = p1 * (__uint_as_float(dr[4 * c4 + 1]) - dl.y) * P.scale;
-                const float g2 = p2 * (__uint_as_float(dr[4 * c4 + 2]) - dl.z) * P.scale;
-                const float g3 = p3 * (__uint_as_float(dr[4 * c4 + 3]) - dl.w) * P.scale;
-                if (kMode == 1) {
-                    xp[2 * c4] = pack2(kBf16, p0, p1);
-                    xp[2 * c4 + 1] = pack2(kBf16, p2, p3);
-                }
-                xd[2 * c4] = pack2(kBf16, g0, g1);
-                xd[2 * c4 + 1] = pack2(kBf16, g2, g3);
-            }
-        };
         bool ok = true;
-        if (kMode == 0) {
+        // The own tiles go from shared memory to TMEM, where they are the A operands of every S and dP: with both operands in shared
+        // memory an M=64 S reads as many bytes of the own tile as of the streamed one.  A thread moves (half of) a row.
+        if (n > 0) {
+            ok = mbar_wait_warp(bar_a_full, 0, ctl, 228, 0);
+            if (ok) {
+                tc_fence_after();
+                const int arow = kM == 128 ? wq * 32 + lane : wq * 16 + (lane & 15);
+                // kM = 64: warpgroup g moves half g of A1 (lanes 0-15) and of A2 (lanes 16-31); kM = 128: A1 and A2, or half g of A1
+                const int tile = kM == 64 ? lane >> 4 : (kOwn2Smem ? 0 : wg);
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    if ((kM == 64 || kOwn2Smem) && half != wg) continue;
+                    const unsigned char* src = smem + kOffA + tile * kATile + half * kAHalf + arow * 128;
+                    uint32_t ar[32];
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 v = *reinterpret_cast<const uint4*>(src + ((c ^ (arow & 7)) << 4));
+                        ar[4 * c + 0] = v.x;
+                        ar[4 * c + 1] = v.y;
+                        ar[4 * c + 2] = v.z;
+                        ar[4 * c + 3] = v.w;
+                    }
+                    tc_st32(tmem + (kM == 128 && tile == 1 ? C::own2 : C::own1) + 32u * half + t_lane, ar);
+                }
+                tc_wait_st();
+                tc_fence_before();
+                mbar_arrive_elect(bar_at_full);
+            }
+        }
+        // Two columns of S and dP -> one 16-bit pair of P and one of dS, two columns per instruction where the machine has packed
+        // fp32 forms.  nl, nd: -lse * log2(e) and -delta.
+        const float2 sc2 = make_float2(P.scale2, P.scale2), sc = make_float2(P.scale, P.scale);
+        auto pair = [&](uint32_t s0, uint32_t s1, uint32_t d0, uint32_t d1, float2 nl, float2 nd, uint32_t& xp, uint32_t& xd) {
+            const float2 x = __ffma2_rn(make_float2(__uint_as_float(s0), __uint_as_float(s1)), sc2, nl);
+            const float2 p = make_float2(ex2(x.x), ex2(x.y));
+            const float2 t = __fadd2_rn(make_float2(__uint_as_float(d0), __uint_as_float(d1)), nd);
+            const float2 g = __fmul2_rn(__fmul2_rn(p, t), sc);
+            if (kMode == 1) xp = pack2(kBf16, p.x, p.y);
+            xd = pack2(kBf16, g.x, g.y);
+        };
+        // dQ pass: -lse * log2(e) and -delta of this thread's query rows, one pair for the whole list; rows outside the grid: 0
+        auto row_stats = [&](int r, float2& nl, float2& nd) {
+            nl = nd = make_float2(0.f, 0.f);
+            if (kMode != 0 || n <= 0) return;
+            int lt, lh, lw, bt, bhh, bw;
+            slot_coords(P.ga, r, lt, lh, lw);
+            block_coords(P.ga, own, bt, bhh, bw);
+            const int tt = bt * P.ga.ct + lt, hh = bhh * P.ga.ch + lh, ww = bw * P.ga.cw + lw;
+            if (tt >= P.ga.T || hh >= P.ga.H || ww >= P.ga.W) return;
+            const long long at = (long long)bh * P.Sq + ((long long)tt * P.ga.H + hh) * P.ga.W + ww;
+            const float l2 = -(P.lse[at] * 1.4426950408889634f), dl = -P.delta[at];
+            nl = make_float2(l2, l2);
+            nd = make_float2(dl, dl);
+        };
+        if constexpr (kM == 64) {
+            // A warp takes its quadrant's 16 rows with all lanes: rows lane / 4 and lane / 4 + 8, columns 8 k + 2 (lane % 4) + 0, 1.
+            float2 nl0, nd0, nl1, nd1;
+            row_stats(wq * 16 + (lane >> 2), nl0, nd0);
+            row_stats(wq * 16 + (lane >> 2) + 8, nl1, nd1);
+            unsigned r = 0;
+            for (int i = wg; i < n && ok; i += 2, ++r) {  // buffer i & 1 = wg
+                const int slot = i % kSlots;
+                // dK/dV pass: the slot's lse and delta values came with its tiles
+                if (kMode == 1) ok = mbar_wait_warp(bar_full(slot), (i / kSlots) & 1, ctl, 234 + wg, i);
+                if (ok) ok = mbar_wait_warp(bar_s_full(wg), r & 1, ctl, 230 + wg, i);
+                if (!ok) break;
+                tc_fence_after();
+                uint32_t xp[16], xd[16], sr[32], dr[32];
+                tc_ld_half64(tmem + C::s(wg) + t_lane, sr);
+                tc_ld_half64(tmem + C::dp(wg) + t_lane, dr);
+                tc_wait_ld();
+                tc_fence_before();
+                mbar_arrive_elect(bar_s_free(wg));  // S and dP may be overwritten by those of entry i + 2
+                const float2* st2 = reinterpret_cast<const float2*>(smem + kOffStats + slot * kStatsBytes) + (lane & 3);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    if (kMode == 1) {  // columns are query rows
+                        nl0 = nl1 = st2[4 * k];
+                        nd0 = nd1 = st2[4 * k + kBlk / 2];
+                    }
+                    pair(sr[4 * k], sr[4 * k + 1], dr[4 * k], dr[4 * k + 1], nl0, nd0, xp[2 * k], xd[2 * k]);
+                    pair(sr[4 * k + 2], sr[4 * k + 3], dr[4 * k + 2], dr[4 * k + 3], nl1, nd1, xp[2 * k + 1], xd[2 * k + 1]);
+                }
+                // TS of entry i - 2 has read the columns
+                ok = mbar_wait_warp(bar_ts_done(wg), (r & 1) ^ 1, ctl, 236 + wg, i);
+                if (!ok) break;
+                tc_fence_after();
+                if (kMode == 1) tc_st_half32(tmem + C::xp(wg) + t_lane, xp);
+                tc_st_half32(tmem + C::xd(wg) + t_lane, xd);
+                tc_wait_st();
+                tc_fence_before();
+                mbar_arrive_elect(bar_x_full(wg));
+            }
+        } else if constexpr (kMode == 0) {
+            float2 nl, nd;
+            row_stats(wq * 32 + lane, nl, nd);
             unsigned r = 0;
             for (int i = wg; i < n && ok; i += 2, ++r) {  // buffer i & 1 = wg
                 ok = mbar_wait_warp(bar_s_full(wg), r & 1, ctl, 230 + wg, i);
                 if (!ok) break;
                 tc_fence_after();
-                uint32_t xd[32];
+                uint32_t xp[1], xd[32], sr[64], dr[64];
+                tc_ld64(tmem + C::s(wg) + t_lane, sr);
+                tc_ld64(tmem + C::dp(wg) + t_lane, dr);
+                tc_wait_ld();
+                tc_fence_before();
+                mbar_arrive_elect(bar_s_free(wg));  // dP may be overwritten by that of entry i + 1, S by that of entry i + 2
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    uint32_t sr[32], dr[32];
-                    tc_ld32(tmem + C::s(wg) + 32u * half + t_lane, sr);
-                    tc_ld32(tmem + C::dp(wg) + 32u * half + t_lane, dr);
-                    tc_wait_ld();
-                    columns32(sr, dr, nullptr, nullptr, nullptr, xd + 16 * half);
-                }
+                for (int k = 0; k < 32; ++k) pair(sr[2 * k], sr[2 * k + 1], dr[2 * k], dr[2 * k + 1], nl, nd, xp[0], xd[k]);
+                // TS of entry i - 2 has read the columns
+                ok = mbar_wait_warp(bar_ts_done(wg), (r & 1) ^ 1, ctl, 236 + wg, i);
+                if (!ok) break;
+                tc_fence_after();
                 tc_st32(tmem + C::xd(wg) + t_lane, xd);
                 tc_wait_st();
                 tc_fence_before();
                 mbar_arrive_elect(bar_x_full(wg));
             }
         } else {
-            for (int i = 0; i < n && ok; ++i) {
-                const int slot = i % kSlots, buf = i & 1;
-                ok = mbar_wait_warp(bar_s_full(0), i & 1, ctl, 232 + wg, i);
-                // the slot's lse and delta values came with its tiles (a completed phase answers at once)
-                if (ok) ok = mbar_wait_warp(bar_full(slot), (i / kSlots) & 1, ctl, 234 + wg, i);
+            for (int i = 0; i < n && ok; ++i) {  // columns 32 wg .. 32 wg + 31 of every entry
+                const int slot = i % kSlots;
+                // the slot's lse and delta values came with its tiles
+                ok = mbar_wait_warp(bar_full(slot), (i / kSlots) & 1, ctl, 234 + wg, i);
+                if (ok) ok = mbar_wait_warp(bar_s_full(0), i & 1, ctl, 232 + wg, i);
                 if (!ok) break;
                 tc_fence_after();
                 uint32_t sr[32], dr[32];
@@ -440,33 +563,38 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
                 tc_ld32(tmem + C::dp(0) + 32u * wg + t_lane, dr);
                 tc_wait_ld();
                 tc_fence_before();
-                mbar_arrive_elect(bar_s_free);  // S^T and dP^T may be overwritten by the next entry's
-                const float4* st4 = reinterpret_cast<const float4*>(smem + kOffStats + slot * kStatsBytes);
+                mbar_arrive_elect(bar_s_free(0));  // S^T and dP^T may be overwritten by the next entry's
+                const float2* st2 = reinterpret_cast<const float2*>(smem + kOffStats + slot * kStatsBytes) + 16 * wg;
                 uint32_t xp[16], xd[16];
-                columns32(sr, dr, st4 + wg * 8, st4 + 16 + wg * 8, xp, xd);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) pair(sr[2 * k], sr[2 * k + 1], dr[2 * k], dr[2 * k + 1], st2[k], st2[k + kBlk / 2], xp[k], xd[k]);
+                // TS of entry i - 1 has read the columns
+                ok = mbar_wait_warp(bar_ts_done(0), (i & 1) ^ 1, ctl, 236 + wg, i);
+                if (!ok) break;
+                tc_fence_after();
                 // 32 columns of the tile are 16 columns of 16-bit pairs
-                tc_st16(tmem + C::xp(buf) + 16u * wg + t_lane, xp);
-                tc_st16(tmem + C::xd(buf) + 16u * wg + t_lane, xd);
+                tc_st16(tmem + C::xp(0) + 16u * wg + t_lane, xp);
+                tc_st16(tmem + C::xd(0) + 16u * wg + t_lane, xd);
                 tc_wait_st();
                 tc_fence_before();
-                mbar_arrive_elect(bar_x_full(buf));
+                mbar_arrive_elect(bar_x_full(0));
             }
         }
 
         // ---- the accumulated gradients of the CTA's 64 rows: TMEM -> registers -> global memory (rows in T,H,W order)
         if (n >= 0) {
-            if (n > 0 && ok) {
-                ok = mbar_wait_warp(bar_acc_done, 0, ctl, 240 + kMode, n);
-                tc_fence_after();
-            }
+            if (n > 0 && ok) ok = mbar_wait_warp(bar_acc_done, 0, ctl, 240 + kMode, n);
             if (ok) {
-                // dQ pass: warpgroup g stores columns 64 g .. 64 g + 63 of dQ; dK/dV pass: warpgroup 0 stores dK, 1 dV
-                const bool second = kMode == 1 && wg == 1;
+                tc_fence_after();
+                // Warpgroup g stores columns 64 g .. 64 g + 63 of dQ, or (kM = 64) of dV from lanes 0-15 and of dK from lanes 16-31;
+                // dK/dV pass with kM = 128: warpgroup 0 stores dK, 1 dV.
+                const bool whole = kMode == 1 && kM == 128;
+                const bool second = kMode == 1 && (kM == 128 ? wg == 1 : lane < 16);
                 unsigned char* base = static_cast<unsigned char*>(second ? P.out2 : P.out1);
                 const long long sb = second ? P.o2_sb : P.o1_sb, sh = second ? P.o2_sh : P.o1_sh, ss = second ? P.o2_ss : P.o1_ss;
                 unsigned char* row_ptr = base + ((long long)b * sb + (long long)h * sh + tok * ss) * 2;
-                const uint32_t t_acc = tmem + (second ? C::acc2 : C::acc1) + t_lane;
-                const int col_lo = kMode == 0 ? 64 * wg : 0, n_chunks = kMode == 0 ? 2 : 4;
+                const uint32_t t_acc = tmem + (whole && second ? C::acc2 : 0u) + t_lane;
+                const int col_lo = whole ? 0 : 64 * wg, n_chunks = whole ? 4 : 2;
 #pragma unroll 1
                 for (int ch = 0; ch < n_chunks; ++ch) {
                     uint32_t acc[32];
@@ -477,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
 #pragma unroll
                         for (int j = 0; j < 32; ++j) acc[j] = 0u;  // nothing selected this block: its gradient is zero
                     }
-                    if ((kM == 128 || lane < 16) && row_inside) store_row32<kBf16>(row_ptr, col_lo + 32 * ch, acc);
+                    if ((kM == 128 || kMode == 1 || lane < 16) && row_inside) store_row32<kBf16>(row_ptr, col_lo + 32 * ch, acc);
                 }
             }
         }
