@@ -288,6 +288,22 @@ int lcbsa_norm_rope_ex(const LcbsaTensor* x, const void* weight, const LcbsaGrid
                        float eps, const LcbsaTensor* out, void* stream);
 
 /*
+ * Up to eight such tensors in one launch: everything a layer does to the rows of its q, k and v before the attention
+ * (attention.py:113-121 and 156-171).  They share dtype, batch, heads, head_dim and eps; a batch or head stride may be 0.  Per job
+ * the rules of lcbsa_norm_rope_ex, and: weight == NULL and rope_tab == NULL copies the rows (v into or behind a cache);
+ * out_norm.data != NULL also keeps the normalised rows from before the embedding, which is what return_kv caches
+ * (attention.py:118-119).  Outputs overlap neither each other nor another job's input.
+ */
+typedef struct LcbsaRowJob {
+    LcbsaTensor x, out, out_norm;
+    const void* weight;
+    const float* rope_tab;
+    LcbsaGrid grid;
+    int32_t table_T, t_offset;
+} LcbsaRowJob;
+int lcbsa_norm_rope_jobs(const LcbsaRowJob* jobs, int n_jobs, float eps, void* stream);
+
+/*
  * Enqueue `count` device-to-device copies of `nbytes` each on `stream`: dst[i] <- src[i], one cudaMemcpyAsync per
  * slab, so the copy engines move them; a destination may be another GPU's memory mapped into this process
  * (symmetric memory, CUDA IPC).  The pointer arrays are host memory and are read before the call returns.

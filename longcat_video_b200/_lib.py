@@ -43,6 +43,11 @@ class LcbsaSplit(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int32) for n in ("hw_q", "period_q", "split_q", "hw_k", "period_k", "split_k", "nsel_first")]
 
 
+class LcbsaRowJob(ctypes.Structure):
+    _fields_ = [("x", LcbsaTensor), ("out", LcbsaTensor), ("out_norm", LcbsaTensor), ("weight", ctypes.c_void_p), ("rope_tab", ctypes.c_void_p),
+                ("grid", LcbsaGrid), ("table_T", ctypes.c_int32), ("t_offset", ctypes.c_int32)]
+
+
 # every symbol include/lcbsa.h declares, with its C signature
 _P = ctypes.POINTER
 SIGNATURES = {
@@ -82,6 +87,7 @@ SIGNATURES = {
     "lcbsa_block_select_static": (ctypes.c_int, [_P(LcbsaTensor), _P(LcbsaTensor), _P(LcbsaGrid), _P(LcbsaGrid), ctypes.c_int,
                                                  ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
     "lcbsa_set_attn_sm_reserve": (ctypes.c_int, [ctypes.c_int]),
+    "lcbsa_norm_rope_jobs": (ctypes.c_int, [_P(LcbsaRowJob), ctypes.c_int, ctypes.c_float, ctypes.c_void_p]),
     "lcbsa_norm_rope_ex": (ctypes.c_int, [_P(LcbsaTensor), ctypes.c_void_p, _P(LcbsaGrid), ctypes.c_void_p, ctypes.c_int, ctypes.c_int,
                                           ctypes.c_float, _P(LcbsaTensor), ctypes.c_void_p]),
     "lcbsa_score_cdf": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p] + [ctypes.c_int] * 5 + [ctypes.c_float, ctypes.c_float, ctypes.c_int,

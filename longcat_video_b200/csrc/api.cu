@@ -469,26 +469,69 @@ size_t lcbsa_rope_table_floats(const LcbsaGrid* g, int D) {
     return lcbsa::rope_table_floats(g->T, g->H, g->W, D);
 }
 
+int lcbsa_norm_rope_jobs(const LcbsaRowJob* jobs, int n_jobs, float eps, void* stream) {
+    if (!jobs || n_jobs < 1 || n_jobs > lcbsa::kMaxRowJobs) return fail(LCBSA_EINVAL, "norm_rope: 1..%d jobs", lcbsa::kMaxRowJobs);
+    if (!(eps >= 0.f)) return fail(LCBSA_EINVAL, "norm_rope: eps must be non-negative");
+    lcbsa::RowJobs P;
+    P.n = n_jobs;
+    P.eps = eps;
+    const LcbsaTensor& x0 = jobs[0].x;
+    P.H = (int)x0.size[1];
+    for (int i = 0; i < n_jobs; ++i) {
+        const LcbsaRowJob& j = jobs[i];
+        const LcbsaGrid* g = &j.grid;
+        if (!grid_ok(g)) return fail(LCBSA_EINVAL, "norm_rope: bad grid");
+        if (int rc = check_tensor("norm_rope input", &j.x, g)) return rc;
+        if (int rc = check_tensor("norm_rope output", &j.out, g)) return rc;
+        const bool keep = j.out_norm.data != nullptr;
+        if (keep)
+            if (int rc = check_tensor("norm_rope normalised output", &j.out_norm, g)) return rc;
+        if (keep && (!j.weight || !j.rope_tab)) return fail(LCBSA_EINVAL, "norm_rope: a second output needs a weight and a rope table");
+        if (reinterpret_cast<uintptr_t>(j.rope_tab) % 16 != 0 || reinterpret_cast<uintptr_t>(j.weight) % 16 != 0)
+            return fail(LCBSA_EINVAL, "norm_rope: weight and rope table must be 16-byte aligned");
+        if (j.rope_tab && (j.t_offset < 0 || j.table_T < g->T + j.t_offset))
+            return fail(LCBSA_EINVAL, "norm_rope: frames %d..%d outside the table's %d frames", j.t_offset, g->T + j.t_offset - 1, j.table_T);
+        if (j.x.dtype != j.out.dtype || (keep && j.x.dtype != j.out_norm.dtype)) return fail(LCBSA_EINVAL, "norm_rope: input and output dtypes differ");
+        for (int a = 0; a < 4; ++a)
+            if (j.x.size[a] != j.out.size[a] || (keep && j.x.size[a] != j.out_norm.size[a]))
+                return fail(LCBSA_EINVAL, "norm_rope: input and output shapes differ");
+        if (j.x.dtype != x0.dtype || j.x.size[0] != x0.size[0] || j.x.size[1] != x0.size[1] || j.x.size[3] != x0.size[3])
+            return fail(LCBSA_EINVAL, "norm_rope: the jobs of a launch share dtype, batch, heads and head_dim");
+        lcbsa::RowJob& r = P.job[i];
+        r.x = view_of(&j.x);
+        r.weight = j.weight;
+        r.tab = j.rope_tab;
+        r.out = j.out.data;
+        r.osb = j.out.stride[0]; r.osh = j.out.stride[1]; r.oss = j.out.stride[2];
+        r.out2 = j.out_norm.data;
+        r.o2sb = j.out_norm.stride[0]; r.o2sh = j.out_norm.stride[1]; r.o2ss = j.out_norm.stride[2];
+        r.S = (int)j.x.size[2];
+        r.tab_t = j.table_T; r.t_off = j.t_offset;
+        r.Hg = g->H; r.Wg = g->W;
+        r.first = 0;
+    }
+    const char* why = "";
+    cudaError_t e = lcbsa::launch_norm_rope(x0.dtype, P, (int)x0.size[0], (int)x0.size[3], static_cast<cudaStream_t>(stream), &why);
+    if (e != cudaSuccess) return cuda_fail(e, "norm_rope", why);
+    return LCBSA_OK;
+}
+
 int lcbsa_norm_rope_ex(const LcbsaTensor* x, const void* weight, const LcbsaGrid* g, const float* rope_tab, int table_T, int t_offset,
                        float eps, const LcbsaTensor* out, void* stream) {
     if (!grid_ok(g)) return fail(LCBSA_EINVAL, "norm_rope: bad grid");
     if (int rc = check_tensor("norm_rope input", x, g)) return rc;
     if (int rc = check_tensor("norm_rope output", out, g)) return rc;
     if (!weight && !rope_tab) return fail(LCBSA_EINVAL, "norm_rope: null weight and null rope table: nothing to do");
-    if (reinterpret_cast<uintptr_t>(rope_tab) % 16 != 0 || reinterpret_cast<uintptr_t>(weight) % 16 != 0)
-        return fail(LCBSA_EINVAL, "norm_rope: weight and rope table must be 16-byte aligned");
-    if (rope_tab && (t_offset < 0 || table_T < g->T + t_offset))
-        return fail(LCBSA_EINVAL, "norm_rope: frames %d..%d outside the table's %d frames", t_offset, g->T + t_offset - 1, table_T);
-    if (x->dtype != out->dtype) return fail(LCBSA_EINVAL, "norm_rope: input and output dtypes differ");
-    for (int i = 0; i < 4; ++i)
-        if (x->size[i] != out->size[i]) return fail(LCBSA_EINVAL, "norm_rope: input and output shapes differ");
-    if (!(eps >= 0.f)) return fail(LCBSA_EINVAL, "norm_rope: eps must be non-negative");
-    const char* why = "";
-    cudaError_t e = lcbsa::launch_norm_rope(x->dtype, view_of(x), (int)x->size[0], (int)x->size[1], (int)x->size[2], (int)x->size[3], table_T,
-                                            t_offset, g->H, g->W, weight, rope_tab, eps, out->data, out->stride[0], out->stride[1],
-                                            out->stride[2], static_cast<cudaStream_t>(stream), &why);
-    if (e != cudaSuccess) return cuda_fail(e, "norm_rope", why);
-    return LCBSA_OK;
+    LcbsaRowJob j;
+    memset(&j, 0, sizeof(j));
+    j.x = *x;
+    j.out = *out;
+    j.weight = weight;
+    j.rope_tab = rope_tab;
+    j.grid = *g;
+    j.table_T = table_T;
+    j.t_offset = t_offset;
+    return lcbsa_norm_rope_jobs(&j, 1, eps, stream);
 }
 
 int lcbsa_norm_rope(const LcbsaTensor* x, const void* weight, const LcbsaGrid* g, const float* rope_tab, float eps,

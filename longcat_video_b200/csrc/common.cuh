@@ -184,8 +184,24 @@ int set_attn_sm_reserve(int n_sms);  // SMs the tcgen05 attention kernel leaves 
 // q/k RMSNorm + 3-D rotary embedding in one pass (norm_rope.cu).  The table is the packed separable form
 // cos_t [T, dt] sin_t [T, dt] cos_h [H, dh] sin_h [H, dh] cos_w [W, dh] sin_w [W, dh], dh = 2 * (D / 6), dt = D - 2 * dh.
 size_t rope_table_floats(int Tg, int Hg, int Wg, int D);
-cudaError_t launch_norm_rope(int dtype, const View& x, int B, int H, int S, int D, int tab_t, int t_off, int Hg, int Wg, const void* weight,
-                             const float* tab, float eps, void* out, long long osb, long long osh, long long oss, cudaStream_t st,
-                             const char** why);
+// What one launch does to the rows of one tensor: weight == nullptr: no normalisation; tab == nullptr: no rotary embedding; neither:
+// a copy.  out2 != nullptr (both weight and tab set): also keeps the normalised, not yet embedded rows.  Strides in elements.
+constexpr int kMaxRowJobs = 8;
+struct RowJob {
+    View x;
+    const void* weight;
+    const float* tab;
+    void *out, *out2;
+    long long osb, osh, oss, o2sb, o2sh, o2ss;
+    int S, tab_t, t_off, Hg, Wg;
+    unsigned first;  // first CTA of the job (filled in by the launch)
+};
+struct RowJobs {
+    RowJob job[kMaxRowJobs];
+    int n, H, hpc;  // jobs, heads of every job, heads per CTA (filled in by the launch)
+    unsigned head_groups;
+    float eps;
+};
+cudaError_t launch_norm_rope(int dtype, RowJobs& jobs, int B, int D, cudaStream_t st, const char** why);
 
 }  // namespace lcbsa

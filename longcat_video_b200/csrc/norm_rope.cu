@@ -23,6 +23,11 @@
 // The rotary angles depend on t for the first D - 4*(D/6) elements of the head dimension, on h for the next
 // 2*(D/6) and on w for the last 2*(D/6) (rope_3d.py:62-84), so the [S, D] cos/sin tables of the reference factor
 // into three small ones, [T, dt], [H, dh], [W, dw]; both elements of a pair have the same angle (rope_3d.py:113-115).
+//
+// A launch works on up to kMaxRowJobs tensors at once: all that a layer does to its q, k, v rows before the attention
+// (normalise, embed, also keep the normalised k, copy v into or behind the cache).  The copies ran as library copies of
+// strided views, two bytes per thread and step: 480p grid, 32 heads, bf16, the clone of v took 361 us and v behind its cache
+// 376 us; as jobs they take 118 and 105 us, at the rate of the other rows.
 #include "common.cuh"
 
 namespace lcbsa {
@@ -31,7 +36,7 @@ namespace {
 
 constexpr int kWarps = 8;         // warps per CTA, four tokens each
 constexpr int kTokens = 4;        // tokens per warp: eight lanes each
-constexpr int kHeadsPerCta = 16;  // heads one warp walks over
+constexpr int kHeadsPerCta = 16;  // heads one warp walks over, at most
 
 // Two values of the storage type in one 32-bit word: rounding two floats costs one packed conversion.
 template <typename T>
@@ -71,23 +76,24 @@ struct Pair<__half> {
 // NORM: RMSNorm times weight (off: the input is already normalised, e.g. cached keys); ROPE: the rotary embedding
 // (off: normalised q / k as they are cached before the embedding, attention.py:118-119).  The token at grid position
 // (t, h, w) takes the angles of frame t + t_off; tab_t is the number of frames the table holds (>= T + t_off).
-template <typename T, int D, bool NORM, bool ROPE>
-__global__ void __launch_bounds__(kWarps * 32) norm_rope_kernel(View x, int H, int S, int tab_t, int t_off, int Hg, int Wg,
-                                                               const T* __restrict__ weight, const float* __restrict__ tab, float eps, T* out,
-                                                               long long osb, long long osh, long long oss) {
+// Neither: the rows are copied.  KEEP: the normalised row also goes to out2.
+template <typename T, int D, bool NORM, bool ROPE, bool KEEP>
+__device__ __forceinline__ void do_rows(const RowJob& j, unsigned s_blk, int b, int h0, int h1, float eps) {
+    const View& x = j.x;
+    const int S = j.S, tab_t = j.tab_t, Hg = j.Hg, Wg = j.Wg;
+    const T* __restrict__ weight = static_cast<const T*>(j.weight);
+    const float* __restrict__ tab = j.tab;
     constexpr int PER = D / 8;   // elements per lane: 16 or 8
     constexpr int NV = PER / 8;  // 16-byte vectors per lane
     constexpr int NP = PER / 2;  // rotation pairs per lane
     static_assert(PER == 8 || PER == 16, "a lane owns one or two 16-byte vectors");
     constexpr int DH = 2 * (D / 6), DW = DH, DT = D - DH - DW;
     const int lane = threadIdx.x & 31, sub = lane & 7, tok = lane >> 3;
-    const long long first = ((long long)blockIdx.x * kWarps + (threadIdx.x >> 5)) * kTokens;  // the warp's first token
+    const long long first = ((long long)s_blk * kWarps + (threadIdx.x >> 5)) * kTokens;  // the warp's first token
     if (first >= S) return;
     const bool live = first + tok < S;  // the last warp may have fewer than four tokens
     const int s = live ? (int)(first + tok) : S - 1;
-    const int b = blockIdx.z;
-    const int h0 = blockIdx.y * kHeadsPerCta, h1 = min(H, h0 + kHeadsPerCta);
-    const int w_pos = s % Wg, h_pos = (s / Wg) % Hg, t_pos = s / (Wg * Hg) + t_off;
+    const int w_pos = s % Wg, h_pos = (s / Wg) % Hg, t_pos = s / (Wg * Hg) + j.t_off;
 
     // table layout: cos_t [T, DT] sin_t [T, DT] cos_h [H, DH] sin_h [H, DH] cos_w [W, DW] sin_w [W, DW]
     const float* cos_t = tab;
@@ -113,20 +119,21 @@ __global__ void __launch_bounds__(kWarps * 32) norm_rope_kernel(View x, int H, i
     }
     uint4 wv[NV];  // the lane's weights, packed as they are stored
 #pragma unroll
-    for (int j = 0; j < NV; ++j) wv[j] = NORM ? __ldg(reinterpret_cast<const uint4*>(weight + sub * PER) + j) : make_uint4(0u, 0u, 0u, 0u);
+    for (int i = 0; i < NV; ++i) wv[i] = NORM ? __ldg(reinterpret_cast<const uint4*>(weight + sub * PER) + i) : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t* wp = reinterpret_cast<const uint32_t*>(wv);
 
     const T* sp = reinterpret_cast<const T*>(x.data) + (long long)b * x.sb + (long long)s * x.ss + (long long)h0 * x.sh + sub * PER;
-    T* dp = out + (long long)b * osb + (long long)s * oss + (long long)h0 * osh + sub * PER;
+    T* dp = static_cast<T*>(j.out) + (long long)b * j.osb + (long long)s * j.oss + (long long)h0 * j.osh + sub * PER;
+    T* dp2 = KEEP ? static_cast<T*>(j.out2) + (long long)b * j.o2sb + (long long)s * j.o2ss + (long long)h0 * j.o2sh + sub * PER : nullptr;
     uint4 cur[NV], nxt[NV];
 #pragma unroll
-    for (int j = 0; j < NV; ++j) cur[j] = reinterpret_cast<const uint4*>(sp)[j];
+    for (int i = 0; i < NV; ++i) cur[i] = reinterpret_cast<const uint4*>(sp)[i];
 #pragma unroll 1
     for (int h = h0; h < h1; ++h) {
         sp += x.sh;
         if (h + 1 < h1) {  // the next head's row is in flight during the arithmetic
 #pragma unroll
-            for (int j = 0; j < NV; ++j) nxt[j] = reinterpret_cast<const uint4*>(sp)[j];
+            for (int i = 0; i < NV; ++i) nxt[i] = reinterpret_cast<const uint4*>(sp)[i];
         }
         const uint32_t* cw = reinterpret_cast<const uint32_t*>(cur);
         float rinv = 1.0f;
@@ -142,50 +149,106 @@ __global__ void __launch_bounds__(kWarps * 32) norm_rope_kernel(View x, int H, i
             const float mean = __fmul_rn(ss, 1.0f / (float)D);
             rinv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
         }
-        uint4 res[NV];
-        uint32_t* rw = reinterpret_cast<uint32_t*>(res);
 #pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            uint32_t z = cw[p];
-            if (NORM) {
-                float v0, v1;
-                Pair<T>::unpack(cw[p], v0, v1);
-                z = Pair<T>::mul(Pair<T>::pack(__fmul_rn(v0, rinv), __fmul_rn(v1, rinv)), wp[p]);
+        for (int i = 0; i < NV; ++i) {
+            uint32_t rw[4], rn[4];
+#pragma unroll
+            for (int p4 = 0; p4 < 4; ++p4) {
+                const int p = 4 * i + p4;
+                uint32_t z = cw[p];
+                if (NORM) {
+                    float v0, v1;
+                    Pair<T>::unpack(cw[p], v0, v1);
+                    z = Pair<T>::mul(Pair<T>::pack(__fmul_rn(v0, rinv), __fmul_rn(v1, rinv)), wp[p]);
+                }
+                rn[p4] = z;
+                if (ROPE) {
+                    float z0, z1;
+                    Pair<T>::unpack(z, z0, z1);
+                    z = Pair<T>::pack(__fadd_rn(__fmul_rn(z0, cs[p]), __fmul_rn(-z1, sn[p])),
+                                      __fadd_rn(__fmul_rn(z1, cs[p]), __fmul_rn(z0, sn[p])));
+                }
+                rw[p4] = z;
             }
-            if (ROPE) {
-                float z0, z1;
-                Pair<T>::unpack(z, z0, z1);
-                z = Pair<T>::pack(__fadd_rn(__fmul_rn(z0, cs[p]), __fmul_rn(-z1, sn[p])),
-                                  __fadd_rn(__fmul_rn(z1, cs[p]), __fmul_rn(z0, sn[p])));
+            if (live) {
+                reinterpret_cast<uint4*>(dp)[i] = make_uint4(rw[0], rw[1], rw[2], rw[3]);
+                if (KEEP) reinterpret_cast<uint4*>(dp2)[i] = make_uint4(rn[0], rn[1], rn[2], rn[3]);
             }
-            rw[p] = z;
         }
-        if (live) {
+        if (KEEP) dp2 += j.o2sh;
+        dp += j.osh;
 #pragma unroll
-            for (int j = 0; j < NV; ++j) reinterpret_cast<uint4*>(dp)[j] = res[j];
-        }
-        dp += osh;
-#pragma unroll
-        for (int j = 0; j < NV; ++j) cur[j] = nxt[j];
+        for (int i = 0; i < NV; ++i) cur[i] = nxt[i];
     }
 }
 
-template <typename T, int D, bool NORM, bool ROPE>
-cudaError_t run(const View& x, int B, int H, int S, int tab_t, int t_off, int Hg, int Wg, const void* weight, const float* tab, float eps,
-                void* out, long long osb, long long osh, long long oss, cudaStream_t st) {
-    if ((long long)B * H * S == 0) return cudaSuccess;
-    dim3 grid((unsigned)((S + kTokens * kWarps - 1) / (kTokens * kWarps)), (unsigned)((H + kHeadsPerCta - 1) / kHeadsPerCta), (unsigned)B);
-    norm_rope_kernel<T, D, NORM, ROPE><<<grid, kWarps * 32, 0, st>>>(x, H, S, tab_t, t_off, Hg, Wg, reinterpret_cast<const T*>(weight), tab,
-                                                                    eps, reinterpret_cast<T*>(out), osb, osh, oss);
+// One CTA: 32 tokens and up to `hpc` heads of one batch entry of one job.  The jobs' CTAs follow each other in the grid.
+// kKind: what the only job of the launch does (kCopy ..), or kMixed: any number of jobs of any kind.
+enum { kCopy, kRope, kNorm, kNormRope, kNormRopeKeep, kMixed };
+
+__host__ __device__ __forceinline__ int kind_of(const RowJob& j) {
+    if (j.weight != nullptr && j.tab != nullptr) return j.out2 != nullptr ? kNormRopeKeep : kNormRope;
+    return j.weight != nullptr ? kNorm : j.tab != nullptr ? kRope : kCopy;
+}
+
+template <typename T, int D, int kKind>
+__global__ void __launch_bounds__(kWarps * 32, 4) norm_rope_kernel(const __grid_constant__ RowJobs P) {
+    int i = 0;
+    if (kKind == kMixed)
+        while (i + 1 < P.n && blockIdx.x >= P.job[i + 1].first) ++i;
+    const RowJob& j = P.job[kKind == kMixed ? i : 0];
+    const unsigned r = blockIdx.x - (kKind == kMixed ? j.first : 0u), s_blks = (unsigned)(j.S + kTokens * kWarps - 1) / (kTokens * kWarps);
+    const unsigned rest = r / s_blks, hg = rest % P.head_groups, s_blk = r % s_blks;
+    const int b = (int)(rest / P.head_groups), h0 = (int)hg * P.hpc, h1 = min(P.H, h0 + P.hpc);
+    const int kind = kKind == kMixed ? kind_of(j) : kKind;
+    if (kind == kNormRopeKeep) do_rows<T, D, true, true, true>(j, s_blk, b, h0, h1, P.eps);
+    else if (kind == kNormRope) do_rows<T, D, true, true, false>(j, s_blk, b, h0, h1, P.eps);
+    else if (kind == kNorm) do_rows<T, D, true, false, false>(j, s_blk, b, h0, h1, P.eps);
+    else if (kind == kRope) do_rows<T, D, false, true, false>(j, s_blk, b, h0, h1, P.eps);
+    else do_rows<T, D, false, false, false>(j, s_blk, b, h0, h1, P.eps);
+}
+
+template <typename T, int D>
+cudaError_t launch(RowJobs& P, int kind, int B, cudaStream_t st) {
+    long long total = 0;
+    P.head_groups = (unsigned)((P.H + P.hpc - 1) / P.hpc);
+    for (int i = 0; i < P.n; ++i) {
+        P.job[i].first = (unsigned)total;
+        total += (long long)((P.job[i].S + kTokens * kWarps - 1) / (kTokens * kWarps)) * P.head_groups * B;
+    }
+    if (total == 0) return cudaSuccess;
+    if (total > 0x7fffffffll) return cudaErrorInvalidConfiguration;
+    switch (kind) {
+        case kCopy: norm_rope_kernel<T, D, kCopy><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
+        case kRope: norm_rope_kernel<T, D, kRope><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
+        case kNorm: norm_rope_kernel<T, D, kNorm><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
+        case kNormRope: norm_rope_kernel<T, D, kNormRope><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
+        case kNormRopeKeep: norm_rope_kernel<T, D, kNormRopeKeep><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
+        default: norm_rope_kernel<T, D, kMixed><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
+    }
     return cudaGetLastError();
 }
 
 template <typename T, int D>
-cudaError_t pick(bool norm, bool rope, const View& x, int B, int H, int S, int tab_t, int t_off, int Hg, int Wg, const void* weight,
-                 const float* tab, float eps, void* out, long long osb, long long osh, long long oss, cudaStream_t st) {
-    if (norm && rope) return run<T, D, true, true>(x, B, H, S, tab_t, t_off, Hg, Wg, weight, tab, eps, out, osb, osh, oss, st);
-    if (norm) return run<T, D, true, false>(x, B, H, S, tab_t, t_off, Hg, Wg, weight, tab, eps, out, osb, osh, oss, st);
-    return run<T, D, false, true>(x, B, H, S, tab_t, t_off, Hg, Wg, weight, tab, eps, out, osb, osh, oss, st);
+cudaError_t run(RowJobs& P, int B, cudaStream_t st) {
+    // A warp takes up to 16 heads, which spreads its set-up (position, angles, weights) over that many rows; small calls take
+    // fewer, so that there are some eight CTAs per SM: the heads of a warp are a serial chain of loads.
+    long long tokens = 0;
+    for (int i = 0; i < P.n; ++i) tokens += (P.job[i].S + kTokens * kWarps - 1) / (kTokens * kWarps);
+    P.hpc = kHeadsPerCta;
+    while (P.hpc > 2 && tokens * B * ((P.H + P.hpc - 1) / P.hpc) < 148 * 8) P.hpc /= 2;
+    // Calls that do not fill the chip are bound by their launches: all jobs in one.  Larger ones take a launch per job, whose
+    // kernel has the registers and the code of its kind alone: q and k of a 24x48x80 grid, 32 heads: 519 us in two launches, 582 us
+    // through the kernel that serves all kinds.
+    if (P.n > 1 && tokens * B * ((P.H + P.hpc - 1) / P.hpc) < 148 * 16) return launch<T, D>(P, kMixed, B, st);
+    for (int i = 0; i < P.n; ++i) {
+        RowJobs one = P;
+        one.job[0] = P.job[i];
+        one.n = 1;
+        cudaError_t e = launch<T, D>(one, kind_of(one.job[0]), B, st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace
@@ -195,10 +258,7 @@ size_t rope_table_floats(int Tg, int Hg, int Wg, int D) {
     return 2 * ((size_t)Tg * dt + (size_t)Hg * dh + (size_t)Wg * dh);
 }
 
-// weight == nullptr: no normalisation; tab == nullptr: no rotary embedding (not both)
-cudaError_t launch_norm_rope(int dtype, const View& x, int B, int H, int S, int D, int tab_t, int t_off, int Hg, int Wg, const void* weight,
-                             const float* tab, float eps, void* out, long long osb, long long osh, long long oss, cudaStream_t st,
-                             const char** why) {
+cudaError_t launch_norm_rope(int dtype, RowJobs& jobs, int B, int D, cudaStream_t st, const char** why) {
     if (dtype == LCBSA_FP32 || (D != 64 && D != 128)) {
         *why = "norm_rope takes bf16 or fp16 with head_dim 64 or 128";
         return cudaErrorInvalidValue;
@@ -207,16 +267,9 @@ cudaError_t launch_norm_rope(int dtype, const View& x, int B, int H, int S, int 
         *why = "norm_rope: batch above 65535";
         return cudaErrorInvalidValue;
     }
-    const bool norm = weight != nullptr, rope = tab != nullptr;
-    if (!norm && !rope) {
-        *why = "norm_rope: neither a weight nor a rope table";
-        return cudaErrorInvalidValue;
-    }
-    if (dtype == LCBSA_BF16)
-        return D == 128 ? pick<__nv_bfloat16, 128>(norm, rope, x, B, H, S, tab_t, t_off, Hg, Wg, weight, tab, eps, out, osb, osh, oss, st)
-                        : pick<__nv_bfloat16, 64>(norm, rope, x, B, H, S, tab_t, t_off, Hg, Wg, weight, tab, eps, out, osb, osh, oss, st);
-    return D == 128 ? pick<__half, 128>(norm, rope, x, B, H, S, tab_t, t_off, Hg, Wg, weight, tab, eps, out, osb, osh, oss, st)
-                    : pick<__half, 64>(norm, rope, x, B, H, S, tab_t, t_off, Hg, Wg, weight, tab, eps, out, osb, osh, oss, st);
+    if (B == 0 || jobs.H == 0) return cudaSuccess;
+    if (dtype == LCBSA_BF16) return D == 128 ? run<__nv_bfloat16, 128>(jobs, B, st) : run<__nv_bfloat16, 64>(jobs, B, st);
+    return D == 128 ? run<__half, 128>(jobs, B, st) : run<__half, 64>(jobs, B, st);
 }
 
 }  // namespace lcbsa

@@ -13,8 +13,18 @@ from typing import Optional, Sequence, Tuple
 
 import torch
 
+from .. import _lib as L
 from ..block_sparse_attention.bsa_interface import flash_attn_bsa_3d, flash_attn_bsa_3d_cond
-from .rope_3d import norm_rope, qk_norm_rope_with_kv_cache, rms_norm
+from .rope_3d import RowJob, kv_cache_row_jobs, run_row_jobs
+
+
+def _rows_can_be_copied(src: torch.Tensor, dst: torch.Tensor) -> bool:
+    """Whether the copy of ``src`` into ``dst`` can ride in the launch that handles the layer's q and k rows.  Anything it does not
+    take (another dtype, unaligned rows) and any copy that differentiation has to see is left to PyTorch."""
+    return (type(src) in (torch.Tensor, torch.nn.Parameter) and src.is_cuda and src.device == dst.device and src.dtype == dst.dtype
+            and src.dtype in (torch.bfloat16, torch.float16) and src.dim() == 4 and src.shape == dst.shape and src.shape[3] in (64, 128)
+            and L.abi_ok(src) and L.abi_ok(dst) and not (torch.is_grad_enabled() and src.requires_grad)
+            and torch.autograd.forward_ad._current_level < 0)
 
 
 def self_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor,
@@ -27,10 +37,19 @@ def self_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, q_weight: 
     (attention.py:118-119).  Returns ``x [B, H, N, D]`` or ``(x, (k_cache, v_cache))``."""
     shape = tuple(int(s) for s in shape)
     kv = None
+    q_e, k_e = torch.empty(q.shape, dtype=q.dtype, device=q.device), torch.empty(k.shape, dtype=k.dtype, device=k.device)
+    jobs = [RowJob(q, q_e, q_weight, shape)]
     if return_kv:
-        kv = (rms_norm(k, k_weight, eps), v.clone())
-    q_e = norm_rope(q, q_weight, shape, eps)
-    k_e = norm_rope(k, k_weight, shape, eps)
+        k_c, v_c = torch.empty(k.shape, dtype=k.dtype, device=k.device), torch.empty_like(v)
+        jobs.append(RowJob(k, k_e, k_weight, shape, out_norm=k_c))
+        if _rows_can_be_copied(v, v_c):
+            jobs.append(RowJob(v, v_c, None, shape, rope=False))
+        else:
+            v_c = v.clone()
+        kv = (k_c, v_c)
+    else:
+        jobs.append(RowJob(k, k_e, k_weight, shape))
+    run_row_jobs(jobs, eps)
     if num_cond_latents is not None and num_cond_latents > 0:
         x = flash_attn_bsa_3d_cond(q_e, k_e, v, shape, num_cond_latents, **bsa_params)
     else:
@@ -60,8 +79,13 @@ def self_attention_with_kv_cache(q: torch.Tensor, k: torch.Tensor, v: torch.Tens
         raise ValueError(f"cache batch {k_cache.shape[0]} / {v_cache.shape[0]} against batch {B}")
     if N != T * Hh * W or k_cache.shape[2] != sc or v_cache.shape[2] != sc:
         raise ValueError(f"{N} new tokens and {k_cache.shape[2]} cached ones do not match shape {(T, Hh, W)} with {nc} cached frames")
-    q_e, k_full = qk_norm_rope_with_kv_cache(q, k, q_weight, k_weight, k_cache, (T, Hh, W), nc, eps)
+    q_e, k_full, jobs = kv_cache_row_jobs(q, k, q_weight, k_weight, k_cache, (T, Hh, W), nc)
     v_full = torch.empty(B, H, sc + N, D, dtype=v.dtype, device=v.device)
-    v_full[:, :, :sc].copy_(v_cache if v_cache.shape[0] == B else v_cache.expand(B, -1, -1, -1))
-    v_full[:, :, sc:].copy_(v)
+    for src, dst, frames in ((v_cache if v_cache.shape[0] == B else v_cache.expand(B, -1, -1, -1), v_full[:, :, :sc], nc),
+                             (v, v_full[:, :, sc:], T)):
+        if _rows_can_be_copied(src, dst):
+            jobs.append(RowJob(src, dst, None, (frames, Hh, W), rope=False))
+        else:
+            dst.copy_(src)
+    run_row_jobs(jobs, eps)
     return flash_attn_bsa_3d(q_e, k_full, v_full, (T, Hh, W), (T + nc, Hh, W), **bsa_params)

@@ -7,12 +7,12 @@ Stands in for these lines of ``Attention.forward`` (``longcat_video/modules/atte
 
 which run as six elementwise passes with fp32 temporaries.  ``qk_norm_rope`` reads the strided q and k views of the
 fused qkv projection once and writes ``[B, H, S, D]`` outputs once.  All arithmetic is in liblcbsa.so
-(``lcbsa_norm_rope``); PyTorch builds the small angle table and allocates the outputs.  There is no CPU path.
+(``lcbsa_norm_rope_jobs``); PyTorch builds the small angle table and allocates the outputs.  There is no CPU path.
 """
 from __future__ import annotations
 
 import ctypes
-from typing import Optional, Sequence, Tuple
+from typing import NamedTuple, Optional, Sequence, Tuple
 
 import torch
 
@@ -59,6 +59,62 @@ def rope_table(grid_size: Sequence[int], head_dim: int, device, base: float = 10
     return tab
 
 
+class RowJob(NamedTuple):
+    """What ``run_row_jobs`` does to the rows of one ``[B, H, S, D]`` tensor (any B/H/S strides): RMSNorm times ``weight`` (None: off),
+    the rotary embedding (``rope``), neither: a copy.  ``out_norm`` also keeps the rows as they are before the embedding."""
+    x: torch.Tensor
+    out: torch.Tensor
+    weight: Optional[torch.Tensor]
+    grid_size: Sequence[int]
+    rope: bool = True
+    t_offset: int = 0
+    table_frames: Optional[int] = None
+    pos_offset: Sequence[int] = (0, 0, 0)
+    out_norm: Optional[torch.Tensor] = None
+
+
+_NO_TENSOR = L.LcbsaTensor()
+
+
+def run_row_jobs(jobs: Sequence[RowJob], eps: float = 1e-6, base: float = 10000.0) -> None:
+    """One launch for all jobs that share dtype, batch, heads and head_dim: for all there are, as a layer has them."""
+    kinds = {}
+    for j in jobs:
+        if j.x.dim() != 4:
+            raise ValueError("expected a [B, H, S, D] tensor")
+        kinds.setdefault((j.x.dtype, j.x.device, j.x.shape[0], j.x.shape[1], j.x.shape[3]), []).append(j)
+    for group in kinds.values():
+        _launch_row_jobs(group, eps, base)
+
+
+def _launch_row_jobs(jobs: Sequence[RowJob], eps: float, base: float) -> None:
+    descs = (L.LcbsaRowJob * len(jobs))()
+    keep = []  # weights and tables stay alive until the launch is queued
+    for j, d in zip(jobs, descs):
+        x, D = j.x, j.x.shape[3]
+        if not L.abi_ok(x):
+            x = x.contiguous()
+        T = int(j.grid_size[0])
+        frames = T + int(j.t_offset) if j.table_frames is None else int(j.table_frames)
+        keep.append(x)
+        if j.weight is not None:
+            w = j.weight.to(device=x.device, dtype=x.dtype).contiguous()
+            if w.numel() != D:
+                raise ValueError(f"weight has {w.numel()} elements, head_dim is {D}")
+            keep.append(w)
+            d.weight = w.data_ptr()
+        if j.rope:
+            tab = rope_table((frames, j.grid_size[1], j.grid_size[2]), D, x.device, base, j.pos_offset)
+            keep.append(tab)
+            d.rope_tab = tab.data_ptr()
+        d.x, d.out = L.tensor_desc(x), L.tensor_desc(j.out)
+        d.out_norm = _NO_TENSOR if j.out_norm is None else L.tensor_desc(j.out_norm)
+        d.grid, d.table_T, d.t_offset = L.grid_plan(j.grid_size, (1, 1, 1))[0], frames, int(j.t_offset)
+    dev = jobs[0].x.device
+    with L.on_device(dev):
+        L.check(L.lib().lcbsa_norm_rope_jobs(descs, len(jobs), float(eps), L.current_stream(dev)))
+
+
 def norm_rope(x: torch.Tensor, weight: Optional[torch.Tensor], grid_size: Sequence[int], eps: float = 1e-6, base: float = 10000.0,
               out: Optional[torch.Tensor] = None, rope: bool = True, t_offset: int = 0, table_frames: Optional[int] = None,
               pos_offset: Sequence[int] = (0, 0, 0)) -> torch.Tensor:
@@ -71,27 +127,9 @@ def norm_rope(x: torch.Tensor, weight: Optional[torch.Tensor], grid_size: Sequen
         raise ValueError("expected a [B, H, S, D] tensor")
     if weight is None and not rope:
         raise ValueError("neither normalisation nor rotary embedding requested")
-    if not L.abi_ok(x):
-        x = x.contiguous()
-    B, H, S, D = x.shape
     if out is None:
-        out = torch.empty(B, H, S, D, dtype=x.dtype, device=x.device)
-    w_ptr = None
-    if weight is not None:
-        w = weight.to(device=x.device, dtype=x.dtype).contiguous()
-        if w.numel() != D:
-            raise ValueError(f"weight has {w.numel()} elements, head_dim is {D}")
-        w_ptr = ctypes.c_void_p(w.data_ptr())
-    T = int(grid_size[0])
-    frames = T + int(t_offset) if table_frames is None else int(table_frames)
-    tab_ptr = None
-    if rope:
-        tab = rope_table((frames, grid_size[1], grid_size[2]), D, x.device, base, pos_offset)
-        tab_ptr = ctypes.c_void_p(tab.data_ptr())
-    xd, od, g = L.tensor_desc(x), L.tensor_desc(out), L.grid_desc(grid_size, (1, 1, 1))
-    with torch.cuda.device(x.device):
-        L.check(L.lib().lcbsa_norm_rope_ex(ctypes.byref(xd), w_ptr, ctypes.byref(g), tab_ptr, frames, int(t_offset),
-                                           ctypes.c_float(eps), ctypes.byref(od), L.current_stream(x.device)))
+        out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+    run_row_jobs([RowJob(x, out, weight, grid_size, rope, t_offset, table_frames, pos_offset)], eps, base)
     return out
 
 
@@ -102,8 +140,27 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, out: Opti
 
 def qk_norm_rope(q: torch.Tensor, k: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, grid_size: Sequence[int],
                  eps: float = 1e-6, base: float = 10000.0) -> Tuple[torch.Tensor, torch.Tensor]:
-    """``rope_3d(q_norm(q), k_norm(k), grid_size)`` of attention.py:113-121: two launches, one per tensor."""
-    return norm_rope(q, q_weight, grid_size, eps, base), norm_rope(k, k_weight, grid_size, eps, base)
+    """``rope_3d(q_norm(q), k_norm(k), grid_size)`` of attention.py:113-121 in one launch."""
+    q_out, k_out = torch.empty(q.shape, dtype=q.dtype, device=q.device), torch.empty(k.shape, dtype=k.dtype, device=k.device)
+    run_row_jobs([RowJob(q, q_out, q_weight, grid_size), RowJob(k, k_out, k_weight, grid_size)], eps, base)
+    return q_out, k_out
+
+
+def kv_cache_row_jobs(q: torch.Tensor, k: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, k_cache: torch.Tensor,
+                      grid_size: Sequence[int], num_cond_latents: int) -> Tuple[torch.Tensor, torch.Tensor, list]:
+    """Outputs and row jobs of ``qk_norm_rope_with_kv_cache``."""
+    T, Hh, W = (int(v) for v in grid_size)
+    nc = int(num_cond_latents)
+    B, H, N, D = q.shape
+    sc = nc * Hh * W
+    if k_cache.shape[0] == 1 and B > 1:  # attention.py:160-162
+        k_cache = k_cache.expand(B, -1, -1, -1)
+    assert k_cache.shape[2] == sc and N == T * Hh * W
+    k_full = torch.empty(B, H, sc + N, D, dtype=k.dtype, device=k.device)
+    q_out = torch.empty(B, H, N, D, dtype=q.dtype, device=q.device)
+    jobs = [RowJob(k_cache, k_full[:, :, :sc], None, (nc, Hh, W), table_frames=T + nc),
+            RowJob(k, k_full[:, :, sc:], k_weight, grid_size, t_offset=nc), RowJob(q, q_out, q_weight, grid_size, t_offset=nc)]
+    return q_out, k_full, jobs
 
 
 def qk_norm_rope_with_kv_cache(q: torch.Tensor, k: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, k_cache: torch.Tensor,
@@ -113,16 +170,7 @@ def qk_norm_rope_with_kv_cache(q: torch.Tensor, k: torch.Tensor, q_weight: torch
     ``k_full [B,H,(NC+T)HW,D]``.  The reference concatenates the cache and the new keys, pads q in front with an empty
     tensor of the cache's size, embeds both over ``(T + NC, H, W)`` and cuts q's tail off again; here the cached keys
     are embedded into the head of ``k_full``, the new keys are normalised and embedded into its tail, and q is
-    normalised and embedded at frame offset NC: three launches, no padding and no concatenation."""
-    T, Hh, W = (int(v) for v in grid_size)
-    nc = int(num_cond_latents)
-    B, H, N, D = q.shape
-    sc = nc * Hh * W
-    if k_cache.shape[0] == 1 and B > 1:  # attention.py:160-162
-        k_cache = k_cache.expand(B, -1, -1, -1)
-    assert k_cache.shape[2] == sc and N == T * Hh * W
-    k_full = torch.empty(B, H, sc + N, D, dtype=k.dtype, device=k.device)
-    norm_rope(k_cache, None, (nc, Hh, W), eps, base, out=k_full[:, :, :sc], table_frames=T + nc)
-    norm_rope(k, k_weight, grid_size, eps, base, out=k_full[:, :, sc:], t_offset=nc)
-    q_out = norm_rope(q, q_weight, grid_size, eps, base, t_offset=nc)
+    normalised and embedded at frame offset NC: one launch, no padding and no concatenation."""
+    q_out, k_full, jobs = kv_cache_row_jobs(q, k, q_weight, k_weight, k_cache, grid_size, num_cond_latents)
+    run_row_jobs(jobs, eps, base)
     return q_out, k_full
