@@ -759,7 +759,7 @@ namespace {
 
 // The workspace is laid out for the finest form the lists can take: 64-token units (a block of 64 * U tokens counts U times).
 struct BwdLayout {
-    size_t delta, tcnt, toff, tidx, bitmap, stats, idx_u, cnt_u, idx_t, cnt_t, total;
+    size_t delta, tcnt, toff, tidx, bitmap, stats, next_item, idx_u, cnt_u, idx_t, cnt_t, total;
 };
 
 BwdLayout bwd_layout(long long BH, const Geom& gq, const Geom& gk, int cap) {
@@ -776,6 +776,7 @@ BwdLayout bwd_layout(long long BH, const Geom& gq, const Geom& gk, int cap) {
     l.bitmap = off; off += up((size_t)BH * Nk * ((Nq + 31) / 32) * sizeof(uint32_t));
     // one pair per slot of every block: on a ragged grid more slots than tokens
     l.stats = off;  off += up((size_t)BH * gq.nblk * gq.bs * 2 * sizeof(float));
+    l.next_item = off; off += 256;
     const size_t rewritten = Uq * Uk > 1 ? 1 : 0;  // 64-token blocks on both sides: the lists are used as they are
     l.idx_u = off;  off += up(rewritten * BH * Nq * capu * sizeof(int32_t));
     l.cnt_u = off;  off += up(rewritten * BH * Nq * sizeof(int32_t));
@@ -798,6 +799,7 @@ cudaError_t launch_attn_bwd(BwdArgs a, void* workspace, cudaStream_t st, const c
     a.tidx = reinterpret_cast<int32_t*>(w + l.tidx);
     a.bitmap = reinterpret_cast<uint32_t*>(w + l.bitmap);
     a.stats = reinterpret_cast<float*>(w + l.stats);
+    a.next_item = reinterpret_cast<int*>(w + l.next_item);
     a.idx_u = reinterpret_cast<int32_t*>(w + l.idx_u);
     a.cnt_u = reinterpret_cast<int32_t*>(w + l.cnt_u);
     a.idx_t = reinterpret_cast<int32_t*>(w + l.idx_t);
