@@ -50,6 +50,7 @@
 // its list, its first tiles and its gradients; now the own tiles, the list and the row values of the next block are fetched
 // under the entries of this one, and some 3500 are left.  The blocks are taken off a counter, since the transposed lists differ in
 // length.  Backward of 8 heads, 39 of 624 64-token blocks: 1889 -> 1704 us; 16 of 832: 570 -> 445 us.
+// With 128-token blocks a long launch runs at 1.28 PFLOP/s of issued MMAs, nine tenths of what the GPU's power cap sustains.
 // Every mbarrier wait is bounded; when one runs out the CTA flags the status word, drains its copies, frees TMEM, returns.
 #include <algorithm>
 #include <cstdlib>
@@ -429,11 +430,6 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
                         if (ok && !kOneDp) ok = mbar_wait_warp(bar_s_free(sbuf), ((s / kSBufs) & 1) ^ 1, ctl, 226, s);
                         if (!ok) break;
                     }
-                    bool nf = false, ns = kOneDp;  // look ahead: probe the next entry's barriers now, read the answer after the MMAs
-                    if (e + 1 < it.n) {
-                        nf = mbar_test(bar_full((s + 1) % kSlots), ((s + 1) / kSlots) & 1);
-                        if (!kOneDp) ns = mbar_test(bar_s_free((s + 1) % kSBufs), (((s + 1) / kSBufs) & 1) ^ 1);
-                    }
                     tc_fence_after();
                     const uint32_t tile = sbase + kOffB + slot * kSlotBytes;
                     const uint64_t b1d = smem_desc(tile, 16, 1024), b2d = smem_desc(tile + kTileBytes, 16, 1024);
@@ -443,6 +439,15 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
                         const uint64_t off = (uint64_t)(((j >> 2) * kHalfBytes + (j & 3) * 32) >> 4);
                         tc_mma_ts(tmem + C::s(sbuf), tmem + C::own1 + 8u * j, b1d + off, idesc_ss, j > 0);
                     }
+                    // Look ahead: probe the next entry's barriers between the two contractions and read the answer after them.  Before the
+                    // first one the arithmetic warps do not have the S and dP of the entry before yet.  (8 heads, 39 of 624 blocks: 1705 us
+                    // with the probe in front, 1662 us.)
+                    bool nf = false, ns = kOneDp;
+                    if (e + 1 < it.n) {
+                        nf = mbar_test(bar_full((s + 1) % kSlots), ((s + 1) / kSlots) & 1);
+                        if (!kOneDp) ns = mbar_test(bar_s_free((s + 1) % kSBufs), (((s + 1) / kSBufs) & 1) ^ 1);
+                    }
+                    tc_fence_after();
                     if (kOneDp && s > 0) {  // dP of the entry before is in registers
                         ok = mbar_wait_warp(bar_s_free((s - 1) & 1), ((s - 1) >> 1) & 1, ctl, 227, s);
                         if (!ok) break;
