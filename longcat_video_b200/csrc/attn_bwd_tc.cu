@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // provably warp-uniform
     if (tid == 0) {
-        *abort_flag = 0;
+        ctl_init(ctl);
         for (int s = 0; s < kSlots; ++s) {
             mbar_init(bar_full(s), 2);  // one arrival per producer
             mbar_init(bar_empty(s), 1);
@@ -754,6 +754,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
     // ---- teardown
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) ctl_report(ctl);
     if (warp == 9) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));

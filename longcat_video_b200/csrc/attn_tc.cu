@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // the same value, but provably warp-uniform
 
     if (tid == 0) {
-        *abort_flag = 0;
+        ctl_init(ctl);
         for (int s = 0; s < kKSlots; ++s) {
             mbar_init(bar_k_full(s), 1);
             mbar_init(bar_k_empty(s), 1);
@@ -824,6 +824,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     // ---- teardown
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) ctl_report(ctl);
     if (warp == 9) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));

@@ -12,8 +12,7 @@ namespace lcbsa {
 namespace tc {
 
 constexpr int kMaxOutDst = 8;
-constexpr unsigned kSpinsBeforeClock = 1u << 12;     // failed try_waits before the clock is consulted
-constexpr long long kWaitLimitCycles = 4000000000ll;  // about 2 s
+constexpr uint32_t kWaitLimitCycles = 3000000000u;  // 1.5 to 2 s; compared with the low word of the cycle counter
 
 // ------------------------------------------------------------------------------------------ PTX
 
@@ -65,39 +64,42 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 #define LCBSA_UNLIKELY(x) __builtin_expect(!!(x), 0)
 
 struct Ctl {
-    volatile int* abort;    // shared flag
+    volatile int* abort;    // shared memory: [0] flag that all roles poll, [4] code, [5] thread, [6] iteration of the wait that ran out
     unsigned int* status;   // global status words
 };
 
-// Reached only after many failed tries: bound the wait by the cycle counter and flag a timeout.
-__device__ __forceinline__ bool mbar_wait_timeout(uint32_t bar, uint32_t parity, const Ctl& c, unsigned code, unsigned it) {
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int k = 0; k < 64; ++k)
-            if (mbar_try(bar, parity)) return true;
-        if (*c.abort) return false;
-        if (clock64() - t0 > kWaitLimitCycles) {
-            *c.abort = 1;
-            if (atomicCAS(c.status, 0u, code) == 0u) {
-                c.status[1] = blockIdx.x;
-                c.status[2] = threadIdx.x;
-                c.status[3] = it;
+__device__ __forceinline__ void ctl_init(const Ctl& c) { c.abort[0] = c.abort[4] = 0; }
+
+// Bounded wait of one thread. Returns false when the CTA is aborting (this wait or another one ran out).
+// try_wait itself blocks for a hardware-defined interval, so the loop turns over rarely.
+// Every role of every kernel waits in a dozen places, so what is inlined here is most of a kernel's code: with the report to
+// global memory and a loop of its own for the clock in each of them the kernels had 145 to 165 KB, more than the
+// instruction caches hold, and whatever ran once per work item came from L2 (75 KB now).
+__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, const Ctl& c, unsigned code, unsigned it) {
+    if (mbar_try(bar, parity)) return true;
+    const uint32_t t0 = (uint32_t)clock();
+    while (!mbar_try(bar, parity)) {
+        if (LCBSA_UNLIKELY(c.abort[0])) return false;
+        if (LCBSA_UNLIKELY((uint32_t)clock() - t0 > kWaitLimitCycles)) {
+            if (atomicCAS(const_cast<int*>(c.abort), 0, 1) == 0) {
+                c.abort[5] = threadIdx.x;
+                c.abort[6] = it;
+                c.abort[4] = code;
             }
-            __threadfence();
             return false;
         }
     }
-}
-// Bounded wait of one thread. Returns false when the CTA is aborting (this wait or another one ran out).
-// try_wait itself blocks for a hardware-defined interval, so the loop turns over rarely.
-__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, const Ctl& c, unsigned code, unsigned it) {
-    unsigned spins = 0;
-    while (!mbar_try(bar, parity)) {
-        if (LCBSA_UNLIKELY(*c.abort)) return false;
-        if (LCBSA_UNLIKELY(++spins >= kSpinsBeforeClock)) return mbar_wait_timeout(bar, parity, c, code, it);
-    }
     return true;
+}
+// One thread of the CTA, behind its last barrier: passes on what the first wait that ran out left in shared memory.
+__device__ __forceinline__ void ctl_report(const Ctl& c) {
+    if (LCBSA_UNLIKELY(c.abort[4])) {
+        if (atomicCAS(c.status, 0u, (unsigned)c.abort[4]) == 0u) {
+            c.status[1] = blockIdx.x;
+            c.status[2] = c.abort[5];
+            c.status[3] = c.abort[6];
+        }
+    }
 }
 // The same for all 32 lanes of a warp; the verdict is made warp-uniform so that the warp-collective
 // tcgen05 instructions that follow are never reached by only some of the lanes.
