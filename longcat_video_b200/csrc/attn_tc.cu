@@ -7,7 +7,7 @@
 //
 // Shape handled: head_dim 128 or 64, query and key blocks of 64 tokens, bf16 or fp16.  The figures below are those of
 // head_dim 128; at 64 a tile is one 64-column half, the rings have six slots, an S is half as many MMAs and a P V half as wide
-// (2 x 16 heads of a 12x16x24 grid in fp16, 18 of 72 blocks: 120 us, 255 us on the warp-level kernel that served it before).
+// (2 x 16 heads of a 12x16x24 grid in fp16, 18 of 72 blocks, whole call: 130 us, 151 us with the merge on the softmax warps).
 //
 // One persistent CTA per SM.  A work item is a pair of consecutive query blocks of one head.  Each
 // query block is a 64-row tile, i.e. an M=64 tcgen05 MMA whose accumulator occupies 16 lanes of every
@@ -16,14 +16,14 @@
 //
 // The selected K/V blocks of the pair are dealt alternately to two softmax warpgroups (even blocks to
 // warpgroup 0, odd blocks to warpgroup 1).  Each keeps its own running maximum, row sum and O accumulator,
-// and the two partial results are merged once at the end of the work item (as in split-KV decoding), so
-// the warpgroups never synchronise with each other inside the loop and one computes while the other waits.
+// and the two partial results are merged once at the end of the work item (as in split-KV decoding) by four warps of
+// their own, so the warpgroups never synchronise with each other inside the loop and one computes while the other waits.
 //
 //   warps 0-3, 4-7 : softmax warpgroups 0 and 1     warp 8  : TMA producer of Q and K
 //   warp 9         : S = Q K^T issuer               warp 10 : O += P V issuer
-//   warp 11        : TMA producer of V, output TMA stores
+//   warp 11        : TMA producer of V               warps 12-15 : Q to TMEM, merge and store of O (epilogue warps)
 //
-// Once per item the softmax warpgroups move the Q rows from shared memory to TMEM, where they are the A operand of
+// Once per item the epilogue warps move the Q rows from shared memory to TMEM, where they are the A operand of
 // every S of the item: with Q in shared memory an S reads as many bytes of Q as of K for every block.
 // Per block i (warpgroup g = i & 1):  S = Q K^T  (M64 N64 K128, A from TMEM, fp32 result in the warpgroup's S columns)
 // ->  the warpgroup reads S into registers with tcgen05.ld and releases the columns, so that the S of its next block is
@@ -35,9 +35,13 @@
 // divergent branch, needed about 950 cycles per ring slot and was what the rest waited for (V was requested 1700 cycles
 // after its P was ready).
 // What bounds it: M=64 MMAs, 16 x 32 + 8 x 64 = 1024 cycles of tensor pipe per block of a pair (an M=64 tile occupies the
-// pipe like an M=128 one); inside an item a block takes 1025 to 1040 cycles.  An item boundary costs some 8000 more, last PV
-// to first PV (the softmax warps merge and store O before they take up the next item).  Attention launch, 480p grid, 32
-// heads, 39 of 624 blocks: 2.25 ms with one producer warp and P over S, 1.91 ms now.
+// pipe like an M=128 one); inside an item a block takes 1025 to 1040 cycles.  K and V of the block come in at 64 bytes per
+// cycle and SM meanwhile, so tiles at the full rate would wait for L2.  An item boundary costs some 2700 cycles more (480p grid, 39
+// blocks per item: 42700 cycles per item by time stamps): PV of the next item waits for the epilogue warps to have read O.
+// It was 8000 when the softmax warps merged and stored O before they took up the next item and the kernel had 162 KB of code, more than
+// the instruction caches hold (68 KB now).  480p, 39 of 624 blocks, whole call with 8 heads: 565 us with both, 549 us with
+// the smaller code, 532 us with epilogue warps; 720p grid of 45 rows (ragged, masks in the softmax warps), 32 heads: 13095,
+// 12880, 11560 us.
 //
 // The MMAs are issued by whole converged warps with one elected lane (about 23 cycles per MMA for the
 // warp; a single lane inside a divergent branch needs 50 and more).
@@ -49,10 +53,10 @@
 // TMEM columns: O of warpgroup g at 128 * g (128 columns), its S at 256 + 64 * g, its P at 384 + 32 * g (two 16-bit
 // values per column), Q at 448 (64 columns of 16-bit pairs); the second tile of the pair 16 lanes up in each.
 //
-// At the end of a work item both warpgroups exchange (maximum, row sum) through shared memory, each merges
-// and normalises one 64-column half of O and stages it in the V slot that the last PV has released; it
-// leaves by TMA store.  The next item's Q goes to TMEM as soon as the last S of the item has been computed, so the
-// next item's K and S are in flight while this one finishes.
+// At the end of a work item the softmax warpgroups leave (maximum, row sum) in shared memory and go on with the next item, whose
+// Q the epilogue warps have moved to TMEM as soon as the last S of the item was computed.  The epilogue warps then merge and
+// normalise O, stage it in the Q buffer (which that Q has just left) and send it off by TMA store, after which the buffer
+// takes the Q of the item after the next.  PV of the next item starts when they have O in registers.
 //
 // Every wait on an mbarrier is bounded: when a wait runs out the CTA records where, raises an abort
 // flag that all roles poll, drains its outstanding bulk copies, frees its TMEM and returns.
@@ -68,12 +72,14 @@ using namespace tc;
 constexpr int kBlk = 64;                    // tokens per query / key block
 constexpr int kHalfBytes = kBlk * 128;      // one 64-column half of a tile: 64 rows x 128 B, 128B-swizzled
 constexpr int kTilesPerWork = 2;            // the two query blocks of a pair
-constexpr int kThreads = 384;
+constexpr int kThreads = 512;
 // Reference of a row whose blocks so far scored -inf throughout: finite, so that their probabilities are 0 and not NaN, and far
 // enough below every score that the first one above -inf replaces it.
 constexpr float kNoScore = -1e30f;
-// setmaxnreg per warpgroup: (208 + 208 + 88) * 128 threads <= the 64 K registers of the SM
-constexpr int kRegsSoftmax = 208, kRegsOther = 88;
+// setmaxnreg per warpgroup: (168 + 168 + 48 + 128) * 128 threads = the 64 K registers of the SM, 128 per thread at launch.  The
+// epilogue warps hold 32 columns of both accumulators: with 96 registers (and 184 for the softmax warps) the 720p grid takes 11300 us
+// instead of 11070.
+constexpr int kRegsSoftmax = 168, kRegsOther = 48, kRegsEpilogue = 128;
 
 // TMEM columns: O accumulator of warpgroup g at 128 * g, its S at 256 + 64 * g, its P (16-bit pairs) at 384 + 32 * g; Q (16-bit pairs)
 constexpr uint32_t kTmO = 0, kTmS = 256, kTmP = 384, kTmQ = 448;
@@ -93,7 +99,7 @@ template <int kD> struct Lay {
     static constexpr int offK = offQ + kTilesPerWork * tile;
     static constexpr int offV = offK + slots * slot;
     static constexpr int offBar = offV + slots * slot;
-    // barriers: k_full[slots] k_empty[slots] v_full[slots] v_empty[slots] q_full q_empty s_full[2] s_free[2] p_full[2] pv_done[2]
+    // barriers: k_full[slots] k_empty[slots] v_full[slots] v_empty[slots] q_full q_free s_full[2] s_free[2] p_full[2] pv_done[2]
     //           ml_ready o_free o_staged qt_full qt_free
     static constexpr int numBars = 4 * slots + 2 + 8 + 5;
     static constexpr int offMisc = offBar + numBars * 8;  // abort flag, TMEM base
@@ -103,7 +109,7 @@ template <int kD> struct Lay {
 };
 
 struct TcParams {
-    CUtensorMap tm_q, tm_k, tm_v;
+    CUtensorMap tm_q, tm_kv[2];  // [0]: K, [1]: V
     // Output maps.  Normally one (tm_o[0]).  With o_frames > 0 the query grid is the rank-major grid of a
     // context-parallel group: frames [r * o_frames, (r + 1) * o_frames) are the tokens of rank r, and the rows of a
     // query block are stored straight into rank r's result buffer (its own map, over this GPU's or a peer's memory).
@@ -146,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     auto bar_v_full = [&](int s) { return bar0 + 8u * (2 * kKSlots + s); };
     auto bar_v_empty = [&](int s) { return bar0 + 8u * (2 * kKSlots + kVSlots + s); };
     constexpr int kB0 = 2 * kKSlots + 2 * kVSlots;
-    const uint32_t bar_q_full = bar0 + 8u * kB0, bar_q_empty = bar0 + 8u * (kB0 + 1);
+    const uint32_t bar_q_full = bar0 + 8u * kB0, bar_q_free = bar0 + 8u * (kB0 + 1);
     auto bar_s_full = [&](int wg) { return bar0 + 8u * (kB0 + 2 + wg); };
     auto bar_s_free = [&](int wg) { return bar0 + 8u * (kB0 + 4 + wg); };
     auto bar_p_full = [&](int wg) { return bar0 + 8u * (kB0 + 6 + wg); };
@@ -174,18 +180,18 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             mbar_init(bar_v_empty(s), 1);
         }
         mbar_init(bar_q_full, 1);
-        mbar_init(bar_q_empty, 8);
+        mbar_init(bar_q_free, 1);
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar_s_full(b), kRagged ? 2 : 1);  // the MMAs; ragged grids: and the issuer, for the masks
             mbar_init(bar_s_free(b), 4);
             mbar_init(bar_p_full(b), 4);  // one elected arrival per softmax warp
             mbar_init(bar_pv_done(b), 1);
         }
-        mbar_init(bar_qt_full, 8);
+        mbar_init(bar_qt_full, 4);
         mbar_init(bar_qt_free, 1);
         mbar_init(bar_ml_ready, 8);
-        mbar_init(bar_o_free, 8);
-        mbar_init(bar_o_staged, 8);
+        mbar_init(bar_o_free, 4);
+        mbar_init(bar_o_staged, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // The tiles are 128B-swizzled, which ties their layout to address bits 7-9: without a 1024-byte aligned
         // base nothing below is valid.  The declaration asks for it; refuse to run if it was not honoured.
@@ -209,7 +215,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     const bool start_ok = *abort_flag == 0;
 
     const int groups = (P.nq + kTilesPerWork - 1) / kTilesPerWork;
-    const long long total_work = start_ok ? (long long)P.bh_total * groups : 0;
+    const int total_work = start_ok ? P.bh_total * groups : 0;  // q alone has 32 KB per item, so this is far below 2^31
     // The CTA's items are blockIdx.x, blockIdx.x + gridDim.x, ...; every role steps through them as (head, group) pairs, since a
     // 64-bit division per role and item costs more than a round.
     const int first_bh = (int)(blockIdx.x / (unsigned)groups), first_g = (int)(blockIdx.x % (unsigned)groups);
@@ -227,27 +233,139 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
     // All roles walk the same list of work items and blocks.  Block number gb (counted over the whole kernel)
     // uses slot gb % slots of the K ring and of the V ring.  Within an item block i belongs to warpgroup i & 1, which numbers its own rounds rr
     // over the whole kernel.
-    if (warp >= 8) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-      if (warp == 8 || warp == 11) {
-        // ================================================================== TMA producers: warp 8 Q and K, warp 11 V and the output
-        // The output rows of an item are staged in the V slot its last PV released.  Warp 11 sends them off when it needs
-        // that slot again, at the latest before it requests the last V of the item behind it (the epilogue of that item
-        // completes the next phase of o_staged, so the wait is never a phase behind).
-        const bool is_k = warp == 8;
-        unsigned gk = 0, gv = 0, wk = 0, nq_issued = 0;
-        int s_bh = first_bh, s_g = first_g;  // item whose output is stored next
-        unsigned ws_end = 0, ks = 0;        // blocks up to and including it, its number
+    if (warp >= 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
+        // ================================================================== epilogue warps
+        // Between two items: Q of the next one from shared memory to TMEM as soon as the last S of the current one has read
+        // the columns, then the merge of the two partial results, staged in the Q buffer that has just become free (a thread
+        // writes the row that it read Q from) and sent off by TMA store.  The softmax warps meanwhile go on with the next item.
+        const int wq = warp & 3;          // TMEM quadrant of this warp
+        const int hf = lane >> 4;         // tile of the pair this lane serves
+        const int row = wq * 16 + (lane & 15);  // row of that tile
+        const uint32_t t_lane = (uint32_t)(wq * 32) << 16;
+        const int ml_idx = wq * 32 + lane;
+        unsigned char* const buf = smem + kOffQ + hf * kTileBytes + row * 128;  // this thread's row: chunk c at 16 * (c ^ (row & 7)), halves kHalfBytes apart
+        unsigned wk = 0, rr0 = 0, rr1 = 0;  // rounds of the two softmax warpgroups over the whole kernel
         bool ok = true;
-        auto store_item = [&]() -> bool {
-            const int bh = s_bh, g = s_g;
-            const int b = bh / P.heads, h = bh % P.heads;
-            if (!mbar_wait_warp(bar_o_staged, ks & 1, ctl, 110, ks)) return false;
-            if (lane == 0) {
-                const unsigned last = ws_end - 1;
-                for (int hf = 0; hf < 2; ++hf) {
-                    const int qq = g * kTilesPerWork + hf;
-                    if (qq >= P.nq) continue;
+        auto q_to_tmem = [&](unsigned item) -> bool {  // Q of the CTA's work item number `item`
+            // the last S of the item before has read the columns
+            if (item > 0 && !mbar_wait_warp(bar_qt_free, (item - 1) & 1, ctl, 106, item)) return false;
+            if (!mbar_wait_warp(bar_q_full, item & 1, ctl, 108, item)) return false;
+            tc_fence_after();
+#pragma unroll 1
+            for (int half = 0; half < kHalves; ++half) {
+                uint32_t qr[32];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(buf + half * kHalfBytes + ((c ^ (row & 7)) << 4));
+                    qr[4 * c + 0] = v.x;
+                    qr[4 * c + 1] = v.y;
+                    qr[4 * c + 2] = v.z;
+                    qr[4 * c + 3] = v.w;
+                }
+                tc_st32(tmem + kTmQ + 32u * half + t_lane, qr);
+            }
+            tc_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            mbar_arrive_elect(bar_qt_full);
+            return true;
+        };
+        int bh = 0, g = 0, nx_bh = first_bh, nx_g = first_g, my_n = 0, other_n = 0;
+        auto peek = [&](bool there) {  // list lengths of item nx, read one item ahead
+            if (there) {
+                my_n = clamp_cnt(P, nx_bh, nx_g * kTilesPerWork + hf);
+                other_n = clamp_cnt(P, nx_bh, nx_g * kTilesPerWork + (hf ^ 1));
+            }
+        };
+        peek(blockIdx.x < total_work);
+        int my_cnt = 0, n_iter = 0;
+        for (int w = blockIdx.x;; w += gridDim.x) {  // item w gets its Q, the one before (number wk) is finished
+            const bool there = w < total_work;
+            const bool start = w == blockIdx.x;
+            if (there && !q_to_tmem(start ? 0 : wk + 1)) break;
+            if (!start) {
+            rr0 += (n_iter + 1) >> 1;
+            rr1 += n_iter >> 1;
+
+            // Both warpgroups have stored their last P, hence seen every PV but their last finish; no PV of the next item starts
+            // before o_free, so the waits below are for exactly the item's last PVs.
+            ok = mbar_wait_warp(bar_ml_ready, wk & 1, ctl, 104, wk);
+            if (!ok) break;
+            const float2 ml0 = ml[ml_idx], ml1 = ml[128 + ml_idx];
+            // merged scale of both partial sums: everything relative to the larger reference maximum.  A row with a NaN or an
+            // infinite score has a NaN sum and comes out as NaN, like on the warp-level kernel; a warpgroup that saw no block has
+            // the maximum -inf, hence the weight 0.
+            const float m_all = fmaxf(ml0.x, ml1.x), m_base = m_all == -INFINITY ? 0.f : m_all;
+            const float w0 = ex2(ml0.x - m_base), w1 = ex2(ml1.x - m_base);
+            // the accumulator of a warpgroup that saw no block holds garbage and is not used
+            const bool saw0 = my_cnt > 0, saw1 = my_cnt > 1;
+            const bool rd0 = __any_sync(0xffffffffu, saw0), rd1 = __any_sync(0xffffffffu, saw1);
+            const bool both = __all_sync(0xffffffffu, saw1);  // the usual case: no lane has to be masked
+            const float l_all = ml0.y * w0 + ml1.y * w1;
+            const float inv = l_all == 0.f ? 0.f : 1.f / l_all;
+            const float f0 = w0 * inv, f1 = w1 * inv;
+            const float2 f0_2 = make_float2(f0, f0), f1_2 = make_float2(f1, f1);
+            ok = mbar_wait_warp(bar_pv_done(0), (rr0 - 1) & 1, ctl, 100, wk);
+            if (ok && n_iter > 1) ok = mbar_wait_warp(bar_pv_done(1), (rr1 - 1) & 1, ctl, 101, wk);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t tm_o = tmem + kTmO + t_lane;
+#pragma unroll 1
+            for (int cch = 0; cch < kD / 32; ++cch) {
+                uint32_t oa[32], ob[32];
+                if (rd0) tc_ld32(tm_o + 32 * cch, oa);
+                if (rd1) tc_ld32(tm_o + 128 + 32 * cch, ob);
+                tc_wait_ld();
+                if (cch == kD / 32 - 1) {  // both O accumulators may be overwritten by the next item's first PVs
+                    tc_fence_before();
+                    __syncwarp();
+                    mbar_arrive_elect(bar_o_free);
+                }
+                if (LCBSA_UNLIKELY(!both)) {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        if (!saw0) oa[j] = 0u;
+                        if (!saw1) ob[j] = 0u;
+                    }
+                }
+                // the rows of a second tile that does not exist are written too; nobody stores them
+                unsigned char* const half = buf + (cch >> 1) * kHalfBytes;
+#pragma unroll
+                for (int q8 = 0; q8 < 4; ++q8) {
+                    uint32_t pw[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int e = q8 * 8 + 2 * j;
+                        const float2 a2 = __fmul2_rn(make_float2(__uint_as_float(oa[e]), __uint_as_float(oa[e + 1])), f0_2);
+                        const float2 v2 = __ffma2_rn(make_float2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), f1_2, a2);
+                        pw[j] = pack2(bf16, v2.x, v2.y);
+                    }
+                    const int chunk = (cch & 1) * 4 + q8;
+                    *reinterpret_cast<uint4*>(half + ((chunk ^ (row & 7)) << 4)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
+                }
+            }
+            fence_proxy_async();
+            __syncwarp();
+            mbar_arrive_elect(bar_o_staged);
+            const int qt = g * kTilesPerWork + hf;
+            if (P.lse != nullptr && qt < P.nq) {
+                int lt, lh, lw, bt, bhh, bw;
+                slot_coords(P.gq, row, lt, lh, lw);
+                block_coords(P.gq, qt, bt, bhh, bw);
+                const int tt = bt * P.gq.ct + lt, hh = bhh * P.gq.ch + lh, ww = bw * P.gq.cw + lw;
+                if (tt < P.gq.T && hh < P.gq.H && ww < P.gq.W) {
+                    const long long Sq = (long long)P.gq.T * P.gq.H * P.gq.W;
+                    const long long tok = ((long long)tt * P.gq.H + hh) * P.gq.W + ww;
+                    P.lse[(long long)bh * Sq + tok] = l_all > 0.f ? (m_all + log2f(l_all)) * 0.6931471805599453f : -INFINITY;
+                }
+            }
+            if (warp == 12) {  // the rows of all four warps are staged: off they go, then the buffer takes the Q after the next
+                ok = mbar_wait_warp(bar_o_staged, wk & 1, ctl, 110, wk);
+                if (!ok) break;
+                const int qq = g * kTilesPerWork + lane;
+                if (lane < 2 && qq < P.nq) {  // a tile each
+                    const int b = bh / P.heads, h = bh - b * P.heads;
                     Coord cc = block_coord(P.gq, qq, b, h, P.heads, P.merge_o, P.Tq);
                     const CUtensorMap* tmo = &P.tm_o[0];
                     if (P.o_frames > 0) {  // blocks never straddle ranks: o_frames is a multiple of the block's frames
@@ -255,19 +373,53 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                         cc.c3 -= dst * P.o_frames;
                         tmo = &P.tm_o[dst];
                     }
-                    const uint32_t src = sbase + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes;
+                    const uint32_t src = sbase + kOffQ + lane * kTileBytes;
                     tma_store_5d(tmo, src, 0, cc.c1, cc.c2, cc.c3, cc.c4);
                     if (kHalves == 2) tma_store_5d(tmo, src + kHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+                    tma_store_commit();
+                    tma_store_wait_read();
                 }
-                tma_store_commit();
-                tma_store_wait_read();
-                mbar_arrive(bar_v_empty(last % kVSlots));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_q_free);
             }
+            ++wk;
+            }
+            if (!there) break;
+            bh = nx_bh;
+            g = nx_g;
+            my_cnt = my_n;
+            n_iter = max(1, max(my_n, other_n));
+            next_item(nx_bh, nx_g);
+            peek(w + gridDim.x < total_work);
+        }
+        if (warp == 12 && lane < 2) tma_store_wait_all();
+    } else if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
+      if (warp == 8 || warp == 11) {
+        // ================================================================== TMA producers: warp 8 Q and K, warp 11 V
+        const bool is_k = warp == 8;
+        // One code path for both rings: they have the same number of slots of the same size.
+        const uint32_t ring = sbase + (is_k ? kOffK : kOffV), full0 = is_k ? bar_k_full(0) : bar_v_full(0), empty0 = is_k ? bar_k_empty(0) : bar_v_empty(0);
+        unsigned gk = 0, wk = 0, nq_issued = 0;  // gk: blocks requested over the whole kernel
+        int slot = 0;
+        unsigned parity = 1;  // of the wait on an empty slot: the ring starts empty
+        bool ok = true;
+        // Q tiles of item (bh, g) into the Q buffer, one by lane 0 and one by lane 1
+        auto request_q = [&](int bh, int g) {
+            const int qt = g * kTilesPerWork + lane;
+            if (lane == 0) mbar_arrive_tx(bar_q_full, min(P.nq - qt, 2) * kTileBytes);
             __syncwarp();
-            next_item(s_bh, s_g);
-            ++ks;
-            return true;
+            if (lane < 2 && qt < P.nq) {
+                const int b = bh / P.heads, h = bh - b * P.heads;
+                const Coord cc = block_coord(P.gq, qt, b, h, P.heads, P.merge_q, P.Tq);
+                const uint32_t dst = sbase + kOffQ + lane * kTileBytes;
+                tma_load_5d(dst, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
+                if (kHalves == 2) tma_load_5d(dst + kHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+            }
+            ++nq_issued;
+            __syncwarp();
         };
+        if (is_k && blockIdx.x < total_work) request_q(first_bh, first_g);
         int bh = first_bh, g = first_g, nx_bh = first_bh, nx_g = first_g;
         int ca_n = 0, cb_n = 0;
         auto peek = [&](bool there) {  // list lengths of item nx, read one item ahead
@@ -277,9 +429,18 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             }
         };
         peek(blockIdx.x < total_work);
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, g = nx_g) {
+        // The first two windows of an item's list are read while the item before is under way: reading them at its start
+        // kept the ring waiting for some 800 cycles.
+        int raw0 = 0, raw1 = 0;
+        auto load_ahead = [&](int bh, int g, int ca, int cb) {
+            const int t = lane & 1, it = lane >> 1, c = t ? cb : ca;
+            const int32_t* l = P.idx + ((long long)bh * P.nq + min(g * kTilesPerWork + t, P.nq - 1)) * P.cap;
+            if (it < c) raw0 = l[it];
+            if (16 + it < c) raw1 = l[16 + it];
+        };
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, g = nx_g) {
             const int b = bh / P.heads, h = bh % P.heads;
-            const int qa = g * kTilesPerWork, qb = qa + 1;
+            const int qa = g * kTilesPerWork;
             const int ca = ca_n, cb = cb_n;
             const int n_iter = max(1, max(ca, cb));
             // Block coordinates are fetched and decoded by the whole warp: lane L holds, for tile (L & 1) and
@@ -288,9 +449,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             const int my_t = lane & 1, my_s = lane >> 1;
             const int my_c = my_t ? cb : ca;
             const int32_t* my_l = P.idx + ((long long)bh * P.nq + min(qa + my_t, P.nq - 1)) * P.cap;
-            auto fetch = [&](int it) {
+            auto decode = [&](int blk, int it) {  // list entry `it` of the lane's tile
                 if (it >= my_c) return 0;
-                const int blk = my_l[it];
                 if ((unsigned)blk >= (unsigned)P.gk.nblk) {
                     // A list entry outside [0, Nk) never becomes an address: its box is placed at w = W, wholly
                     // outside the tensor map, so TMA fills the tile with zeros; the call is flagged.
@@ -305,91 +465,74 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                 block_coords(P.gk, blk, bt, bhh, bw);
                 return ((bt * P.gk.ct) << 20) | ((bhh * P.gk.ch) << 10) | (bw * P.gk.cw);
             };
-            int cur = fetch(my_s);
-            int nxt = fetch(16 + my_s);
+            if (wk == 0) load_ahead(bh, g, ca, cb);
+            int cur = decode(raw0, my_s);
+            int nxt = decode(raw1, 16 + my_s);
             next_item(nx_bh, nx_g);
-            peek(w + gridDim.x < total_work);
+            const bool more_items = w + gridDim.x < total_work;
+            peek(more_items);
             const bool mrg = is_k ? P.merge_k : P.merge_v;
             const int c3 = mrg ? b * P.Tk : 0, c4 = mrg ? h : b * P.heads + h;
             // the boxes of both query blocks' tiles of list position j into ring slot `dst`
             auto request = [&](int j, const CUtensorMap* tm, uint32_t bar, uint32_t dst) {
                 const int pa = __shfl_sync(0xffffffffu, cur, (j & 15) << 1), pb = __shfl_sync(0xffffffffu, cur, ((j & 15) << 1) | 1);
                 mbar_arrive_tx_elect(bar, ((j < ca) + (j < cb)) * kTileBytes);
-                if (j < ca) {
-                    tma_load_5d_elect(dst, tm, bar, 0, pa & 1023, (pa >> 10) & 1023, (pa >> 20) + c3, c4);
-                    if (kHalves == 2) tma_load_5d_elect(dst + kHalfBytes, tm, bar, 64, pa & 1023, (pa >> 10) & 1023, (pa >> 20) + c3, c4);
+#pragma unroll 1
+                for (int t = 0; t < 2; ++t, dst += kTileBytes) {
+                    if (j >= (t ? cb : ca)) continue;
+                    const int pt = t ? pb : pa;
+                    tma_load_5d_elect(dst, tm, bar, 0, pt & 1023, (pt >> 10) & 1023, (pt >> 20) + c3, c4);
+                    if (kHalves == 2) tma_load_5d_elect(dst + kHalfBytes, tm, bar, 64, pt & 1023, (pt >> 10) & 1023, (pt >> 20) + c3, c4);
                 }
-                if (j < cb) {
-                    tma_load_5d_elect(dst + kTileBytes, tm, bar, 0, pb & 1023, (pb >> 10) & 1023, (pb >> 20) + c3, c4);
-                    if (kHalves == 2) tma_load_5d_elect(dst + kTileBytes + kHalfBytes, tm, bar, 64, pb & 1023, (pb >> 10) & 1023, (pb >> 20) + c3, c4);
+            };
+            // ragged grids: which keys of this lane's list entry lie inside the grid (decoded here once per entry; the softmax
+            // warps spent two divisions per round and thread on it)
+            auto entry_mask = [&]() {
+                return slot_mask64(P.gk.ct, P.gk.ch, P.gk.cw, P.gk.T - (cur >> 20), P.gk.H - ((cur >> 10) & 1023), P.gk.W - (cur & 1023));
+            };
+            unsigned long long my_mask = kRagged ? entry_mask() : 0ull;
+            bool q_due = is_k && more_items;  // Q of the next item has not been requested yet
+#pragma unroll 1
+            for (int j = 0; j < n_iter; ++j) {
+                // Q of the next item as soon as the buffer is free again (see the epilogue warps), which is early in this
+                // item; behind the last chance for it comes the item's last K.
+                if (q_due) {
+                    const uint32_t bar = wk == 0 ? bar_qt_full : bar_q_free, ph = wk == 0 ? 0 : (wk - 1) & 1;
+                    bool go = __all_sync(0xffffffffu, mbar_test(bar, ph));
+                    if (!go && j == n_iter - 1) {
+                        ok = go = mbar_wait_warp(bar, ph, ctl, 10, wk);
+                        if (!ok) break;
+                    }
+                    if (go) {
+                        request_q(nx_bh, nx_g);
+                        q_due = false;
+                    }
+                }
+                if (j == min(2, n_iter - 1) && more_items) load_ahead(nx_bh, nx_g, ca_n, cb_n);
+                ok = mbar_wait_warp(empty0 + 8u * slot, parity, ctl, is_k ? 20 : 22, gk);
+                if (!ok) break;
+                if (kRagged && is_k) {
+                    if (my_s == (j & 15)) masks[(gk % kMaskRing) * 2 + my_t] = my_mask;
+                    __syncwarp();
+                }
+                request(j, &P.tm_kv[is_k ? 0 : 1], full0 + 8u * slot, ring + slot * kSlotBytes);
+                ++gk;
+                if (++slot == kKSlots) {
+                    slot = 0;
+                    parity ^= 1;
                 }
                 if ((j & 15) == 15) {
                     cur = nxt;
-                    nxt = fetch(j + 17 + my_s);
+                    nxt = decode(j + 17 + my_s < my_c ? my_l[j + 17 + my_s] : 0, j + 17 + my_s);
+                    if (kRagged) my_mask = entry_mask();
                 }
-            };
-            if (is_k) {
-                // Q tiles: the buffer is free once the softmax warps have moved the previous item's Q to TMEM
-                ok = mbar_wait_warp(bar_q_empty, (wk & 1) ^ 1, ctl, 10, wk);
-                if (!ok) break;
-                ++nq_issued;
-                if (lane == 0) {
-                    const int ntile = (qa < P.nq) + (qb < P.nq);
-                    mbar_arrive_tx(bar_q_full, ntile * kTileBytes);
-                    for (int hf = 0; hf < 2; ++hf) {
-                        const int qt = qa + hf;
-                        if (qt >= P.nq) continue;
-                        const Coord cc = block_coord(P.gq, qt, b, h, P.heads, P.merge_q, P.Tq);
-                        const uint32_t dst = sbase + kOffQ + hf * kTileBytes;
-                        tma_load_5d(dst, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                        if (kHalves == 2) tma_load_5d(dst + kHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
-                    }
-                }
-                __syncwarp();
-                // ragged grids: which keys of this lane's list entry lie inside the grid (decoded here once per entry; the softmax
-                // warps spent two divisions per round and thread on it: 720p with 45 rows, 8 heads, 2.73 ms, 2.61 ms with masks
-                // from here and the single copy of the pass below)
-                auto entry_mask = [&]() {
-                    return slot_mask64(P.gk.ct, P.gk.ch, P.gk.cw, P.gk.T - (cur >> 20), P.gk.H - ((cur >> 10) & 1023), P.gk.W - (cur & 1023));
-                };
-                unsigned long long my_mask = kRagged ? entry_mask() : 0ull;
-                for (int j = 0; j < n_iter; ++j) {
-                    const int slot = gk % kKSlots;
-                    ok = mbar_wait_warp(bar_k_empty(slot), ((gk / kKSlots) & 1) ^ 1, ctl, 20, gk);
-                    if (!ok) break;
-                    if (kRagged) {
-                        if (my_s == (j & 15)) masks[(gk % kMaskRing) * 2 + my_t] = my_mask;
-                        __syncwarp();
-                    }
-                    ++gk;
-                    request(j, &P.tm_k, bar_k_full(slot), sbase + kOffK + slot * kSlotBytes);
-                    if (kRagged && (j & 15) == 15) my_mask = entry_mask();
-                }
-            } else {
-                for (int j = 0; j < n_iter; ++j) {
-                    if (ks < wk && (gv >= ws_end - 1 + kVSlots || j == n_iter - 1)) {
-                        ok = store_item();
-                        if (!ok) break;
-                    }
-                    const int slot = gv % kVSlots;
-                    ok = mbar_wait_warp(bar_v_empty(slot), ((gv / kVSlots) & 1) ^ 1, ctl, 22, gv);
-                    if (!ok) break;
-                    ++gv;
-                    request(j, &P.tm_v, bar_v_full(slot), sbase + kOffV + slot * kSlotBytes);
-                }
-                ws_end = gv;  // the item before has been stored
             }
         }
-        if (!is_k && ok && ks < wk) ok = store_item();
-        if (!is_k && lane == 0) tma_store_wait_all();
         if (!ok && lane == 0) {
             // drain: give the copies this warp issued a bounded time to land before the CTA exits
             const long long t0 = clock64();
             for (unsigned r = gk > kKSlots ? gk - kKSlots : 0; r < gk; ++r)
-                while (!mbar_try(bar_k_full(r % kKSlots), (r / kKSlots) & 1) && clock64() - t0 < 40000000ll) {
-                }
-            for (unsigned r = gv > kVSlots ? gv - kVSlots : 0; r < gv; ++r)
-                while (!mbar_try(bar_v_full(r % kVSlots), (r / kVSlots) & 1) && clock64() - t0 < 40000000ll) {
+                while (!mbar_try(full0 + 8u * (r % kKSlots), (r / kKSlots) & 1) && clock64() - t0 < 40000000ll) {
                 }
             if (nq_issued > 0)
                 while (!mbar_try(bar_q_full, (nq_issued - 1) & 1) && clock64() - t0 < 40000000ll) {
@@ -408,7 +551,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             next_item(bh, g);
         };
         peek(blockIdx.x < total_work);
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
             const int ca = ca_n, cb = cb_n;
             peek(w + gridDim.x < total_work);
             const int n_iter = max(1, max(ca, cb));
@@ -469,7 +612,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             next_item(bh, g);
         };
         peek(blockIdx.x < total_work);
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
             const int ca = ca_n, cb = cb_n;
             peek(w + gridDim.x < total_work);
             const int n_iter = max(1, max(ca, cb));
@@ -504,8 +647,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
                     for (int j = 0; j < kBlk / 16; ++j)
                         tc_mma_ts(d, pa + 8u * j, vd + (uint64_t)((j * 2048) >> 4), idesc_pv, (i > 1 || j > 0) ? 1u : 0u);
                 }
-                // the V slot of the item's last block goes to the epilogue, which stages O in it and frees it
-                if (i < n_iter - 1) tc_commit(bar_v_empty(slot));
+                tc_commit(bar_v_empty(slot));
                 tc_commit(bar_pv_done(wg));
                 __syncwarp();
                 if (wg) ++rr1; else ++rr0;
@@ -519,43 +661,12 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
         const int wg = warp >> 2;         // warpgroup: takes blocks wg, wg + 2, ... of every work item
         const int wq = warp & 3;          // TMEM quadrant of this warp
         const int hf = lane >> 4;         // tile of the pair this lane serves
-        const int row = wq * 16 + (lane & 15);  // row of that tile
         const uint32_t t_lane = (uint32_t)(wq * 32) << 16;
         const uint32_t tm_s = tmem + kTmS + 64u * wg + t_lane, tm_p = tmem + kTmP + 32u * wg + t_lane;
-        const uint32_t tm_o_mine = tmem + kTmO + 128u * wg + t_lane, tm_o_other = tmem + kTmO + 128u * (wg ^ 1) + t_lane;
+        const uint32_t tm_o_mine = tmem + kTmO + 128u * wg + t_lane;
         const int ml_idx = wq * 32 + lane;
         unsigned wk = 0, gb = 0, rr = 0;  // rr: rounds of this warpgroup over the whole kernel
         bool ok = true;
-
-        // Q of the CTA's work item number `item` from shared memory to TMEM: a thread moves its row, the warpgroup half of the columns.
-        auto q_to_tmem = [&](unsigned item) -> bool {
-            // the last S of the item before has read the columns
-            if (item > 0 && !mbar_wait_warp(bar_qt_free, (item - 1) & 1, ctl, 106 + wg, item)) return false;
-            if (!mbar_wait_warp(bar_q_full, item & 1, ctl, 108 + wg, item)) return false;
-            tc_fence_after();
-            // head_dim 128: the warpgroup's 64-column half, eight chunks of 16 bytes; 64: its four chunks of the only half
-            constexpr int kChunks = kD / 16;
-            const unsigned char* src = smem + kOffQ + hf * kTileBytes + (kD == 128 ? wg * kHalfBytes : 0) + row * 128;
-            const int c0 = kD == 128 ? 0 : 4 * wg;
-            uint32_t qr[4 * kChunks];
-#pragma unroll
-            for (int c = 0; c < kChunks; ++c) {
-                const uint4 v = *reinterpret_cast<const uint4*>(src + (((c0 + c) ^ (row & 7)) << 4));
-                qr[4 * c + 0] = v.x;
-                qr[4 * c + 1] = v.y;
-                qr[4 * c + 2] = v.z;
-                qr[4 * c + 3] = v.w;
-            }
-            if constexpr (kD == 128) tc_st32(tmem + kTmQ + 32u * wg + t_lane, qr);
-            else tc_st16(tmem + kTmQ + 16u * wg + t_lane, qr);
-            tc_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            mbar_arrive_elect(bar_q_empty);
-            mbar_arrive_elect(bar_qt_full);
-            return true;
-        };
-        if (blockIdx.x < total_work) ok = q_to_tmem(0);
 
         int bh = first_bh, g = first_g, nx_bh = first_bh, nx_g = first_g, my_n = 0, other_n = 0;
         auto peek = [&](bool there) {  // list lengths of item nx, read one item ahead
@@ -565,9 +676,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             }
         };
         peek(blockIdx.x < total_work);
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, g = nx_g) {
-            const int qt = g * kTilesPerWork + hf;
-            const bool tile_valid = qt < P.nq;
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, g = nx_g) {
             const int my_cnt = my_n, other_cnt = other_n;
             next_item(nx_bh, nx_g);
             peek(w + gridDim.x < total_work);
@@ -734,90 +843,17 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             }
             if (!ok) break;
             gb += n_iter;
-            // Q of the next item, so that its S runs under this item's epilogue
-            if (w + gridDim.x < total_work && !q_to_tmem(wk + 1)) break;
-
-            // ---- epilogue of this work item.  The warpgroup's PVs are finished once its last one is; it then
-            // publishes (maximum, row sum) of its rows and waits for the other warpgroup to do the same.
-            if (n_iter > wg) {
-                ok = mbar_wait_warp(bar_pv_done(wg), (rr - 1) & 1, ctl, 100 + wg, rr);
-                if (!ok) break;
-            }
-            // the other warpgroup has read this warpgroup's entry of the previous item before it arrived on o_free
+            // The epilogue warps merge this item's partial results; they have read the (maximum, row sum) of the item before once
+            // they have arrived on o_free.
             if (wk > 0) {
-                ok = mbar_wait_warp(bar_o_free, (wk - 1) & 1, ctl, 102 + wg, wk);
-                if (!ok) break;
+                if (!__all_sync(0xffffffffu, mbar_test(bar_o_free, (wk - 1) & 1))) {
+                    ok = mbar_wait_warp(bar_o_free, (wk - 1) & 1, ctl, 102 + wg, wk);
+                    if (!ok) break;
+                }
             }
             ml[wg * 128 + ml_idx] = make_float2(m_ref, l_sum);
             __syncwarp();
             mbar_arrive_elect(bar_ml_ready);
-            ok = mbar_wait_warp(bar_ml_ready, wk & 1, ctl, 104 + wg, wk);
-            if (!ok) break;
-            tc_fence_after();
-            const float2 oth = ml[(wg ^ 1) * 128 + ml_idx];
-            // merged scale of both partial sums: everything relative to the larger reference maximum.  A row with a NaN or an
-            // infinite score has a NaN sum and comes out as NaN, like on the warp-level kernel; a warpgroup that saw no block has
-            // the maximum -inf, hence the weight 0.
-            const float m_all = fmaxf(m_ref, oth.x), m_base = m_all == -INFINITY ? 0.f : m_all;
-            const float w_mine = ex2(m_ref - m_base), w_oth = ex2(oth.x - m_base);
-            const float l_all = l_sum * w_mine + oth.y * w_oth;
-            const float inv = l_all == 0.f ? 0.f : 1.f / l_all;
-            const float f_mine = w_mine * inv, f_oth = w_oth * inv;
-            // This warpgroup merges and stages half of the columns of O (input dtype, 128B-swizzled rows of 64 columns) in the V slot that the item's last PV has just released.
-            const unsigned last = gb - 1;
-            unsigned char* o_half = smem + kOffV + (last % kVSlots) * kSlotBytes + hf * kTileBytes + (kD == 128 ? wg * kHalfBytes : 0);
-            constexpr int kMine = kD / 2;  // columns kMine * wg ..
-            // the accumulator of a warpgroup that saw no block holds garbage and is not used
-            const bool saw_mine = my_cnt > wg, saw_oth = my_cnt > (wg ^ 1);
-            const bool rd_mine = __any_sync(0xffffffffu, saw_mine), rd_oth = __any_sync(0xffffffffu, saw_oth);
-            const bool both = __all_sync(0xffffffffu, saw_mine && saw_oth);  // the usual case: no lane has to be masked
-            const float2 fm2 = make_float2(f_mine, f_mine), fo2 = make_float2(f_oth, f_oth);
-#pragma unroll
-            for (int cch = 0; cch < kMine / 32; ++cch) {
-                uint32_t oa[32], ob[32];
-                if (rd_mine) tc_ld32(tm_o_mine + kMine * wg + 32 * cch, oa);
-                if (rd_oth) tc_ld32(tm_o_other + kMine * wg + 32 * cch, ob);
-                tc_wait_ld();
-                if (LCBSA_UNLIKELY(!both)) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        if (!saw_mine) oa[j] = 0u;
-                        if (!saw_oth) ob[j] = 0u;
-                    }
-                }
-                if (tile_valid) {
-#pragma unroll
-                    for (int q8 = 0; q8 < 4; ++q8) {
-                        uint32_t pw[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int e = q8 * 8 + 2 * j;
-                            const float2 a2 = __fmul2_rn(make_float2(__uint_as_float(oa[e]), __uint_as_float(oa[e + 1])), fm2);
-                            const float2 v2 = __ffma2_rn(make_float2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), fo2, a2);
-                            pw[j] = pack2(bf16, v2.x, v2.y);
-                        }
-                        const int chunk = (kD == 128 ? 0 : 4 * wg) + cch * 4 + q8;
-                        *reinterpret_cast<uint4*>(o_half + row * 128 + ((chunk ^ (row & 7)) << 4)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            mbar_arrive_elect(bar_o_free);  // both O accumulators may be overwritten by the next item's first PVs
-            if (wg == 0 && P.lse != nullptr && tile_valid) {
-                int lt, lh, lw, bt, bhh, bw;
-                slot_coords(P.gq, row, lt, lh, lw);
-                block_coords(P.gq, qt, bt, bhh, bw);
-                const int tt = bt * P.gq.ct + lt, hh = bhh * P.gq.ch + lh, ww = bw * P.gq.cw + lw;
-                if (tt < P.gq.T && hh < P.gq.H && ww < P.gq.W) {
-                    const long long Sq = (long long)P.gq.T * P.gq.H * P.gq.W;
-                    const long long tok = ((long long)tt * P.gq.H + hh) * P.gq.W + ww;
-                    P.lse[(long long)bh * Sq + tok] = l_all > 0.f ? (m_all + log2f(l_all)) * 0.6931471805599453f : -INFINITY;
-                }
-            }
-            fence_proxy_async();
-            __syncwarp();
-            mbar_arrive_elect(bar_o_staged);  // the store warp takes it from here
         }
     }
 
@@ -887,8 +923,8 @@ cudaError_t launch_attn_tc(const AttnArgs& a, cudaStream_t st, const char** why)
     TcParams P;
     const int mq = merge_mode(a.q, a.B, a.H, a.gq), mk = merge_mode(a.k, a.B, a.H, a.gk);
     const int mv = merge_mode(a.v, a.B, a.H, a.gk), mo = merge_mode(a.o, a.B, a.H, a.gq);
-    if (!make_map(&P.tm_q, a.dtype, a.q, a.B, a.H, a.gq, mq, a.D) || !make_map(&P.tm_k, a.dtype, a.k, a.B, a.H, a.gk, mk, a.D) ||
-        !make_map(&P.tm_v, a.dtype, a.v, a.B, a.H, a.gk, mv, a.D)) {
+    if (!make_map(&P.tm_q, a.dtype, a.q, a.B, a.H, a.gq, mq, a.D) || !make_map(&P.tm_kv[0], a.dtype, a.k, a.B, a.H, a.gk, mk, a.D) ||
+        !make_map(&P.tm_kv[1], a.dtype, a.v, a.B, a.H, a.gk, mv, a.D)) {
         *why = "cuTensorMapEncodeTiled rejected a tensor";
         return cudaErrorInvalidValue;
     }

@@ -12,7 +12,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "longcat_video_b200", "csrc")
-TOKEN = re.compile(r"[{}]|\b(?:mbar_wait_warp|mbar_wait_thread|mbar_test|mbar_try|tc_fence_after|tc_ld32|tc_ld64|tc_ld_half64|tc_st_half32|tc_st16|tc_st32|tc_mma|tc_mma_ts)(?=\()")
+TOKEN = re.compile(r"[{}]|\b(?:mbar_wait_warp|mbar_wait_thread|mbar_test|mbar_try|tc_fence_after|tc_ld16|tc_ld32|tc_ld64|tc_ld_half64|tc_st_half32|tc_st16|tc_st32|tc_mma|tc_mma_ts)(?=\()")
 
 
 def _unfenced(text):
