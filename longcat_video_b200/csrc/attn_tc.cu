@@ -284,6 +284,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc_kernel(const __grid_const
             const bool there = w < total_work;
             const bool start = w == blockIdx.x;
             if (there && !q_to_tmem(start ? 0 : wk + 1)) break;
+            // Behind the last item comes no Q, whose arrival would mean that the store of the item before has left the buffer.
+            if (!there && wk > 0 && !mbar_wait_warp(bar_q_free, (wk - 1) & 1, ctl, 112, wk)) break;
             if (!start) {
             rr0 += (n_iter + 1) >> 1;
             rr1 += n_iter >> 1;
