@@ -15,21 +15,24 @@
 // 64-token kernel:
 //
 //   warps 0-3, 4-7 : softmax warpgroups 0 and 1 (units of even / odd number; thread = one query row)
-//   warp 8 : TMA producer of Q and K   warp 9 : S = Q K^T issuer   warp 10 : O += P V issuer
-//   warp 11: TMA producer of V, output TMA stores
+//   warp 8 : TMA producer of Q and K   warp 9 : S = Q K^T issuer   warp 10 : O += P V issuer   warp 11: TMA producer of V
+//   warps 12-15 : Q to TMEM, merge and store of O (epilogue warps)
 //
 // Per unit i (warpgroup g = i & 1):  S = Q K^T (M128 N64 K128, A = Q from TMEM) -> tcgen05.ld, exp2 online softmax in registers, P in the input dtype into TMEM columns of its own ->
 // O_g += P V (M128 N128 K64, A from TMEM).  The two warpgroups keep separate maxima, row sums and accumulators and
-// are merged once per work item.  K and V rings: six slots of one 64-key tile (16 KiB) each.  The finished O
-// (128 rows x 256 B) is staged in the V slots of the item's last two units and leaves by TMA store.
+// are merged once per work item by the epilogue warps, while the softmax warps go on with the next item.  K and V rings: six slots of one
+// 64-key tile (16 KiB) each.  The finished O (128 rows x 256 B) is staged in the Q buffer and leaves by TMA store.
 //
 // Q in TMEM: an S with both operands in shared memory reads 48 KB of them per unit, which takes longer than its MMAs
 // (M128 N64 K128: 256 cycles); with A from TMEM it reads 16 KB.
 // What bounds it: the softmax warps.  A unit's MMAs take 512 cycles, its exponentials 512 cycles of the transcendental
 // unit, and a warpgroup needs about 1900 cycles per round (two rounds per pair of units at the same time): the two
 // warpgroups run in step, so nobody uses the transcendental unit while both store P and fetch S.  720p grid, 90 of 720
-// blocks, 8 heads, attention launch: 5.08 ms with one producer warp, Q in shared memory and P over S; 4.0 ms now; with 32
-// heads (17 ms) the launch runs into the power cap of the GPU.
+// blocks, 8 heads, attention launch: 5.08 ms with one producer warp, Q in shared memory and P over S; 4.0 ms without; with 32
+// heads (16.5 ms) the launch runs into the power cap of the GPU.  Turns for the transcendental unit (a warp waits until the one
+// that shares its scheduler is through with its exponentials) make it 5 % slower: alone, a warp needs 1000 cycles for them.
+// Epilogue warps and code that fits the instruction caches (55 KB, 144 KB before): 720p, 32 heads, whole call 17450 -> 16570 us;
+// training step 480p, 8 heads, 3950 -> 3670 us.
 //
 // Every wait on an mbarrier is bounded, as in attn_tc.cu.
 #include "tc_common.cuh"
@@ -50,10 +53,10 @@ constexpr int kTileBytes = kBlk * kD * 2;          // 16 KiB: one K or V tile of
 constexpr int kHalfBytes = kTileBytes / 2;         // one 64-column half: 64 rows x 128 B
 constexpr int kSlotBytes = kTileBytes;             // a ring slot holds one unit's tile
 constexpr int kMaxUnits = 8;                       // units of 64 keys per key block: blocks of up to 512 tokens
-constexpr int kKSlots = 6, kVSlots = 6;            // even, like the number of units of an item: the last two units sit in a slot pair
-constexpr int kThreads = 384;
-// setmaxnreg per warpgroup: (208 + 208 + 88) * 128 threads <= the 64 K registers of the SM
-constexpr int kRegsSoftmax = 208, kRegsOther = 88;
+constexpr int kKSlots = 6, kVSlots = 6;            // the same number: one code path serves both producers
+constexpr int kThreads = 512;
+// setmaxnreg per warpgroup: (176 + 176 + 48 + 112) * 128 threads = the 64 K registers of the SM, 128 per thread at launch
+constexpr int kRegsSoftmax = 176, kRegsOther = 48, kRegsEpilogue = 112;
 
 // TMEM columns: O accumulator of warpgroup g at 128 * g, its S at 256 + 64 * g, its P (16-bit pairs) at 384 + 32 * g; Q (16-bit pairs)
 constexpr uint32_t kTmO = 0, kTmS = 256, kTmP = 384, kTmQ = 448;
@@ -63,7 +66,7 @@ constexpr int kOffQ = 0;
 constexpr int kOffK = kOffQ + kQTileBytes;
 constexpr int kOffV = kOffK + kKSlots * kSlotBytes;
 constexpr int kOffBar = kOffV + kVSlots * kSlotBytes;
-// barriers: k_full[6] k_empty[6] v_full[6] v_empty[6] q_full q_empty s_full[2] s_free[2] p_full[2] pv_done[2]
+// barriers: k_full[6] k_empty[6] v_full[6] v_empty[6] q_full q_free s_full[2] s_free[2] p_full[2] pv_done[2]
 //           ml_ready o_free o_staged qt_full qt_free
 constexpr int kNumBars = 2 * kKSlots + 2 * kVSlots + 2 + 8 + 5;
 constexpr int kOffMisc = kOffBar + kNumBars * 8;      // abort flag, TMEM base
@@ -71,7 +74,7 @@ constexpr int kOffMl = kOffMisc + 64;                 // [2 warpgroups][128 lane
 constexpr int kSmemBytes = kOffMl + 2 * 128 * 8;
 
 struct TcParams {
-    CUtensorMap tm_q, tm_k, tm_v;
+    CUtensorMap tm_q, tm_kv[2];  // [0]: K, [1]: V
     // Output maps.  Normally one (tm_o[0]).  With o_frames > 0 the query grid is the rank-major grid of a
     // context-parallel group: frames [r * o_frames, (r + 1) * o_frames) are the tokens of rank r, and the rows of a
     // query block are stored straight into rank r's result buffer (its own map, over this GPU's or a peer's memory).
@@ -115,7 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
     auto bar_v_full = [&](int s) { return bar0 + 8u * (2 * kKSlots + s); };
     auto bar_v_empty = [&](int s) { return bar0 + 8u * (2 * kKSlots + kVSlots + s); };
     constexpr int kB0 = 2 * kKSlots + 2 * kVSlots;
-    const uint32_t bar_q_full = bar0 + 8u * kB0, bar_q_empty = bar0 + 8u * (kB0 + 1);
+    const uint32_t bar_q_full = bar0 + 8u * kB0, bar_q_free = bar0 + 8u * (kB0 + 1);
     auto bar_s_full = [&](int wg) { return bar0 + 8u * (kB0 + 2 + wg); };
     auto bar_s_free = [&](int wg) { return bar0 + 8u * (kB0 + 4 + wg); };
     auto bar_p_full = [&](int wg) { return bar0 + 8u * (kB0 + 6 + wg); };
@@ -142,18 +145,18 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
             mbar_init(bar_v_empty(s), 1);
         }
         mbar_init(bar_q_full, 1);
-        mbar_init(bar_q_empty, 8);
+        mbar_init(bar_q_free, 1);
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar_s_full(b), 1);
             mbar_init(bar_s_free(b), 4);
             mbar_init(bar_p_full(b), 4);  // one elected arrival per softmax warp
             mbar_init(bar_pv_done(b), 1);
         }
-        mbar_init(bar_qt_full, 8);
+        mbar_init(bar_qt_full, 4);
         mbar_init(bar_qt_free, 1);
         mbar_init(bar_ml_ready, 8);
-        mbar_init(bar_o_free, 8);
-        mbar_init(bar_o_staged, 8);
+        mbar_init(bar_o_free, 4);
+        mbar_init(bar_o_staged, 4);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         // The tiles are 128B-swizzled, which ties their layout to address bits 7-9: without a 1024-byte aligned
         // base nothing below is valid.  The declaration asks for it; refuse to run if it was not honoured.
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
     const bool start_ok = *abort_flag == 0;
 
     const int groups = P.nq;  // one work item per query block
-    const long long total_work = start_ok ? (long long)P.bh_total * groups : 0;
+    const int total_work = start_ok ? P.bh_total * groups : 0;  // q alone has 32 KB per item, so this is far below 2^31
     // The CTA's items are blockIdx.x, blockIdx.x + gridDim.x, ...; every role steps through them as (head, query block) pairs, since a
     // 64-bit division per role and item costs more than a round.
     const int first_bh = (int)(blockIdx.x / (unsigned)groups), first_g = (int)(blockIdx.x % (unsigned)groups);
@@ -194,51 +197,189 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
 
     // All roles walk the same list of work items and units.  Unit number gb (counted over the whole kernel)
     // uses K slot gb % 6 and V slot gb % 6.  Within an item unit i belongs to warpgroup i & 1.
-    if (warp >= 8) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-      if (warp == 8 || warp == 11) {
-        // ================================================================== TMA producers: warp 8 Q and K, warp 11 V and the output
-        // The output rows of an item are staged in the two V slots its last PVs released.  Warp 11 sends them off when it needs
-        // the first of them again, at the latest before it requests the last V of the item behind it (the epilogue of that item
-        // completes the next phase of o_staged, so the wait is never a phase behind).
-        const bool is_k = warp == 8;
-        unsigned gk = 0, gv = 0, wk = 0, nq_issued = 0;
-        int s_bh = first_bh, s_g = first_g;  // item whose output is stored next
-        unsigned ws_end = 0, ks = 0;        // units up to and including it, its number
+    if (warp >= 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
+        // ================================================================== epilogue warps (as in attn_tc.cu)
+        // Between two items: Q of the next one from shared memory to TMEM as soon as the last S of the current one has read
+        // the columns, then the merge of the two partial results, staged in the Q buffer that has just become free (a thread
+        // writes the row that it read Q from) and sent off by TMA store.  The softmax warps meanwhile go on with the next item.
+        const int wq = warp & 3;          // TMEM quadrant of this warp
+        const int row = wq * 32 + lane;   // row of the query block = TMEM lane
+        const uint32_t t_lane = (uint32_t)(wq * 32) << 16;
+        unsigned char* const buf = smem + kOffQ + row * 128;  // this thread's row: chunk c at 16 * (c ^ (row & 7)), halves kQHalfBytes apart
+        unsigned wk = 0, rr = 0;  // rr: rounds of either softmax warpgroup over the whole kernel
         bool ok = true;
-        auto store_item = [&]() -> bool {
-            const int bh = s_bh, qb = s_g;
-            const int b = bh / P.heads, h = bh % P.heads;
-            const int s0 = (int)((ws_end - 2) % kVSlots);  // ws_end is even and so is the ring: slots s0 and s0 + 1
-            if (!mbar_wait_warp(bar_o_staged, ks & 1, ctl, 110, ks)) return false;
-            if (lane == 0) {
-                Coord cc = block_coord(P.gq, qb, b, h, P.heads, P.merge_o, P.Tq);
-                const CUtensorMap* tmo = &P.tm_o[0];
-                if (P.o_frames > 0) {  // blocks never straddle ranks: o_frames is a multiple of the block's frames
-                    const int dst = cc.c3 / P.o_frames;
-                    cc.c3 -= dst * P.o_frames;
-                    tmo = &P.tm_o[dst];
+        auto q_to_tmem = [&](unsigned item) -> bool {  // Q of the CTA's work item number `item`
+            // the last S of the item before has read the columns
+            if (item > 0 && !mbar_wait_warp(bar_qt_free, (item - 1) & 1, ctl, 106, item)) return false;
+            if (!mbar_wait_warp(bar_q_full, item & 1, ctl, 108, item)) return false;
+            tc_fence_after();
+#pragma unroll 1
+            for (int half = 0; half < 2; ++half) {
+                uint32_t qr[32];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(buf + half * kQHalfBytes + ((c ^ (row & 7)) << 4));
+                    qr[4 * c + 0] = v.x;
+                    qr[4 * c + 1] = v.y;
+                    qr[4 * c + 2] = v.z;
+                    qr[4 * c + 3] = v.w;
                 }
-                const uint32_t src = sbase + kOffV + s0 * kSlotBytes;
-                tma_store_5d(tmo, src, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                tma_store_5d(tmo, src + kQHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
-                tma_store_commit();
-                tma_store_wait_read();
-                mbar_arrive(bar_v_empty(s0));
-                mbar_arrive(bar_v_empty(s0 + 1));
+                tc_st32(tmem + kTmQ + 32u * half + t_lane, qr);
             }
+            tc_wait_st();
+            tc_fence_before();
             __syncwarp();
-            next_item(s_bh, s_g);
-            ++ks;
+            mbar_arrive_elect(bar_qt_full);
             return true;
         };
+
+        int bh = 0, qt = 0, nx_bh = first_bh, nx_g = first_g, cnt_n = 0, n_act = 0;
+        auto peek = [&](bool there) {  // list length of item nx, read one item ahead
+            if (there) cnt_n = clamp_cnt(P, nx_bh, nx_g);
+        };
+        peek(blockIdx.x < total_work);
+        for (int w = blockIdx.x;; w += gridDim.x) {  // item w gets its Q, the one before (number wk) is finished
+            const bool there = w < total_work;
+            const bool start = w == blockIdx.x;
+            if (there && !q_to_tmem(start ? 0 : wk + 1)) break;
+            // Behind the last item comes no Q, whose arrival would mean that the store of the item before has left the buffer.
+            if (!there && wk > 0 && !mbar_wait_warp(bar_q_free, (wk - 1) & 1, ctl, 112, wk)) break;
+            if (!start) {
+                rr += max(2, n_act) >> 1;  // the units of an item are even in number and at least two
+                // Both warpgroups have stored their last P, hence seen every PV but their last finish; no PV of the next item
+                // starts before o_free, so the waits below are for exactly the item's last PVs.
+                ok = mbar_wait_warp(bar_ml_ready, wk & 1, ctl, 104, wk);
+                if (!ok) break;
+                const float2 ml0 = ml[row], ml1 = ml[128 + row];
+                // merged scale of both partial sums: everything relative to the larger reference maximum.  A row with a NaN or an
+                // infinite score has a NaN sum and comes out as NaN, like on the warp-level kernel; a side that saw no key has the
+                // maximum -inf, hence the weight 0.
+                const float m_all = fmaxf(ml0.x, ml1.x), m_base = m_all == -INFINITY ? 0.f : m_all;
+                const float w0 = ex2(ml0.x - m_base), w1 = ex2(ml1.x - m_base);
+                const float l_all = ml0.y * w0 + ml1.y * w1;
+                const float inv = l_all == 0.f ? 0.f : 1.f / l_all;
+                const float f0 = w0 * inv, f1 = w1 * inv;
+                const float2 f0_2 = make_float2(f0, f0), f1_2 = make_float2(f1, f1);
+                const bool saw = n_act > 0;  // an empty list: the accumulators hold garbage and are not used
+                ok = mbar_wait_warp(bar_pv_done(0), (rr - 1) & 1, ctl, 100, wk);
+                if (ok) ok = mbar_wait_warp(bar_pv_done(1), (rr - 1) & 1, ctl, 101, wk);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t tm_o = tmem + kTmO + t_lane;
+#pragma unroll 1
+                for (int cch = 0; cch < kD / 32; ++cch) {
+                    uint32_t oa[32], ob[32];
+                    if (saw) {
+                        tc_ld32(tm_o + 32 * cch, oa);
+                        tc_ld32(tm_o + 128 + 32 * cch, ob);
+                    }
+                    tc_wait_ld();
+                    if (cch == kD / 32 - 1) {  // both O accumulators may be overwritten by the next item's first PVs
+                        tc_fence_before();
+                        __syncwarp();
+                        mbar_arrive_elect(bar_o_free);
+                    }
+                    if (LCBSA_UNLIKELY(!saw)) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) oa[j] = ob[j] = 0u;
+                    }
+                    unsigned char* const half = buf + (cch >> 1) * kQHalfBytes;
+#pragma unroll
+                    for (int q8 = 0; q8 < 4; ++q8) {
+                        uint32_t pw[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int e = q8 * 8 + 2 * j;
+                            const float2 a2 = __fmul2_rn(make_float2(__uint_as_float(oa[e]), __uint_as_float(oa[e + 1])), f0_2);
+                            const float2 v2 = __ffma2_rn(make_float2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), f1_2, a2);
+                            pw[j] = pack2(bf16, v2.x, v2.y);
+                        }
+                        const int chunk = (cch & 1) * 4 + q8;
+                        *reinterpret_cast<uint4*>(half + ((chunk ^ (row & 7)) << 4)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
+                    }
+                }
+                fence_proxy_async();
+                __syncwarp();
+                mbar_arrive_elect(bar_o_staged);
+                if (P.lse != nullptr) {
+                    int lt, lh, lw, bt, bhh, bw;
+                    slot_coords(P.gq, row, lt, lh, lw);
+                    block_coords(P.gq, qt, bt, bhh, bw);
+                    const int tt = bt * P.gq.ct + lt, hh = bhh * P.gq.ch + lh, ww = bw * P.gq.cw + lw;
+                    if (tt < P.gq.T && hh < P.gq.H && ww < P.gq.W) {
+                        const long long Sq = (long long)P.gq.T * P.gq.H * P.gq.W;
+                        const long long tok = ((long long)tt * P.gq.H + hh) * P.gq.W + ww;
+                        P.lse[(long long)bh * Sq + tok] = l_all > 0.f ? (m_all + log2f(l_all)) * 0.6931471805599453f : -INFINITY;
+                    }
+                }
+                if (warp == 12) {  // the rows of all four warps are staged: off they go, then the buffer takes the Q after the next
+                    ok = mbar_wait_warp(bar_o_staged, wk & 1, ctl, 110, wk);
+                    if (!ok) break;
+                    if (lane == 0) {
+                        const int b = bh / P.heads, h = bh - b * P.heads;
+                        Coord cc = block_coord(P.gq, qt, b, h, P.heads, P.merge_o, P.Tq);
+                        const CUtensorMap* tmo = &P.tm_o[0];
+                        if (P.o_frames > 0) {  // blocks never straddle ranks: o_frames is a multiple of the block's frames
+                            const int dst = cc.c3 / P.o_frames;
+                            cc.c3 -= dst * P.o_frames;
+                            tmo = &P.tm_o[dst];
+                        }
+                        tma_store_5d(tmo, sbase + kOffQ, 0, cc.c1, cc.c2, cc.c3, cc.c4);
+                        tma_store_5d(tmo, sbase + kOffQ + kQHalfBytes, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+                        tma_store_commit();
+                        tma_store_wait_read();
+                        mbar_arrive(bar_q_free);
+                    }
+                    __syncwarp();
+                }
+                ++wk;
+            }
+            if (!there) break;
+            bh = nx_bh;
+            qt = nx_g;
+            n_act = cnt_n << P.lg_units;
+            next_item(nx_bh, nx_g);
+            peek(w + gridDim.x < total_work);
+        }
+        if (warp == 12 && lane == 0) tma_store_wait_all();
+    } else if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
+      if (warp == 8 || warp == 11) {
+        // ================================================================== TMA producers: warp 8 Q and K, warp 11 V
+        const bool is_k = warp == 8;
+        // One code path for both rings: they have the same number of slots of the same size.
+        const uint32_t ring = sbase + (is_k ? kOffK : kOffV), full0 = is_k ? bar_k_full(0) : bar_v_full(0), empty0 = is_k ? bar_k_empty(0) : bar_v_empty(0);
+        unsigned gk = 0, wk = 0, nq_issued = 0;  // gk: units requested over the whole kernel
+        int slot = 0;
+        unsigned parity = 1;  // of the wait on an empty slot: the ring starts empty
+        bool ok = true;
+        auto request_q = [&](int bh, int qb) {  // Q tile of item (bh, qb) into the Q buffer
+            if (lane == 0) {
+                mbar_arrive_tx(bar_q_full, kQTileBytes);
+                const int b = bh / P.heads, h = bh - b * P.heads;
+                const Coord cc = block_coord(P.gq, qb, b, h, P.heads, P.merge_q, P.Tq);
+                tma_load_5d(sbase + kOffQ, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
+                tma_load_5d(sbase + kOffQ + kQHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
+            }
+            ++nq_issued;
+            __syncwarp();
+        };
+        if (is_k && blockIdx.x < total_work) request_q(first_bh, first_g);
         int bh = first_bh, qb = first_g, nx_bh = first_bh, nx_g = first_g;
         int cnt_n = 0;
         auto peek = [&](bool there) {  // list length of item nx, read one item ahead
             if (there) cnt_n = clamp_cnt(P, nx_bh, nx_g);
         };
         peek(blockIdx.x < total_work);
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, qb = nx_g) {
+        // The first two windows of an item's list are read while the item before is under way.
+        int raw0 = 0, raw1 = 0;
+        auto load_ahead = [&](int bh, int qb, int cnt) {
+            const int32_t* l = P.idx + ((long long)bh * P.nq + qb) * P.cap;
+            if (lane < cnt) raw0 = l[lane];
+            if (32 + lane < cnt) raw1 = l[32 + lane];
+        };
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, qb = nx_g) {
             const int b = bh / P.heads, h = bh % P.heads;
             const int cnt = cnt_n;
             const int n_act = cnt << P.lg_units;  // units that exist: 2, 4 or 8 per listed key block
@@ -246,9 +387,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
             // Block coordinates are fetched and decoded by the whole warp: lane L holds list entry 32 n + L as the
             // block's first token packed t << 20 | h << 10 | w.  `nxt` holds the thirty-two entries behind the current ones.
             const int32_t* my_l = P.idx + ((long long)bh * P.nq + qb) * P.cap;
-            auto fetch = [&](int e) {
+            auto decode = [&](int blk, int e) {  // list entry e
                 if (e >= cnt) return 0;
-                const int blk = my_l[e];
                 if ((unsigned)blk >= (unsigned)P.gk.nblk) {
                     // A list entry outside [0, Nk) never becomes an address: its box is placed at w = W, wholly
                     // outside the tensor map, so TMA fills the tile with zeros; the call is flagged.
@@ -263,10 +403,12 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                 block_coords(P.gk, blk, bt, bhh, bw);
                 return ((bt * P.gk.ct) << 20) | ((bhh * P.gk.ch) << 10) | (bw * P.gk.cw);
             };
-            int cur = fetch(lane);
-            int nxt = fetch(32 + lane);
+            if (wk == 0) load_ahead(bh, qb, cnt);
+            int cur = decode(raw0, lane);
+            int nxt = decode(raw1, 32 + lane);
             next_item(nx_bh, nx_g);
-            peek(w + gridDim.x < total_work);
+            const bool more_items = w + gridDim.x < total_work;
+            peek(more_items);
             const bool mrg = is_k ? P.merge_k : P.merge_v;
             const int c3 = mrg ? b * P.Tk : 0, c4 = mrg ? h : b * P.heads + h;
             // the boxes of unit j: its block's first token plus the offset of the unit inside the block
@@ -281,53 +423,42 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                 }
                 if ((e & 31) == 31 && u == (1 << P.lg_units) - 1) {
                     cur = nxt;
-                    nxt = fetch(e + 33 + lane);
+                    nxt = decode(e + 33 + lane < cnt ? my_l[e + 33 + lane] : 0, e + 33 + lane);
                 }
             };
-            if (is_k) {
-                // Q tile: the buffer is free once the softmax warps have moved the previous item's Q to TMEM
-                ok = mbar_wait_warp(bar_q_empty, (wk & 1) ^ 1, ctl, 10, wk);
-                if (!ok) break;
-                ++nq_issued;
-                if (lane == 0) {
-                    mbar_arrive_tx(bar_q_full, kQTileBytes);
-                    const Coord cc = block_coord(P.gq, qb, b, h, P.heads, P.merge_q, P.Tq);
-                    tma_load_5d(sbase + kOffQ, &P.tm_q, bar_q_full, 0, cc.c1, cc.c2, cc.c3, cc.c4);
-                    tma_load_5d(sbase + kOffQ + kQHalfBytes, &P.tm_q, bar_q_full, 64, cc.c1, cc.c2, cc.c3, cc.c4);
-                }
-                __syncwarp();
-                for (int j = 0; j < n_iter; ++j) {
-                    const int slot = gk % kKSlots;
-                    ok = mbar_wait_warp(bar_k_empty(slot), ((gk / kKSlots) & 1) ^ 1, ctl, 20, gk);
-                    if (!ok) break;
-                    ++gk;
-                    request(j, &P.tm_k, bar_k_full(slot), sbase + kOffK + slot * kSlotBytes);
-                }
-            } else {
-                for (int j = 0; j < n_iter; ++j) {
-                    if (ks < wk && (gv >= ws_end - 2 + kVSlots || j == n_iter - 1)) {
-                        ok = store_item();
+            bool q_due = is_k && more_items;  // Q of the next item has not been requested yet
+#pragma unroll 1
+            for (int j = 0; j < n_iter; ++j) {
+                // Q of the next item as soon as the buffer is free again (see the epilogue warps), which is early in this
+                // item; behind the last chance for it comes the item's last K.
+                if (q_due) {
+                    const uint32_t bar = wk == 0 ? bar_qt_full : bar_q_free, ph = wk == 0 ? 0 : (wk - 1) & 1;
+                    bool go = __all_sync(0xffffffffu, mbar_test(bar, ph));
+                    if (!go && j == n_iter - 1) {
+                        ok = go = mbar_wait_warp(bar, ph, ctl, 10, wk);
                         if (!ok) break;
                     }
-                    const int slot = gv % kVSlots;
-                    ok = mbar_wait_warp(bar_v_empty(slot), ((gv / kVSlots) & 1) ^ 1, ctl, 22, gv);
-                    if (!ok) break;
-                    ++gv;
-                    request(j, &P.tm_v, bar_v_full(slot), sbase + kOffV + slot * kSlotBytes);
+                    if (go) {
+                        request_q(nx_bh, nx_g);
+                        q_due = false;
+                    }
                 }
-                ws_end = gv;  // the item before has been stored
+                if (j == min(2, n_iter - 1) && more_items) load_ahead(nx_bh, nx_g, cnt_n);
+                ok = mbar_wait_warp(empty0 + 8u * slot, parity, ctl, is_k ? 20 : 22, gk);
+                if (!ok) break;
+                request(j, &P.tm_kv[is_k ? 0 : 1], full0 + 8u * slot, ring + slot * kSlotBytes);
+                ++gk;
+                if (++slot == kKSlots) {
+                    slot = 0;
+                    parity ^= 1;
+                }
             }
         }
-        if (!is_k && ok && ks < wk) ok = store_item();
-        if (!is_k && lane == 0) tma_store_wait_all();
         if (!ok && lane == 0) {
             // drain: give the copies this warp issued a bounded time to land before the CTA exits
             const long long t0 = clock64();
             for (unsigned r = gk > kKSlots ? gk - kKSlots : 0; r < gk; ++r)
-                while (!mbar_try(bar_k_full(r % kKSlots), (r / kKSlots) & 1) && clock64() - t0 < 40000000ll) {
-                }
-            for (unsigned r = gv > kVSlots ? gv - kVSlots : 0; r < gv; ++r)
-                while (!mbar_try(bar_v_full(r % kVSlots), (r / kVSlots) & 1) && clock64() - t0 < 40000000ll) {
+                while (!mbar_try(full0 + 8u * (r % kKSlots), (r / kKSlots) & 1) && clock64() - t0 < 40000000ll) {
                 }
             if (nq_issued > 0)
                 while (!mbar_try(bar_q_full, (nq_issued - 1) & 1) && clock64() - t0 < 40000000ll) {
@@ -345,7 +476,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
             next_item(bh, g);
         };
         peek(blockIdx.x < total_work);
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
             const int n_act = cnt_n << P.lg_units;
             peek(w + gridDim.x < total_work);
             const int n_iter = max(2, n_act);
@@ -398,7 +529,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
             next_item(bh, g);
         };
         peek(blockIdx.x < total_work);
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk) {
             const int n_act = cnt_n << P.lg_units;
             peek(w + gridDim.x < total_work);
             const int n_iter = max(2, n_act);
@@ -430,8 +561,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                     for (int j = 0; j < kBlk / 16; ++j)
                         tc_mma_ts(d, pa + 8u * j, vd + (uint64_t)((j * 2048) >> 4), idesc_pv, (i > 1 || j > 0) ? 1u : 0u);
                 }
-                // the V slots of the item's last two units go to the epilogue, which stages O in them and frees them
-                if (i < n_iter - 2) tc_commit(bar_v_empty(slot));
+                tc_commit(bar_v_empty(slot));
                 tc_commit(bar_pv_done(wg));
                 __syncwarp();
                 if (wg) ++rr1; else ++rr0;
@@ -447,40 +577,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
         const int row = wq * 32 + lane;   // row of the query block = TMEM lane
         const uint32_t t_lane = (uint32_t)(wq * 32) << 16;
         const uint32_t tm_s = tmem + kTmS + 64u * wg + t_lane, tm_p = tmem + kTmP + 32u * wg + t_lane;
-        const uint32_t tm_o_mine = tmem + kTmO + 128u * wg + t_lane, tm_o_other = tmem + kTmO + 128u * (wg ^ 1) + t_lane;
-        const int ml_idx = row;
-        unsigned wk = 0, gb = 0, rr = 0;  // rr: rounds of this warpgroup over the whole kernel
+        const uint32_t tm_o_mine = tmem + kTmO + 128u * wg + t_lane;
+        unsigned wk = 0, rr = 0;  // rr: rounds of this warpgroup over the whole kernel
         bool ok = true;
-
-        // Q of the CTA's work item number `item` from shared memory to TMEM: a thread moves its row, the warpgroup 64 of the 128 columns.
-        auto q_to_tmem = [&](unsigned item) -> bool {
-            // the last S of the item before has read the columns
-            if (item > 0 && !mbar_wait_warp(bar_qt_free, (item - 1) & 1, ctl, 106 + wg, item)) return false;
-            if (!mbar_wait_warp(bar_q_full, item & 1, ctl, 108 + wg, item)) return false;
-            tc_fence_after();
-            const unsigned char* src = smem + kOffQ + wg * kQHalfBytes + row * 128;
-            uint32_t qr[32];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const uint4 v = *reinterpret_cast<const uint4*>(src + ((c ^ (row & 7)) << 4));
-                qr[4 * c + 0] = v.x;
-                qr[4 * c + 1] = v.y;
-                qr[4 * c + 2] = v.z;
-                qr[4 * c + 3] = v.w;
-            }
-            tc_st32(tmem + kTmQ + 32u * wg + t_lane, qr);
-            tc_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            mbar_arrive_elect(bar_q_empty);
-            mbar_arrive_elect(bar_qt_full);
-            return true;
-        };
-        if (blockIdx.x < total_work) ok = q_to_tmem(0);
 
         int bh = first_bh, qt = first_g, nx_bh = first_bh, nx_g = first_g, cnt_n = 0;
         if (blockIdx.x < total_work) cnt_n = clamp_cnt(P, bh, qt);
-        for (long long w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, qt = nx_g) {
+        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++wk, bh = nx_bh, qt = nx_g) {
             const int n_act = cnt_n << P.lg_units;
             next_item(nx_bh, nx_g);
             if (w + gridDim.x < total_work) cnt_n = clamp_cnt(P, nx_bh, nx_g);  // read one item ahead
@@ -637,88 +740,17 @@ __global__ void __launch_bounds__(kThreads, 1) attn_tc128_kernel(const __grid_co
                 }
             }
             if (!ok) break;
-            gb += n_iter;
-            // Q of the next item, so that its S runs under this item's epilogue
-            if (w + gridDim.x < total_work && !q_to_tmem(wk + 1)) break;
-
-            // ---- epilogue of this work item.  The warpgroup's PVs are finished once its last one is; it then
-            // publishes (maximum, row sum) of its rows and waits for the other warpgroup to do the same.
-            {   // n_iter is even and at least 2: every warpgroup has had a round
-                ok = mbar_wait_warp(bar_pv_done(wg), (rr - 1) & 1, ctl, 100 + wg, rr);
-                if (!ok) break;
-            }
-            // the other warpgroup has read this warpgroup's entry of the previous item before it arrived on o_free
+            // The epilogue warps merge this item's partial results; they have read the (maximum, row sum) of the item before once
+            // they have arrived on o_free.
             if (wk > 0) {
-                ok = mbar_wait_warp(bar_o_free, (wk - 1) & 1, ctl, 102 + wg, wk);
-                if (!ok) break;
+                if (!__all_sync(0xffffffffu, mbar_test(bar_o_free, (wk - 1) & 1))) {
+                    ok = mbar_wait_warp(bar_o_free, (wk - 1) & 1, ctl, 102 + wg, wk);
+                    if (!ok) break;
+                }
             }
-            const float m_pub = first ? -INFINITY : m_ref;  // no key seen: m_ref is a placeholder
-            ml[wg * 128 + ml_idx] = make_float2(m_pub, l_sum);
+            ml[wg * 128 + row] = make_float2(first ? -INFINITY : m_ref, l_sum);  // no key seen: m_ref is a placeholder
             __syncwarp();
             mbar_arrive_elect(bar_ml_ready);
-            ok = mbar_wait_warp(bar_ml_ready, wk & 1, ctl, 104 + wg, wk);
-            if (!ok) break;
-            tc_fence_after();
-            const float2 oth = ml[(wg ^ 1) * 128 + ml_idx];
-            // merged scale of both partial sums: everything relative to the larger reference maximum.  A row with a NaN or an
-            // infinite score has a NaN sum and comes out as NaN, like on the warp-level kernel; a side that saw no key has the
-            // maximum -inf, hence the weight 0.
-            const float m_all = fmaxf(m_pub, oth.x), m_base = m_all == -INFINITY ? 0.f : m_all;
-            const float w_mine = ex2(m_pub - m_base), w_oth = ex2(oth.x - m_base);
-            const float l_all = l_sum * w_mine + oth.y * w_oth;
-            const float inv = l_all == 0.f ? 0.f : 1.f / l_all;
-            const float f_mine = w_mine * inv, f_oth = w_oth * inv;
-            // This warpgroup merges and stages columns 64*wg .. 64*wg+63 of O (input dtype, one 128B-swizzled
-            // half-tile row per thread) in the V slot that its own last PV has just released: the last two units of
-            // the item sit in slots s0 (warpgroup 0) and s0 + 1 (warpgroup 1), s0 even.
-            unsigned char* o_half = smem + kOffV + ((gb - 2) % kVSlots + wg) * kSlotBytes;
-            const bool saw = n_act > 0;  // an empty list: the accumulators hold garbage and are not used
-            const float2 fm2 = make_float2(f_mine, f_mine), fo2 = make_float2(f_oth, f_oth);
-#pragma unroll
-            for (int cch = 0; cch < 2; ++cch) {
-                uint32_t oa[32], ob[32];
-                if (saw) {
-                    tc_ld32(tm_o_mine + 64 * wg + 32 * cch, oa);
-                    tc_ld32(tm_o_other + 64 * wg + 32 * cch, ob);
-                }
-                tc_wait_ld();
-                if (LCBSA_UNLIKELY(!saw)) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) oa[j] = ob[j] = 0u;
-                }
-                {
-#pragma unroll
-                    for (int q8 = 0; q8 < 4; ++q8) {
-                        uint32_t pw[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int e = q8 * 8 + 2 * j;
-                            const float2 a2 = __fmul2_rn(make_float2(__uint_as_float(oa[e]), __uint_as_float(oa[e + 1])), fm2);
-                            const float2 v2 = __ffma2_rn(make_float2(__uint_as_float(ob[e]), __uint_as_float(ob[e + 1])), fo2, a2);
-                            pw[j] = pack2(bf16, v2.x, v2.y);
-                        }
-                        const int chunk = cch * 4 + q8;
-                        *reinterpret_cast<uint4*>(o_half + row * 128 + ((chunk ^ (row & 7)) << 4)) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            mbar_arrive_elect(bar_o_free);  // both O accumulators may be overwritten by the next item's first PVs
-            if (wg == 0 && P.lse != nullptr) {
-                int lt, lh, lw, bt, bhh, bw;
-                slot_coords(P.gq, row, lt, lh, lw);
-                block_coords(P.gq, qt, bt, bhh, bw);
-                const int tt = bt * P.gq.ct + lt, hh = bhh * P.gq.ch + lh, ww = bw * P.gq.cw + lw;
-                if (tt < P.gq.T && hh < P.gq.H && ww < P.gq.W) {
-                    const long long Sq = (long long)P.gq.T * P.gq.H * P.gq.W;
-                    const long long tok = ((long long)tt * P.gq.H + hh) * P.gq.W + ww;
-                    P.lse[(long long)bh * Sq + tok] = l_all > 0.f ? (m_all + log2f(l_all)) * 0.6931471805599453f : -INFINITY;
-                }
-            }
-            fence_proxy_async();
-            __syncwarp();
-            mbar_arrive_elect(bar_o_staged);  // the store warp takes it from here
         }
     }
 
@@ -804,8 +836,8 @@ cudaError_t launch_attn_tc128(const AttnArgs& a, cudaStream_t st, const char** w
     P.gu = gu;
     const int mq = merge_mode(a.q, a.B, a.H, a.gq), mk = merge_mode(a.k, a.B, a.H, a.gk);
     const int mv = merge_mode(a.v, a.B, a.H, a.gk), mo = merge_mode(a.o, a.B, a.H, a.gq);
-    if (!make_map(&P.tm_q, a.dtype, a.q, a.B, a.H, a.gq, mq) || !make_map(&P.tm_k, a.dtype, a.k, a.B, a.H, gu, mk) ||
-        !make_map(&P.tm_v, a.dtype, a.v, a.B, a.H, gu, mv)) {
+    if (!make_map(&P.tm_q, a.dtype, a.q, a.B, a.H, a.gq, mq) || !make_map(&P.tm_kv[0], a.dtype, a.k, a.B, a.H, gu, mk) ||
+        !make_map(&P.tm_kv[1], a.dtype, a.v, a.B, a.H, gu, mv)) {
         *why = "cuTensorMapEncodeTiled rejected a tensor";
         return cudaErrorInvalidValue;
     }
