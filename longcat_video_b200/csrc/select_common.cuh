@@ -6,6 +6,7 @@
 namespace lcbsa {
 namespace sel {
 
+constexpr uint32_t kFirstStep = 128;  // of the search for the threshold of a row of 16-bit keys (select_row_regs)
 constexpr int kRegWords = 24;  // 32-bit words of a 16-bit key row that a lane may keep in registers (select_row_regs: rows up to 1536 keys)
 
 template <typename T> struct KeyOf { using type = uint16_t; };
@@ -66,12 +67,14 @@ struct KeyMask {
 // ascending block indices by one warp; the cap - nsel trailing entries are set to -1.  nk_pad (a multiple of 64, at most
 // 64 * NW) entries are readable and those past Nk hold key 0, which no block that may be selected has.
 //
-// Issue bound: the row is read once (2 bytes per key) and then counted up to 16 times.  Every lane keeps its share of the
+// Issue bound: the row is read once (2 bytes per key) and then counted some seven times (16 bits of a plain bisection took 12 to 17).  Every lane keeps its share of the
 // row in registers (word i: keys 2 (lane + 32 i) and the one behind it), the low key of a word shifted up in a register of
 // its own, so that a count is a compare and an add per key; NW follows the row (a fixed 24 words spent 60 % of the work of a 624-key row on padding); the
 // bisection ends as soon as a candidate is reached by exactly nsel keys; and the indices are emitted from the registers.
 // Before, with 24 words for every row, five shuffles per count, all 17 counts and a second read of the row: 19 968 rows of
-// 624 keys 76 us, now 33 us; 46 080 rows of 1440 keys 199 us, now 185 us (there 23 of the 24 words were needed all along).
+// 624 keys 76 us, now 33 us; 46 080 rows of 1440 keys 199 us, then
+// 185 us (there 23 of the 24 words were needed all along).  Searching from the largest key down: scores and selection of those
+// 46 080 rows 620 us, now 561 us; of 19 968 rows of 624 keys 127 us, now 115 us.
 template <int NW>
 __device__ __forceinline__ void select_row_regs(const uint16_t* row, int nk_pad, int nsel, int cap, int32_t* out, int32_t* cnt_out, int lane,
                                                 const KeyMask mask = KeyMask{1, 0, 0}) {
@@ -98,20 +101,36 @@ __device__ __forceinline__ void select_row_regs(const uint16_t* row, int nk_pad,
             for (int i = 0; i < NW; ++i) n += (int)(hi[i] >= cc) + (int)(lo[i] >= cc);
             return warp_sum(n);
         };
-        uint32_t thr = 0;
+        // The threshold lies a little below the row's largest key: steps down from there, of an octave of bf16 scores at first, then twice
+        // as long each time, until nsel keys are reached, and bisects the last step.  count(lo) >= nsel > count(hi) throughout.
+        uint32_t top = 0;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) top = max(top, max(hi[i], lo[i]));
+        uint32_t below = 0, above = (__reduce_max_sync(0xffffffffu, top) >> 16) + 1u, reach = kFirstStep;
+        int n_above = 0;     // keys that reach `above`
         bool exact = false;  // exactly nsel keys reach the threshold
 #pragma unroll 1
-        for (int bit = 15; bit >= 0; --bit) {
-            const uint32_t cand = thr | (1u << bit);
+        while (above - below > 1u) {
+            uint32_t cand = (below + above) >> 1;
+            if (below == 0u) {
+                cand = above > reach ? above - reach : 1u;
+                if (n_above > 0) reach *= 2u;
+            }
             const int n = count(cand);
-            if (n >= nsel) thr = cand;
-            if (n == nsel) {
-                exact = true;
-                break;
+            if (n >= nsel) {
+                below = cand;
+                if (n == nsel) {
+                    exact = true;
+                    break;
+                }
+            } else {
+                above = cand;
+                n_above = n;
             }
         }
-        // otherwise thr is the nsel-th largest key and more than nsel keys reach it
-        const int take_eq = exact ? 0 : nsel - (thr < 0xffffu ? count(thr + 1u) : 0);  // ties to keep, lowest block index first
+        // otherwise the threshold is the nsel-th largest key and more than nsel keys reach it
+        const uint32_t thr = below;
+        const int take_eq = exact ? 0 : nsel - n_above;  // ties to keep, lowest block index first
         const uint32_t tt = thr << 16;
         const unsigned lt_mask = (1u << lane) - 1u;
         int n_out = 0, n_eq = 0;
