@@ -5,7 +5,7 @@
 // arithmetic:  score(i,j) = fp32 FMA chain over d = 0..D-1 (ascending), rounded to the input dtype.  The FMA pipe
 // can only be kept busy if every operand word read from shared memory feeds several FMAs (shared memory hands a
 // warp 32 words per cycle, the FMA pipes take 128 lanes per cycle), and that needs a two-dimensional register
-// tile: here 8 x 8 scores per thread, 128 x 128 per CTA, 16 FMAs per 128-bit operand read.  A tile of that shape
+// tile: here 8 x 8 scores per thread, 128 x 128 per CTA, 16 FMAs per 128-bit operand read (4 x 4 or 2 x 2 on small calls).  A tile of that shape
 // cannot keep whole rows of scores on chip, so the rounded scores go to a workspace as order-preserving 16-bit keys
 // (2 bytes per score, written once and read once: 0.27 GB of traffic at 720p with 32 heads) and a second kernel
 // selects per row, one warp per row with the row in registers.  Used by lcbsa_block_select when the caller's
@@ -18,16 +18,19 @@ namespace {
 
 using namespace sel;
 
-constexpr int kTile = 128;          // scores per CTA: kTile x kTile
-constexpr int kBK = 16;             // head-dimension elements per shared-memory slab
-constexpr int kPitch = kTile + 4;   // slab row pitch in floats
-constexpr int kGemmThreads = 256;   // 16 x 16 threads, 8 x 8 scores each
+constexpr int kGemmThreads = 256;   // 16 x 16 threads, R x R scores each
 
-// q: [BH, Nq, D], k: [BH, Nk, D] pooled rows in the input dtype; keys: [BH, Nq, nk_pad]
-template <typename T, int D>
+// q: [BH, Nq, D], k: [BH, Nk, D] pooled rows in the input dtype; keys: [BH, Nq, nk_pad].  R: scores per thread and direction, 8, 4
+// or 2 (tiles of 128, 64 or 32 scores; see launch_gemm)
+template <typename T, int D, int R>
 __global__ void __launch_bounds__(kGemmThreads, 2) score_gemm_kernel(const T* __restrict__ qc, const T* __restrict__ kc, int Nq, int Nk,
                                                                     int nk_pad, uint16_t* __restrict__ keys) {
-    static_assert(sizeof(T) == 2 && D % kBK == 0, "16-bit inputs, head_dim a multiple of 16");
+    constexpr int kTile = 16 * R;              // scores per CTA: kTile x kTile
+    constexpr int kBK = 2048 / kTile;          // head-dimension elements per shared-memory slab: a 128-bit load per thread and operand
+    constexpr int kPitch = kTile + 4;          // slab row pitch in floats
+    constexpr int kG = R == 8 ? 2 : 1;         // groups of neighbouring rows (columns) of a thread, 64 apart
+    constexpr int kW = R / kG;                 // rows (columns) per group: 4, 4 or 2
+    static_assert(sizeof(T) == 2 && D % kBK == 0, "16-bit inputs, head_dim a multiple of the slab");
     __shared__ __align__(16) float qs[2][kBK][kPitch];  // [slab][d][row]: transposed, so that a thread's rows are contiguous
     __shared__ __align__(16) float ks[2][kBK][kPitch];
 
@@ -37,8 +40,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) score_gemm_kernel(const T* __
     const T* qbase = qc + (long long)bh * Nq * D;
     const T* kbase = kc + (long long)bh * Nk * D;
 
-    // global -> registers: thread t brings 8 consecutive d of row t / 2 of the Q tile and of the K tile
-    const int lrow = tid >> 1, ldh = (tid & 1) * 8;
+    // global -> registers: a thread brings 8 consecutive d of one row of the Q tile and of the K tile
+    constexpr int kPer = kBK / 8;  // threads per row
+    const int lrow = tid / kPer, ldh = (tid % kPer) * 8;
     const bool q_ok = i0 + lrow < Nq, k_ok = j0 + lrow < Nk;
     const T* qsrc = qbase + (long long)(q_ok ? i0 + lrow : 0) * D + ldh;
     const T* ksrc = kbase + (long long)(k_ok ? j0 + lrow : 0) * D + ldh;
@@ -57,14 +61,14 @@ __global__ void __launch_bounds__(kGemmThreads, 2) score_gemm_kernel(const T* __
         }
     };
 
-    // this thread's scores: rows {4 ty .. 4 ty + 3, 64 + 4 ty ..}, columns {4 tx .. 4 tx + 3, 64 + 4 tx ..}
+    // this thread's scores: rows kW ty .. (and 64 + 4 ty ..), columns kW tx .. (and 64 + 4 tx ..)
     // column pairs: two fused multiply-adds per instruction, each rounded like a scalar one (32 x 1440 x 1440 scores: 476 us with
     // scalar ones, 443 us; 236 us is what the FMA pipes need)
-    float2 acc[8][4];
+    float2 acc[R][R / 2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
+        for (int j = 0; j < R / 2; ++j) acc[i][j] = make_float2(0.f, 0.f);
 
     fetch(0);
     stash(0);
@@ -74,20 +78,30 @@ __global__ void __launch_bounds__(kGemmThreads, 2) score_gemm_kernel(const T* __
     for (int slab = 0; slab < kSlabs; ++slab) {
         const int buf = slab & 1;
         if (slab + 1 < kSlabs) fetch(slab + 1);
-        // four steps of 16 per turn: unrolled whole, the loop is 36 KB of code and waits for instructions (32 x 1440 x 1440 scores: 26 us of
-        // 400; a 16 x 8 tile per thread, with fewer operand reads but half the warps, is 5 to 8 % slower than this one)
-#pragma unroll 4
+        // unrolled whole, the loop of the large tile is 36 KB of code and waits for instructions (32 x 1440 x 1440 scores: 26 us of
+        // 400; a 16 x 8 tile per thread, with fewer operand reads but half the warps, is 5 to 8 % slower than 8 x 8)
+#pragma unroll (32 / R)
         for (int d = 0; d < kBK; ++d) {  // ascending d: every score is one chain acc = fmaf(q[d], k[d], acc)
-            const float4 qa = *reinterpret_cast<const float4*>(&qs[buf][d][4 * ty]);
-            const float4 qb = *reinterpret_cast<const float4*>(&qs[buf][d][64 + 4 * ty]);
-            const float4 ka = *reinterpret_cast<const float4*>(&ks[buf][d][4 * tx]);
-            const float4 kb = *reinterpret_cast<const float4*>(&ks[buf][d][64 + 4 * tx]);
-            const float qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-            const float2 kv[4] = {make_float2(ka.x, ka.y), make_float2(ka.z, ka.w), make_float2(kb.x, kb.y), make_float2(kb.z, kb.w)};
+            float qv[R];
+            float2 kv[R / 2];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int g = 0; g < kG; ++g) {
+                if constexpr (kW == 4) {
+                    const float4 q4 = *reinterpret_cast<const float4*>(&qs[buf][d][64 * g + 4 * ty]);
+                    const float4 k4 = *reinterpret_cast<const float4*>(&ks[buf][d][64 * g + 4 * tx]);
+                    qv[4 * g] = q4.x; qv[4 * g + 1] = q4.y; qv[4 * g + 2] = q4.z; qv[4 * g + 3] = q4.w;
+                    kv[2 * g] = make_float2(k4.x, k4.y);
+                    kv[2 * g + 1] = make_float2(k4.z, k4.w);
+                } else {
+                    const float2 q2 = *reinterpret_cast<const float2*>(&qs[buf][d][2 * ty]);
+                    qv[0] = q2.x; qv[1] = q2.y;
+                    kv[0] = *reinterpret_cast<const float2*>(&ks[buf][d][2 * tx]);
+                }
+            }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = __ffma2_rn(make_float2(qv[i], qv[i]), kv[j], acc[i][j]);
+            for (int i = 0; i < R; ++i)
+#pragma unroll
+                for (int j = 0; j < R / 2; ++j) acc[i][j] = __ffma2_rn(make_float2(qv[i], qv[i]), kv[j], acc[i][j]);
         }
         if (slab + 1 < kSlabs) stash(buf ^ 1);
         __syncthreads();
@@ -95,24 +109,22 @@ __global__ void __launch_bounds__(kGemmThreads, 2) score_gemm_kernel(const T* __
 
     // rounded scores -> keys; columns past Nk get the smallest key, columns past nk_pad do not exist
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int row = i0 + (i < 4 ? 4 * ty + i : 64 + 4 * ty + (i - 4));
+    for (int i = 0; i < R; ++i) {
+        const int row = i0 + 64 * (i / kW) + kW * ty + i % kW;
         if (row >= Nq) continue;
         uint16_t* out = keys + ((long long)bh * Nq + row) * nk_pad;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int col = j0 + 64 * h + 4 * tx;
-            if (col >= nk_pad) continue;  // nk_pad is a multiple of 64, so a group of four columns is all in or all out
-            uint16_t kk[4];
+        for (int g = 0; g < kG; ++g) {
+            const int col = j0 + 64 * g + kW * tx;
+            if (col >= nk_pad) continue;  // nk_pad is a multiple of 64, so a group of columns is all in or all out
+            uint32_t kk[kW];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 a2 = acc[i][2 * h + (j >> 1)];
-                kk[j] = (col + j < Nk) ? make_key(DType<T>::from_f32((j & 1) ? a2.y : a2.x)) : (uint16_t)0;
+            for (int j = 0; j < kW; ++j) {
+                const float2 a2 = acc[i][(kW * g + j) >> 1];
+                kk[j] = (col + j < Nk) ? (uint32_t)make_key(DType<T>::from_f32((j & 1) ? a2.y : a2.x)) : 0u;
             }
-            uint2 pk;
-            pk.x = (uint32_t)kk[0] | ((uint32_t)kk[1] << 16);
-            pk.y = (uint32_t)kk[2] | ((uint32_t)kk[3] << 16);
-            *reinterpret_cast<uint2*>(out + col) = pk;
+            if constexpr (kW == 4) *reinterpret_cast<uint2*>(out + col) = make_uint2(kk[0] | (kk[1] << 16), kk[2] | (kk[3] << 16));
+            else *reinterpret_cast<uint32_t*>(out + col) = kk[0] | (kk[1] << 16);
         }
     }
 }
@@ -175,9 +187,20 @@ cudaError_t launch_topk_for(const uint16_t* keys, long long rows, int Nq, int Nk
 
 template <typename T, int D>
 cudaError_t launch_gemm(const void* qc, const void* kc, int BH, int Nq, int Nk, int nk_pad, uint16_t* keys, cudaStream_t st) {
-    dim3 grid((nk_pad + kTile - 1) / kTile, (Nq + kTile - 1) / kTile, BH);
-    score_gemm_kernel<T, D><<<grid, kGemmThreads, 0, st>>>(reinterpret_cast<const T*>(qc), reinterpret_cast<const T*>(kc), Nq, Nk, nk_pad, keys);
-    return cudaGetLastError();
+    auto tiles = [&](int t) { return (long long)((nk_pad + t - 1) / t) * ((Nq + t - 1) / t) * BH; };
+    auto run = [&](auto kern, int t) {
+        const dim3 grid((nk_pad + t - 1) / t, (Nq + t - 1) / t, BH);
+        kern<<<grid, kGemmThreads, 0, st>>>(reinterpret_cast<const T*>(qc), reinterpret_cast<const T*>(kc), Nq, Nk, nk_pad, keys);
+        return cudaGetLastError();
+    };
+    // A tile of 128 takes 9 us whatever is in it, so small calls take small tiles as long as those fit the chip in two (32) or three
+    // (64) waves of one per SM; operand reads per multiply-add double from one size to the next.  Scores and selection, us, tiles of
+    // 128 / 64 / 32:  2 x 12 x 12 scores 15.9 / 8.7 / 5.8;  1 x 312 x 312 (100 tiles of 32) 21.3 / 11.0 / 7.6;  1 x 624 x 624
+    // (400 tiles of 32) 23.0 / 12.4 / 14.9;  4 x 624 x 624 (400 tiles of 64) 25.2 / 24.2 / 38.8;  1 x 1440 x 1440 (529) 28.8 / 32.6 / 50.8.
+    constexpr long long kSms = 148;
+    if (tiles(32) <= 2 * kSms) return run(score_gemm_kernel<T, D, 2>, 32);
+    if (tiles(64) <= 3 * kSms) return run(score_gemm_kernel<T, D, 4>, 64);
+    return run(score_gemm_kernel<T, D, 8>, 128);
 }
 
 }  // namespace
