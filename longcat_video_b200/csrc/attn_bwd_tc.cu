@@ -21,9 +21,11 @@
 // memory between the contractions, and no gradient is accumulated with atomics.
 //
 // Ragged grids (64-token blocks, bf16): the boxes of partial blocks are zero-filled by TMA outside the grid; a key outside
-// the grid then has K = V = 0 and a query row outside has Q = dO = 0, so every term they enter is a finite number times
-// zero and needs no mask (P of such a key is 2^(-lse * log2 e), finite in fp32 and bf16; fp16 could overflow, so fp16 keeps
-// ragged grids on the warp-level kernels); rows outside the grid are not stored.
+// the grid then has K = V = 0 and a query row outside has Q = dO = 0, so every term they enter is a number times zero and
+// needs no mask as long as that number is finite.  A streamed query row outside the grid has P = 1 and dS = 0.  A streamed key
+// outside the grid (dQ pass) has S = dP = 0, hence P = 2^(-lse * log2 e), which overflows for rows whose scores are all far
+// below zero: where the key grid has partial blocks the exponent is capped (kCap).  A dS of fp16 overflows long before
+// that, so fp16 keeps ragged grids on the warp-level kernels, which mask such keys.  Rows outside the grid are not stored.
 //
 //   warps 0-7 : arithmetic.  A thread serves one TMEM lane = one row of the kM x 64 tile (an M=128 accumulator has row r in
 //               lane r, an M=64 one occupies lanes 0-15 of every 32-lane quadrant)
@@ -154,6 +156,16 @@ struct BwdTcParams {
     float scale, scale2;   // sm_scale, sm_scale * log2(e)
 };
 
+// Cap of the exponents on ragged key grids.  A present key has S * scale <= lse, so its exponent is at most rounding above 0 (2^-22
+// of |lse|: the cap is out of its reach below |lse| = 2^27); a key outside the grid gets P <= 2^64, whose dS = -P * delta * scale is
+// finite in fp32 and bf16.  A NaN stays a NaN.
+constexpr float kMaxExponent = 64.f;
+__device__ __forceinline__ float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // called by a whole converged warp with warp-uniform operands, like the _elect copies of tc_common.cuh
 __device__ __forceinline__ void bulk_load_elect(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile(
@@ -166,7 +178,7 @@ __device__ __forceinline__ void bulk_load_elect(uint32_t dst, const void* src, u
 
 // -lse * log2(e) and -delta of every query row, laid out per 64-token block in slot order, so that a block's 128 values are
 // one contiguous 512-byte piece.  Slots of a partial block that lie outside the grid get zeros (their q and dO rows are
-// zero-filled by TMA, so every term they enter is a finite number times zero).
+// zero-filled by TMA, so that P is 1 and dS 0, and every term they enter is zero).
 __global__ void __launch_bounds__(256) bwd_stats_kernel(const float* lse, const float* delta, Geom g, long long Sq, long long total,
                                                         float* stats, int* next_item) {
     const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -201,8 +213,8 @@ __device__ __forceinline__ void store_row64(unsigned char* row_ptr, int col0, co
     }
 }
 
-// kMode 0: dQ pass, 1: dK/dV pass.  Persistent, one CTA per SM.
-template <bool kBf16, int kMode, int kM>
+// kMode 0: dQ pass, 1: dK/dV pass.  kCap: dQ pass over a key grid with partial blocks.  Persistent, one CTA per SM.
+template <bool kBf16, int kMode, int kM, bool kCap>
 __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_constant__ BwdTcParams P) {
     using C = Cols<kMode, kM>;
     using Ly = Lay<kM>;
@@ -559,7 +571,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
         // fp32 forms.  nl, nd: -lse * log2(e) and -delta.
         const float2 sc2 = make_float2(P.scale2, P.scale2), sc = make_float2(P.scale, P.scale);
         auto pair = [&](uint32_t s0, uint32_t s1, uint32_t d0, uint32_t d1, float2 nl, float2 nd, uint32_t& xp, uint32_t& xd) {
-            const float2 x = __ffma2_rn(make_float2(__uint_as_float(s0), __uint_as_float(s1)), sc2, nl);
+            float2 x = __ffma2_rn(make_float2(__uint_as_float(s0), __uint_as_float(s1)), sc2, nl);
+            if (kCap) x = make_float2(min_nan(x.x, kMaxExponent), min_nan(x.y, kMaxExponent));
             const float2 p = make_float2(ex2(x.x), ex2(x.y));
             const float2 t = __fadd2_rn(make_float2(__uint_as_float(d0), __uint_as_float(d1)), nd);
             const float2 g = __fmul2_rn(__fmul2_rn(p, t), sc);
@@ -761,7 +774,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
     }
 }
 
-template <bool kBf16, int kMode, int kM>
+template <bool kBf16, int kMode, int kM, bool kCap = false>
 cudaError_t launch_pass(const BwdTcParams& P, cudaStream_t st) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -775,14 +788,16 @@ cudaError_t launch_pass(const BwdTcParams& P, cudaStream_t st) {
         sms.store(sm_count, std::memory_order_relaxed);
     }
     // the attribute is per device and per kernel; setting it on every call costs a microsecond and keeps this stateless
-    e = cudaFuncSetAttribute(bwd_tc_kernel<kBf16, kMode, kM>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay<kM>::smem);
+    e = cudaFuncSetAttribute(bwd_tc_kernel<kBf16, kMode, kM, kCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay<kM>::smem);
     if (e != cudaSuccess) return e;
-    bwd_tc_kernel<kBf16, kMode, kM><<<(unsigned)std::min(P.n_items, sm_count), kThreads, Lay<kM>::smem, st>>>(P);
+    bwd_tc_kernel<kBf16, kMode, kM, kCap><<<(unsigned)std::min(P.n_items, sm_count), kThreads, Lay<kM>::smem, st>>>(P);
     return cudaGetLastError();
 }
 
 template <int kMode>
 cudaError_t launch_pass_any(bool bf16, int rows, const BwdTcParams& P, cudaStream_t st) {
+    if constexpr (kMode == 0)
+        if (P.gb.ragged) return rows == 128 ? launch_pass<true, 0, 128, true>(P, st) : launch_pass<true, 0, 64, true>(P, st);  // bf16 only
     if (rows == 128) return bf16 ? launch_pass<true, kMode, 128>(P, st) : launch_pass<false, kMode, 128>(P, st);
     return bf16 ? launch_pass<true, kMode, 64>(P, st) : launch_pass<false, kMode, 64>(P, st);
 }
