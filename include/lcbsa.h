@@ -238,8 +238,8 @@ int lcbsa_block_select_static(const LcbsaTensor* q, const LcbsaTensor* k, const 
                               int nsel, int cap, int32_t* idx, int32_t* cnt, void* stream);
 
 /*
- * Number of SMs that lcbsa_attn_fwd leaves idle (0..64, default 0; process-wide).  The attention kernel is
- * persistent with one CTA per SM and all of an SM's shared memory, so nothing else can start beside it; a caller
+ * Number of SMs that lcbsa_attn_fwd and lcbsa_attn_bwd leave idle (0..64, default 0; process-wide).  The attention kernels are
+ * persistent with one CTA per SM and all of an SM's shared memory, so nothing else can start beside them; a caller
  * that overlaps it with communication kernels on another stream (the all-to-all of
  * longcat_video/context_parallel/ulysses_wrapper.py:7-83) reserves a few SMs for them.  No counterpart in the
  * reference.  Returns the previous value, or LCBSA_EINVAL.

@@ -790,7 +790,9 @@ cudaError_t launch_pass(const BwdTcParams& P, cudaStream_t st) {
     // the attribute is per device and per kernel; setting it on every call costs a microsecond and keeps this stateless
     e = cudaFuncSetAttribute(bwd_tc_kernel<kBf16, kMode, kM, kCap>, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay<kM>::smem);
     if (e != cudaSuccess) return e;
-    bwd_tc_kernel<kBf16, kMode, kM, kCap><<<(unsigned)std::min(P.n_items, sm_count), kThreads, Lay<kM>::smem, st>>>(P);
+    // a CTA holds its SM for the whole pass: those that the caller keeps free for other streams stay free here too
+    const int usable = std::max(sm_count - attn_sm_reserve(), 1);
+    bwd_tc_kernel<kBf16, kMode, kM, kCap><<<(unsigned)std::min(P.n_items, usable), kThreads, Lay<kM>::smem, st>>>(P);
     return cudaGetLastError();
 }
 

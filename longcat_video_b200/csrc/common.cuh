@@ -180,7 +180,7 @@ cudaError_t launch_score_keys(int dtype, const void* qc, const void* kc, int BH,
 // cdf_threshold selectors on the keys of launch_score_keys (select_cdf.cu): idx [rows, Nk] sorted by descending weight, cnt [rows]
 cudaError_t launch_cdf_rows(int dtype, const void* keys, long long rows, int Nk, float sm_scale, float threshold, int nsel_min,
                             int32_t* idx, int32_t* cnt, cudaStream_t st, const char** why);
-int set_attn_sm_reserve(int n_sms);  // SMs the tcgen05 attention kernel leaves idle; returns the previous value
+int set_attn_sm_reserve(int n_sms);  // SMs the tcgen05 attention kernels leave idle; returns the previous value
 
 // q/k RMSNorm + 3-D rotary embedding in one pass (norm_rope.cu).  The table is the packed separable form
 // cos_t [T, dt] sin_t [T, dt] cos_h [H, dh] sin_h [H, dh] cos_w [W, dh] sin_w [W, dh], dh = 2 * (D / 6), dt = D - 2 * dh.

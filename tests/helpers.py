@@ -30,6 +30,16 @@ def max_abs(a, b):
 def kernels_of_capture(fn):
     """Mangled names of the kernels that ``fn`` launches, from the nodes of a graph captured around a second call."""
     import re
+    return re.findall(r"_Z\w+", _dot_of_capture(fn))
+
+
+def grids_of_capture(fn):
+    """(mangled name, CTAs along x) of the kernels that ``fn`` launches."""
+    import re
+    return [(n, int(x)) for n, x in re.findall(r"(_Z\w+)[\\<]+(\d+)", _dot_of_capture(fn))]
+
+
+def _dot_of_capture(fn):
     import tempfile
     fn()
     torch.cuda.synchronize()
@@ -40,4 +50,4 @@ def kernels_of_capture(fn):
         path = os.path.join(d, "graph.dot")
         graph.debug_dump(path)
         with open(path) as f:
-            return re.findall(r"_Z\w+", f.read())
+            return f.read()

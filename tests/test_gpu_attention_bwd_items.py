@@ -5,6 +5,7 @@ import torch
 
 from longcat_video_b200 import _lib as L
 from longcat_video_b200.block_sparse_attention import bsa_interface as B
+from tests.helpers import grids_of_capture
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,32 @@ def test_many_items_per_cta(monkeypatch, grid, block, dtype, cap, bits):
         else:  # fp32 sums in another order, rounded to the dtype: one unit in the last place here and there
             err = (g.double() - w.double()).norm() / w.double().norm()
             assert float(err) <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11)
+
+
+@pytest.mark.parametrize("block", [(4, 4, 4), (4, 4, 8)])
+def test_reserved_sms_stay_free(block):
+    """Each pass launches one CTA per SM less the reserve, and gives the same bits with another number of CTAs."""
+    grid, heads, D = (8, 32, 48), 3, 128
+    gen = torch.Generator().manual_seed(3)
+    S = grid[0] * grid[1] * grid[2]
+    n = L.grid_plan(grid, block)[1]
+    q, k, v, do = (torch.randn(1, heads, S, D, generator=gen).to(torch.bfloat16).cuda() for _ in range(4))
+    idx, cnt = (t.cuda() for t in _lists(gen, heads, n, n, 5, [0, n - 1]))
+    o, lse = B.attn_fwd_bsa_varlen(q, k, v, D ** -0.5, idx, cnt, grid, grid, block, block, return_lse=True)
+    args = (do, q, k, v, o, lse, D ** -0.5, idx, cnt, grid, grid, block, block)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert heads * n >= sms
+    want = B.attn_bwd_bsa_varlen(*args)
+    for reserve in (2, 64):
+        old = L.lib().lcbsa_set_attn_sm_reserve(reserve)
+        try:
+            assert old >= 0
+            got = B.attn_bwd_bsa_varlen(*args)
+            passes = [ctas for name, ctas in grids_of_capture(lambda: B.attn_bwd_bsa_varlen(*args)) if "bwd_tc_kernel" in name]
+        finally:
+            L.lib().lcbsa_set_attn_sm_reserve(old)
+        torch.cuda.synchronize()
+        L.check(L.lib().lcbsa_check_device_status())
+        assert passes == [sms - reserve] * 2
+        for g, w in zip(got, want):
+            assert torch.equal(g, w)
