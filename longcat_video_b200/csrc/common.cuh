@@ -148,7 +148,7 @@ struct BwdArgs {
     int32_t* tidx;        // [B*H, Nq * cap] query blocks of key block j at toff[j] .. toff[j + 1], ascending
     uint32_t* bitmap;     // [B*H, Nk, ceil(Nq / 32)] bit i of row j: query block i selected key block j
     float* stats;         // [B*H, blocks * 128] per 64-token query block: lse * log2(e) [64], delta [64] (tcgen05 passes)
-    int* next_item;       // [2] items taken by the dQ and the dK/dV pass (tcgen05 passes)
+    int* next_item;       // [2] items the dQ and the dK/dV pass took, less the first of each CTA (tcgen05 passes)
     int32_t* idx_u;       // [B*H, Nq_u, cap * Uk] rewritten lists of the dQ pass (tcgen05 passes, blocks split into units)
     int32_t* cnt_u;       // [B*H, Nq_u]
     int32_t* idx_t;       // the same for the lists that are transposed for the dK/dV pass
