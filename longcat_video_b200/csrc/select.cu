@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kThreads) score_topk_kernel(const T* __restric
         int32_t* n_out = cnt + (long long)bh * Nq + qrow;
         if constexpr (sizeof(Key) == 2) {
             if (nk_pad <= 64 * kRegWords) {
-                select_row_regs<kRegWords>(row, nk_pad, nsel, cap, out, n_out, lane);
+                select_row_regs<kRegWords>(row, Nk, nk_pad, nsel, cap, FirstStep<T>::value, out, n_out, lane);
                 continue;
             }
         }

@@ -6,7 +6,10 @@
 namespace lcbsa {
 namespace sel {
 
-constexpr uint32_t kFirstStep = 128;  // of the search for the threshold of a row of 16-bit keys (select_row_regs)
+// First step of the search for the threshold of a row of 16-bit keys (select_row_regs): an octave of scores
+template <typename T> struct FirstStep { static constexpr uint32_t value = 0; };
+template <> struct FirstStep<__nv_bfloat16> { static constexpr uint32_t value = 1u << 7; };
+template <> struct FirstStep<__half> { static constexpr uint32_t value = 1u << 10; };
 constexpr int kRegWords = 24;  // 32-bit words of a 16-bit key row that a lane may keep in registers (select_row_regs: rows up to 1536 keys)
 
 template <typename T> struct KeyOf { using type = uint16_t; };
@@ -67,17 +70,24 @@ struct KeyMask {
 // ascending block indices by one warp; the cap - nsel trailing entries are set to -1.  nk_pad (a multiple of 64, at most
 // 64 * NW) entries are readable and those past Nk hold key 0, which no block that may be selected has.
 //
-// Issue bound: the row is read once (2 bytes per key) and then counted some seven times (16 bits of a plain bisection took 12 to 17).  Every lane keeps its share of the
-// row in registers (word i: keys 2 (lane + 32 i) and the one behind it), the low key of a word shifted up in a register of
-// its own, so that a count is a compare and an add per key; NW follows the row (a fixed 24 words spent 60 % of the work of a 624-key row on padding); the
-// bisection ends as soon as a candidate is reached by exactly nsel keys; and the indices are emitted from the registers.
-// Before, with 24 words for every row, five shuffles per count, all 17 counts and a second read of the row: 19 968 rows of
-// 624 keys 76 us, now 33 us; 46 080 rows of 1440 keys 199 us, then
-// 185 us (there 23 of the 24 words were needed all along).  Searching from the largest key down: scores and selection of those
-// 46 080 rows 620 us, now 561 us; of 19 968 rows of 624 keys 127 us, now 115 us.
+// n_keys: keys the row may select from (it decides how the threshold is looked for, not the result).
+//
+// Issue bound: the row is read once (2 bytes per key) and then counted some seven times (16 bits of a plain bisection take 12
+// to 17).  Every lane keeps its share of the row in registers (word i: keys 2 (lane + 32 i) and the one behind it), the low key
+// of a word shifted up in a register of its own, so that a count is a compare and an add per key; NW follows the row (a fixed 24
+// words spent 60 % of the work of a 624-key row on padding); the search ends as soon as a candidate is reached by exactly
+// nsel keys; and the indices are emitted from the registers.  Before, with 24 words for every row, five shuffles per count, all
+// 17 counts and a second read of the row: 19 968 rows of 624 keys 76 us, then 33 us; 46 080 rows of 1440 keys 199 us, then 185 us
+// (there 23 of the 24 words were needed all along).
+//
+// Where the threshold is looked for.  Fewer than half of the keys selected: a little below the largest key.  Half or more: it
+// may lie on the other side of zero, half of all 16-bit values away, so it is bisected between the smallest and the largest key.
+// Scores and selection, us: always from 16 bits down / always from the largest key, by an octave of bf16 / as here:
+//   46 080 rows of 1440 keys, bf16, head_dim 128: 1/16 selected 630 / 556 / 556, half 595 / 607 / 575, three quarters 632 / 673 / 608
+//   the same in fp16, head_dim 64:                1/16 selected 423 / 400 / 380, half 389 / 423 / 380, three quarters 425 / 478 / 415
 template <int NW>
-__device__ __forceinline__ void select_row_regs(const uint16_t* row, int nk_pad, int nsel, int cap, int32_t* out, int32_t* cnt_out, int lane,
-                                                const KeyMask mask = KeyMask{1, 0, 0}) {
+__device__ __forceinline__ void select_row_regs(const uint16_t* row, int n_keys, int nk_pad, int nsel, int cap, uint32_t first_step, int32_t* out,
+                                                int32_t* cnt_out, int lane, const KeyMask mask = KeyMask{1, 0, 0}) {
     if (lane == 0) *cnt_out = nsel;
     if (nsel > 0) {
         const uint32_t* r32 = reinterpret_cast<const uint32_t*>(row);
@@ -101,16 +111,26 @@ __device__ __forceinline__ void select_row_regs(const uint16_t* row, int nk_pad,
             for (int i = 0; i < NW; ++i) n += (int)(hi[i] >= cc) + (int)(lo[i] >= cc);
             return warp_sum(n);
         };
-        // The threshold lies a little below the row's largest key: steps down from there, of an octave of bf16 scores at first, then twice
-        // as long each time, until nsel keys are reached, and bisects the last step.  count(lo) >= nsel > count(hi) throughout.
+        // Few keys: steps down from the largest one, of an octave of scores at first, then twice as long each time, until nsel keys are
+        // reached, and bisects the last step.  Many: bisects from the smallest key up.  count(below) >= nsel > count(above) throughout.
         uint32_t top = 0;
 #pragma unroll
         for (int i = 0; i < NW; ++i) top = max(top, max(hi[i], lo[i]));
-        uint32_t below = 0, above = (__reduce_max_sync(0xffffffffu, top) >> 16) + 1u, reach = kFirstStep;
+        uint32_t below = 0, above = (__reduce_max_sync(0xffffffffu, top) >> 16) + 1u, reach = first_step;
         int n_above = 0;     // keys that reach `above`
         bool exact = false;  // exactly nsel keys reach the threshold
+        if (2 * nsel >= n_keys) {
+            uint32_t low = 0xffffffffu;  // key 0 is no key
+#pragma unroll
+            for (int i = 0; i < NW; ++i) {
+                low = min(low, hi[i] >= 0x10000u ? hi[i] : 0xffffffffu);
+                low = min(low, lo[i] != 0u ? lo[i] : 0xffffffffu);
+            }
+            below = __reduce_min_sync(0xffffffffu, low) >> 16;
+            exact = nsel >= n_keys && count(below) == nsel;  // all of them
+        }
 #pragma unroll 1
-        while (above - below > 1u) {
+        while (!exact && above - below > 1u) {
             uint32_t cand = (below + above) >> 1;
             if (below == 0u) {
                 cand = above > reach ? above - reach : 1u;
@@ -119,10 +139,7 @@ __device__ __forceinline__ void select_row_regs(const uint16_t* row, int nk_pad,
             const int n = count(cand);
             if (n >= nsel) {
                 below = cand;
-                if (n == nsel) {
-                    exact = true;
-                    break;
-                }
+                exact = n == nsel;
             } else {
                 above = cand;
                 n_above = n;

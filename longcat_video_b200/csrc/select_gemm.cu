@@ -132,12 +132,12 @@ __global__ void __launch_bounds__(kGemmThreads, 2) score_gemm_kernel(const T* __
 // one warp per row of keys; NW: words a lane keeps (rows of up to 64 * NW keys), 0: a row of any length, counted where it lies
 template <int NW>
 __global__ void __launch_bounds__(256) topk_rows_kernel(const uint16_t* __restrict__ keys, long long rows, int Nk, int nk_pad, int nsel,
-                                                       int cap, int32_t* __restrict__ idx, int32_t* __restrict__ cnt) {
+                                                       int cap, uint32_t first_step, int32_t* __restrict__ idx, int32_t* __restrict__ cnt) {
     const int lane = threadIdx.x & 31;
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     if constexpr (NW > 0)
-        select_row_regs<NW>(keys + row * nk_pad, nk_pad, nsel, cap, idx + row * cap, cnt + row, lane);
+        select_row_regs<NW>(keys + row * nk_pad, Nk, nk_pad, nsel, cap, first_step, idx + row * cap, cnt + row, lane);
     else
         select_row<uint16_t>(keys + row * nk_pad, Nk, nk_pad, nsel, cap, idx + row * cap, cnt + row, lane);
 }
@@ -145,29 +145,30 @@ __global__ void __launch_bounds__(256) topk_rows_kernel(const uint16_t* __restri
 // The same for a grid with a "first part" (the conditioning frames of video continuation): query blocks of the first
 // part take nsel_first blocks among the key blocks of the first part, all other query blocks nsel blocks among all.
 template <int NW>
-__global__ void __launch_bounds__(256) topk_rows_split_kernel(const uint16_t* __restrict__ keys, long long rows, int Nq, int nk_pad,
-                                                             SelectSplit sp, int nsel, int cap, int32_t* __restrict__ idx,
-                                                             int32_t* __restrict__ cnt) {
+__global__ void __launch_bounds__(256) topk_rows_split_kernel(const uint16_t* __restrict__ keys, long long rows, int Nq, int Nk, int nk_pad,
+                                                             SelectSplit sp, int nsel, int cap, uint32_t first_step,
+                                                             int32_t* __restrict__ idx, int32_t* __restrict__ cnt) {
     const int lane = threadIdx.x & 31;
     const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int qblk = (int)(row % Nq);
     const bool first = ((qblk / sp.hw_q) % sp.period_q) < sp.split_q;
     const KeyMask mask{sp.hw_k, first ? sp.period_k : 0, sp.split_k};
-    select_row_regs<NW>(keys + row * nk_pad, nk_pad, first ? sp.nsel_first : nsel, cap, idx + row * cap, cnt + row, lane, mask);
+    const int n_keys = first ? Nk / sp.hw_k / sp.period_k * sp.split_k * sp.hw_k : Nk;
+    select_row_regs<NW>(keys + row * nk_pad, n_keys, nk_pad, first ? sp.nsel_first : nsel, cap, first_step, idx + row * cap, cnt + row, lane, mask);
 }
 
 template <int NW>
-cudaError_t launch_topk(const uint16_t* keys, long long rows, int Nq, int Nk, int nk_pad, const SelectSplit* split, int nsel, int cap, int32_t* idx,
-                        int32_t* cnt, cudaStream_t st) {
+cudaError_t launch_topk(const uint16_t* keys, long long rows, int Nq, int Nk, int nk_pad, const SelectSplit* split, int nsel, int cap,
+                        uint32_t first_step, int32_t* idx, int32_t* cnt, cudaStream_t st) {
     const unsigned grid = (unsigned)((rows + 7) / 8);
     if constexpr (NW > 0) {
         if (split != nullptr) {
-            topk_rows_split_kernel<NW><<<grid, 256, 0, st>>>(keys, rows, Nq, nk_pad, *split, nsel, cap, idx, cnt);
+            topk_rows_split_kernel<NW><<<grid, 256, 0, st>>>(keys, rows, Nq, Nk, nk_pad, *split, nsel, cap, first_step, idx, cnt);
             return cudaGetLastError();
         }
     }
-    topk_rows_kernel<NW><<<grid, 256, 0, st>>>(keys, rows, Nk, nk_pad, nsel, cap, idx, cnt);
+    topk_rows_kernel<NW><<<grid, 256, 0, st>>>(keys, rows, Nk, nk_pad, nsel, cap, first_step, idx, cnt);
     return cudaGetLastError();
 }
 
@@ -175,13 +176,13 @@ cudaError_t launch_topk(const uint16_t* keys, long long rows, int Nq, int Nk, in
 // lane keeps, and with two words a step no row counts more than one word of padding.  Rows above 64 * kRegWords keys are
 // counted where they lie.
 template <int NW>
-cudaError_t launch_topk_for(const uint16_t* keys, long long rows, int Nq, int Nk, int nk_pad, const SelectSplit* split, int nsel, int cap, int32_t* idx,
-                            int32_t* cnt, cudaStream_t st) {
+cudaError_t launch_topk_for(const uint16_t* keys, long long rows, int Nq, int Nk, int nk_pad, const SelectSplit* split, int nsel, int cap,
+                            uint32_t first_step, int32_t* idx, int32_t* cnt, cudaStream_t st) {
     if constexpr (NW <= kRegWords) {
-        if (nk_pad <= 64 * NW) return launch_topk<NW>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
-        return launch_topk_for<NW + 2>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
+        if (nk_pad <= 64 * NW) return launch_topk<NW>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, first_step, idx, cnt, st);
+        return launch_topk_for<NW + 2>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, first_step, idx, cnt, st);
     } else {
-        return launch_topk<0>(keys, rows, Nq, Nk, nk_pad, nullptr, nsel, cap, idx, cnt, st);
+        return launch_topk<0>(keys, rows, Nq, Nk, nk_pad, nullptr, nsel, cap, first_step, idx, cnt, st);
     }
 }
 
@@ -248,7 +249,8 @@ cudaError_t launch_score_gemm_topk(int dtype, const void* qc, const void* kc, in
         *why = "the split selection handles up to 1536 key blocks";
         return cudaErrorInvalidValue;
     }
-    return launch_topk_for<2>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, idx, cnt, st);
+    const uint32_t first_step = dtype == LCBSA_BF16 ? FirstStep<__nv_bfloat16>::value : FirstStep<__half>::value;
+    return launch_topk_for<2>(keys, rows, Nq, Nk, nk_pad, split, nsel, cap, first_step, idx, cnt, st);
 }
 
 }  // namespace lcbsa
