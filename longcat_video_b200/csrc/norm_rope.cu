@@ -149,9 +149,11 @@ __device__ __forceinline__ void do_rows(const RowJob& j, unsigned s_blk, int b, 
             const float mean = __fmul_rn(ss, 1.0f / (float)D);
             rinv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
         }
+        uint4 res[NV];
+        uint32_t* rw = reinterpret_cast<uint32_t*>(res);
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-            uint32_t rw[4], rn[4];
+            uint32_t rn[4];
 #pragma unroll
             for (int p4 = 0; p4 < 4; ++p4) {
                 const int p = 4 * i + p4;
@@ -168,12 +170,13 @@ __device__ __forceinline__ void do_rows(const RowJob& j, unsigned s_blk, int b, 
                     z = Pair<T>::pack(__fadd_rn(__fmul_rn(z0, cs[p]), __fmul_rn(-z1, sn[p])),
                                       __fadd_rn(__fmul_rn(z1, cs[p]), __fmul_rn(z0, sn[p])));
                 }
-                rw[p4] = z;
+                rw[p] = z;
             }
-            if (live) {
-                reinterpret_cast<uint4*>(dp)[i] = make_uint4(rw[0], rw[1], rw[2], rw[3]);
-                if (KEEP) reinterpret_cast<uint4*>(dp2)[i] = make_uint4(rn[0], rn[1], rn[2], rn[3]);
-            }
+            if (KEEP && live) reinterpret_cast<uint4*>(dp2)[i] = make_uint4(rn[0], rn[1], rn[2], rn[3]);
+        }
+        if (live) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) reinterpret_cast<uint4*>(dp)[i] = res[i];
         }
         if (KEEP) dp2 += j.o2sh;
         dp += j.osh;
@@ -191,21 +194,32 @@ __host__ __device__ __forceinline__ int kind_of(const RowJob& j) {
     return j.weight != nullptr ? kNorm : j.tab != nullptr ? kRope : kCopy;
 }
 
+// CTAs per SM that a kernel's registers have to allow: memory bound, so as many as fit without spilling in the loop.  A uniform 4, with the
+// CTA's place worked out from a one-dimensional grid in every kind: 24x48x80 grid, 32 heads, bf16, RMSNorm and embedding 262 us,
+// RMSNorm alone 248, embedding alone 252 (head_dim 64: 154); as here 258, 242, 244 (141).
+constexpr int min_ctas(int D, int kind) {
+    return kind == kCopy ? 8 : kind == kRope ? (D == 128 ? 5 : 8) : kind == kNorm ? (D == 128 ? 5 : 6) : (D == 128 ? 4 : 5);
+}
+
 template <typename T, int D, int kKind>
-__global__ void __launch_bounds__(kWarps * 32, 4) norm_rope_kernel(const __grid_constant__ RowJobs P) {
+__global__ void __launch_bounds__(kWarps * 32, min_ctas(D, kKind)) norm_rope_kernel(const __grid_constant__ RowJobs P) {
     int i = 0;
-    if (kKind == kMixed)
+    unsigned s_blk = blockIdx.x, hg = blockIdx.y, b = blockIdx.z;
+    if (kKind == kMixed) {
         while (i + 1 < P.n && blockIdx.x >= P.job[i + 1].first) ++i;
+        const unsigned r = blockIdx.x - P.job[i].first, s_blks = (unsigned)(P.job[i].S + kTokens * kWarps - 1) / (kTokens * kWarps);
+        s_blk = r % s_blks;
+        hg = r / s_blks % P.head_groups;
+        b = r / s_blks / P.head_groups;
+    }
     const RowJob& j = P.job[kKind == kMixed ? i : 0];
-    const unsigned r = blockIdx.x - (kKind == kMixed ? j.first : 0u), s_blks = (unsigned)(j.S + kTokens * kWarps - 1) / (kTokens * kWarps);
-    const unsigned rest = r / s_blks, hg = rest % P.head_groups, s_blk = r % s_blks;
-    const int b = (int)(rest / P.head_groups), h0 = (int)hg * P.hpc, h1 = min(P.H, h0 + P.hpc);
+    const int h0 = (int)hg * P.hpc, h1 = min(P.H, h0 + P.hpc);
     const int kind = kKind == kMixed ? kind_of(j) : kKind;
-    if (kind == kNormRopeKeep) do_rows<T, D, true, true, true>(j, s_blk, b, h0, h1, P.eps);
-    else if (kind == kNormRope) do_rows<T, D, true, true, false>(j, s_blk, b, h0, h1, P.eps);
-    else if (kind == kNorm) do_rows<T, D, true, false, false>(j, s_blk, b, h0, h1, P.eps);
-    else if (kind == kRope) do_rows<T, D, false, true, false>(j, s_blk, b, h0, h1, P.eps);
-    else do_rows<T, D, false, false, false>(j, s_blk, b, h0, h1, P.eps);
+    if (kind == kNormRopeKeep) do_rows<T, D, true, true, true>(j, s_blk, (int)b, h0, h1, P.eps);
+    else if (kind == kNormRope) do_rows<T, D, true, true, false>(j, s_blk, (int)b, h0, h1, P.eps);
+    else if (kind == kNorm) do_rows<T, D, true, false, false>(j, s_blk, (int)b, h0, h1, P.eps);
+    else if (kind == kRope) do_rows<T, D, false, true, false>(j, s_blk, (int)b, h0, h1, P.eps);
+    else do_rows<T, D, false, false, false>(j, s_blk, (int)b, h0, h1, P.eps);
 }
 
 template <typename T, int D>
@@ -217,14 +231,15 @@ cudaError_t launch(RowJobs& P, int kind, int B, cudaStream_t st) {
         total += (long long)((P.job[i].S + kTokens * kWarps - 1) / (kTokens * kWarps)) * P.head_groups * B;
     }
     if (total == 0) return cudaSuccess;
-    if (total > 0x7fffffffll) return cudaErrorInvalidConfiguration;
+    if (kind == kMixed ? total > 0x7fffffffll : P.head_groups > 65535u) return cudaErrorInvalidConfiguration;
+    const dim3 grid = kind == kMixed ? dim3((unsigned)total) : dim3((unsigned)(total / P.head_groups / B), P.head_groups, (unsigned)B);
     switch (kind) {
-        case kCopy: norm_rope_kernel<T, D, kCopy><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
-        case kRope: norm_rope_kernel<T, D, kRope><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
-        case kNorm: norm_rope_kernel<T, D, kNorm><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
-        case kNormRope: norm_rope_kernel<T, D, kNormRope><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
-        case kNormRopeKeep: norm_rope_kernel<T, D, kNormRopeKeep><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
-        default: norm_rope_kernel<T, D, kMixed><<<(unsigned)total, kWarps * 32, 0, st>>>(P); break;
+        case kCopy: norm_rope_kernel<T, D, kCopy><<<grid, kWarps * 32, 0, st>>>(P); break;
+        case kRope: norm_rope_kernel<T, D, kRope><<<grid, kWarps * 32, 0, st>>>(P); break;
+        case kNorm: norm_rope_kernel<T, D, kNorm><<<grid, kWarps * 32, 0, st>>>(P); break;
+        case kNormRope: norm_rope_kernel<T, D, kNormRope><<<grid, kWarps * 32, 0, st>>>(P); break;
+        case kNormRopeKeep: norm_rope_kernel<T, D, kNormRopeKeep><<<grid, kWarps * 32, 0, st>>>(P); break;
+        default: norm_rope_kernel<T, D, kMixed><<<grid, kWarps * 32, 0, st>>>(P); break;
     }
     return cudaGetLastError();
 }
@@ -238,7 +253,7 @@ cudaError_t run(RowJobs& P, int B, cudaStream_t st) {
     P.hpc = kHeadsPerCta;
     while (P.hpc > 2 && tokens * B * ((P.H + P.hpc - 1) / P.hpc) < 148 * 8) P.hpc /= 2;
     // Calls that do not fill the chip are bound by their launches: all jobs in one.  Larger ones take a launch per job, whose
-    // kernel has the registers and the code of its kind alone: q and k of a 24x48x80 grid, 32 heads: 519 us in two launches, 582 us
+    // kernel has the registers and the code of its kind alone: q and k of a 24x48x80 grid, 32 heads: 509 us in two launches, 582 us
     // through the kernel that serves all kinds.
     if (P.n > 1 && tokens * B * ((P.H + P.hpc - 1) / P.hpc) < 148 * 16) return launch<T, D>(P, kMixed, B, st);
     for (int i = 0; i < P.n; ++i) {

@@ -19,6 +19,7 @@ def _bits(t):
     (2, 17, 64, (3, 5, 7)),      # remainders in tokens and heads
     (2, 2, 128, (1, 1, 33)),
     (1, 33, 128, (8, 33, 41)),   # enough CTAs for a launch per job
+    (3, 18, 64, (6, 33, 41)),
 ])
 def test_jobs_together_equal_jobs_alone(dtype, B, H, D, grid):
     S = grid[0] * grid[1] * grid[2]
