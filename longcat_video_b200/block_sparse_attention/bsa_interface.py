@@ -217,10 +217,16 @@ def attn_bwd_bsa_varlen(do, q, k, v, o, lse, sm_scale, block_indices, block_indi
     return dq, dk, dv
 
 
+# Up to this size the selection's workspace is part of the scratch tensor of a call and lives as long: one allocation less where the host
+# is what the time goes into.  A larger one (133 MB for 32 heads of 1440 x 1440 blocks) goes back to the allocator before the output is
+# allocated, which can then have the memory.
+_SHARED_WORKSPACE_BYTES = 1 << 20
+
+
 def _select_and_attend(q, k, v, latent_shape_q, latent_shape_k, sparsity, chunk_q, chunk_k) -> torch.Tensor:
     """``get_select_indices`` and ``attn_fwd_bsa_varlen`` behind each other, with what the two have in common done once: on
-    the smallest calls the host is what the time goes into (2 heads of 8x8x12 tokens, a call among others: 76 us as two calls, 52 us here).  The lists and the selection's
-    workspace are parts of one scratch tensor, which lives as long as this call."""
+    the smallest calls the host is what the time goes into (2 heads of 8x8x12 tokens, a call among others: 76 us as two calls,
+    52 us here).  The lists and a small workspace are parts of one scratch tensor, which lives as long as this call."""
     q, k, v = _as_abi(q), _as_abi(k), _as_abi(v)
     B, H, Sq, D = q.shape
     (gq, nq), (gk, nk) = L.grid_plan(latent_shape_q, chunk_q), L.grid_plan(latent_shape_k, chunk_k)
@@ -230,13 +236,16 @@ def _select_and_attend(q, k, v, latent_shape_q, latent_shape_k, sparsity, chunk_
     lib, ref, dev = L.lib(), ctypes.byref, q.device
     rq, rk, rgq, rgk = ref(qd), ref(kd), ref(gq), ref(gk)
     ws_bytes = lib.lcbsa_select_workspace_bytes_fast(rq, rk, rgq, rgk)
-    at_idx = -(-ws_bytes // 256) * 256
+    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=dev) if ws_bytes > _SHARED_WORKSPACE_BYTES else None
+    at_idx = -(-ws_bytes // 256) * 256 if ws is None else 0
     at_cnt = at_idx + -(-B * H * nq * cap // 64) * 256
     scratch = torch.empty(at_cnt + max(B * H * nq, 1) * 4, dtype=torch.uint8, device=dev)
     base = scratch.data_ptr()
     with L.on_device(dev):
         stream = L.current_stream(dev)
-        L.check(lib.lcbsa_block_select(rq, rk, rgq, rgk, nsel, cap, base + at_idx, base + at_cnt, base, ws_bytes, stream))
+        L.check(lib.lcbsa_block_select(rq, rk, rgq, rgk, nsel, cap, base + at_idx, base + at_cnt,
+                                       base if ws is None else ws.data_ptr(), ws_bytes, stream))
+        del ws
         if STAGE_HOOK is not None:
             STAGE_HOOK()
         out = torch.empty(B, H, Sq, D, dtype=q.dtype, device=dev)
