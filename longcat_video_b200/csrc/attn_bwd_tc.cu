@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
                 const Item it = take_item(k);
                 if (it.id < 0) break;
                 if (it.n == 0) continue;
-                ok = mbar_wait_warp(bar_acc_free, (kk & 1) ^ 1, ctl, 221, kk);  // the gradients of the item before have been read
+                ok = mbar_wait_warp(bar_acc_free, (kk & 1) ^ 1, ctl, 244, kk);  // the gradients of the item before have been read
                 ++kk;
                 bool pre = false;
                 for (int e = 0; e < it.n && ok; ++e, ++s) {
@@ -546,8 +546,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tc_kernel(const __grid_consta
         // The own tiles go from shared memory to TMEM, where they are the A operands of every S and dP: with both operands in shared
         // memory an M=64 S reads as many bytes of the own tile as of the streamed one.  A thread moves (half of) a row.
         auto own_to_tmem = [&](unsigned item) -> bool {
-            if (!mbar_wait_warp(bar_a_full, item & 1, ctl, 228, item)) return false;
-            if (item > 0 && !mbar_wait_warp(bar_at_free, (item - 1) & 1, ctl, 229, item)) return false;
+            if (!mbar_wait_warp(bar_a_full, item & 1, ctl, 242, item)) return false;
+            if (item > 0 && !mbar_wait_warp(bar_at_free, (item - 1) & 1, ctl, 243, item)) return false;
             tc_fence_after();
             // kM = 64: warpgroup g moves half g of A1 (lanes 0-15) and of A2 (lanes 16-31); kM = 128: A1 and A2, or half g of A1
             const int tile = kM == 64 ? lane >> 4 : (kOwn2Smem ? 0 : wg);

@@ -70,3 +70,24 @@ def test_key_masks_are_handed_on_by_arrivals_of_threads():
     issue = src[src.index("mbar_wait_warp(bar_k_full(slot)"):src.index("tc_commit(bar_s_full(wg))")]
     assert "if (kRagged) mbar_arrive_elect(bar_s_full(wg));" in issue
     assert "mbar_init(bar_s_full(b), kRagged ? 2 : 1);" in src
+
+
+def _codes_of_waits(text):
+    """code -> barriers whose waits report it when they run out; codes are expressions of kMode, wg and is_k."""
+    text = re.sub(r"//[^\n]*", "", text)
+    out = {}
+    for bar, code in re.findall(r"\bmbar_wait_warp\((\w+)[^;]*?, ctl, ([^,]+),", text):
+        yes, no = re.fullmatch(r"(?:\w+ \? )?([^:]+?)(?: : (.+))?", code).groups()
+        for expr in filter(None, (yes, no)):
+            for mode in (0, 1):
+                for wg in (0, 1):
+                    out.setdefault(eval(expr, {"kMode": mode, "wg": wg}), set()).add(bar)
+    return out
+
+
+@pytest.mark.parametrize("name", ["attn_tc.cu", "attn_tc128.cu", "attn_bwd_tc.cu"])
+def test_a_reported_code_names_one_barrier(name):
+    """The status word of a wait that ran out is the wait's code: waits on different barriers have different ones."""
+    codes = _codes_of_waits(_source(name))
+    assert len(codes) > 15
+    assert {c: b for c, b in codes.items() if len(b) > 1} == {}
