@@ -12,7 +12,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "longcat_video_b200", "csrc")
-TOKEN = re.compile(r"[{}]|\b(?:mbar_wait_warp|mbar_wait_thread|mbar_test|mbar_try|tc_fence_after|tc_ld16|tc_ld32|tc_ld64|tc_ld_half64|tc_st_half32|tc_st16|tc_st32|tc_mma|tc_mma_ts)(?=\()")
+TOKEN = re.compile(r"[{}]|\b(?:mbar_wait_warp|mbar_wait_thread|mbar_test|mbar_try|tc_fence_after|tc_ld32|tc_ld64|tc_ld_half64|tc_st_half32|tc_st16|tc_st32|tc_mma|tc_mma_ts)(?=\()")
 
 
 def _unfenced(text):
@@ -91,3 +91,14 @@ def test_a_reported_code_names_one_barrier(name):
     codes = _codes_of_waits(_source(name))
     assert len(codes) > 15
     assert {c: b for c, b in codes.items() if len(b) > 1} == {}
+
+
+def test_the_scan_knows_the_accesses_there_are():
+    """Every wrapper of a tcgen05 load, store or MMA is scanned for and used."""
+    wrappers = set(re.findall(r"void (tc_(?:ld|st|mma)\w*)\(", _source("tc_common.cuh")))
+    used = "".join(_source(n) for n in ("attn_tc.cu", "attn_tc128.cu", "attn_bwd_tc.cu", "tc_common.cuh"))
+    for w in wrappers:
+        assert len(re.findall(rf"\b{w}\(", used)) > 1, f"nothing calls {w}"
+        assert TOKEN.search(f" {w}("), f"the scan does not know {w}"
+    for w in re.findall(r"tc_(?:ld|st|mma)\w*", TOKEN.pattern):
+        assert w in wrappers, f"the scan looks for {w}, which does not exist"
