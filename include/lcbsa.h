@@ -288,7 +288,7 @@ int lcbsa_norm_rope_ex(const LcbsaTensor* x, const void* weight, const LcbsaGrid
                        float eps, const LcbsaTensor* out, void* stream);
 
 /*
- * Up to eight such tensors in one launch: everything a layer does to the rows of its q, k and v before the attention
+ * Up to eight such tensors in one call (one launch where they do not fill the chip, else one each): everything a layer does to the rows of its q, k and v before the attention
  * (attention.py:113-121 and 156-171).  They share dtype, batch, heads, head_dim and eps; a batch or head stride may be 0.  Per job
  * the rules of lcbsa_norm_rope_ex, and: weight == NULL and rope_tab == NULL copies the rows (v into or behind a cache);
  * out_norm.data != NULL also keeps the normalised rows from before the embedding, which is what return_kv caches

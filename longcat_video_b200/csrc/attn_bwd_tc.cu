@@ -13,8 +13,8 @@
 //   dK/dV pass (CTA = key block j, list = the query blocks i that selected it):  A1 = K_j  A2 = V_j  B1 = Q_i  B2 = dO_i
 //       S^T = A1 B1^T       dP^T = A2 B2^T       P^T, dS^T as above, transposed          dV_j += P^T B2   dK_j += dS^T B1
 //
-// with P = exp2(S * scale * log2(e) - lse * log2(e)).  S and dP are (M = kM) N64 K128 MMAs with both operands in shared
-// memory (fp32 in TMEM); P and dS are written back to TMEM in the input dtype and are the A operands of the N128 K64 MMAs
+// with P = exp2(S * scale * log2(e) - lse * log2(e)).  S and dP are (M = kM) N64 K128 MMAs, own tile from TMEM,
+// streamed tile from shared memory, fp32 result in TMEM (kM = 128, dK/dV pass: V too comes from shared memory); P and dS are written back to TMEM in the input dtype and are the A operands of the N128 K64 MMAs
 // that accumulate the gradients in TMEM over the whole list, with the streamed tile as MN-major B operand: a tile is
 // loaded once (two 5-D TMA boxes of 64 columns, 128-byte swizzle) and serves as K-major operand of the first
 // contraction and as MN-major operand of the last.  Nothing is recomputed within a pass, nothing goes through shared
@@ -27,20 +27,21 @@
 // below zero: where the key grid has partial blocks the exponent is capped (kCap).  A dS of fp16 overflows long before
 // that, so fp16 keeps ragged grids on the warp-level kernels, which mask such keys.  Rows outside the grid are not stored.
 //
-//   warps 0-7 : arithmetic.  A thread serves one TMEM lane = one row of the kM x 64 tile (an M=128 accumulator has row r in
-//               lane r, an M=64 one occupies lanes 0-15 of every 32-lane quadrant)
+//   warps 0-7 : arithmetic.  kM = 128: a thread serves one TMEM lane = one row of the 128 x 64 tile.  kM = 64: the tile occupies lanes
+//               0-15 of every 32-lane quadrant, and a warp takes its 16 rows with all threads, two rows and 32 values each
 //   warps 8, 11 : TMA producers of B1 and of B2 into a ring of five (four for kM = 128) slots; warp 8 also brings the CTA's
 //               own tiles once, and in the dK/dV pass the query block's 64 (lse * log2 e) and 64 delta values per slot, by a
 //               bulk copy onto the same barrier (bwd_stats_kernel lays them out, negated, per block)
-//   warp 9    : issues S and dP (SS)    warp 10 : issues the gradient MMAs (TS); one elected lane each
+//   warp 9    : issues S and dP    warp 10 : issues the gradient MMAs; one elected lane each
 //
-// TMEM and the order of the MMAs.  P and dS (16-bit pairs) have columns of their own, twice, in both passes: the values
-// of entry s + 2 go where those of entry s were, once TS(s) has read them (ts_done).
-//   dQ pass (448 columns): S and dP have two buffers; warps 0-3 take the even entries, warps 4-7 the odd ones.
-//   dK/dV pass (512 columns, two accumulators): S^T and dP^T have ONE buffer; all eight warps work on every entry (warps
-//       0-3 columns 0-31, warps 4-7 columns 32-63).
-//   In both, SS of the entry that takes the buffer next waits until the arithmetic warps hold S and dP in registers
-//   (s_free), and TS(s) for x_full(s), the P and dS of entry s.
+// TMEM and the order of the MMAs (see Cols).  P and dS (16-bit pairs) have columns of their own; those of entry s are overwritten
+// once the gradient MMAs of s have read them (ts_done).
+//   kM = 64, both passes: two buffers of everything; warps 0-3 take the even entries, warps 4-7 the odd ones.
+//   kM = 128, dQ pass: two buffers of S and of dS, one of dP; the same split of the entries.
+//   kM = 128, dK/dV pass (two accumulators): ONE buffer each of S^T, dP^T, P^T and dS^T; all eight warps work on every entry
+//       (warps 0-3 columns 0-31, warps 4-7 columns 32-63).
+//   S and dP of the entry that takes a buffer next wait until the arithmetic warps hold the last ones in registers (s_free), and the
+//   gradient MMAs of s for x_full(s), its P and dS.
 // The own tiles are moved to TMEM once, where they are the A operands of every S and dP (kM = 128, dK/dV pass: only K, TMEM is
 // full): an M=64 S with both operands in shared memory reads 128 bytes a cycle of it, all that it gives, beside the incoming
 // tiles.  At kM = 64 the second of two things sits in the lanes 16-31 that an M=64 tile leaves free (see Cols).
@@ -51,8 +52,11 @@
 // Persistent, one CTA per SM: a CTA per block spent some 10000 cycles before its first and behind its last entry, on barriers, TMEM,
 // its list, its first tiles and its gradients; now the own tiles, the list and the row values of the next block are fetched
 // under the entries of this one, and some 3500 are left.  The blocks are taken off a counter, since the transposed lists differ in
-// length.  Backward of 8 heads, 39 of 624 64-token blocks: 1889 -> 1704 us; 16 of 832: 570 -> 445 us.
-// With 128-token blocks a long launch runs at 1.28 PFLOP/s of issued MMAs, nine tenths of what the GPU's power cap sustains.
+// length.  Backward of 8 heads, 39 of 624 64-token blocks: 1889 -> 1704 us; 16 of 832: 570 -> 445 us.  With 128-token blocks, 42
+// of 336, the step took 2497 -> 2590 us (2653 us before the issuer's look-ahead, 2470 to 2540 us now); short calls of a few blocks
+// are some 3 us slower for it.
+// Counters over whole launches (8 heads, 480p grids): tensor pipe 82 % (dQ) and 88 % (dK/dV) with 64-token blocks, 957 and 1190 cycles
+// per entry; 70 % and 73 % with 128-token blocks, 1126 and 1431 cycles.
 // Every mbarrier wait is bounded; when one runs out the CTA flags the status word, drains its copies, frees TMEM, returns.
 #include <algorithm>
 #include <cstdlib>

@@ -36,8 +36,9 @@
 // after its P was ready).
 // What bounds it: M=64 MMAs, 16 x 32 + 8 x 64 = 1024 cycles of tensor pipe per block of a pair (an M=64 tile occupies the
 // pipe like an M=128 one); inside an item a block takes 1025 to 1040 cycles.  K and V of the block come in at 64 bytes per
-// cycle and SM meanwhile, so tiles at the full rate would wait for L2.  An item boundary costs some 2700 cycles more (480p grid, 39
-// blocks per item: 42700 cycles per item by time stamps): PV of the next item waits for the epilogue warps to have read O.
+// cycle and SM meanwhile; tiles at the full rate would ask L2 for twice that (what it can deliver has not been measured).  An item
+// boundary costs some 2700 cycles more (480p grid, 39 blocks per item: 42700 cycles per item by time stamps): PV of the next item
+// waits for the epilogue warps to have read O.
 // It was 8000 when the softmax warps merged and stored O before they took up the next item and the kernel had 162 KB of code, more than
 // the instruction caches hold (68 KB now).  480p, 39 of 624 blocks, whole call with 8 heads: 565 us with both, 549 us with
 // the smaller code, 532 us with epilogue warps; 720p grid of 45 rows (ragged, masks in the softmax warps), 32 heads: 13095,
@@ -78,7 +79,8 @@ constexpr int kThreads = 512;
 constexpr float kNoScore = -1e30f;
 // setmaxnreg per warpgroup: (168 + 168 + 48 + 128) * 128 threads = the 64 K registers of the SM, 128 per thread at launch.  The
 // epilogue warps hold 32 columns of both accumulators: with 96 registers (and 184 for the softmax warps) the 720p grid takes 11300 us
-// instead of 11070.
+// instead of 11070.  ptxas reports 88 bytes of spill stores and 164 of loads per thread (ragged head_dim 128: 56 and 120), whatever
+// the split of the budgets: 64 for the producers or 144 for the epilogue warps leave them much the same.
 constexpr int kRegsSoftmax = 168, kRegsOther = 48, kRegsEpilogue = 128;
 
 // TMEM columns: O accumulator of warpgroup g at 128 * g, its S at 256 + 64 * g, its P (16-bit pairs) at 384 + 32 * g; Q (16-bit pairs)

@@ -82,7 +82,8 @@ struct KeyMask {
 //
 // Where the threshold is looked for.  Fewer than half of the keys selected: a little below the largest key.  Half or more: it
 // may lie on the other side of zero, half of all 16-bit values away, so it is bisected between the smallest and the largest key.
-// Scores and selection, us: always from 16 bits down / always from the largest key, by an octave of bf16 / as here:
+// Scores and selection, us: always from 16 bits down (with a score kernel some 25 us slower) / always from the largest key, by an
+// octave of bf16 / as here:
 //   46 080 rows of 1440 keys, bf16, head_dim 128: 1/16 selected 630 / 556 / 556, half 595 / 607 / 575, three quarters 632 / 673 / 608
 //   the same in fp16, head_dim 64:                1/16 selected 423 / 400 / 380, half 389 / 423 / 380, three quarters 425 / 478 / 415
 template <int NW>

@@ -74,7 +74,7 @@ __device__ __forceinline__ void ctl_init(const Ctl& c) { c.abort[0] = c.abort[4]
 // try_wait itself blocks for a hardware-defined interval, so the loop turns over rarely.
 // Every role of every kernel waits in a dozen places, so what is inlined here is most of a kernel's code: with the report to
 // global memory and a loop of its own for the clock in each of them the kernels had 145 to 165 KB, more than the
-// instruction caches hold, and whatever ran once per work item came from L2 (75 KB now).
+// instruction caches hold, and whatever ran once per work item came from L2 (68 and 55 KB without).
 __device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, const Ctl& c, unsigned code, unsigned it) {
     if (mbar_try(bar, parity)) return true;
     const uint32_t t0 = (uint32_t)clock();
@@ -267,7 +267,7 @@ __device__ __forceinline__ uint32_t pack2(bool bf16, float lo, float hi) {
 
 // Multiply this thread's row of a kCols-column fp32 accumulator in TMEM by alpha.  Warp-collective.  A rolled loop: at head_dim
 // 128 it is the rare path of the online softmax and should take little room in the instruction stream of the loop; at
-// head_dim 64, where most rounds come here, an unrolled one costs 11 spilled registers.
+// head_dim 64, where most rounds come here, both halves of a row at once do not fit the registers of the softmax warps.
 template <int kCols>
 __device__ __forceinline__ void tc_scale_row(uint32_t taddr, float alpha) {
     tc_fence_after();

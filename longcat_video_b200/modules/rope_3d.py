@@ -77,7 +77,8 @@ _NO_TENSOR = L.LcbsaTensor()
 
 
 def run_row_jobs(jobs: Sequence[RowJob], eps: float = 1e-6, base: float = 10000.0) -> None:
-    """One launch for all jobs that share dtype, batch, heads and head_dim: for all there are, as a layer has them."""
+    """One call for all jobs that share dtype, batch, heads and head_dim: for all there are, as a layer has them.  It is one launch
+    where the jobs do not fill the chip, else a launch per job."""
     kinds = {}
     for j in jobs:
         if j.x.dim() != 4:
@@ -140,7 +141,7 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, out: Opti
 
 def qk_norm_rope(q: torch.Tensor, k: torch.Tensor, q_weight: torch.Tensor, k_weight: torch.Tensor, grid_size: Sequence[int],
                  eps: float = 1e-6, base: float = 10000.0) -> Tuple[torch.Tensor, torch.Tensor]:
-    """``rope_3d(q_norm(q), k_norm(k), grid_size)`` of attention.py:113-121 in one launch."""
+    """``rope_3d(q_norm(q), k_norm(k), grid_size)`` of attention.py:113-121 in one call (see ``run_row_jobs``)."""
     q_out, k_out = torch.empty(q.shape, dtype=q.dtype, device=q.device), torch.empty(k.shape, dtype=k.dtype, device=k.device)
     run_row_jobs([RowJob(q, q_out, q_weight, grid_size), RowJob(k, k_out, k_weight, grid_size)], eps, base)
     return q_out, k_out
@@ -170,7 +171,7 @@ def qk_norm_rope_with_kv_cache(q: torch.Tensor, k: torch.Tensor, q_weight: torch
     ``k_full [B,H,(NC+T)HW,D]``.  The reference concatenates the cache and the new keys, pads q in front with an empty
     tensor of the cache's size, embeds both over ``(T + NC, H, W)`` and cuts q's tail off again; here the cached keys
     are embedded into the head of ``k_full``, the new keys are normalised and embedded into its tail, and q is
-    normalised and embedded at frame offset NC: one launch, no padding and no concatenation."""
+    normalised and embedded at frame offset NC: one call, no padding and no concatenation."""
     q_out, k_full, jobs = kv_cache_row_jobs(q, k, q_weight, k_weight, k_cache, grid_size, num_cond_latents)
     run_row_jobs(jobs, eps, base)
     return q_out, k_full

@@ -1,7 +1,7 @@
 """The last items of a CTA, one block long each: the result of the last is staged where the store of the one before is still read.
 
-Every query block lists one key block; the check is against the fp32 oracle, rel-L2 <= 1e-2 (bf16 probabilities).  84 CTAs, two or three items each, five calls: the order in
-which stores and merges meet differs from call to call."""
+Every query block lists one key block; the check is against the fp32 oracle, rel-L2 <= 1e-2 (bf16 probabilities).  84 CTAs, two or
+three items each, five calls: the order in which stores and merges meet differs from call to call."""
 import pytest
 import torch
 
