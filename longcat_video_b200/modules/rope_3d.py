@@ -83,6 +83,8 @@ def run_row_jobs(jobs: Sequence[RowJob], eps: float = 1e-6, base: float = 10000.
     for j in jobs:
         if j.x.dim() != 4:
             raise ValueError("expected a [B, H, S, D] tensor")
+        if j.out_norm is not None and (j.weight is None or not j.rope):
+            raise ValueError("normalised rows are kept beside embedded ones: that takes a weight and the embedding")
         kinds.setdefault((j.x.dtype, j.x.device, j.x.shape[0], j.x.shape[1], j.x.shape[3]), []).append(j)
     for group in kinds.values():
         _launch_row_jobs(group, eps, base)

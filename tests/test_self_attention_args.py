@@ -37,3 +37,10 @@ def test_no_cpu_path():
     w = torch.ones(128)
     with pytest.raises(Exception):
         A.self_attention(q, k, v, w, w, (4, 8, 8), PARAMS)
+
+
+def test_caching_normalised_keys_needs_a_weight():
+    """``return_kv`` without a k_norm weight is a ValueError, as ``rms_norm`` without one is."""
+    q = torch.zeros(1, 2, 32, 128, dtype=torch.bfloat16)
+    with pytest.raises(ValueError):
+        A.self_attention(q, q, q, q[0, 0, 0], None, (2, 4, 4), {}, return_kv=True)
